@@ -26,7 +26,8 @@ struct ArenaSim {
     PadSim pads[NUM_PADS];
 };
 
-RSB_HD void ballFinishTick(World& W, V3 velCache) {
+template <class WT>
+RSB_HD void ballFinishTick(WT& W, V3 velCache) {
     Body& b = W.b[0];
     if (!isZero(velCache)) b.lin = b.lin + velCache;
     float ms = W.P->ballMaxSpeedBt;
@@ -38,7 +39,8 @@ RSB_HD void ballFinishTick(World& W, V3 velCache) {
 }
 
 // Arena::IsBallScored for soccar (Arena.cpp:949-957): the ball centre past a goal line.
-RSB_HD bool ballScored(const World& W, float goalBaseY, float ballRadiusUu) {
+template <class WT>
+RSB_HD bool ballScored(const WT& W, float goalBaseY, float ballRadiusUu) {
     float y = W.b[0].xf.o.y * kBtToUu;
     return fabsf(y) > (goalBaseY + ballRadiusUu);
 }
@@ -54,29 +56,26 @@ RSB_HD uint32_t mixHash(uint32_t a, uint32_t b, uint32_t c) {
     return h;
 }
 
-// BoostPad::_CheckCollide for one car
-RSB_HD void padCheckCollide(ArenaSim& A, int p, int ci) {
-    const World& W = A.W;
-    const Body& cb = W.b[1 + ci];
-    PadSim& pad = A.pads[p];
+// BoostPad::_CheckCollide of pad p for a car at xf; `locked`: the car locked the pad last tick
+RSB_HD bool padCollides(const WorldParams& P, int p, const Xf& xf, bool locked) {
     bool big = p < NUM_BIG_PADS;
     PadLoc pl = padLoc(p);
     V3 posBT = V3{pl.x, pl.y, pl.z} * kUuToBt;
-    V3 carPos = cb.xf.o;
-    bool colliding = false;
-    if (pad.prevLocked == W.c[ci].id) {
+    V3 carPos = xf.o;
+    if (locked) {
         V3 mn, mx;
-        carCompoundAabb(W.P->car, cb.xf, mn, mx);
+        carCompoundAabb(P.car, xf, mn, mx);
         float boxRad = (big ? PAD_BOX_RAD_BIG : PAD_BOX_RAD_SMALL) * kUuToBt;
         V3 boxMin = posBT - V3{boxRad, boxRad, 0};
         V3 boxMax = posBT + V3{boxRad, boxRad, PAD_BOX_HEIGHT * kUuToBt};
-        colliding = (boxMax.x > mn.x && boxMax.y > mn.y && boxMax.z > mn.z) && (boxMin.x < mx.x && boxMin.y < mx.y && boxMin.z < mx.z);
-    } else {
-        float rad = (big ? PAD_CYL_RAD_BIG : PAD_CYL_RAD_SMALL) * kUuToBt;
-        float dx = carPos.x - posBT.x, dy = carPos.y - posBT.y;
-        if (dx * dx + dy * dy < rad * rad) colliding = fabsf(carPos.z - posBT.z) < PAD_CYL_HEIGHT * kUuToBt;
+        return (boxMax.x > mn.x && boxMax.y > mn.y && boxMax.z > mn.z) && (boxMin.x < mx.x && boxMin.y < mx.y && boxMin.z < mx.z);
     }
-    if (colliding) pad.curLocked = ci;
+    float rad = (big ? PAD_CYL_RAD_BIG : PAD_CYL_RAD_SMALL) * kUuToBt;
+    float dx = carPos.x - posBT.x, dy = carPos.y - posBT.y;
+    return dx * dx + dy * dy < rad * rad && fabsf(carPos.z - posBT.z) < PAD_CYL_HEIGHT * kUuToBt;
+}
+RSB_HD void padCheckCollide(ArenaSim& A, int p, int ci) {
+    if (padCollides(*A.W.P, p, A.W.b[1 + ci].xf, A.pads[p].prevLocked == A.W.c[ci].id)) A.pads[p].curLocked = ci;
 }
 
 // BoostPadGrid::CheckCollision

@@ -60,7 +60,8 @@ struct GroundRef {
     float invMass;
     const Body* body;
 };
-RSB_HD GroundRef groundRef(const World& W, int o) {
+template <class WT>
+RSB_HD GroundRef groundRef(const WT& W, int o) {
     GroundRef g;
     if (o < OBJ_BALL) {
         g.com = o < MAX_MESHES ? v3zero() : W.S->planeOrigin[o - MAX_MESHES];
@@ -103,7 +104,8 @@ RSB_HD float resolveBilateral(const Body& b1, V3 pos1, const GroundRef& g, V3 po
 }
 
 // resolveSingleCollision (btContactConstraint.cpp:60-105), impulses not applied
-RSB_HD float resolveCollision(const Body& b1, int obj, const World& W, V3 contact, V3 normal, float distance, float timeStep) {
+template <class WT>
+RSB_HD float resolveCollision(const Body& b1, int obj, const WT& W, V3 contact, V3 normal, float distance, float timeStep) {
     GroundRef g = groundRef(W, obj);
     V3 rel1 = contact - b1.xf.o;
     V3 rel2 = contact - g.com;
@@ -153,22 +155,24 @@ RSB_HD void wheelTransform(const CarParams& C, const Body& cb, WheelTick& w, int
 RSB_HD V3 chassisUp(const Body& cb) { return cb.xf.b.col(2); }
 RSB_HD V3 chassisFwd(const Body& cb) { return cb.xf.b.col(0); }
 
-// btVehicleRL::rayCast (btVehicleRL.cpp:118-206)
-RSB_HD void wheelRayCast(World& W, int ci, int i) {
+// The segment of wheel i's ray (btVehicleRL::rayCast, btVehicleRL.cpp:118-130).
+RSB_HD void wheelSegment(const CarParams& C, const Body& cb, WheelTick& w, int i, V3& source, V3& target) {
+    wheelTransformsWS(C, cb, w, i);
+    source = w.hardPoint;
+    target = source + w.dirWS * C.rayLen[i];
+}
+
+// btVehicleRL::rayCast (btVehicleRL.cpp:131-206) after the cast: object `obj` hit at hp with
+// normal hn, or obj < 0.  The wheel's hard point and direction are set by wheelSegment.
+template <class WT>
+RSB_HD void wheelFromHit(WT& W, int ci, int i, V3 target, int obj, V3 hp, V3 hn) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     WheelTick& w = c.w[i];
-    wheelTransformsWS(C, cb, w, i);
     float travel = C.susTravel;
-    float rayLen = C.rayLen[i];
-    V3 source = w.hardPoint;
-    V3 target = source + w.dirWS * rayLen;
     w.contactPoint = target;
     w.ground = -1;
-    V3 hp, hn;
-    float frac;
-    int obj = castRay(W, source, target, OBJ_CAR0 + ci, hp, hn, frac);
     if (obj >= 0) {
         w.contactPoint = hp;
         w.contactNormal = hn;
@@ -211,8 +215,18 @@ RSB_HD void wheelRayCast(World& W, int ci, int i) {
     }
 }
 
+template <class WT>
+RSB_HD void wheelRayCast(WT& W, int ci, int i) {
+    V3 source, target, hp, hn;
+    float frac;
+    wheelSegment(W.P->car, W.b[1 + ci], W.c[ci].w[i], i, source, target);
+    const int obj = castRay(W, source, target, OBJ_CAR0 + ci, hp, hn, frac);
+    wheelFromHit(W, ci, i, target, obj, hp, hn);
+}
+
 // btVehicleRL::calcFrictionImpulses (btVehicleRL.cpp:307-370)
-RSB_HD void calcFrictionImpulses(World& W, int ci, float timeStep) {
+template <class WT>
+RSB_HD void calcFrictionImpulses(WT& W, int ci, float timeStep) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -258,7 +272,8 @@ RSB_HD void calcFrictionImpulses(World& W, int ci, float timeStep) {
 }
 
 // btVehicleRL::updateSuspension (btVehicleRL.cpp:275-305)
-RSB_HD void updateSuspension(World& W, int ci, float dt) {
+template <class WT>
+RSB_HD void updateSuspension(WT& W, int ci, float dt) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -286,7 +301,8 @@ RSB_HD void updateSuspension(World& W, int ci, float dt) {
 }
 
 // btVehicleRL::applyFrictionImpulses (btVehicleRL.cpp:372-387)
-RSB_HD void applyFrictionImpulses(World& W, int ci, float dt) {
+template <class WT>
+RSB_HD void applyFrictionImpulses(WT& W, int ci, float dt) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     V3 up = chassisUp(cb);
@@ -302,7 +318,8 @@ RSB_HD void applyFrictionImpulses(World& W, int ci, float dt) {
 }
 
 // btVehicleRL::getUpwardsDirFromWheelContacts
-RSB_HD V3 upwardsDirFromWheels(const World& W, int ci) {
+template <class WT>
+RSB_HD V3 upwardsDirFromWheels(const WT& W, int ci) {
     const CarSim& c = W.c[ci];
     V3 sum = v3zero();
     for (int i = 0; i < 4; i++)
@@ -323,7 +340,8 @@ RSB_HD bool cflag(const CarSim& c, uint32_t f) { return (c.flags & f) != 0; }
 RSB_HD void setFlag(CarSim& c, uint32_t f, bool on) { c.flags = on ? (c.flags | f) : (c.flags & ~f); }
 
 // Car::SetState applied to a fresh CarState with the given placement (Car.cpp:24-36)
-RSB_HD void carSetSpawnState(World& W, int ci, V3 posUu, const M3& rot, float boost) {
+template <class WT>
+RSB_HD void carSetSpawnState(WT& W, int ci, V3 posUu, const M3& rot, float boost) {
     CarSim& c = W.c[ci];
     Body& b = W.b[1 + ci];
     b.xf.o = posUu * kUuToBt;
@@ -347,23 +365,31 @@ RSB_HD void carSetSpawnState(World& W, int ci, V3 posUu, const M3& rot, float bo
     c.lastCtlBits = 0;
 }
 
-// Car::Respawn for soccar; `pick` selects one of CAR_RESPAWN_LOCATIONS_SOCCAR
-RSB_HD void carRespawn(World& W, int ci, int pick) {
-    W.cull &= ~(1u << (1 + ci));  // the spawn is next to the floor: no culling this launch
+// Placement of Car::Respawn for soccar; `pick` selects one of CAR_RESPAWN_LOCATIONS_SOCCAR
+RSB_HD void respawnPlacement(int team, int pick, V3& posUu, M3& rot) {
     const double kRespawnYaw = 3.14159265358979323846 / 2;
     const float xs[4] = {-2304.f, -2688.f, 2304.f, 2688.f};
-    CarSim& c = W.c[ci];
-    bool blue = c.team == 0;
+    bool blue = team == 0;
     float y = -4608.f * (blue ? 1.f : -1.f);
-    V3 pos{xs[pick], y, CAR_RESPAWN_Z};
+    posUu = V3{xs[pick], y, CAR_RESPAWN_Z};
     float yaw = (float)(kRespawnYaw + (blue ? 0.0 : 3.14159265358979323846));
     // Angle(yaw, 0, 0).ToRotMat() = setEulerYPR(yaw, -0, -0) = setEulerZYX(-0, -0, yaw)
-    M3 rot = m3fromEulerZYX(-0.f, -0.f, yaw);
+    rot = m3fromEulerZYX(-0.f, -0.f, yaw);
+}
+
+// Car::Respawn
+template <class WT>
+RSB_HD void carRespawn(WT& W, int ci, int pick) {
+    W.cull &= ~(1u << (1 + ci));  // the spawn is next to the floor: no culling this launch
+    V3 pos;
+    M3 rot;
+    respawnPlacement(W.c[ci].team, pick, pos, rot);
     carSetSpawnState(W, ci, pos, rot, W.P->car.spawnBoost);
 }
 
 // Car::_UpdateWheels (Car.cpp:323-461)
-RSB_HD void updateWheels(World& W, int ci, float dt, int numContact, float fwdSpeedUu) {
+template <class WT>
+RSB_HD void updateWheels(WT& W, int ci, float dt, int numContact, float fwdSpeedUu) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     float absFwd = fabsf(fwdSpeedUu);
@@ -445,7 +471,8 @@ RSB_HD void updateWheels(World& W, int ci, float dt, int numContact, float fwdSp
 }
 
 // Car::_UpdateAirTorque (Car.cpp:558-646)
-RSB_HD void updateAirTorque(World& W, int ci, bool updateAirControl) {
+template <class WT>
+RSB_HD void updateAirTorque(WT& W, int ci, bool updateAirControl) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     V3 dirPitch = -c.rotMat.col(1), dirYaw = c.rotMat.col(2), dirRoll = -c.rotMat.col(0);
@@ -499,7 +526,8 @@ RSB_HD void updateAirTorque(World& W, int ci, bool updateAirControl) {
 }
 
 // Car::_UpdateJump (Car.cpp:496-556)
-RSB_HD void updateJump(World& W, int ci, float dt, bool jumpPressed) {
+template <class WT>
+RSB_HD void updateJump(WT& W, int ci, float dt, bool jumpPressed) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -529,7 +557,8 @@ RSB_HD void updateJump(World& W, int ci, float dt, bool jumpPressed) {
 }
 
 // Car::_UpdateAutoFlip (Car.cpp:770-803)
-RSB_HD void updateAutoFlip(World& W, int ci, float dt, bool jumpPressed) {
+template <class WT>
+RSB_HD void updateAutoFlip(WT& W, int ci, float dt, bool jumpPressed) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     if (jumpPressed && cflag(c, CF_WORLD_CONTACT) && c.worldContactNormal.z > CAR_AUTOFLIP_NORMZ_THRESH) {
@@ -564,7 +593,8 @@ RSB_HD void updateAutoFlip(World& W, int ci, float dt, bool jumpPressed) {
 }
 
 // Car::_UpdateDoubleJumpOrFlip (Car.cpp:648-768)
-RSB_HD void updateDoubleJumpOrFlip(World& W, int ci, float dt, bool jumpPressed, float fwdSpeedUu) {
+template <class WT>
+RSB_HD void updateDoubleJumpOrFlip(WT& W, int ci, float dt, bool jumpPressed, float fwdSpeedUu) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -630,7 +660,8 @@ RSB_HD void updateDoubleJumpOrFlip(World& W, int ci, float dt, bool jumpPressed,
 }
 
 // Car::_UpdateAutoRoll (Car.cpp:805-832)
-RSB_HD void updateAutoRoll(World& W, int ci, int numContact) {
+template <class WT>
+RSB_HD void updateAutoRoll(WT& W, int ci, int numContact) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     V3 groundUp = numContact > 0 ? upwardsDirFromWheels(W, ci) : c.worldContactNormal;
@@ -649,7 +680,8 @@ RSB_HD void updateAutoRoll(World& W, int ci, int numContact) {
 }
 
 // Car::_UpdateBoost (Car.cpp:463-494)
-RSB_HD void updateBoost(World& W, int ci, float dt) {
+template <class WT>
+RSB_HD void updateBoost(WT& W, int ci, float dt) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -668,8 +700,10 @@ RSB_HD void updateBoost(World& W, int ci, float dt) {
     c.boost = fmin_(c.boost, BOOST_MAX);
 }
 
-// Car::_PreTickUpdate
-RSB_HD void carPreTick(World& W, int ci, uint32_t respawnPick) {
+// Car::_PreTickUpdate up to the vehicle update (Car.cpp:58-83): control clamps, demo timer and
+// respawn.  Returns false for a car that stays demoed, whose update ends here.
+template <class WT>
+RSB_HD bool carPreTickStatus(WT& W, int ci, uint32_t respawnPick) {
     const float dt = W.P->dt;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
@@ -683,11 +717,15 @@ RSB_HD void carPreTick(World& W, int ci, uint32_t respawnPick) {
         cb.act = ACT_ACTIVE;
         cb.noResp = 0;
     }
-    if (cflag(c, CF_DEMOED)) return;
+    return !cflag(c, CF_DEMOED);
+}
 
-    // btVehicleRL::updateVehicleFirst
-    for (int i = 0; i < 4; i++) wheelTransform(W.P->car, cb, c.w[i], i, i < 2 ? c.steerAngle : 0.f);
-    for (int i = 0; i < 4; i++) wheelRayCast(W, ci, i);
+// The rest of Car::_PreTickUpdate (Car.cpp:84-128) once the wheel rays are cast.
+template <class WT>
+RSB_HD void carDrive(WT& W, int ci) {
+    const float dt = W.P->dt;
+    Body& cb = W.b[1 + ci];
+    CarSim& c = W.c[ci];
     calcFrictionImpulses(W, ci, dt);
 
     bool jump = (c.ctlBits & 1u) != 0, lastJump = (c.lastCtlBits & 1u) != 0;
@@ -714,8 +752,21 @@ RSB_HD void carPreTick(World& W, int ci, uint32_t respawnPick) {
     updateBoost(W, ci, dt);
 }
 
+// Car::_PreTickUpdate
+template <class WT>
+RSB_HD void carPreTick(WT& W, int ci, uint32_t respawnPick) {
+    if (!carPreTickStatus(W, ci, respawnPick)) return;
+    Body& cb = W.b[1 + ci];
+    CarSim& c = W.c[ci];
+    // btVehicleRL::updateVehicleFirst
+    for (int i = 0; i < 4; i++) wheelTransform(W.P->car, cb, c.w[i], i, i < 2 ? c.steerAngle : 0.f);
+    for (int i = 0; i < 4; i++) wheelRayCast(W, ci, i);
+    carDrive(W, ci);
+}
+
 // Car::_PostTickUpdate + Car::_FinishPhysicsTick
-RSB_HD void carPostTick(World& W, int ci) {
+template <class WT>
+RSB_HD void carPostTick(WT& W, int ci) {
     const float dt = W.P->dt;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];

@@ -1,6 +1,7 @@
-// Per-arena body of the step kernel: load the arena's records from the word planes,
-// run the requested ticks, store the records back.  The kernel in rsb_engine.cu calls
-// stepArena() once per arena.
+// A whole step of one arena: load the arena's records from the word planes, run the requested
+// ticks, store the records back.  The step kernels run the same tick cut into phases
+// (step_phases.h); stepArena() is the tick in the reference's own order, which the host tests
+// compare with the reference and the phases.
 #pragma once
 #include "arena.h"
 
@@ -27,7 +28,7 @@ struct EngineView {
     const uint32_t* cull;          // per-arena body bits from the learned culler, or null
     int32_t cullAudit;             // run culled static tests anyway and count what they find
     unsigned long long* counters;  // [static tests run, tests culled, culled tests that hit, solver rows], or null
-    unsigned int* work;            // next unclaimed arena of a persistent launch (zeroed before it)
+    unsigned int* work;            // queue counters of the step phases (step_phases.h)
 };
 
 RSB_HD void initBodyCommon(Body& b) {

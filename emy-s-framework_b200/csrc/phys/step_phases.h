@@ -1,0 +1,1361 @@
+// One physics tick of the whole batch as a sequence of phases.
+//
+// stepArena() (engine_core.h) runs a tick of one arena from start to end on one thread.  Here
+// the same computation is cut where the work changes shape, so that each phase runs on the
+// threads that fit it: a thread per wheel ray, per body, per contact pair, per arena with
+// contacts.  Rare and expensive work (rays near meshes or other bodies, box-mesh and
+// convex-convex contacts, islands to solve) goes through queues, so that a warp holds 32 items
+// of it instead of the few that 32 arenas happen to have at the same time.
+//
+//   rays ....... every wheel ray of every car: the planes here, the rest into the ray queue
+//   heavy rays . the queued rays: meshes, planes, other bodies (castRay)
+//   bodies ..... respawns, vehicle update, gravity, predicted motion, broadphase pairs, plane
+//                contacts; queues the other contact pairs and the arenas that have any
+//   contacts ... one queued pair per thread: box-mesh, sphere-mesh, box-sphere, box-box
+//   islands .... the queued arenas: contact callbacks, islands, solver (solveIslands)
+//   finish ..... integration, post-tick updates, boost pads, goal and tick counters
+//
+// Between the phases a tick lives in the persistent records (state.h) and in StepTemp.  What
+// orders the reference's results is kept: rays of a car see the cars that pre-tick before it
+// (higher slots) as those left them and the others as the last tick left them; manifolds,
+// callbacks and solver rows follow the pair order of computePairs.  Every operation on a value
+// is the one stepArena applies, in the same order, so the results are the same bit for bit.
+#pragma once
+#include <stddef.h>
+
+#include "engine_core.h"
+
+namespace rsb {
+
+// Words of the body information planes ([word][MAX_BODIES][N]).
+enum : int {
+    BI_PAIRS = 0,   // static pairs (20 bits) | activation << 20 | BI_* flags
+    BI_MANI,        // static pairs that have a manifold (20 bits)
+    BI_TASKS,       // meshes with a queued contact pair (16 bits) | planes with a contact << 16
+    BI_MESHRES,     // result of the first queued mesh pair (the others follow)
+    BI_PLANERES,    // results of the plane contacts (4 words)
+    BI_DYN = BI_PLANERES + NUM_PLANES,  // dynamic pairs in visiting order, 3 bits each, count << 24
+    BI_DYNMANI,     // bodies of higher index with which this body has a manifold (7 bits)
+    BI_WORDS
+};
+constexpr int BI_ACT_SHIFT = 20;
+constexpr uint32_t BI_ACT_MASK = 7u << BI_ACT_SHIFT;
+constexpr uint32_t BI_SOLVED = 1u << 24;    // velocities and transform were written by the islands phase
+constexpr uint32_t BI_CACHE = 1u << 25;     // the body's velocity cache holds an impulse
+constexpr uint32_t BI_RESPONDS = 1u << 26;  // contact response on (cars)
+
+// Dynamic pairs (lo < hi) of seven bodies.
+constexpr int NUM_DYN_PAIRS = MAX_BODIES * (MAX_BODIES - 1) / 2;
+RSB_HD int dynPair(int lo, int hi) { return lo * (2 * MAX_BODIES - lo - 1) / 2 + (hi - lo - 1); }
+
+// Queue counters.
+enum : int { QC_RAY = 0, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_WORDS };
+constexpr int NUM_TASK_TYPES = 4;  // QC_CARMESH .. QC_CARCAR
+// The most pairs of each type that an arena can have, and contact blocks (MAX_BLOCKS manifolds
+// hold contacts in one tick; more are dropped, as in the one-thread tick).
+constexpr int CAP_CARMESH = MAX_CARS * MAX_MESHES, CAP_BALLMESH = MAX_MESHES, CAP_CARBALL = MAX_CARS,
+              CAP_CARCAR = MAX_CARS * (MAX_CARS - 1) / 2, CAP_PLANE = MAX_BODIES * NUM_PLANES;
+constexpr int CAP_RESULTS = CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL + CAP_CARCAR + CAP_PLANE;
+RSB_HD int resultBase(int type) {  // per arena: first result of the type
+    return type == QC_CARMESH ? 0
+         : type == QC_BALLMESH ? CAP_CARMESH
+         : type == QC_CARBALL ? CAP_CARMESH + CAP_BALLMESH
+         : type == QC_CARCAR ? CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL
+                             : CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL + CAP_CARCAR;
+}
+
+struct PairTask {
+    uint32_t a;
+    uint16_t o0, o1;
+};
+
+// Outcome of one contact pair.
+struct PairResult {
+    int32_t n;        // points left in the manifold
+    uint32_t flags;   // PR_*
+    uint32_t block;   // its points (when PR_BLOCK is set)
+    float normal[3];  // normal of the last world contact reported to the car
+};
+enum : uint32_t {
+    PR_BLOCK = 1u,  // a contact was added, so the manifold owns a point block
+    PR_WORLD = 2u   // ... and the car-world callback saw it
+};
+
+struct StepTemp {
+    // wheel rays, [4][MAX_CARS][N]: object hit (-1 none), fraction, normal (3 planes)
+    int32_t* rayObj;
+    float* rayFrac;
+    float* rayN;
+    uint32_t* info;      // BI_WORDS planes of [MAX_BODIES][N]
+    float* force;        // force, torque of the tick: 6 planes of [MAX_BODIES][N]
+    float* box;          // broadphase AABB: 6 planes of [MAX_BODIES][N]
+    float* cache;        // velocity impulse caches: 3 planes of [MAX_BODIES][N]
+    uint32_t* dynRes;    // result of each dynamic pair: [NUM_DYN_PAIRS][N]
+    uint32_t* count;     // QC_WORDS counters
+    uint32_t* rayQ;      // [4 * MAX_CARS * N]
+    PairTask* tasks;     // per type, [cap * N], at resultBase(type) * N
+    PairResult* results;
+    MPoint* blocks;      // [MAX_BLOCKS * N][MAX_POINTS]
+    uint32_t blockCap;
+    uint32_t* solveQ;    // [N]
+};
+
+// Static-test counters of one thread (rsb_stats).
+struct PhaseStats {
+    uint32_t nStatic, nCulled, nMissed, nRows;
+};
+
+RSB_HD uint32_t phaseAtomicAdd(uint32_t* p, uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    return atomicAdd(p, v);
+#else
+    const uint32_t o = *p;
+    *p += v;
+    return o;
+#endif
+}
+RSB_HD void phaseAtomicOr(uint32_t* p, uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    atomicOr(p, v);
+#else
+    *p |= v;
+#endif
+}
+RSB_HD void phaseAtomicAnd(uint32_t* p, uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    atomicAnd(p, v);
+#else
+    *p &= v;
+#endif
+}
+
+#define RSB_PW(T, f) ((int)(offsetof(T, f) / 4))
+
+// ------------------------------------------------------------------ record access
+
+RSB_HD uint32_t ballWord(const EngineView& D, int a, int w) { return D.ball[(size_t)w * D.N + a]; }
+RSB_HD uint32_t carWord(const EngineView& D, int a, int s, int w) { return D.car[((size_t)w * MAX_CARS + s) * D.N + a]; }
+RSB_HD float carFloat(const EngineView& D, int a, int s, int w) { return u2f(carWord(D, a, s, w)); }
+RSB_HD void putCarWord(const EngineView& D, int a, int s, int w, uint32_t v) {
+    D.car[((size_t)w * MAX_CARS + s) * D.N + a] = v;
+}
+RSB_HD void putCarFloat(const EngineView& D, int a, int s, int w, float v) { putCarWord(D, a, s, w, f2u(v)); }
+RSB_HD V3 carV3(const EngineView& D, int a, int s, int w) {
+    return V3{carFloat(D, a, s, w), carFloat(D, a, s, w + 1), carFloat(D, a, s, w + 2)};
+}
+RSB_HD void putCarV3(const EngineView& D, int a, int s, int w, V3 v) {
+    putCarFloat(D, a, s, w, v.x);
+    putCarFloat(D, a, s, w + 1, v.y);
+    putCarFloat(D, a, s, w + 2, v.z);
+}
+RSB_HD uint32_t arenaWord(const EngineView& D, int a, int w) { return D.arena[(size_t)w * D.N + a]; }
+RSB_HD uint64_t arenaTickCount(const EngineView& D, int a) {
+    return (uint64_t)arenaWord(D, a, RSB_PW(ArenaP, tick)) | ((uint64_t)arenaWord(D, a, RSB_PW(ArenaP, tick) + 1) << 32);
+}
+RSB_HD uint32_t* arenaStatus(const EngineView& D, int a) { return D.arena + (size_t)RSB_PW(ArenaP, status) * D.N + a; }
+
+// Pose and velocity words lie at the same offsets in the ball and the car records.
+static_assert(offsetof(BallP, ang) == offsetof(CarP, ang) && offsetof(BallP, regStamp) == offsetof(CarP, regStamp),
+              "common head of the body records");
+RSB_HD uint32_t bodyWord(const EngineView& D, int a, int b, int w) {
+    return b == 0 ? ballWord(D, a, w) : carWord(D, a, b - 1, w);
+}
+RSB_HD float bodyFloat(const EngineView& D, int a, int b, int w) { return u2f(bodyWord(D, a, b, w)); }
+RSB_HD void putBodyWord(const EngineView& D, int a, int b, int w, uint32_t v) {
+    if (b == 0) D.ball[(size_t)w * D.N + a] = v;
+    else putCarWord(D, a, b - 1, w, v);
+}
+RSB_HD V3 bodyV3(const EngineView& D, int a, int b, int w) {
+    return V3{bodyFloat(D, a, b, w), bodyFloat(D, a, b, w + 1), bodyFloat(D, a, b, w + 2)};
+}
+RSB_HD void putBodyV3(const EngineView& D, int a, int b, int w, V3 v) {
+    putBodyWord(D, a, b, w, f2u(v.x));
+    putBodyWord(D, a, b, w + 1, f2u(v.y));
+    putBodyWord(D, a, b, w + 2, f2u(v.z));
+}
+RSB_HD Xf bodyXf(const EngineView& D, int a, int b) {
+    Xf x;
+    x.o = bodyV3(D, a, b, RSB_PW(CarP, pos));
+    for (int r = 0; r < 3; r++) x.b.r[r] = bodyV3(D, a, b, RSB_PW(CarP, rot) + 3 * r);
+    return x;
+}
+RSB_HD void putBodyXf(const EngineView& D, int a, int b, const Xf& x) {
+    putBodyV3(D, a, b, RSB_PW(CarP, pos), x.o);
+    for (int r = 0; r < 3; r++) putBodyV3(D, a, b, RSB_PW(CarP, rot) + 3 * r, x.b.r[r]);
+}
+
+RSB_HD size_t bodyIdx(const EngineView& D, int a, int b) { return (size_t)b * D.N + a; }
+RSB_HD uint32_t& infoWord(const EngineView& D, const StepTemp& T, int a, int b, int w) {
+    return T.info[(size_t)w * MAX_BODIES * D.N + bodyIdx(D, a, b)];
+}
+RSB_HD V3 tempV3(const EngineView& D, const float* p, int a, int b, int k) {
+    const size_t st = (size_t)MAX_BODIES * D.N, i = (size_t)k * st + bodyIdx(D, a, b);
+    return V3{p[i], p[i + st], p[i + 2 * st]};
+}
+RSB_HD void putTempV3(const EngineView& D, float* p, int a, int b, int k, V3 v) {
+    const size_t st = (size_t)MAX_BODIES * D.N, i = (size_t)k * st + bodyIdx(D, a, b);
+    p[i] = v.x;
+    p[i + st] = v.y;
+    p[i + 2 * st] = v.z;
+}
+
+// Constants of a body at transform x (the pose-independent part of loadBall / loadCar).
+RSB_HD void bodyConstants(const EngineView& D, int b, Body& o) {
+    initBodyCommon(o);
+    if (b == 0) {
+        o.invMass = D.P.ballInvMass;
+        o.grav = D.P.ballGrav;
+        o.invIl = D.P.ballInvInertia;
+        o.linDampFactor = D.P.ballLinDampFactor;
+        o.friction = D.P.ballFriction;
+        o.restitution = D.P.ballRestitution;
+    } else {
+        o.invMass = D.P.car.invMass;
+        o.grav = D.P.car.grav;
+        o.invIl = D.P.car.invInertiaLocal;
+        o.linDampFactor = 1.f;
+        o.friction = CAR_COLLISION_FRICTION;
+        o.restitution = CAR_COLLISION_RESTITUTION;
+    }
+}
+
+RSB_HD int arenaBodies(const EngineView& D, int a) { return 1 + 2 * D.teamSize[a]; }
+RSB_HD int respawnPick(const EngineView& D, int a, uint64_t tick, int ci) {
+    return (int)(mixHash(mixHash(D.seed, (uint32_t)a, 0x5EEDu), (uint32_t)tick, (uint32_t)ci) & 3u);
+}
+// Whether car s, demoed before the tick, respawns in it.
+RSB_HD bool respawns(const EngineView& D, int a, int s) {
+    return fmax_(carFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer)) - D.P.dt, 0) == 0;
+}
+RSB_HD Xf respawnXf(const EngineView& D, int a, int s, uint32_t flags, uint64_t tick) {
+    V3 pos;
+    M3 rot;
+    respawnPlacement((flags & CF_TEAM_ORANGE) ? 1 : 0, respawnPick(D, a, tick, s), pos, rot);
+    return Xf{rot, pos * kUuToBt};
+}
+
+// ------------------------------------------------------------------ wheel rays
+
+// What castRay reads of the world, for the rays of car `viewer`, from the records as the last
+// tick left them.  Cars of higher slots have pre-ticked before the viewer's rays are cast: a
+// respawning one stands at its spawn, and a demoed one has no contact response.
+struct RayBody {
+    Xf xf;
+    int noResp;
+};
+struct RayWorld;
+struct RayBodies {
+    const EngineView* D;
+    int a, viewer;
+    uint64_t tick;
+    RSB_HD RayBody operator[](int b) const {
+        RayBody r;
+        r.noResp = 0;
+        if (b > 0) {
+            const int s = b - 1;
+            const uint32_t f = carWord(*D, a, s, RSB_PW(CarP, flags));
+            if (s > viewer) {
+                r.noResp = (f & CF_DEMOED) ? 1 : 0;
+                if ((f & CF_DEMOED) && respawns(*D, a, s)) {
+                    r.xf = respawnXf(*D, a, s, f, tick);
+                    return r;
+                }
+            } else {
+                r.noResp = (f & CF_NO_RESPONSE) ? 1 : 0;
+            }
+        }
+        r.xf = rsb::bodyXf(*D, a, b);
+        return r;
+    }
+};
+struct RayWorld {
+    const ArenaStatic* S;
+    const WorldParams* P;
+    RayBodies b;
+    int nb;
+    uint32_t cull;
+    int32_t cullAudit;
+    mutable uint32_t nStatic, nCulled, nMissed, cullMissed;
+    RegOrder reg;
+};
+
+// Registration order of the arena's bodies from their records (buildRegOrder).
+template <class StampF, class CellF>
+RSB_HD void regOrderOf(RegOrder& R, int nb, StampF&& stamp, CellF&& cell) {
+    R.n = 0;
+    for (int e = 0; e < nb; e++) {
+        const int32_t st = stamp(e);
+        int i, j, k;
+        cell(e, i, j, k);
+        int r = R.n++;
+        while (r > 0 && R.stamp[r - 1] > (uint32_t)st) {
+            R.body[r] = R.body[r - 1];
+            R.stamp[r] = R.stamp[r - 1];
+            R.ci[r] = R.ci[r - 1];
+            R.cj[r] = R.cj[r - 1];
+            R.ck[r] = R.ck[r - 1];
+            r--;
+        }
+        R.body[r] = (int8_t)e;
+        R.stamp[r] = (uint32_t)st;
+        R.ci[r] = (int16_t)i;
+        R.cj[r] = (int16_t)j;
+        R.ck[r] = (int16_t)k;
+    }
+}
+
+RSB_HD size_t rayIdx(const EngineView& D, int a, int s, int w) { return ((size_t)w * MAX_CARS + s) * D.N + a; }
+RSB_HD void storeRay(const EngineView& D, const StepTemp& T, size_t r, int obj, float frac, V3 n) {
+    T.rayObj[r] = obj;
+    if (obj < 0) return;
+    const size_t st = (size_t)4 * MAX_CARS * D.N;
+    T.rayFrac[r] = frac;
+    T.rayN[r] = n.x;
+    T.rayN[r + st] = n.y;
+    T.rayN[r + 2 * st] = n.z;
+}
+
+// The casting car at the start of its pre-tick: false when it stays demoed (casts no rays).
+RSB_HD bool rayCar(const EngineView& D, int a, int s, Xf& xf, bool& culled) {
+    const uint32_t f = carWord(D, a, s, RSB_PW(CarP, flags));
+    culled = D.cull && ((D.cull[a] >> (1 + s)) & 1u);
+    if (f & CF_DEMOED) {
+        if (!respawns(D, a, s)) return false;
+        xf = respawnXf(D, a, s, f, arenaTickCount(D, a));
+        culled = false;
+    } else {
+        xf = bodyXf(D, a, 1 + s);
+    }
+    return true;
+}
+
+// Wheel w of car s: casts the ray if only planes can be near, else returns true (queue it).
+// `near(i, j, k)`: whether a body other than the car is registered around that cell.
+template <class NearF>
+RSB_HD bool rayPhase(const EngineView& D, const StepTemp& T, int a, int s, int w, const Xf& xf, bool culled,
+                     NearF&& near, PhaseStats& st) {
+    const ArenaStatic& S = D.S;
+    Body cb;
+    WheelTick wt;
+    V3 from, to;
+    cb.xf = xf;
+    wheelSegment(D.P.car, cb, wt, w, from, to);
+    if (culled || !(dist2(from, to) < S.bp.cellSize * S.bp.cellSize)) return true;
+    int i, j, k;
+    bpCellIndices(S.bp, from, i, j, k);
+    uint32_t mask = S.bpCells[i * S.bp.cellsY * S.bp.cellsZ + j * S.bp.cellsZ + k];
+    if (near(i, j, k)) return true;
+    const uint32_t kMeshBits = (1u << MAX_MESHES) - 1u;
+    if (mask & kMeshBits) {
+        const V3 tolv{kOccTol, kOccTol, kOccTol};
+        if (mask & kMeshBits & occMask(S, vmin(from, to) - tolv, vmax(from, to) + tolv)) return true;
+    }
+    RayHit hit;
+    hit.fraction = 1.f;
+    hit.obj = -1;
+    hit.normal = v3zero();
+    for (mask >>= MAX_MESHES; mask; mask &= mask - 1u) {
+        if (hit.fraction == 0.f) break;
+        st.nStatic++;
+        rayVsPlane(S, MAX_MESHES + lowestBit(mask), from, to, hit);
+    }
+    storeRay(D, T, rayIdx(D, a, s, w), hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
+    return false;
+}
+
+// A queued ray: castRay over everything around it.
+RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
+    const int a = (int)(r % (uint32_t)D.N), q = (int)(r / (uint32_t)D.N), s = q % MAX_CARS, w = q / MAX_CARS;
+    Xf xf;
+    bool culled;
+    if (!rayCar(D, a, s, xf, culled)) return;  // never queued
+    Body cb;
+    WheelTick wt;
+    V3 from, to;
+    cb.xf = xf;
+    wheelSegment(D.P.car, cb, wt, w, from, to);
+    RayWorld W;
+    W.S = &D.S;
+    W.P = &D.P;
+    W.nb = arenaBodies(D, a);
+    W.b.D = &D;
+    W.b.a = a;
+    W.b.viewer = s;
+    W.b.tick = arenaTickCount(D, a);
+    W.cull = culled ? 1u << (1 + s) : 0u;
+    W.cullAudit = D.cullAudit;
+    W.nStatic = W.nCulled = W.nMissed = W.cullMissed = 0;
+    regOrderOf(W.reg, W.nb, [&](int e) { return (int32_t)bodyWord(D, a, e, RSB_PW(CarP, regStamp)); },
+               [&](int e, int& i, int& j, int& k) {
+                   i = (int)bodyWord(D, a, e, RSB_PW(CarP, ci));
+                   j = (int)bodyWord(D, a, e, RSB_PW(CarP, cj));
+                   k = (int)bodyWord(D, a, e, RSB_PW(CarP, ck));
+               });
+    V3 hp, hn = v3zero();
+    float frac = 1.f;
+    const int obj = castRay(W, from, to, OBJ_CAR0 + s, hp, hn, frac);
+    storeRay(D, T, r, obj, frac, hn);
+    st.nStatic += W.nStatic;
+    st.nCulled += W.nCulled;
+    st.nMissed += W.nMissed;
+    if (W.cullMissed) phaseAtomicOr(arenaStatus(D, a), W.cullMissed);
+}
+
+// ------------------------------------------------------------------ bodies
+
+// What the threads of one arena's bodies exchange during the bodies phase, one column per arena.
+constexpr int PHASE_ARENAS = 32;
+struct BodyShared {
+    float pre[MAX_CARS][6][PHASE_ARENAS];   // linear and angular velocity before the car's pre-tick
+    float post[MAX_CARS][6][PHASE_ARENAS];  // ... and after it
+    float box[MAX_BODIES][6][PHASE_ARENAS];
+    int32_t cell[MAX_BODIES][3][PHASE_ARENAS];
+    uint32_t stamp[MAX_BODIES][PHASE_ARENAS];
+    uint32_t pick[MAX_BODIES][PHASE_ARENAS];  // BI_DYN word of each body
+    uint32_t live[MAX_BODIES][PHASE_ARENAS];  // 1: active (objActive)
+    uint32_t done[PHASE_ARENAS];              // cars whose pre-tick is finished
+    uint32_t need[PHASE_ARENAS];              // the arena has contacts or dynamic pairs to solve
+};
+
+struct OneBody {
+    Body v;
+    RSB_HD Body& operator[](int) { return v; }
+    RSB_HD const Body& operator[](int) const { return v; }
+};
+struct OneCar {
+    CarSim v;
+    RSB_HD CarSim& operator[](int) { return v; }
+    RSB_HD const CarSim& operator[](int) const { return v; }
+};
+
+// One car's view of the world in its pre-tick.
+struct CarWorld {
+    const ArenaStatic* S;
+    const WorldParams* P;
+    uint64_t tick;
+    uint32_t cull;
+    OneBody b;
+    OneCar c;
+    const EngineView* D;
+    const BodyShared* sh;
+    int a, la, ci;
+};
+
+// A dynamic ground object of a wheel: cars of higher slots have finished their pre-tick.
+RSB_HD GroundRef groundRef(const CarWorld& W, int o) {
+    GroundRef g;
+    g.body = nullptr;
+    if (o < OBJ_BALL) {
+        g.com = o < MAX_MESHES ? v3zero() : W.S->planeOrigin[o - MAX_MESHES];
+        g.lin = g.ang = v3zero();
+        g.basis = m3identity();
+        g.invInertiaLocal = v3zero();
+        g.invMass = 0.f;
+        return g;
+    }
+    const int b = o - OBJ_BALL;
+    const Xf x = bodyXf(*W.D, W.a, b);
+    g.com = x.o;
+    g.basis = x.b;
+    if (b == 0) {
+        g.lin = bodyV3(*W.D, W.a, 0, RSB_PW(BallP, lin));
+        g.ang = bodyV3(*W.D, W.a, 0, RSB_PW(BallP, ang));
+        g.invInertiaLocal = W.P->ballInvInertia;
+        g.invMass = W.P->ballInvMass;
+    } else {
+        const float(*v)[PHASE_ARENAS] = (b - 1 > W.ci) ? W.sh->post[b - 1] : W.sh->pre[b - 1];
+        g.lin = V3{v[0][W.la], v[1][W.la], v[2][W.la]};
+        g.ang = V3{v[3][W.la], v[4][W.la], v[5][W.la]};
+        g.invInertiaLocal = W.P->car.invInertiaLocal;
+        g.invMass = W.P->car.invMass;
+    }
+    return g;
+}
+
+// One body's thread of the bodies phase.
+struct BodyThread {
+    int a, la, b, nb;   // b < nb when there is such a body
+    bool live;          // a car whose vehicle update runs (not demoed)
+    bool respawned, finished;
+    uint32_t deps;      // cars whose finished pre-tick this one waits for
+    uint32_t dyn;       // BI_DYN word
+    CarWorld W;
+};
+
+RSB_HD void publishVel(float (*v)[PHASE_ARENAS], int la, const Body& b) {
+    v[0][la] = b.lin.x; v[1][la] = b.lin.y; v[2][la] = b.lin.z;
+    v[3][la] = b.ang.x; v[4][la] = b.ang.y; v[5][la] = b.ang.z;
+}
+
+// Loads the body; a car runs its status update.  Nothing is written to the records before
+// every thread of the arena has published what others read.
+RSB_HD void bodyLoad(const EngineView& D, const StepTemp& T, BodyThread& t, BodyShared& sh) {
+    CarWorld& W = t.W;
+    Body& b = W.b.v;
+    CarSim& c = W.c.v;
+    W.S = &D.S;
+    W.P = &D.P;
+    W.D = &D;
+    W.sh = &sh;
+    W.a = t.a;
+    W.la = t.la;
+    W.ci = t.b - 1;
+    W.tick = arenaTickCount(D, t.a);
+    W.cull = 0;
+    t.live = t.respawned = false;
+    t.finished = true;
+    t.deps = 0;
+    t.dyn = 0;
+    const int a = t.a, s = t.b - 1;
+    bodyConstants(D, t.b, b);
+    b.xf = bodyXf(D, a, t.b);
+    b.lin = bodyV3(D, a, t.b, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, t.b, RSB_PW(CarP, ang));
+    b.cell = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cell));
+    b.ci = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ci));
+    b.cj = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cj));
+    b.ck = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ck));
+    b.regStamp = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, regStamp));
+    updateInertia(b);
+    if (t.b == 0) {
+        // ball zero-velocity sleeping (Arena.cpp:721-727)
+        b.act = (length2(b.lin) == 0.f && length2(b.ang) == 0.f) ? ACT_SLEEPING : ACT_ACTIVE;
+        return;
+    }
+    publishVel(sh.pre[s], t.la, b);
+    c.flags = carWord(D, a, s, RSB_PW(CarP, flags));
+    c.team = (c.flags & CF_TEAM_ORANGE) ? 1 : 0;
+    c.id = (uint32_t)s + 1u;
+    c.boost = carFloat(D, a, s, RSB_PW(CarP, boost));
+    c.timeSpentBoosting = carFloat(D, a, s, RSB_PW(CarP, timeSpentBoosting));
+    c.jumpTime = carFloat(D, a, s, RSB_PW(CarP, jumpTime));
+    c.flipTime = carFloat(D, a, s, RSB_PW(CarP, flipTime));
+    c.airTime = carFloat(D, a, s, RSB_PW(CarP, airTime));
+    c.airTimeSinceJump = carFloat(D, a, s, RSB_PW(CarP, airTimeSinceJump));
+    c.handbrakeVal = carFloat(D, a, s, RSB_PW(CarP, handbrakeVal));
+    c.autoFlipTimer = carFloat(D, a, s, RSB_PW(CarP, autoFlipTimer));
+    c.autoFlipTorqueScale = carFloat(D, a, s, RSB_PW(CarP, autoFlipTorqueScale));
+    c.demoRespawnTimer = carFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer));
+    c.flipRelTorque = carV3(D, a, s, RSB_PW(CarP, flipRelTorque));
+    c.worldContactNormal = carV3(D, a, s, RSB_PW(CarP, worldContactNormal));
+    for (int r = 0; r < 3; r++) c.rotMat.r[r] = carV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r);
+    c.lastCtlBits = carWord(D, a, s, RSB_PW(CarP, lastCtlBits));
+    c.steerAngle = carFloat(D, a, s, RSB_PW(CarP, steerAngle));
+    c.engineForce = carFloat(D, a, s, RSB_PW(CarP, engineForce));
+    c.brake = carFloat(D, a, s, RSB_PW(CarP, brake));
+    for (int i = 0; i < 4; i++) {
+        c.latF[i] = carFloat(D, a, s, RSB_PW(CarP, latFriction) + i);
+        c.longF[i] = carFloat(D, a, s, RSB_PW(CarP, longFriction) + i);
+        c.extraPush[i] = carFloat(D, a, s, RSB_PW(CarP, extraPushback) + i);
+    }
+    const CtlRec& ctl = D.controls[D.carOffset[a] + s];
+    for (int k = 0; k < 5; k++) c.ctl[k] = ctl.v[k];
+    c.ctlBits = (ctl.jump ? 1u : 0u) | (ctl.boost ? 2u : 0u) | (ctl.handbrake ? 4u : 0u);
+    const bool wasDemoed = (c.flags & CF_DEMOED) != 0;
+    t.live = carPreTickStatus(W, s, mixHash(mixHash(D.seed, (uint32_t)a, 0x5EEDu), (uint32_t)W.tick, (uint32_t)s));
+    t.respawned = wasDemoed && t.live;
+    t.finished = !t.live;
+    if (t.finished) publishVel(sh.post[s], t.la, b);
+    if (t.respawned && D.cull) phaseAtomicAnd(const_cast<uint32_t*>(D.cull) + a, ~(1u << t.b));
+    if (!t.live) return;
+    // wheels: steering basis and the rays' results
+    const size_t rst = (size_t)4 * MAX_CARS * D.N;
+    for (int i = 0; i < 4; i++) {
+        wheelTransform(D.P.car, b, c.w[i], i, i < 2 ? c.steerAngle : 0.f);
+        V3 from, to, hp = v3zero(), hn = v3zero();
+        wheelSegment(D.P.car, b, c.w[i], i, from, to);
+        const size_t r = rayIdx(D, a, s, i);
+        const int obj = T.rayObj[r];
+        if (obj >= 0) {
+            const float f = T.rayFrac[r], f1 = 1.f - f;
+            hp = from * f1 + to * f;
+            hn = V3{T.rayN[r], T.rayN[r + rst], T.rayN[r + 2 * rst]};
+            if (obj > OBJ_CAR0 + s) t.deps |= 1u << (obj - OBJ_CAR0);
+        }
+        wheelFromHit(W, s, i, to, obj, hp, hn);
+    }
+}
+
+// The vehicle update, once the cars it stands on have finished theirs.
+RSB_HD void bodyDrive(BodyThread& t, BodyShared& sh) {
+    carDrive(t.W, t.b - 1);
+    publishVel(sh.post[t.b - 1], t.la, t.W.b.v);
+    t.finished = true;
+}
+
+// Gravity, predicted motion, broadphase box and registration; writes the record.
+RSB_HD void bodyMove(const EngineView& D, const StepTemp& T, BodyThread& t, BodyShared& sh, bool firstTick) {
+    Body& b = t.W.b.v;
+    CarSim& c = t.W.c.v;
+    const int a = t.a, s = t.b - 1, la = t.la;
+    const float dt = D.P.dt;
+    if (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) b.force = b.force + b.grav;
+    b.lin = b.lin * b.linDampFactor;
+    b.ixf = t.b == 0 ? integrateTransformNoRot(b.xf, b.lin, dt) : integrateTransform(b.xf, b.lin, b.ang, dt);
+    // the box of the last tick stays when this one's is not finite
+    b.bpMin = b.bpMax = b.xf.o;
+    struct {
+        const ArenaStatic* S;
+        const WorldParams* P;
+        int nb;
+        OneBody* bp;
+        uint32_t stampBase, status;
+        struct Ref {
+            OneBody* p;
+            RSB_HD Body& operator[](int i) { return (*p)[i]; }
+        } b;
+    } M{&D.S, &D.P, t.nb, nullptr, (uint32_t)((t.W.tick + 1) * 8u), 0u, {&t.W.b}};
+    updateBodyAabb(M, t.b);
+    if (M.status) {
+        phaseAtomicOr(arenaStatus(D, a), M.status);
+        if (!firstTick) {
+            b.bpMin = tempV3(D, T.box, a, t.b, 0);
+            b.bpMax = tempV3(D, T.box, a, t.b, 3);
+        }
+    }
+    putTempV3(D, T.box, a, t.b, 0, b.bpMin);
+    putTempV3(D, T.box, a, t.b, 3, b.bpMax);
+    putTempV3(D, T.force, a, t.b, 0, b.force);
+    putTempV3(D, T.force, a, t.b, 3, b.torque);
+    const float bx[6] = {b.bpMin.x, b.bpMin.y, b.bpMin.z, b.bpMax.x, b.bpMax.y, b.bpMax.z};
+    for (int k = 0; k < 6; k++) sh.box[t.b][k][la] = bx[k];
+    sh.cell[t.b][0][la] = b.ci;
+    sh.cell[t.b][1][la] = b.cj;
+    sh.cell[t.b][2][la] = b.ck;
+    sh.stamp[t.b][la] = (uint32_t)b.regStamp;
+    sh.live[t.b][la] = (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) ? 1u : 0u;
+
+    putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
+    putBodyWord(D, a, t.b, RSB_PW(CarP, cell), (uint32_t)b.cell);
+    putBodyWord(D, a, t.b, RSB_PW(CarP, ci), (uint32_t)b.ci);
+    putBodyWord(D, a, t.b, RSB_PW(CarP, cj), (uint32_t)b.cj);
+    putBodyWord(D, a, t.b, RSB_PW(CarP, ck), (uint32_t)b.ck);
+    putBodyWord(D, a, t.b, RSB_PW(CarP, regStamp), (uint32_t)b.regStamp);
+    if (t.b == 0) return;
+    putCarWord(D, a, s, RSB_PW(CarP, flags), (c.flags & ~CF_NO_RESPONSE) | (b.noResp ? CF_NO_RESPONSE : 0u));
+    putCarFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer), c.demoRespawnTimer);
+    if (!t.live) return;
+    putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+    putCarFloat(D, a, s, RSB_PW(CarP, boost), c.boost);
+    putCarFloat(D, a, s, RSB_PW(CarP, timeSpentBoosting), c.timeSpentBoosting);
+    putCarFloat(D, a, s, RSB_PW(CarP, jumpTime), c.jumpTime);
+    putCarFloat(D, a, s, RSB_PW(CarP, flipTime), c.flipTime);
+    putCarFloat(D, a, s, RSB_PW(CarP, airTime), c.airTime);
+    putCarFloat(D, a, s, RSB_PW(CarP, airTimeSinceJump), c.airTimeSinceJump);
+    putCarFloat(D, a, s, RSB_PW(CarP, handbrakeVal), c.handbrakeVal);
+    putCarFloat(D, a, s, RSB_PW(CarP, autoFlipTimer), c.autoFlipTimer);
+    putCarFloat(D, a, s, RSB_PW(CarP, autoFlipTorqueScale), c.autoFlipTorqueScale);
+    putCarV3(D, a, s, RSB_PW(CarP, flipRelTorque), c.flipRelTorque);
+    putCarFloat(D, a, s, RSB_PW(CarP, steerAngle), c.steerAngle);
+    putCarFloat(D, a, s, RSB_PW(CarP, engineForce), c.engineForce);
+    putCarFloat(D, a, s, RSB_PW(CarP, brake), c.brake);
+    for (int i = 0; i < 4; i++) {
+        putCarFloat(D, a, s, RSB_PW(CarP, latFriction) + i, c.latF[i]);
+        putCarFloat(D, a, s, RSB_PW(CarP, longFriction) + i, c.longF[i]);
+        putCarFloat(D, a, s, RSB_PW(CarP, extraPushback) + i, c.extraPush[i]);
+    }
+    if (!t.respawned) return;
+    // Car::SetState of the spawn: the rest of the record
+    putBodyXf(D, a, t.b, b.xf);
+    putCarFloat(D, a, s, RSB_PW(CarP, supersonicTime), 0.f);
+    putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), 0.f);
+    putCarV3(D, a, s, RSB_PW(CarP, worldContactNormal), v3zero());
+    putCarWord(D, a, s, RSB_PW(CarP, carContactOtherId), 0u);
+    for (int k = 0; k < 2; k++) {
+        putCarWord(D, a, s, RSB_PW(CarP, ballHitTick) + k, ~0u);
+        putCarWord(D, a, s, RSB_PW(CarP, ballHitExtraTick) + k, ~0u);
+    }
+    putCarV3(D, a, s, RSB_PW(CarP, ballHitRelPos), v3zero());
+    putCarV3(D, a, s, RSB_PW(CarP, ballHitBallPos), v3zero());
+    putCarV3(D, a, s, RSB_PW(CarP, ballHitExtraVel), v3zero());
+    for (int r = 0; r < 3; r++) putCarV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r, c.rotMat.r[r]);
+}
+
+RSB_HD V3 sharedV3(const float (*v)[PHASE_ARENAS], int k, int la) { return V3{v[k][la], v[k + 1][la], v[k + 2][la]}; }
+
+// The dynamic pairs of this body in visiting order (the second half of computePairs).
+RSB_HD void bodyPick(const EngineView& D, BodyThread& t, BodyShared& sh) {
+    const Body& b = t.W.b.v;
+    const BpGrid& g = D.S.bp;
+    const int la = t.la;
+    t.dyn = 0;
+    if (t.nb > 1) {
+        const int ci = b.cell / (g.cellsY * g.cellsZ), cj = (b.cell / g.cellsZ) % g.cellsY, ck = b.cell % g.cellsZ;
+        auto near = [&](int e) {
+            const int i = sh.cell[e][0][la], j = sh.cell[e][1][la], k = sh.cell[e][2][la];
+            return ci >= i - 1 && ci <= i + 1 && cj >= j - 1 && cj <= j + 1 && ck >= k - 1 && ck <= k + 1;
+        };
+        uint32_t cand = 0;
+        for (int e = 0; e < t.nb; e++) cand |= near(e) ? 1u << e : 0u;
+        // in registration order; a proxy whose stamp equals the one just visited is passed over
+        if (cand & (cand - 1u)) {
+            uint32_t last = 0, n = 0;
+            bool first = true;
+            while (cand) {
+                int pick = -1;
+                uint32_t ps = 0;
+                for (int e = 0; e < t.nb; e++) {
+                    if (!((cand >> e) & 1u)) continue;
+                    const uint32_t st = sh.stamp[e][la];
+                    if (pick < 0 || st < ps) {
+                        pick = e;
+                        ps = st;
+                    }
+                }
+                cand &= ~(1u << pick);
+                if (!first && ps <= last) continue;
+                first = false;
+                last = ps;
+                if (pick == t.b) continue;
+                if (aabbOverlap(b.bpMin, b.bpMax, sharedV3(sh.box[pick], 0, la), sharedV3(sh.box[pick], 3, la)))
+                    t.dyn |= (uint32_t)pick << (3 * n++);
+            }
+            t.dyn |= n << 24;
+        }
+    }
+    sh.pick[t.b][la] = t.dyn;
+}
+
+// Contact world of one pair: at most two bodies.
+struct LocalPool {
+    int32_t n;
+    uint32_t* status;
+    MPoint pts[MAX_POINTS];
+};
+struct PairBodies {
+    Body v0, v1;
+    int i0;
+    RSB_HD Body& operator[](int i) { return i == i0 ? v0 : v1; }
+    RSB_HD const Body& operator[](int i) const { return i == i0 ? v0 : v1; }
+};
+template <class BodiesT>
+struct PairWorldT {
+    const ArenaStatic* S;
+    const WorldParams* P;
+    BodiesT b;
+    OneCar c;
+    LocalPool pool;
+    uint32_t status;
+    EpaWork* epa;
+    uint32_t cull;
+    int32_t cullAudit;
+    mutable uint32_t nStatic, nCulled, nMissed, cullMissed;
+};
+template <class WT>
+RSB_HD void pairWorldInit(const EngineView& D, WT& W, EpaWork* epa, uint32_t cull) {
+    W.S = &D.S;
+    W.P = &D.P;
+    W.pool.n = 0;
+    W.pool.status = &W.status;
+    W.status = 0;
+    W.epa = epa;
+    W.cull = cull;
+    W.cullAudit = D.cullAudit;
+    W.nStatic = W.nCulled = W.nMissed = W.cullMissed = 0;
+    W.c.v.flags = 0;
+    W.c.v.worldContactNormal = v3zero();
+}
+RSB_HD void pairManifold(Manifold& m, int o0, int o1, float cbt) {
+    m.o0 = o0;
+    m.o1 = o1;
+    m.cbt = cbt;
+    m.n = 0;
+    m.pt = nullptr;
+}
+template <class WT>
+RSB_HD void storePair(const EngineView& D, const StepTemp& T, int a, WT& W, const Manifold& m, uint32_t res) {
+    PairResult r;
+    r.n = m.n;
+    r.flags = (m.pt ? PR_BLOCK : 0u) | ((W.c.v.flags & CF_WORLD_CONTACT) ? PR_WORLD : 0u);
+    r.block = 0;
+    r.normal[0] = W.c.v.worldContactNormal.x;
+    r.normal[1] = W.c.v.worldContactNormal.y;
+    r.normal[2] = W.c.v.worldContactNormal.z;
+    if (m.n > 0) {
+        r.block = phaseAtomicAdd(&T.count[QC_BLOCK], 1u);
+        if (r.block < T.blockCap) {
+            MPoint* dst = T.blocks + (size_t)MAX_POINTS * r.block;
+            for (int k = 0; k < m.n; k++) dst[k] = m.pt[k];
+        } else {
+            r.n = 0;  // more blocks than the whole batch may hold: the contacts are dropped
+            r.block = r.flags = 0;
+            W.status |= WS_OVERFLOW;
+        }
+    }
+    T.results[res] = r;
+    if (W.status | W.cullMissed) phaseAtomicOr(arenaStatus(D, a), W.status | W.cullMissed);
+}
+
+// Static pairs: manifolds, plane contacts, queued meshes (the mesh bits are returned; the
+// caller allocates their places and stores them with bodyStaticStore).
+struct BodyStatics {
+    uint32_t pairs, mani, meshes, planes;
+    uint32_t planeRes[NUM_PLANES];
+};
+RSB_HD BodyStatics bodyStatics(const EngineView& D, const StepTemp& T, BodyThread& t, PhaseStats& st) {
+    BodyStatics o;
+    o.pairs = o.mani = o.meshes = o.planes = 0;
+    for (int p = 0; p < NUM_PLANES; p++) o.planeRes[p] = 0;
+    const ArenaStatic& S = D.S;
+    const Body& b = t.W.b.v;
+    const CarParams& C = D.P.car;
+    const bool active = b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM;
+    const uint32_t cull = D.cull ? (D.cull[t.a] & (1u << t.b)) : 0u;
+    // the box the narrowphase tests: the ball's, or the hitbox at its place in the car
+    Xf childXf = t.b == 0 ? b.xf : carChildXf(C, b.xf);
+    V3 bmn, bmx;
+    if (t.b == 0) ballAabb(D.P, b.xf, bmn, bmx);
+    else carBoxAabb(C, childXf, bmn, bmx);
+    uint32_t occ = 0;
+    bool occKnown = false;
+    for (uint32_t mask = S.bpCells[b.cell]; mask; mask &= mask - 1u) {
+        const int s = lowestBit(mask);
+        V3 smn, smx;
+        if (s < MAX_MESHES) { smn = S.meshes[s].bpMin; smx = S.meshes[s].bpMax; }
+        else { smn = S.planeBpMin[s - MAX_MESHES]; smx = S.planeBpMax[s - MAX_MESHES]; }
+        if (!aabbOverlap(b.bpMin, b.bpMax, smn, smx)) continue;
+        o.pairs |= 1u << s;
+        if (!active) continue;
+        if (t.b != 0) {
+            if (s < MAX_MESHES) { smn = S.meshes[s].shapeMin; smx = S.meshes[s].shapeMax; }
+            else { smn = S.planeShapeMin[s - MAX_MESHES]; smx = S.planeShapeMax[s - MAX_MESHES]; }
+            if (!aabbOverlap(bmn, bmx, smn, smx)) continue;  // its manifold is released again
+        }
+        o.mani |= 1u << s;
+        if (s < MAX_MESHES) {
+            // cullSkip's bookkeeping, then the occupancy reject of the mesh walk
+            if (cull) {
+                st.nCulled++;
+                if (!D.cullAudit) continue;
+            }
+            st.nStatic++;
+            if (!occKnown) {
+                const V3 tolv{kOccTol, kOccTol, kOccTol};
+                occ = occMask(S, bmn - tolv, bmx + tolv);
+                occKnown = true;
+            }
+            if ((occ >> s) & 1u) o.meshes |= 1u << s;
+        } else {
+            PairWorldT<OneBody> W;
+            pairWorldInit(D, W, nullptr, cull);
+            W.b.v = b;
+            Manifold m;
+            if (t.b == 0) {
+                pairManifold(m, OBJ_BALL, s, D.P.ballCbt);
+                collideBallPlane(W, s, m);
+            } else {
+                pairManifold(m, OBJ_CAR0 + t.b - 1, s, C.cbt);
+                collideBoxPlane(W, s, t.b - 1, childXf, m);
+            }
+            st.nStatic += W.nStatic;
+            st.nCulled += W.nCulled;
+            st.nMissed += W.nMissed;
+            if (m.pt) {
+                const uint32_t k = phaseAtomicAdd(&T.count[QC_PLANE], 1u);
+                const uint32_t r = (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + k;
+                o.planes |= 1u << (s - MAX_MESHES);
+                o.planeRes[s - MAX_MESHES] = r;
+                storePair(D, T, t.a, W, m, r);
+            } else if (W.cullMissed) {
+                phaseAtomicOr(arenaStatus(D, t.a), W.cullMissed);
+            }
+        }
+    }
+    return o;
+}
+
+// The dynamic pairs (b, hi > b) that have a manifold: bit hi.
+RSB_HD uint32_t bodyDynamics(const EngineView& D, const BodyThread& t, const BodyShared& sh) {
+    const CarParams& C = D.P.car;
+    const Body& b = t.W.b.v;
+    uint32_t m = 0;
+    auto picked = [&](int x, int y) {
+        const uint32_t d = sh.pick[x][t.la];
+        for (uint32_t k = 0; k < (d >> 24); k++)
+            if (((d >> (3 * k)) & 7u) == (uint32_t)y) return true;
+        return false;
+    };
+    for (int hi = t.b + 1; hi < t.nb; hi++) {
+        if (!picked(t.b, hi) && !picked(hi, t.b)) continue;
+        if (!sh.live[t.b][t.la] && !sh.live[hi][t.la]) continue;
+        // the other body's transform: a car that respawned wrote its spawn to its record, which
+        // every thread of the arena has finished by now
+        const Xf hx = bodyXf(D, t.a, hi);
+        V3 mn, mx, mn2, mx2;
+        if (t.b == 0) {
+            carBoxAabb(C, carChildXf(C, hx), mn, mx);
+            ballAabb(D.P, b.xf, mn2, mx2);
+            if (aabbOverlap(mn, mx, mn2, mx2)) m |= 1u << hi;
+        } else {
+            // car a = lower slot, car b = higher slot (collideCarCar)
+            carBoxAabb(C, carChildXf(C, b.xf), mn, mx);
+            carCompoundAabb(C, hx, mn2, mx2);
+            if (!aabbOverlap(mn, mx, mn2, mx2)) continue;
+            carBoxAabb(C, carChildXf(C, hx), mn2, mx2);
+            if (aabbOverlap(mn2, mx2, mn, mx)) m |= 1u << hi;
+        }
+    }
+    return m;
+}
+
+// Stores the body's pair information and fills its queue places: `mesh0` the first of its mesh
+// pairs in their queue, `dyn0` the first of its dynamic pairs in theirs.
+RSB_HD void bodyStore(const EngineView& D, const StepTemp& T, const BodyThread& t, BodyShared& sh,
+                      const BodyStatics& o, uint32_t dynMani, uint32_t mesh0, uint32_t dyn0) {
+    const int a = t.a;
+    const Body& b = t.W.b.v;
+    const int meshType = t.b == 0 ? QC_BALLMESH : QC_CARMESH, dynType = t.b == 0 ? QC_CARBALL : QC_CARCAR;
+    infoWord(D, T, a, t.b, BI_PAIRS) = o.pairs | ((uint32_t)b.act << BI_ACT_SHIFT) | (b.noResp ? 0u : BI_RESPONDS);
+    infoWord(D, T, a, t.b, BI_DYN) = t.dyn;
+    if (o.pairs | t.dyn | dynMani) {
+        infoWord(D, T, a, t.b, BI_MANI) = o.mani;
+        infoWord(D, T, a, t.b, BI_TASKS) = o.meshes | (o.planes << 16);
+        infoWord(D, T, a, t.b, BI_DYNMANI) = dynMani;
+    }
+    const uint32_t mb = (uint32_t)resultBase(meshType) * (uint32_t)D.N + mesh0;
+    if (o.meshes) infoWord(D, T, a, t.b, BI_MESHRES) = mb;
+    uint32_t k = 0;
+    for (uint32_t m = o.meshes; m; m &= m - 1u, k++)
+        T.tasks[mb + k] = PairTask{(uint32_t)a, (uint16_t)lowestBit(m), (uint16_t)(OBJ_BALL + t.b)};
+    for (int p = 0; p < NUM_PLANES; p++)
+        if ((o.planes >> p) & 1u) infoWord(D, T, a, t.b, BI_PLANERES + p) = o.planeRes[p];
+    const uint32_t db = (uint32_t)resultBase(dynType) * (uint32_t)D.N + dyn0;
+    k = 0;
+    for (uint32_t m = dynMani; m; m &= m - 1u, k++) {
+        const int hi = lowestBit(m);
+        T.tasks[db + k] = PairTask{(uint32_t)a, (uint16_t)(OBJ_BALL + t.b), (uint16_t)(OBJ_BALL + hi)};
+        T.dynRes[(size_t)dynPair(t.b, hi) * D.N + a] = db + k;
+    }
+    // an arena without contacts and without dynamic pairs has nothing to solve
+    if (o.meshes | o.planes | dynMani | t.dyn) phaseAtomicOr(&sh.need[t.la], 1u);
+}
+
+// ------------------------------------------------------------------ contacts
+
+RSB_HD void pairBody(const EngineView& D, int a, int b, Body& o) {
+    bodyConstants(D, b, o);
+    o.xf = bodyXf(D, a, b);
+    o.noResp = b > 0 && (carWord(D, a, b - 1, RSB_PW(CarP, flags)) & CF_NO_RESPONSE) ? 1 : 0;
+}
+
+// One queued pair; `res` is its place in the task and result arrays.
+RSB_HD void carMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, EpaWork* epa, PhaseStats& st) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a, b = k.o1 - OBJ_BALL;
+    PairWorldT<OneBody> W;
+    pairWorldInit(D, W, epa, D.cull ? (D.cull[a] & (1u << b)) : 0u);
+    pairBody(D, a, b, W.b.v);
+    Manifold m;
+    pairManifold(m, k.o1, k.o0, D.P.car.cbt);
+    collideBoxMesh(W, k.o0, b - 1, carChildXf(D.P.car, W.b.v.xf), m);
+    st.nMissed += W.nMissed;
+    storePair(D, T, a, W, m, res);
+}
+RSB_HD void ballMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, PhaseStats& st) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a;
+    PairWorldT<OneBody> W;
+    pairWorldInit(D, W, nullptr, D.cull ? (D.cull[a] & 1u) : 0u);
+    pairBody(D, a, 0, W.b.v);
+    Manifold m;
+    pairManifold(m, OBJ_BALL, k.o0, D.P.ballCbt);
+    collideBallMesh(W, k.o0, m);
+    st.nMissed += W.nMissed;
+    storePair(D, T, a, W, m, res);
+}
+// Car pairs keep their points as added: the islands phase runs the callbacks on them before
+// refreshContactPoints.
+RSB_HD void carBallPhase(const EngineView& D, const StepTemp& T, uint32_t res, EpaWork* epa) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a, b = k.o1 - OBJ_BALL;
+    PairWorldT<PairBodies> W;
+    pairWorldInit(D, W, epa, 0u);
+    W.b.i0 = 0;
+    pairBody(D, a, 0, W.b.v0);
+    pairBody(D, a, b, W.b.v1);
+    Manifold m;
+    pairManifold(m, k.o1, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt));
+    carBallContact(W, b - 1, carChildXf(D.P.car, W.b.v1.xf), m);
+    storePair(D, T, a, W, m, res);
+}
+RSB_HD void carCarPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a, ba = k.o0 - OBJ_BALL, bb = k.o1 - OBJ_BALL;
+    PairWorldT<PairBodies> W;
+    pairWorldInit(D, W, nullptr, 0u);
+    W.b.i0 = ba;
+    pairBody(D, a, ba, W.b.v0);
+    pairBody(D, a, bb, W.b.v1);
+    Manifold m;
+    pairManifold(m, k.o1, k.o0, D.P.car.cbt);
+    BoxContacts bc;
+    carCarContacts(W, ba - 1, bb - 1, bc);
+    ObjRef rA = objRef(W, k.o0), rB = objRef(W, k.o1);
+    for (int c = 0; c < bc.n; c++)
+        addContact(m, W.pool, k.o0, rA, k.o1, rB, bc.c[c].normalOnB, bc.c[c].point, bc.c[c].depth);
+    storePair(D, T, a, W, m, res);
+}
+
+// ------------------------------------------------------------------ islands
+
+struct SolveCars {
+    CarSim v[2];
+    int i0;
+    RSB_HD CarSim& operator[](int i) { return v[i == i0 ? 0 : 1]; }
+    RSB_HD const CarSim& operator[](int i) const { return v[i == i0 ? 0 : 1]; }
+};
+// The arena as the contact callbacks and solveIslands see it.
+struct SolveWorld {
+    const ArenaStatic* S;
+    const WorldParams* P;
+    int nb;
+    Body b[MAX_BODIES];
+    int noRot[MAX_BODIES];
+    int np;
+    int16_t po0[MAX_PAIRS], po1[MAX_PAIRS];
+    int nm;
+    Manifold m[MAX_MANIFOLDS];
+    uint32_t status;
+    SolveCars c;
+    uint64_t tick;
+    V3 ballVelCache;
+    uint32_t nRows;
+};
+
+// The car fields that the car-ball and car-car callbacks read and write.
+RSB_HD void loadContactCar(const EngineView& D, int a, int s, CarSim& c, V3 velCache) {
+    c.flags = carWord(D, a, s, RSB_PW(CarP, flags));
+    c.team = (c.flags & CF_TEAM_ORANGE) ? 1 : 0;
+    c.id = (uint32_t)s + 1u;
+    c.carContactOtherId = carWord(D, a, s, RSB_PW(CarP, carContactOtherId));
+    c.carContactCooldown = carFloat(D, a, s, RSB_PW(CarP, carContactCooldown));
+    c.demoRespawnTimer = carFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer));
+    c.ballHitExtraTick = (uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitExtraTick)) |
+                         ((uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitExtraTick) + 1) << 32);
+    for (int r = 0; r < 3; r++) c.rotMat.r[r] = carV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r);
+    c.velCache = velCache;
+}
+
+// Callbacks, islands and solver of one arena.
+RSB_HD void solvePhase(const EngineView& D, const StepTemp& T, int a, PhaseStats& st) {
+    SolveWorld W;
+    W.S = &D.S;
+    W.P = &D.P;
+    W.nb = arenaBodies(D, a);
+    W.status = 0;
+    W.nRows = 0;
+    W.tick = arenaTickCount(D, a);
+    W.ballVelCache = v3zero();
+    W.np = W.nm = 0;
+    uint32_t actBits[MAX_BODIES], cached = 0, dynDone = 0;
+    for (int i = 0; i < W.nb; i++) {
+        Body& b = W.b[i];
+        bodyConstants(D, i, b);
+        const uint32_t p = infoWord(D, T, a, i, BI_PAIRS);
+        actBits[i] = p;
+        b.act = (int32_t)((p & BI_ACT_MASK) >> BI_ACT_SHIFT);
+        b.noResp = i > 0 && !(p & BI_RESPONDS) ? 1 : 0;
+        b.xf = bodyXf(D, a, i);
+        b.lin = bodyV3(D, a, i, RSB_PW(CarP, lin));
+        b.ang = bodyV3(D, a, i, RSB_PW(CarP, ang));
+        b.force = tempV3(D, T.force, a, i, 0);
+        b.torque = tempV3(D, T.force, a, i, 3);
+        updateInertia(b);
+        W.noRot[i] = i == 0 ? 1 : 0;
+    }
+    int blocks = 0;
+    auto addPairTo = [&](int lo, int hi) -> bool {
+        if (W.np >= MAX_PAIRS) {
+            W.status |= WS_OVERFLOW;
+            return false;
+        }
+        W.po0[W.np] = (int16_t)lo;
+        W.po1[W.np] = (int16_t)hi;
+        W.np++;
+        return true;
+    };
+    auto active = [&](int i) { return W.b[i].act != ACT_SLEEPING && W.b[i].act != ACT_DISABLE_SIM; };
+    // a manifold in dispatch order, with the points of its result (null: none)
+    auto addManifold = [&](int o0, int o1, float cbt, const PairResult* r) -> Manifold* {
+        if (W.nm >= MAX_MANIFOLDS) {
+            W.status |= WS_OVERFLOW;
+            return nullptr;
+        }
+        Manifold& m = W.m[W.nm++];
+        pairManifold(m, o0, o1, cbt);
+        if (r && (r->flags & PR_BLOCK)) {
+            if (blocks >= MAX_BLOCKS) {
+                W.status |= WS_OVERFLOW;
+                return nullptr;
+            }
+            blocks++;
+            m.n = r->n;
+            m.pt = T.blocks + (size_t)MAX_POINTS * r->block;
+            return &m;
+        }
+        return nullptr;
+    };
+    for (int i = 0; i < W.nb; i++) {
+        const uint32_t pairs = actBits[i] & ((1u << NUM_STATICS) - 1u), dyn = infoWord(D, T, a, i, BI_DYN);
+        const uint32_t mani = pairs ? infoWord(D, T, a, i, BI_MANI) : 0u;
+        const uint32_t tasks = pairs ? infoWord(D, T, a, i, BI_TASKS) : 0u;
+        for (uint32_t k = pairs; k; k &= k - 1u) {
+            const int s = lowestBit(k);
+            if (!addPairTo(s, OBJ_BALL + i)) continue;
+            if (!((mani >> s) & 1u)) continue;
+            const PairResult* r = nullptr;
+            if (s < MAX_MESHES) {
+                if ((tasks >> s) & 1u)
+                    r = T.results + infoWord(D, T, a, i, BI_MESHRES) + bitCount(tasks & ((1u << s) - 1u));
+            } else if ((tasks >> s) & 1u) {
+                r = T.results + infoWord(D, T, a, i, BI_PLANERES + s - MAX_MESHES);
+            }
+            if (addManifold(OBJ_BALL + i, s, i == 0 ? D.P.ballCbt : D.P.car.cbt, r) && (r->flags & PR_WORLD)) {
+                // onCarWorld's state; its material is in the points already
+                putCarV3(D, a, i - 1, RSB_PW(CarP, worldContactNormal), V3{r->normal[0], r->normal[1], r->normal[2]});
+                putCarWord(D, a, i - 1, RSB_PW(CarP, flags), carWord(D, a, i - 1, RSB_PW(CarP, flags)) | CF_WORLD_CONTACT);
+            }
+        }
+        for (uint32_t q = 0; q < (dyn >> 24); q++) {
+            const int j = (int)((dyn >> (3 * q)) & 7u), lo = imin_(i, j), hi = imax_(i, j);
+            const uint32_t bit = 1u << dynPair(lo, hi);
+            if (dynDone & bit) continue;
+            if (!addPairTo(OBJ_BALL + lo, OBJ_BALL + hi)) continue;
+            dynDone |= bit;
+            if (!active(lo) && !active(hi)) continue;
+            if (!((infoWord(D, T, a, lo, BI_DYNMANI) >> hi) & 1u)) continue;
+            const PairResult* r = T.results + T.dynRes[(size_t)dynPair(lo, hi) * D.N + a];
+            if (lo == 0) {
+                Manifold* m = addManifold(OBJ_BALL + hi, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt), r);
+                if (!m) continue;
+                if (!W.b[hi].noResp) {
+                    W.c.i0 = hi - 1;
+                    CarSim& c = W.c.v[0];
+                    loadContactCar(D, a, hi - 1, c, v3zero());
+                    c.ballHitExtraVel = v3zero();
+                    onCarBall(W, hi - 1, m->pt[0], false);
+                    putCarWord(D, a, hi - 1, RSB_PW(CarP, flags), c.flags);
+                    putCarV3(D, a, hi - 1, RSB_PW(CarP, ballHitRelPos), c.ballHitRelPos);
+                    putCarWord(D, a, hi - 1, RSB_PW(CarP, ballHitTick), (uint32_t)c.ballHitTick);
+                    putCarWord(D, a, hi - 1, RSB_PW(CarP, ballHitTick) + 1, (uint32_t)(c.ballHitTick >> 32));
+                    putCarV3(D, a, hi - 1, RSB_PW(CarP, ballHitBallPos), c.ballHitBallPos);
+                    putCarV3(D, a, hi - 1, RSB_PW(CarP, ballHitExtraVel), c.ballHitExtraVel);
+                    putCarWord(D, a, hi - 1, RSB_PW(CarP, ballHitExtraTick), (uint32_t)c.ballHitExtraTick);
+                    putCarWord(D, a, hi - 1, RSB_PW(CarP, ballHitExtraTick) + 1, (uint32_t)(c.ballHitExtraTick >> 32));
+                    cached |= 1u;
+                }
+                if (m->n) refreshContactPoints(*m, W.b[hi].xf, W.b[0].xf);
+            } else {
+                Manifold* m = addManifold(OBJ_BALL + hi, OBJ_BALL + lo, D.P.car.cbt, r);
+                if (!m) continue;
+                const int ca = lo - 1, cb = hi - 1;
+                if (!W.b[lo].noResp && !W.b[hi].noResp) {
+                    W.c.i0 = ca;
+                    loadContactCar(D, a, ca, W.c.v[0], (cached >> lo) & 1u ? tempV3(D, T.cache, a, lo, 0) : v3zero());
+                    loadContactCar(D, a, cb, W.c.v[1], (cached >> hi) & 1u ? tempV3(D, T.cache, a, hi, 0) : v3zero());
+                    for (int k = 0; k < m->n; k++) onCarCar(W, cb, ca, m->pt[k]);
+                    for (int e = 0; e < 2; e++) {
+                        const int s = e ? cb : ca;
+                        const CarSim& c = W.c.v[e];
+                        putCarWord(D, a, s, RSB_PW(CarP, flags), c.flags);
+                        putCarFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer), c.demoRespawnTimer);
+                        putCarWord(D, a, s, RSB_PW(CarP, carContactOtherId), c.carContactOtherId);
+                        putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), c.carContactCooldown);
+                        putTempV3(D, T.cache, a, 1 + s, 0, c.velCache);
+                        cached |= 2u << s;
+                    }
+                }
+                if (m->n) refreshContactPoints(*m, W.b[hi].xf, W.b[lo].xf);
+            }
+        }
+    }
+    solveIslands(W);
+    for (int i = 0; i < W.nb; i++) {
+        const Body& b = W.b[i];
+        putBodyXf(D, a, i, b.xf);
+        putBodyV3(D, a, i, RSB_PW(CarP, lin), b.lin);
+        putBodyV3(D, a, i, RSB_PW(CarP, ang), b.ang);
+        infoWord(D, T, a, i, BI_PAIRS) = (actBits[i] & ~BI_ACT_MASK) | ((uint32_t)b.act << BI_ACT_SHIFT) | BI_SOLVED |
+                                         ((cached >> i) & 1u ? BI_CACHE : 0u);
+    }
+    if (cached & 1u) putTempV3(D, T.cache, a, 0, 0, W.ballVelCache);
+    st.nRows += W.nRows;
+    if (W.status) phaseAtomicOr(arenaStatus(D, a), W.status);
+}
+
+// ------------------------------------------------------------------ finish
+
+struct FinishShared {
+    int32_t locked[NUM_PADS][PHASE_ARENAS];        // car that locked the pad this tick, MAX_CARS none
+    uint32_t prevLocked[NUM_PADS][PHASE_ARENAS];   // car id of the last tick
+    uint32_t picked[MAX_CARS][PHASE_ARENAS];       // pads taken: small | big << 16
+    uint32_t touched[PHASE_ARENAS];
+};
+
+RSB_HD void padLoad(const EngineView& D, int a, int la, int p, FinishShared& sh) {
+    sh.locked[p][la] = MAX_CARS;
+    sh.prevLocked[p][la] = D.pad[((size_t)RSB_PW(PadP, bits) * NUM_PADS + p) * D.N + a] >> 8;
+}
+
+struct FinishThread {
+    int a, la, b, nb;
+    Body body;
+    CarSim c;
+    uint64_t tick;
+    bool pads;  // the car may collide with pads
+};
+
+// Integration and post-tick of one body (integrateBodies, updateActivation, carPostTick,
+// ballFinishTick), then the pads around a car.
+RSB_HD void finishBody(const EngineView& D, const StepTemp& T, FinishThread& t, FinishShared& sh) {
+    Body& b = t.body;
+    CarSim& c = t.c;
+    const int a = t.a, s = t.b - 1;
+    const float dt = D.P.dt;
+    const uint32_t info = infoWord(D, T, a, t.b, BI_PAIRS);
+    t.tick = arenaTickCount(D, a);
+    t.pads = false;
+    bodyConstants(D, t.b, b);
+    b.act = (int32_t)((info & BI_ACT_MASK) >> BI_ACT_SHIFT);
+    b.xf = bodyXf(D, a, t.b);
+    b.lin = bodyV3(D, a, t.b, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, t.b, RSB_PW(CarP, ang));
+    const bool moves = b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM;
+    if (!(info & BI_SOLVED) && moves) {
+        // an island of one body without contacts: the solver adds the external impulses only
+        updateInertia(b);
+        b.force = tempV3(D, T.force, a, t.b, 0);
+        b.torque = tempV3(D, T.force, a, t.b, 3);
+        const V3 extF = (b.force * b.invMass) * dt, extT = tmul(b.torque, b.invIw) * dt;
+        b.lin = (b.lin + v3zero()) + extF;
+        b.ang = (b.ang + v3zero()) + extT;
+    }
+    if (moves) b.xf = t.b == 0 ? integrateTransformNoRot(b.xf, b.lin, dt) : integrateTransform(b.xf, b.lin, b.ang, dt);
+    if (b.act == ACT_SLEEPING) b.lin = b.ang = v3zero();
+    if (moves) {
+        putBodyV3(D, a, t.b, RSB_PW(CarP, pos), b.xf.o);
+        if (t.b != 0)
+            for (int r = 0; r < 3; r++) putBodyV3(D, a, t.b, RSB_PW(CarP, rot) + 3 * r, b.xf.b.r[r]);
+    }
+    if (t.b == 0) {
+        struct {
+            const WorldParams* P;
+            OneBody b;
+        } W{&D.P, {b}};
+        ballFinishTick(W, (info & BI_CACHE) ? tempV3(D, T.cache, a, 0, 0) : v3zero());
+        putBodyV3(D, a, 0, RSB_PW(BallP, lin), W.b.v.lin);
+        putBodyV3(D, a, 0, RSB_PW(BallP, ang), W.b.v.ang);
+        return;
+    }
+    c.flags = carWord(D, a, s, RSB_PW(CarP, flags));
+    c.boost = carFloat(D, a, s, RSB_PW(CarP, boost));
+    if (!(c.flags & CF_DEMOED)) {
+        c.supersonicTime = carFloat(D, a, s, RSB_PW(CarP, supersonicTime));
+        c.carContactCooldown = carFloat(D, a, s, RSB_PW(CarP, carContactCooldown));
+        const CtlRec& ctl = D.controls[D.carOffset[a] + s];
+        for (int k = 0; k < 5; k++) c.ctl[k] = clampf(ctl.v[k], -1, 1);
+        c.ctlBits = (ctl.jump ? 1u : 0u) | (ctl.boost ? 2u : 0u) | (ctl.handbrake ? 4u : 0u);
+        c.velCache = (info & BI_CACHE) ? tempV3(D, T.cache, a, t.b, 0) : v3zero();
+        struct {
+            const WorldParams* P;
+            OneBody b;
+            OneCar c;
+        } W{&D.P, {b}, {c}};
+        carPostTick(W, s);
+        b = W.b.v;
+        c = W.c.v;
+        putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
+        putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+        for (int r = 0; r < 3; r++) putCarV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r, c.rotMat.r[r]);
+        putCarWord(D, a, s, RSB_PW(CarP, flags), c.flags);
+        putCarFloat(D, a, s, RSB_PW(CarP, supersonicTime), c.supersonicTime);
+        putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), c.carContactCooldown);
+        for (int k = 0; k < 5; k++) putCarFloat(D, a, s, RSB_PW(CarP, lastCtl) + k, c.lastCtl[k]);
+        putCarWord(D, a, s, RSB_PW(CarP, lastCtlBits), c.lastCtlBits);
+        t.pads = c.boost < 100;
+    } else if (moves) {
+        // demoed in this tick: integrated, then left alone
+        putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
+        putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+    }
+    const uint64_t hit = (uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitTick)) |
+                         ((uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitTick) + 1) << 32);
+    if (hit == t.tick) phaseAtomicOr(&sh.touched[t.la], 1u << s);
+}
+
+// BoostPadGrid::CheckCollision of one car: the pads it locks (the lowest slot wins a pad, as
+// the last writer of the reference's loop over the cars in reverse creation order).
+RSB_HD void finishPads(const EngineView& D, FinishThread& t, FinishShared& sh) {
+    if (!t.pads) return;
+    const V3 carPos = t.body.xf.o * kBtToUu;
+    if (carPos.z > PAD_CYL_HEIGHT + 250.f) return;
+    const int ix = (int)(carPos.x / 1024.f + 4.f), iy = (int)(carPos.y / 1024.f + 5.f);
+    for (int i = imax_(ix - 1, 0); i <= imin_(ix + 1, 7); i++)
+        for (int j = imax_(iy - 1, 0); j <= imin_(iy + 1, 9); j++) {
+            const int p = D.P.padGrid[i * 10 + j];
+            if (p < 0) continue;
+            if (padCollides(D.P, p, t.body.xf, sh.prevLocked[p][t.la] == (uint32_t)t.b)) {
+#if defined(__CUDA_ARCH__)
+                atomicMin(&sh.locked[p][t.la], t.b - 1);
+#else
+                sh.locked[p][t.la] = imin_(sh.locked[p][t.la], t.b - 1);
+#endif
+            }
+        }
+}
+
+// One pad's cooldown and pickup.
+RSB_HD void finishPad(const EngineView& D, int a, int la, int p, FinishShared& sh) {
+    uint32_t* cool = D.pad + ((size_t)RSB_PW(PadP, cooldown) * NUM_PADS + p) * D.N + a;
+    uint32_t* bits = D.pad + ((size_t)RSB_PW(PadP, bits) * NUM_PADS + p) * D.N + a;
+    const uint32_t cool0 = *cool;
+    float cd = u2f(cool0);
+    if (cd > 0) cd = fmax_(cd - D.P.dt, 0);
+    uint32_t isActive = cd == 0 ? 1u : 0u, locked = 0;
+    const int car = sh.locked[p][la];
+    if (car < MAX_CARS) {
+        locked = (uint32_t)car + 1u;
+        if (isActive) {
+            phaseAtomicAdd(&sh.picked[car][la], p < NUM_BIG_PADS ? 0x10000u : 1u);
+            isActive = 0;
+            cd = p < NUM_BIG_PADS ? D.P.car.padCooldownBig : D.P.car.padCooldownSmall;
+        }
+    }
+    if (f2u(cd) != cool0) *cool = f2u(cd);
+    *bits = isActive | (locked << 8);
+}
+
+// The boost of the pads a car took.  The amounts are added one by one and clamped, so their
+// order does not matter: equal amounts commute, and a big pad fills the tank.
+RSB_HD void finishBoost(const EngineView& D, const FinishThread& t, const FinishShared& sh) {
+    const int s = t.b - 1;
+    const uint32_t n = sh.picked[s][t.la];
+    if (!n) return;
+    float boost = t.c.boost;
+    for (uint32_t k = 0; k < (n & 0xffffu); k++) boost = fmin_(boost + PAD_BOOST_AMOUNT_SMALL, BOOST_MAX);
+    for (uint32_t k = 0; k < (n >> 16); k++) boost = fmin_(boost + PAD_BOOST_AMOUNT_BIG, BOOST_MAX);
+    putCarFloat(D, t.a, s, RSB_PW(CarP, boost), boost);
+}
+
+// Arena counters, by the ball's thread.
+RSB_HD void finishArena(const EngineView& D, const FinishThread& t, const FinishShared& sh) {
+    const int a = t.a;
+    struct {
+        OneBody b;
+    } W{{t.body}};
+    const bool scored = ballScored(W, D.P.goalBaseY, D.P.ballRadiusUu);
+    const int side = W.b.v.xf.o.y > 0 ? 0 : 1;
+    auto put = [&](int w, uint32_t v) { D.arena[(size_t)w * D.N + a] = v; };
+    if (scored && (int32_t)arenaWord(D, a, RSB_PW(ArenaP, goalTeam)) < 0) put(RSB_PW(ArenaP, goalTeam), (uint32_t)side);
+    put(RSB_PW(ArenaP, scored), scored ? (side == 0 ? 1u : 2u) : 0u);
+    const uint64_t tk = t.tick + 1;
+    put(RSB_PW(ArenaP, tick), (uint32_t)tk);
+    put(RSB_PW(ArenaP, tick) + 1, (uint32_t)(tk >> 32));
+    put(RSB_PW(ArenaP, episodeTicks), arenaWord(D, a, RSB_PW(ArenaP, episodeTicks)) + 1u);
+    const uint32_t touched = sh.touched[t.la];
+    if (touched) put(RSB_PW(ArenaP, touchedMask), arenaWord(D, a, RSB_PW(ArenaP, touchedMask)) | touched);
+}
+
+#undef RSB_PW
+
+}  // namespace rsb

@@ -108,7 +108,8 @@ constexpr float kOccTol = 2.f * kUuToBt;
 
 // Bookkeeping of one static test of body b: returns true when the test must be skipped.
 // (nCulled counts the tests the bound clears, also in audit mode where they still run.)
-RSB_HD bool cullSkip(const World& W, int b) {
+template <class WT>
+RSB_HD bool cullSkip(const WT& W, int b) {
     if ((W.cull >> b) & 1u) {
         W.nCulled++;
         if (!W.cullAudit) return true;
@@ -116,7 +117,8 @@ RSB_HD bool cullSkip(const World& W, int b) {
     W.nStatic++;
     return false;
 }
-RSB_HD void cullCheck(const World& W, int b, bool found) {
+template <class WT>
+RSB_HD void cullCheck(const WT& W, int b, bool found) {
     if (found && ((W.cull >> b) & 1u)) {
         W.nMissed++;
         W.cullMissed = WS_CULL_MISS;
@@ -128,7 +130,8 @@ RSB_HD void cullCheck(const World& W, int b, bool found) {
 RSB_HD bool objIsStatic(int o) { return o < OBJ_BALL; }
 RSB_HD bool objIsPlane(int o) { return o >= MAX_MESHES && o < NUM_STATICS; }
 
-RSB_HD ObjRef objRef(const World& W, int o) {
+template <class WT>
+RSB_HD ObjRef objRef(const WT& W, int o) {
     ObjRef r;
     if (o < MAX_MESHES) {
         r.xf = xfIdentity();
@@ -150,7 +153,8 @@ RSB_HD ObjRef objRef(const World& W, int o) {
     return r;
 }
 
-RSB_HD bool objActive(const World& W, int o) {
+template <class WT>
+RSB_HD bool objActive(const WT& W, int o) {
     if (objIsStatic(o)) return false;  // static objects are ISLAND_SLEEPING
     int a = W.b[o - OBJ_BALL].act;
     return a != ACT_SLEEPING && a != ACT_DISABLE_SIM;
@@ -174,7 +178,8 @@ RSB_HD void carBoxAabb(const CarParams& C, const Xf& childXf, V3& mn, V3& mx) {
 }
 RSB_HD ConvexShape carBoxShape(const CarParams& C) { return makeBox(C.boxHe, C.boxMargin); }
 
-RSB_HD void bodyShapeAabb(const World& W, int bi, const Xf& xf, V3& mn, V3& mx) {
+template <class WT>
+RSB_HD void bodyShapeAabb(const WT& W, int bi, const Xf& xf, V3& mn, V3& mx) {
     if (bi == 0) ballAabb(*W.P, xf, mn, mx);
     else carCompoundAabb(W.P->car, xf, mn, mx);
 }
@@ -191,7 +196,8 @@ RSB_HD void bpCellIndices(const BpGrid& g, V3 pos, int& i, int& j, int& k) {
 }
 
 // btCollisionWorld::updateSingleAabb + btRSBroadphase::setAabb (dynamic proxies)
-RSB_HD void updateBodyAabb(World& W, int bi) {
+template <class WT>
+RSB_HD void updateBodyAabb(WT& W, int bi) {
     Body& b = W.b[bi];
     V3 mn, mx, mn2, mx2;
     bodyShapeAabb(W, bi, b.xf, mn, mx);
@@ -419,7 +425,8 @@ RSB_HD bool sphereTriCollide(const V3* v, V3 center, float radius, float cbt, V3
 
 // Ball vs one arena mesh: btConvexConcaveCollisionAlgorithm (swapped: the pair is
 // (mesh, ball)) -> per triangle early-out + btSphereTriangleCollisionAlgorithm.
-RSB_HD void collideBallMesh(World& W, int mesh, Manifold& man) {
+template <class WT>
+RSB_HD void collideBallMesh(WT& W, int mesh, Manifold& man) {
     const WorldParams& P = *W.P;
     const Body& ball = W.b[0];
     ObjRef rMesh = objRef(W, mesh), rBall = objRef(W, OBJ_BALL);
@@ -464,7 +471,8 @@ RSB_HD void collideBallMesh(World& W, int mesh, Manifold& man) {
 }
 
 // Ball vs static plane: btConvexPlaneCollisionAlgorithm (swapped pair (plane, ball))
-RSB_HD void collideBallPlane(World& W, int plane, Manifold& man) {
+template <class WT>
+RSB_HD void collideBallPlane(WT& W, int plane, Manifold& man) {
     const WorldParams& P = *W.P;
     ObjRef rPlane = objRef(W, plane), rBall = objRef(W, OBJ_BALL);
     V3 pn = W.S->planeNormal[plane - MAX_MESHES];
@@ -489,10 +497,12 @@ RSB_HD void collideBallPlane(World& W, int plane, Manifold& man) {
 
 // ------------------------------------------------------------------ contact callbacks
 
-RSB_HD bool carResponds(const World& W, int ci) { return !W.b[1 + ci].noResp; }
+template <class WT>
+RSB_HD bool carResponds(const WT& W, int ci) { return !W.b[1 + ci].noResp; }
 
 // Arena::_BtCallback_OnCarWorldCollision (Arena.cpp:420-427)
-RSB_HD void onCarWorld(World& W, int ci, MPoint& cp) {
+template <class WT>
+RSB_HD void onCarWorld(WT& W, int ci, MPoint& cp) {
     CarSim& c = W.c[ci];
     c.flags |= CF_WORLD_CONTACT;
     c.worldContactNormal = cp.normal;
@@ -501,7 +511,8 @@ RSB_HD void onCarWorld(World& W, int ci, MPoint& cp) {
 }
 
 // Arena::_BtCallback_OnCarBallCollision (Arena.cpp:278-332)
-RSB_HD void onCarBall(World& W, int ci, MPoint& cp, bool ballIsBodyA) {
+template <class WT>
+RSB_HD void onCarBall(WT& W, int ci, MPoint& cp, bool ballIsBodyA) {
     const CarParams& C = W.P->car;
     CarSim& c = W.c[ci];
     const Body& cb = W.b[1 + ci];
@@ -532,7 +543,8 @@ RSB_HD void onCarBall(World& W, int ci, MPoint& cp, bool ballIsBodyA) {
 }
 
 // Arena::_BtCallback_OnCarCarCollision (Arena.cpp:334-418); car1 is the manifold's body 0
-RSB_HD void onCarCar(World& W, int car1, int car2, MPoint& cp) {
+template <class WT>
+RSB_HD void onCarCar(WT& W, int car1, int car2, MPoint& cp) {
     const CarParams& C = W.P->car;
     cp.fric = CARCAR_COLLISION_FRICTION;
     cp.rest = CARCAR_COLLISION_RESTITUTION;
@@ -631,7 +643,8 @@ RSB_HD bool boxTriFar(const Xf& x, V3 he, const V3* v, float limit) {
 // Car box vs one arena mesh: the compound's child algorithm is btConvexConcaveCollisionAlgorithm
 // (btConvexConcaveCollisionAlgorithm.cpp:60-250), each overlapping triangle through
 // btConvexConvexAlgorithm's GJK (btConvexConvexAlgorithm.cpp:268-590).
-RSB_HD void collideBoxMesh(World& W, int mesh, int ci, const Xf& childXf, Manifold& man) {
+template <class WT>
+RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold& man) {
     const CarParams& C = W.P->car;
     int carObj = OBJ_CAR0 + ci;
     ObjRef rMesh = objRef(W, mesh), rCar = objRef(W, carObj);
@@ -679,7 +692,8 @@ RSB_HD void collideBoxMesh(World& W, int mesh, int ci, const Xf& childXf, Manifo
 }
 
 // Car box vs a static plane: btConvexPlaneCollisionAlgorithm owning its manifold
-RSB_HD void collideBoxPlane(World& W, int plane, int ci, const Xf& childXf, Manifold& man) {
+template <class WT>
+RSB_HD void collideBoxPlane(WT& W, int plane, int ci, const Xf& childXf, Manifold& man) {
     const CarParams& C = W.P->car;
     int carObj = OBJ_CAR0 + ci;
     ObjRef rPlane = objRef(W, plane), rCar = objRef(W, carObj);
@@ -724,6 +738,21 @@ RSB_HD void collideCarStatic(World& W, int s, int ci) {
     }
 }
 
+// GJK contact of car ci's box (at childXf) with the ball, added to `man`; the point's slot or -1.
+template <class WT>
+RSB_HD int carBallContact(WT& W, int ci, const Xf& childXf, Manifold& man) {
+    const WorldParams& P = *W.P;
+    const CarParams& C = P.car;
+    int carObj = OBJ_CAR0 + ci;
+    ObjRef rBall = objRef(W, OBJ_BALL), rCar = objRef(W, carObj);
+    ConvexShape box = carBoxShape(C), sph = makeSphere(P.ballRadius);
+    float maxDist2 = sq((C.boxMargin + P.ballMargin) + man.cbt);
+    GjkOut g = gjkPairDetector(W.epa, box, childXf, sph, rBall.xf, maxDist2);
+    if (g.overflow) W.status |= WS_EPA_OVERFLOW;
+    if (!g.has) return -1;
+    return addContact(man, W.pool, OBJ_BALL, rBall, carObj, rCar, g.normal, g.point, g.dist);
+}
+
 // (ball, car) pair: swapped compound over a btConvexConvexAlgorithm that creates its
 // manifold on first use
 RSB_HD void collideCarBall(World& W, int ci) {
@@ -738,16 +767,17 @@ RSB_HD void collideCarBall(World& W, int ci) {
     int mi = newManifold(W, carObj, OBJ_BALL, fmin_(C.cbt, P.ballCbt));
     if (mi < 0) return;
     Manifold& man = W.m[mi];
-    ObjRef rBall = objRef(W, OBJ_BALL), rCar = objRef(W, carObj);
-    ConvexShape box = carBoxShape(C), sph = makeSphere(P.ballRadius);
-    float maxDist2 = sq((C.boxMargin + P.ballMargin) + man.cbt);
-    GjkOut g = gjkPairDetector(W.epa, box, childXf, sph, W.b[0].xf, maxDist2);
-    if (g.overflow) W.status |= WS_EPA_OVERFLOW;
-    if (g.has) {
-        int idx = addContact(man, W.pool, OBJ_BALL, rBall, carObj, rCar, g.normal, g.point, g.dist);
-        if (idx >= 0 && carResponds(W, ci)) onCarBall(W, ci, man.pt[idx], false);
-    }
-    if (man.n) refreshContactPoints(man, rCar.xf, rBall.xf);
+    const int idx = carBallContact(W, ci, childXf, man);
+    if (idx >= 0 && carResponds(W, ci)) onCarBall(W, ci, man.pt[idx], false);
+    if (man.n) refreshContactPoints(man, W.b[1 + ci].xf, W.b[0].xf);
+}
+
+// Box-box contacts of cars ca < cb, with car cb as the first box.
+template <class WT>
+RSB_HD void carCarContacts(const WT& W, int ca, int cb, BoxContacts& bc) {
+    const CarParams& C = W.P->car;
+    Xf xa = carChildXf(C, W.b[1 + ca].xf), xb = carChildXf(C, W.b[1 + cb].xf);
+    boxBoxContacts(xb, C.boxHeM, xa, C.boxHeM, bc);
 }
 
 // (car a, car b), a < b: btCompoundCompoundCollisionAlgorithm without child trees falls back to
@@ -772,7 +802,7 @@ RSB_HD void collideCarCar(World& W, int ca, int cb) {
             Manifold& man = W.m[mi];
             ObjRef rA = objRef(W, objA), rB = objRef(W, objB);
             BoxContacts bc;
-            boxBoxContacts(xb, C.boxHeM, xa, C.boxHeM, bc);
+            carCarContacts(W, ca, cb, bc);
             bool responds = carResponds(W, ca) && carResponds(W, cb);
             for (int k = 0; k < bc.n; k++) {
                 int idx = addContact(man, W.pool, objA, rA, objB, rB, bc.c[k].normalOnB, bc.c[k].point, bc.c[k].depth);
@@ -820,7 +850,8 @@ RSB_HD void buildRayOrder(World& W) { buildRegOrder(W); }
 // (btRSBroadphase::rayTest, btRSBroadphase.cpp:325-356): statics in registration order,
 // then dynamic bodies in registration order; objects are tested without AABB culling.
 // Returns the object hit, or -1 (also when the closest object has no contact response).
-RSB_HD int castRay(const World& W, V3 from, V3 to, int ignoreObj, V3& hitPoint, V3& hitNormal, float& hitFrac) {
+template <class WT>
+RSB_HD int castRay(const WT& W, V3 from, V3 to, int ignoreObj, V3& hitPoint, V3& hitNormal, float& hitFrac) {
     const ArenaStatic& S = *W.S;
     const WorldParams& P = *W.P;
     RayHit hit;
@@ -857,7 +888,7 @@ RSB_HD int castRay(const World& W, V3 from, V3 to, int ignoreObj, V3& hitPoint, 
             else rayVsPlane(S, o, from, to, hit);
         } else {
             int bi = o - OBJ_BALL;
-            const Body& b = W.b[bi];
+            const auto& b = W.b[bi];
             ConvexShape sh;
             Xf x;
             if (bi == 0) {
@@ -986,7 +1017,8 @@ RSB_HD void quickSortKV(int* key, int* val, int lo, int hi, uint32_t& status) {
 }
 
 // btSimulationIslandManager + InplaceSolverIslandCallback + btSequentialImpulseConstraintSolver
-RSB_HD void solveIslands(World& W) {
+template <class WT>
+RSB_HD void solveIslands(WT& W) {
     const float dt = W.P->dt;
     UnionFind uf;
     uf.reset(W.nb);

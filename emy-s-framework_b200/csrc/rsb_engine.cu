@@ -1,9 +1,8 @@
 // CUDA engine behind the C ABI of include/rsb.h.
 //
-// One kernel thread advances one arena through all requested ticks with the arena's
-// state held in registers / thread-local memory; state is read from and written back to
-// the word-plane layout of phys/state.h at the launch boundaries.  Static arena data
-// (meshes, BVHs, grids) is built once on the host and shared by every handle on a device.
+// A step is a sequence of kernels per tick (step_kernels.cuh) over the word-plane records of
+// phys/state.h.  Static arena data (meshes, BVHs, grids) is built once on the host and shared
+// by every handle on a device.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,6 +20,7 @@
 #include "arena_build.h"
 #include "engine_host.h"
 #include "env_kernels.cuh"
+#include "step_kernels.cuh"
 #include "culler.cuh"
 #include "vanta.cuh"
 
@@ -130,11 +130,12 @@ struct rsb_handle {
     float* dTris = nullptr;                // mesh triangles in uu (9 floats each)
     int numTris = 0;
     std::shared_ptr<ArenaStaticHost> host;
-    // launch configuration of the step kernel (indices into kStepVariants / kStepBlocks)
+    // launch configuration of the step's queue kernels (indices into kStepVariants / kStepBlocks)
     int stepVariant = 0, stepBlock = 1, stepResidency = 0;
     uint32_t* dScratch = nullptr;   // the autotuner's copy of the arena records
-    unsigned int* dWork = nullptr;  // claim counter of the persistent step kernel
-    int persistGrid[8][4] = {};     // resident blocks (all SMs) per persistent variant and block size
+    unsigned int* dWork = nullptr;  // queue counters of the step phases (zero between ticks)
+    StepTemp step{};                // what the phases of a tick hand on (one allocation, dStep)
+    char* dStep = nullptr;
     int smCount = 0;
     uint32_t* dStage = nullptr;     // staging of the per-arena getters
     rsb_ball_state* dPred = nullptr;  // ball prediction slices [num_arenas][n_slices]
@@ -183,56 +184,28 @@ static rsb_status cudaFail(rsb_handle* h, const char* what, cudaError_t e) {
 
 // ------------------------------------------------------------------ kernels
 
-// One thread advances one arena.  MINB is the minimum number of 128-thread blocks per SM
-// the compiler must fit, which caps the registers per thread; the autotuner picks the
-// variant and the block size.
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) stepKernel(EngineView D, int ticks) {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= D.N) return;
-    ArenaSim A;
-    EpaWork epa;
-    A.W.epa = &epa;
-    stepArena(D, a, ticks, A);
-}
-
-// Persistent form: the grid holds only as many blocks as fit on the GPU at once, and each warp
-// claims the next 32 arenas from a counter until none are left.  One arena per thread still,
-// and the same per-arena computation; the claims pack the work that one-arena-per-thread
-// blocks leave in a partial last wave (65,536 arenas are about 1.7 waves of resident warps).
-// No waiting: a claim is one atomic add.
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) stepKernelPersistent(EngineView D, int ticks) {
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = (int)atomicAdd(D.work, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= D.N) return;
-        const int a = base + lane;
-        if (a < D.N) {
-            ArenaSim A;
-            EpaWork epa;
-            A.W.epa = &epa;
-            stepArena(D, a, ticks, A);
-        }
-    }
-}
-
+// The queue kernels of a step (heavy rays, contacts, islands) for one register budget: MINB is
+// the minimum number of 128-thread blocks per SM the compiler must fit.  Their grids loop over
+// the queues: either wide enough for every item to get a thread of its own, or (persistent)
+// only as many blocks as are resident at once.  The autotuner picks the variant and the block
+// size.
+typedef void (*StepFn)(EngineView, StepTemp);
 struct StepVariant {
-    void (*fn)(EngineView, int);
+    StepFn ray, contact, solve;
     int minBlocks;
     bool persistent;
 };
-static const StepVariant kStepVariants[] = {{stepKernel<1>, 1, false},          {stepKernel<3>, 3, false},
-                                            {stepKernel<4>, 4, false},          {stepKernelPersistent<1>, 1, true},
-                                            {stepKernelPersistent<3>, 3, true}, {stepKernelPersistent<4>, 4, true}};
+static const StepVariant kStepVariants[] = {
+    {heavyRayKernel<1>, contactKernel<1>, solveKernel<1>, 1, false},
+    {heavyRayKernel<3>, contactKernel<3>, solveKernel<3>, 3, false},
+    {heavyRayKernel<4>, contactKernel<4>, solveKernel<4>, 4, false},
+    {heavyRayKernel<1>, contactKernel<1>, solveKernel<1>, 1, true},
+    {heavyRayKernel<3>, contactKernel<3>, solveKernel<3>, 3, true},
+    {heavyRayKernel<4>, contactKernel<4>, solveKernel<4>, 4, true}};
 constexpr int kNumStepVariants = sizeof(kStepVariants) / sizeof(kStepVariants[0]);
 static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
-// Resident warps per SM of a persistent launch (0 = as many as fit).  The working sets of the
-// arenas in flight share the L2: with every warp slot filled (about 38,000 arenas at a time)
-// they do not fit, and each thread waits on DRAM; fewer arenas in flight stay in L2.
+// Resident warps per SM of a persistent launch (0 = as many as fit).
 static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
 
@@ -477,6 +450,38 @@ static EnvView envView(rsb_handle* h) {
     return E;
 }
 
+// The buffers that the phases of a tick hand on, one allocation per handle.
+static bool allocStep(rsb_handle* h) {
+    StepTemp& T = h->step;
+    const size_t N = h->N, B = MAX_BODIES * N, R = (size_t)4 * MAX_CARS * N;
+    size_t off = 0;
+    auto place = [&](auto*& p, size_t count) {
+        off = (off + 255) / 256 * 256;
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(h->dStep + off);
+        off += count * sizeof(*p);
+    };
+    T.blockCap = (uint32_t)(MAX_BLOCKS * N);
+    for (int pass = 0; pass < 2; pass++) {
+        off = 0;
+        place(T.rayObj, R);
+        place(T.rayFrac, R);
+        place(T.rayN, 3 * R);
+        place(T.info, (size_t)BI_WORDS * B);
+        place(T.force, 6 * B);
+        place(T.box, 6 * B);
+        place(T.cache, 3 * B);
+        place(T.dynRes, (size_t)NUM_DYN_PAIRS * N);
+        place(T.rayQ, R);
+        place(T.tasks, (size_t)CAP_RESULTS * N);
+        place(T.results, (size_t)CAP_RESULTS * N);
+        place(T.blocks, (size_t)T.blockCap * MAX_POINTS);
+        place(T.solveQ, N);
+        if (pass == 0 && cudaMalloc((void**)&h->dStep, off) != cudaSuccess) return false;
+    }
+    T.count = h->dWork;
+    return true;
+}
+
 static cudaStream_t pick(rsb_handle* h, void* s) { return s ? (cudaStream_t)s : h->stream; }
 
 // ------------------------------------------------------------------ C ABI
@@ -621,21 +626,24 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
 
     if (cudaSetDevice(h->device) != cudaSuccess) return fail(nullptr, RSB_ERR_CUDA, "cudaSetDevice failed");
     {
-        // the arena kernel keeps one arena's working set in thread-local memory; make the
-        // per-thread stack limit cover the largest variant's frame (the default limit is
-        // 1 KB), and give the L1 its largest share (the kernels use no shared memory)
+        // kernels with a large thread-local frame (EPA scratch, solver rows, the ball-only world):
+        // make the per-thread stack limit cover the largest (the default limit is 1 KB), and give
+        // the L1 its largest share in those that use no shared memory to speak of
         size_t need = 0;
-        for (const StepVariant& v : kStepVariants) {
+        std::vector<const void*> fns{(const void*)predictBallKernel};
+        for (const StepVariant& v : kStepVariants)
+            for (StepFn f : {v.ray, v.contact, v.solve}) fns.push_back((const void*)f);
+        for (const void* f : fns) {
             cudaFuncAttributes fa{};
-            if (cudaFuncGetAttributes(&fa, v.fn) != cudaSuccess)
+            if (cudaFuncGetAttributes(&fa, f) != cudaSuccess)
                 return fail(nullptr, RSB_ERR_CUDA, "cudaFuncGetAttributes failed");
             need = std::max(need, ((fa.localSizeBytes + 4096) + 1023) / 1024 * 1024);
-            cudaFuncSetAttribute(v.fn, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
         }
         size_t cur = 0;
         cudaDeviceGetLimit(&cur, cudaLimitStackSize);
         if (cur < need && cudaDeviceSetLimit(cudaLimitStackSize, need) != cudaSuccess)
-            return fail(nullptr, RSB_ERR_CUDA, "cannot raise the per-thread stack limit for the arena kernel");
+            return fail(nullptr, RSB_ERR_CUDA, "cannot raise the per-thread stack limit");
     }
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(nullptr, RSB_ERR_CUDA, "stream creation failed");
@@ -652,7 +660,8 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
         !dalloc(h->dMasks, (size_t)h->numCars * RSB_NUM_ACTIONS) ||
         !dalloc(h->dRewards, (size_t)h->numCars * 4) || !dalloc(h->dTerminals, N) ||
         !dalloc(h->dResetIdx, N * 4) || !dalloc(h->dCull, N * 4) ||
-        !dalloc(h->dCounters, 4 * sizeof(unsigned long long)) || !dalloc(h->dWork, sizeof(unsigned int)))
+        !dalloc(h->dCounters, 4 * sizeof(unsigned long long)) || !dalloc(h->dWork, QC_WORDS * sizeof(unsigned int)) ||
+        !allocStep(h) || cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
         return fail(nullptr, RSB_ERR_NOMEM, "device allocation failed");
     cudaMemcpy(h->dTeamSize, h->teamSize.data(), N * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(h->dCarOffset, h->carOffset.data(), (N + 1) * 4, cudaMemcpyHostToDevice);
@@ -676,6 +685,7 @@ rsb_status rsb_destroy(rsb_handle* h) {
     cudaFree(h->dTeamSize); cudaFree(h->dCarOffset); cudaFree(h->dBall); cudaFree(h->dCar);
     cudaFree(h->dPad); cudaFree(h->dArena); cudaFree(h->dControls); cudaFree(h->dLut); cudaFree(h->dActions);
     cudaFree(h->dScratch);
+    cudaFree(h->dStep);
     cudaFree(h->dCw); cudaFree(h->dCwBf); cudaFree(h->dCull); cudaFree(h->dCounters); cudaFree(h->dLog);
     cudaFree(h->dTris);
     cudaFree(h->dObs); cudaFree(h->dMasks); cudaFree(h->dRewards); cudaFree(h->dTerminals); cudaFree(h->dResetIdx);
@@ -707,33 +717,37 @@ rsb_status rsb_obs_stride(const rsb_handle* h, int32_t* stride) {
     return RSB_OK;
 }
 
-// Launches step-kernel variant v with block size index b on stream st (a persistent variant
-// first zeroes its claim counter on the same stream).
+// Launches `ticks` ticks on stream st, the queue kernels as variant v with block size index b.
 static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, int ticks, cudaStream_t st,
                               int residency = 0) {
     const StepVariant& sv = kStepVariants[v];
-    const int block = kStepBlocks[b];
-    int grid = (h->N + block - 1) / block;
-    if (sv.persistent) {
-        int& g = h->persistGrid[v][b];
-        if (g == 0) {
-            int perSm = 0, sms = 0;
-            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, sv.fn, block, 0);
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-            if (e != cudaSuccess) return e;
-            h->smCount = sms;
-            g = std::max(1, perSm * sms);
+    const StepTemp& T = h->step;
+    const int block = kStepBlocks[b], groups = (h->N + PHASE_ARENAS - 1) / PHASE_ARENAS;
+    // blocks of a queue kernel for about `items` items
+    auto grid = [&](StepFn f, int64_t items) -> int {
+        int64_t g = std::max<int64_t>(1, (items + block - 1) / block);
+        if (sv.persistent) {
+            int perSm = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, f, block, 0) != cudaSuccess) perSm = 1;
+            if (kStepResidency[residency] > 0) perSm = std::min(perSm, std::max(1, kStepResidency[residency] * 32 / block));
+            g = std::min<int64_t>(g, (int64_t)std::max(1, perSm) * h->smCount);
         }
-        int cap = g;
-        if (kStepResidency[residency] > 0) {
-            const int blocksPerSm = std::max(1, kStepResidency[residency] * 32 / block);
-            cap = std::min(g, blocksPerSm * h->smCount);
+        return (int)g;
+    };
+    const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars);
+    const int contactGrid = grid(sv.contact, (int64_t)h->numCars + h->N);
+    const int solveGrid = grid(sv.solve, h->N);
+    const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
+    for (int t = 0; t < ticks; t++) {
+        if (h->maxCars > 0) {
+            rayKernel<<<groups, carThreads, 0, st>>>(D, T);
+            sv.ray<<<rayGrid, block, 0, st>>>(D, T);
         }
-        grid = std::min(grid, cap);
-        cudaError_t e = cudaMemsetAsync(h->dWork, 0, sizeof(unsigned int), st);
-        if (e != cudaSuccess) return e;
+        bodyKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
+        sv.contact<<<contactGrid, block, 0, st>>>(D, T);
+        sv.solve<<<solveGrid, block, 0, st>>>(D, T);
+        finishKernel<<<groups, bodyThreads, 0, st>>>(D, T);
     }
-    sv.fn<<<grid, block, 0, st>>>(D, ticks);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,207 @@
+// Kernels of the step: the phases of phys/step_phases.h on the device.
+//
+// A block of the ray, body and finish kernels serves 32 arenas, one warp per car or body: lanes
+// run over arenas, so every record word is read and written coalesced, and the bodies of an
+// arena exchange what the reference's order needs through shared memory.  The queue kernels
+// (heavy rays, contacts, islands) run one queued item per thread; their counts are known on the
+// device only, so their grids loop.
+#pragma once
+#include "phys/step_phases.h"
+
+namespace rsb {
+
+// Adds a thread's counters to the handle's statistics: one atomic per block and counter.
+RSB_D void blockStats(const EngineView& D, const PhaseStats& st) {
+    __shared__ uint32_t sum[4];
+    if (threadIdx.x < 4) sum[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t v[4] = {st.nStatic, st.nCulled, st.nMissed, st.nRows};
+    for (int k = 0; k < 4; k++) {
+        const uint32_t w = __reduce_add_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0 && w) atomicAdd(&sum[k], w);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && sum[threadIdx.x] && D.counters)
+        atomicAdd(&D.counters[threadIdx.x], (unsigned long long)sum[threadIdx.x]);
+}
+
+// Places for n items of this thread in a queue: one atomic per warp.  Called by whole warps.
+RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
+    const int lane = threadIdx.x & 31;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    uint32_t base = 0;
+    if (lane == 31 && incl) base = atomicAdd(counter, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    return base + incl - n;
+}
+
+constexpr int BODY_THREADS = MAX_BODIES * PHASE_ARENAS;
+constexpr int CAR_THREADS = MAX_CARS * PHASE_ARENAS;
+
+__global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__ EngineView D,
+                                                         const __grid_constant__ StepTemp T) {
+    __shared__ int32_t cell[MAX_BODIES][3][PHASE_ARENAS];
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+    const int a = blockIdx.x * PHASE_ARENAS + lane;
+    const int nb = a < D.N ? arenaBodies(D, a) : 0;
+    for (int b = s; b < MAX_BODIES; b += blockDim.x >> 5)
+        if (b < nb)
+            for (int k = 0; k < 3; k++)
+                cell[b][k][lane] = (int32_t)bodyWord(D, a, b, (int)(offsetof(CarP, ci) / 4) + k);
+    __syncthreads();
+    PhaseStats st{0, 0, 0, 0};
+    Xf xf;
+    bool culled = false;
+    const bool live = 1 + s < nb && rayCar(D, a, s, xf, culled);
+    auto near = [&](int i, int j, int k) {
+        bool n = false;
+        for (int b = 0; b < nb; b++) {
+            if (b == 1 + s) continue;
+            const int ci = cell[b][0][lane], cj = cell[b][1][lane], ck = cell[b][2][lane];
+            n |= i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1;
+        }
+        return n;
+    };
+    for (int w = 0; w < 4; w++) {
+        const bool heavy = live && rayPhase(D, T, a, s, w, xf, culled, near, st);
+        const uint32_t at = queueAlloc(&T.count[QC_RAY], heavy ? 1u : 0u);
+        if (heavy) T.rayQ[at] = (uint32_t)rayIdx(D, a, s, w);
+    }
+    blockStats(D, st);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) heavyRayKernel(const __grid_constant__ EngineView D,
+                                                            const __grid_constant__ StepTemp T) {
+    const uint32_t n = T.count[QC_RAY];
+    PhaseStats st{0, 0, 0, 0};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        heavyRayPhase(D, T, T.rayQ[i], st);
+    blockStats(D, st);
+}
+
+__global__ void __launch_bounds__(BODY_THREADS) bodyKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T, bool firstTick) {
+    __shared__ BodyShared sh;
+    const int lane = threadIdx.x & 31;
+    BodyThread t;
+    t.b = threadIdx.x >> 5;
+    t.la = lane;
+    t.a = blockIdx.x * PHASE_ARENAS + lane;
+    t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
+    t.finished = true;
+    t.deps = 0;
+    const bool valid = t.b < t.nb;
+    if (blockIdx.x == 0 && threadIdx.x == 0) T.count[QC_RAY] = 0;  // the queued rays are cast
+    if (threadIdx.x < PHASE_ARENAS) sh.done[lane] = sh.need[lane] = 0;
+    if (valid) bodyLoad(D, T, t, sh);
+    __syncthreads();
+    if (valid && t.b > 0 && t.finished) atomicOr(&sh.done[lane], 1u << (t.b - 1));
+    __syncthreads();
+    // a car waits only for cars of higher slots, so every round finishes the highest one left
+    for (int round = 0; round <= MAX_CARS; round++) {
+        const bool ready = !t.finished && !(t.deps & ~sh.done[lane]);
+        if (ready) bodyDrive(t, sh);
+        const int all = __syncthreads_and(t.finished);
+        if (all) break;
+        if (ready) atomicOr(&sh.done[lane], 1u << (t.b - 1));
+        __syncthreads();
+    }
+    if (valid) bodyMove(D, T, t, sh, firstTick);
+    __syncthreads();
+    if (valid) bodyPick(D, t, sh);
+    __syncthreads();
+    PhaseStats st{0, 0, 0, 0};
+    BodyStatics o;
+    o.meshes = o.planes = 0;
+    uint32_t dyn = 0;
+    if (valid) {
+        o = bodyStatics(D, T, t, st);
+        dyn = bodyDynamics(D, t, sh);
+    }
+    const uint32_t m0 = queueAlloc(&T.count[t.b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)__popc(o.meshes));
+    const uint32_t d0 = queueAlloc(&T.count[t.b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)__popc(dyn));
+    if (valid) bodyStore(D, T, t, sh, o, dyn, m0, d0);
+    __syncthreads();
+    if (threadIdx.x < PHASE_ARENAS) {
+        const bool need = sh.need[lane] != 0;
+        const uint32_t at = queueAlloc(&T.count[QC_SOLVE], need ? 1u : 0u);
+        if (need) T.solveQ[at] = (uint32_t)t.a;
+    }
+    blockStats(D, st);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) contactKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T) {
+    EpaWork epa;
+    PhaseStats st{0, 0, 0, 0};
+    uint32_t n[NUM_TASK_TYPES], tiles = 0;
+    for (int k = 0; k < NUM_TASK_TYPES; k++) {
+        n[k] = T.count[QC_CARMESH + k];
+        tiles += (n[k] + 31u) / 32u;
+    }
+    // a warp takes 32 pairs of one type
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
+        uint32_t q = tile;
+        int type = 0;
+        while (q >= (n[type] + 31u) / 32u) q -= (n[type++] + 31u) / 32u;
+        const uint32_t i = q * 32u + (threadIdx.x & 31u);
+        if (i >= n[type]) continue;
+        const uint32_t res = (uint32_t)resultBase(QC_CARMESH + type) * (uint32_t)D.N + i;
+        switch (QC_CARMESH + type) {
+            case QC_CARMESH: carMeshPhase(D, T, res, &epa, st); break;
+            case QC_BALLMESH: ballMeshPhase(D, T, res, st); break;
+            case QC_CARBALL: carBallPhase(D, T, res, &epa); break;
+            default: carCarPhase(D, T, res); break;
+        }
+    }
+    blockStats(D, st);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) solveKernel(const __grid_constant__ EngineView D,
+                                                         const __grid_constant__ StepTemp T) {
+    const uint32_t n = T.count[QC_SOLVE];
+    PhaseStats st{0, 0, 0, 0};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        solvePhase(D, T, (int)T.solveQ[i], st);
+    blockStats(D, st);
+}
+
+__global__ void __launch_bounds__(BODY_THREADS) finishKernel(const __grid_constant__ EngineView D,
+                                                             const __grid_constant__ StepTemp T) {
+    __shared__ FinishShared sh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    FinishThread t;
+    t.b = warp;
+    t.la = lane;
+    t.a = blockIdx.x * PHASE_ARENAS + lane;
+    t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
+    const bool valid = t.b < t.nb, pads = t.nb > 1;
+    if (blockIdx.x == 0 && threadIdx.x < QC_WORDS && threadIdx.x != QC_RAY) T.count[threadIdx.x] = 0;
+    if (pads)
+        for (int p = warp; p < NUM_PADS; p += warps) padLoad(D, t.a, lane, p, sh);
+    if (warp > 0) sh.picked[warp - 1][lane] = 0;
+    else sh.touched[lane] = 0;
+    __syncthreads();
+    if (valid) {
+        finishBody(D, T, t, sh);
+        if (t.b > 0) finishPads(D, t, sh);
+    }
+    __syncthreads();
+    if (pads)
+        for (int p = warp; p < NUM_PADS; p += warps) finishPad(D, t.a, lane, p, sh);
+    __syncthreads();
+    if (!valid) return;
+    if (t.b > 0) finishBoost(D, t, sh);
+    else finishArena(D, t, sh);
+}
+
+}  // namespace rsb

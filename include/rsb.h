@@ -396,16 +396,17 @@ rsb_status rsb_get_arena_info_at(rsb_handle* h, int32_t arena, rsb_arena_info* o
 rsb_status rsb_predict_ball(rsb_handle* h, const int32_t* slice_ticks, int32_t n_slices, rsb_ball_state* out,
                             size_t out_count, void* stream);
 
-/* One candidate launch configuration of the step kernel and its measured time. */
+/* One candidate launch configuration of the step's queue kernels (wheel rays near meshes or
+ * bodies, contact pairs, islands) and the measured time of the step. */
 typedef struct rsb_tune_entry {
     int32_t min_blocks;   /* register budget: at least this many 128-thread blocks per SM */
-    int32_t block;        /* threads per block (one arena per thread) */
+    int32_t block;        /* threads per block (one queued item per thread) */
     float ms;             /* best of two timed launches of `ticks` ticks */
-    int32_t persistent;   /* 1: a grid whose warps claim 32 arenas at a time until none are left */
+    int32_t persistent;   /* 1: a grid of resident size that loops over the queue */
     int32_t warps_per_sm; /* persistent grids: warps resident per SM (0 = as many as fit) */
 } rsb_tune_entry;
 
-/* Times every launch configuration of the step kernel on a device copy of the current
+/* Times every launch configuration of the step's queue kernels on a device copy of the current
  * arena state (the handle's own state is not advanced), keeps the fastest for later
  * rsb_step calls, and reports every candidate in out[0..cap).  Allocates the scratch copy
  * of the state on its first call.  No counterpart in the reference. */

@@ -1,0 +1,185 @@
+// Host run of the step's phases (emy-s-framework_b200/csrc/phys/step_phases.h) beside the
+// one-thread tick of the host engine, for the CPU test that compares the two byte by byte.
+// The loops below stand for the kernels of step_kernels.cuh: blocks of 32 arenas with one
+// thread per body, queues taken from the back so that nothing depends on their order.
+#include "host_engine.cpp"
+
+#include "phys/step_phases.h"
+
+extern "C" {
+
+// `ticks` ticks of the handle's arenas through the phases.  cull: a body mask per arena, or null.
+// Returns the number of items that went through each queue in counts[QC_WORDS].
+int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int64_t* counts, uint64_t* stats) {
+    const size_t N = h->N, B = MAX_BODIES * N, R = (size_t)4 * MAX_CARS * N;
+    EngineView D;
+    D.S = h->S.view;
+    D.P = h->P;
+    D.N = h->N;
+    D.teamSize = h->teamSize.data();
+    D.carOffset = h->carOffset.data();
+    D.ball = h->ball.data();
+    D.car = h->car.data();
+    D.pad = h->pad.data();
+    D.arena = h->arena.data();
+    D.controls = reinterpret_cast<const CtlRec*>(h->controls.data());
+    D.seed = (uint32_t)(h->seed ^ (h->seed >> 32));
+    D.cull = cull;
+    D.cullAudit = 0;
+    D.counters = nullptr;
+    D.work = nullptr;
+    std::vector<int32_t> rayObj(R);
+    std::vector<float> rayFrac(R), rayN(3 * R), force(6 * B), box(6 * B), cache(3 * B);
+    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(R), solveQ(N);
+    std::vector<PairTask> tasks(CAP_RESULTS * N);
+    std::vector<PairResult> results(CAP_RESULTS * N);
+    std::vector<MPoint> blocks(MAX_BLOCKS * N * MAX_POINTS);
+    StepTemp T;
+    T.rayObj = rayObj.data();
+    T.rayFrac = rayFrac.data();
+    T.rayN = rayN.data();
+    T.info = info.data();
+    T.force = force.data();
+    T.box = box.data();
+    T.cache = cache.data();
+    T.dynRes = dynRes.data();
+    T.count = count.data();
+    T.rayQ = rayQ.data();
+    T.tasks = tasks.data();
+    T.results = results.data();
+    T.blocks = blocks.data();
+    T.blockCap = (uint32_t)(MAX_BLOCKS * N);
+    T.solveQ = solveQ.data();
+    std::unique_ptr<EpaWork> epa(new EpaWork());
+    std::unique_ptr<BodyShared> sh(new BodyShared());
+    std::unique_ptr<FinishShared> fs(new FinishShared());
+    std::vector<BodyThread> bt(MAX_BODIES * PHASE_ARENAS);
+    std::vector<FinishThread> ft(MAX_BODIES * PHASE_ARENAS);
+    PhaseStats st{0, 0, 0, 0};
+    for (int tick = 0; tick < ticks; tick++) {
+        // rays
+        for (int a = 0; a < h->N; a++)
+            for (int s = 0; s < 2 * h->teamSize[a]; s++) {
+                Xf xf;
+                bool culled;
+                if (!rayCar(D, a, s, xf, culled)) continue;
+                auto near = [&](int i, int j, int k) {
+                    for (int b = 0; b < arenaBodies(D, a); b++) {
+                        if (b == 1 + s) continue;
+                        const int w = (int)(offsetof(CarP, ci) / 4);
+                        const int ci = (int)bodyWord(D, a, b, w), cj = (int)bodyWord(D, a, b, w + 1), ck = (int)bodyWord(D, a, b, w + 2);
+                        if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) return true;
+                    }
+                    return false;
+                };
+                for (int w = 0; w < 4; w++)
+                    if (rayPhase(D, T, a, s, w, xf, culled, near, st)) T.rayQ[T.count[QC_RAY]++] = (uint32_t)rayIdx(D, a, s, w);
+            }
+        counts[QC_RAY] += T.count[QC_RAY];
+        while (T.count[QC_RAY] > 0) heavyRayPhase(D, T, T.rayQ[--T.count[QC_RAY]], st);
+        // bodies
+        for (int g = 0; g < h->N; g += PHASE_ARENAS) {
+            auto each = [&](auto&& fn) {
+                for (int b = MAX_BODIES - 1; b >= 0; b--)
+                    for (int la = 0; la < PHASE_ARENAS && g + la < h->N; la++)
+                        if (b < arenaBodies(D, g + la)) fn(bt[b * PHASE_ARENAS + la], b, la);
+            };
+            std::memset(sh->done, 0, sizeof sh->done);
+            std::memset(sh->need, 0, sizeof sh->need);
+            each([&](BodyThread& t, int b, int la) {
+                t.b = b;
+                t.la = la;
+                t.a = g + la;
+                t.nb = arenaBodies(D, t.a);
+                bodyLoad(D, T, t, *sh);
+                if (b > 0 && t.finished) sh->done[la] |= 1u << (b - 1);
+            });
+            for (bool all = false; !all;) {
+                std::vector<BodyThread*> ran;
+                all = true;
+                each([&](BodyThread& t, int, int la) {
+                    if (!t.finished && !(t.deps & ~sh->done[la])) {
+                        bodyDrive(t, *sh);
+                        ran.push_back(&t);
+                    }
+                });
+                for (BodyThread* t : ran) sh->done[t->la] |= 1u << (t->b - 1);
+                each([&](BodyThread& t, int, int) { all &= t.finished; });
+                if (!all && ran.empty()) return -1;
+            }
+            each([&](BodyThread& t, int, int) { bodyMove(D, T, t, *sh, tick == 0); });
+            each([&](BodyThread& t, int, int) { bodyPick(D, t, *sh); });
+            each([&](BodyThread& t, int b, int) {
+                const BodyStatics o = bodyStatics(D, T, t, st);
+                const uint32_t dyn = bodyDynamics(D, t, *sh);
+                const uint32_t m0 = phaseAtomicAdd(&T.count[b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)bitCount(o.meshes));
+                const uint32_t d0 = phaseAtomicAdd(&T.count[b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)bitCount(dyn));
+                bodyStore(D, T, t, *sh, o, dyn, m0, d0);
+            });
+            for (int la = 0; la < PHASE_ARENAS; la++)
+                if (sh->need[la]) T.solveQ[T.count[QC_SOLVE]++] = (uint32_t)(g + la);
+        }
+        // contacts, islands
+        for (int k = 0; k < NUM_TASK_TYPES; k++) {
+            const int type = QC_CARMESH + k;
+            for (uint32_t i = T.count[type]; i-- > 0;) {
+                const uint32_t res = (uint32_t)resultBase(type) * (uint32_t)D.N + i;
+                if (type == QC_CARMESH) carMeshPhase(D, T, res, epa.get(), st);
+                else if (type == QC_BALLMESH) ballMeshPhase(D, T, res, st);
+                else if (type == QC_CARBALL) carBallPhase(D, T, res, epa.get());
+                else carCarPhase(D, T, res);
+            }
+        }
+        for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], st);
+        // finish
+        for (int g = 0; g < h->N; g += PHASE_ARENAS) {
+            auto each = [&](auto&& fn) {
+                for (int b = 0; b < MAX_BODIES; b++)
+                    for (int la = 0; la < PHASE_ARENAS && g + la < h->N; la++)
+                        if (b < arenaBodies(D, g + la)) fn(ft[b * PHASE_ARENAS + la], b, la);
+            };
+            auto eachPad = [&](auto&& fn) {
+                for (int p = 0; p < NUM_PADS; p++)
+                    for (int la = 0; la < PHASE_ARENAS && g + la < h->N; la++)
+                        if (arenaBodies(D, g + la) > 1) fn(p, la);
+            };
+            eachPad([&](int p, int la) { padLoad(D, g + la, la, p, *fs); });
+            std::memset(fs->picked, 0, sizeof fs->picked);
+            std::memset(fs->touched, 0, sizeof fs->touched);
+            each([&](FinishThread& t, int b, int la) {
+                t.b = b;
+                t.la = la;
+                t.a = g + la;
+                t.nb = arenaBodies(D, t.a);
+                finishBody(D, T, t, *fs);
+                if (b > 0) finishPads(D, t, *fs);
+            });
+            eachPad([&](int p, int la) { finishPad(D, g + la, la, p, *fs); });
+            each([&](FinishThread& t, int b, int) {
+                if (b > 0) finishBoost(D, t, *fs);
+                else finishArena(D, t, *fs);
+            });
+        }
+        for (int k = QC_CARMESH; k < QC_WORDS; k++) {
+            counts[k] += T.count[k];
+            T.count[k] = 0;
+        }
+    }
+    stats[0] += st.nStatic;
+    stats[1] += st.nCulled;
+    stats[2] += st.nMissed;
+    stats[3] += st.nRows;
+    return RSB_OK;
+}
+
+// The first word at which the records of two handles differ, as plane * 2^40 + index, or -1.
+int64_t rsb_host_records_differ(const rsb_handle* x, const rsb_handle* y) {
+    const std::vector<uint32_t>* p[4] = {&x->ball, &x->car, &x->pad, &x->arena};
+    const std::vector<uint32_t>* q[4] = {&y->ball, &y->car, &y->pad, &y->arena};
+    for (int k = 0; k < 4; k++)
+        for (size_t i = 0; i < p[k]->size(); i++)
+            if ((*p[k])[i] != (*q[k])[i]) return ((int64_t)k << 40) + (int64_t)i;
+    return -1;
+}
+
+}  // extern "C"
