@@ -363,8 +363,8 @@ struct EpaSolver {
     V3 normal;
     float depth;
     uint32_t nextsv;
-    int16_t hullRoot, stockRoot;
-    uint32_t hullCount, stockCount;
+    int16_t hullRoot, stockRoot, stockNext;
+    uint32_t hullCount;
     bool overflow;
 
     RSB_HD EpaSimplex& simplex() { return simplices[simplexSel]; }
@@ -613,23 +613,34 @@ struct EpaSolver {
                          wk->sv[s.c[2]].w - wk->sv[s.c[3]].w)) > 0;
     }
 
-    // ---- EPA lists
-    RSB_HD void listAppend(bool hull, int16_t f) {
-        int16_t& root = hull ? hullRoot : stockRoot;
+    // ---- EPA lists.  Faces leave the stock at its front and return to it there, and the
+    // reference's stock starts as faces 0, 1, 2, ...: a stack of returned faces over the next
+    // unused face gives the same faces without building the 256-entry list first.
+    RSB_HD void hullAppend(int16_t f) {
         EpaFace& F = wk->fc[f];
         F.l[0] = -1;
-        F.l[1] = root;
-        if (root >= 0) wk->fc[root].l[0] = f;
-        root = f;
-        if (hull) hullCount++; else stockCount++;
+        F.l[1] = hullRoot;
+        if (hullRoot >= 0) wk->fc[hullRoot].l[0] = f;
+        hullRoot = f;
+        hullCount++;
     }
-    RSB_HD void listRemove(bool hull, int16_t f) {
-        int16_t& root = hull ? hullRoot : stockRoot;
+    RSB_HD void hullRemove(int16_t f) {
         EpaFace& F = wk->fc[f];
         if (F.l[1] >= 0) wk->fc[F.l[1]].l[0] = F.l[0];
         if (F.l[0] >= 0) wk->fc[F.l[0]].l[1] = F.l[1];
-        if (f == root) root = F.l[1];
-        if (hull) hullCount--; else stockCount--;
+        if (f == hullRoot) hullRoot = F.l[1];
+        hullCount--;
+    }
+    RSB_HD bool stockEmpty() const { return stockRoot < 0 && stockNext >= EPA_MAX_FACES; }
+    RSB_HD int16_t stockTake() {
+        if (stockRoot < 0) return stockNext++;
+        const int16_t f = stockRoot;
+        stockRoot = wk->fc[f].l[1];
+        return f;
+    }
+    RSB_HD void stockReturn(int16_t f) {
+        wk->fc[f].l[1] = stockRoot;
+        stockRoot = f;
     }
     RSB_HD void bind(int16_t fa, uint32_t ea, int16_t fb, uint32_t eb) {
         wk->fc[fa].e[ea] = (uint8_t)eb;
@@ -656,10 +667,9 @@ struct EpaSolver {
         return false;
     }
     RSB_HD int16_t newface(int ia, int ib, int ic, bool forced) {
-        if (stockRoot >= 0) {
-            int16_t f = stockRoot;
-            listRemove(false, f);
-            listAppend(true, f);
+        if (!stockEmpty()) {
+            int16_t f = stockTake();
+            hullAppend(f);
             EpaFace& F = wk->fc[f];
             F.pass = 0;
             F.c[0] = (uint8_t)ia;
@@ -678,11 +688,11 @@ struct EpaSolver {
             } else {
                 epaStatus = 2;  // Degenerated
             }
-            listRemove(true, f);
-            listAppend(false, f);
+            hullRemove(f);
+            stockReturn(f);
             return -1;
         }
-        epaStatus = (stockRoot >= 0) ? 6 : 5;
+        epaStatus = 5;
         return -1;
     }
     RSB_HD int16_t findbest() const {
@@ -739,8 +749,8 @@ struct EpaSolver {
                 continue;
             }
             if (ret) {
-                listRemove(true, f);
-                listAppend(false, f);
+                hullRemove(f);
+                stockReturn(f);
             }
             sp--;
         }
@@ -751,11 +761,6 @@ struct EpaSolver {
     RSB_HD int epaEvaluate(V3 guess) {
         EpaSimplex& s = simplex();
         if ((s.rank > 1) && encloseOrigin()) {
-            while (hullRoot >= 0) {
-                int16_t f = hullRoot;
-                listRemove(true, f);
-                listAppend(false, f);
-            }
             epaStatus = 0;
             nextsv = 0;
             if (det(wk->sv[s.c[0]].w - wk->sv[s.c[3]].w, wk->sv[s.c[1]].w - wk->sv[s.c[3]].w,
@@ -795,8 +800,8 @@ struct EpaSolver {
                             if (overflow) return 9;
                             if (valid && (hnf >= 3)) {
                                 bind(hcf, 1, hff, 2);
-                                listRemove(true, best);
-                                listAppend(false, best);
+                                hullRemove(best);
+                                stockReturn(best);
                                 best = findbest();
                                 outer = wk->fc[best];
                             } else {
@@ -852,15 +857,15 @@ struct EpaSolver {
         shape.margins = margins;
         overflow = false;
     }
-    // EPA::Initialize: every face starts in the stock list
+    // EPA::Initialize: an empty hull, every face in the stock
     RSB_HD void initEpa() {
         epaStatus = 9;
         normal = v3zero();
         depth = 0;
         nextsv = 0;
         hullRoot = stockRoot = -1;
-        hullCount = stockCount = 0;
-        for (int i = 0; i < EPA_MAX_FACES; ++i) listAppend(false, (int16_t)(EPA_MAX_FACES - i - 1));
+        stockNext = 0;
+        hullCount = 0;
     }
 };
 
@@ -944,18 +949,31 @@ struct GjkOut {
     bool overflow;
 };
 
-RSB_HD GjkOut gjkPairDetector(EpaWork* wk, const ConvexShape& A, const Xf& trA, const ConvexShape& B, const Xf& trB,
-                              float maxDist2) {
-    GjkOut out;
-    out.has = false;
-    out.overflow = false;
+// The detector between its parts: the iteration (gjkIterate), the penetration solver where the
+// iteration found the cores touching or nearly so (gjkPenetrate), and the result (gjkFinish).
+struct GjkState {
+    Xf lA, lB;           // the shapes' transforms about their midpoint
+    V3 positionOffset;
+    V3 normalInB, pointOnB;
+    float distance;
+    bool isValid, needEpa;
+};
+
+RSB_HD void gjkFrames(const Xf& trA, const Xf& trB, GjkState& st) {
+    st.lA = trA;
+    st.lB = trB;
+    st.positionOffset = (st.lA.o + st.lB.o) * 0.5f;
+    st.lA.o = st.lA.o - st.positionOffset;
+    st.lB.o = st.lB.o - st.positionOffset;
+}
+
+RSB_HD void gjkIterate(const ConvexShape& A, const Xf& trA, const ConvexShape& B, const Xf& trB, float maxDist2,
+                       GjkState& st) {
+    gjkFrames(trA, trB, st);
     float distance = 0.f;
     V3 normalInB = v3zero();
     V3 pointOnA = v3zero(), pointOnB = v3zero();
-    Xf lA = trA, lB = trB;
-    V3 positionOffset = (lA.o + lB.o) * 0.5f;
-    lA.o = lA.o - positionOffset;
-    lB.o = lB.o - positionOffset;
+    const Xf &lA = st.lA, &lB = st.lB;
     float marginA = A.margin, marginB = B.margin;
     int curIter = 0;
     const int gGjkMaxIter = 1000;
@@ -1036,62 +1054,83 @@ RSB_HD GjkOut gjkPairDetector(EpaWork* wk, const ConvexShape& A, const Xf& trA, 
         }
     }
     bool catchDegenerate = degenerate && ((distance + margin) < 0.01f);
-    if (!isValid || catchDegenerate) {
-        V3 tA, tB;
-        axis = v3zero();
-        bool ovf = false;
-        bool valid2 = calcPenDepth(wk, A, lA, B, lB, axis, tA, tB, ovf);
-        if (ovf) {
-            out.overflow = true;
-            return out;
+    st.normalInB = normalInB;
+    st.pointOnB = pointOnB;
+    st.distance = distance;
+    st.isValid = isValid;
+    st.needEpa = !isValid || catchDegenerate;
+}
+
+// The penetration solver's result where it is deeper; returns true when it ran out of stack.
+RSB_HD bool gjkPenetrate(EpaWork* wk, const ConvexShape& A, const ConvexShape& B, GjkState& st) {
+    const float marginA = A.margin, marginB = B.margin, margin = marginA + marginB;
+    V3 tA, tB, axis = v3zero();
+    bool ovf = false;
+    bool valid2 = calcPenDepth(wk, A, st.lA, B, st.lB, axis, tA, tB, ovf);
+    if (ovf) return true;
+    if (valid2) {
+        V3 tn = tB - tA;
+        float l2 = length2(tn);
+        if (l2 <= kEpsilon * kEpsilon) {
+            tn = axis;
+            l2 = length2(axis);
         }
-        if (valid2) {
-            V3 tn = tB - tA;
-            float l2 = length2(tn);
-            if (l2 <= kEpsilon * kEpsilon) {
-                tn = axis;
-                l2 = length2(axis);
+        if (l2 > kEpsilon * kEpsilon) {
+            tn = bdiv(tn, fsqrt(l2));
+            float d2 = -length(tA - tB);
+            if (!st.isValid || (d2 < st.distance)) {
+                st.distance = d2;
+                st.pointOnB = tB;
+                st.normalInB = tn;
+                st.isValid = true;
             }
-            if (l2 > kEpsilon * kEpsilon) {
-                tn = bdiv(tn, fsqrt(l2));
-                float d2 = -length(tA - tB);
-                if (!isValid || (d2 < distance)) {
-                    distance = d2;
-                    pointOnA = tA;
-                    pointOnB = tB;
-                    normalInB = tn;
-                    isValid = true;
-                }
-            }
-        } else {
-            if (length2(axis) > 0.f) {
-                float d2 = length(tA - tB) - margin;
-                if (!isValid || (d2 < distance)) {
-                    distance = d2;
-                    pointOnA = tA;
-                    pointOnB = tB;
-                    pointOnA -= axis * marginA;
-                    pointOnB += axis * marginB;
-                    normalInB = normalized(axis);
-                    isValid = true;
-                }
+        }
+    } else {
+        if (length2(axis) > 0.f) {
+            float d2 = length(tA - tB) - margin;
+            if (!st.isValid || (d2 < st.distance)) {
+                st.distance = d2;
+                st.pointOnB = tB;
+                st.pointOnB += axis * marginB;
+                st.normalInB = normalized(axis);
+                st.isValid = true;
             }
         }
     }
-    if (isValid && ((distance < 0) || (distance * distance < maxDist2))) {
-        V3 mn, mx;
-        shapeAabb(A, lA, mn, mx);
+    return false;
+}
+
+RSB_HD GjkOut gjkFinish(const ConvexShape& A, const ConvexShape& B, const GjkState& st, float maxDist2) {
+    GjkOut out;
+    out.has = false;
+    out.overflow = false;
+    if (st.isValid && ((st.distance < 0) || (st.distance * st.distance < maxDist2))) {
+        V3 mn, mx, normalInB = st.normalInB;
+        shapeAabb(A, st.lA, mn, mx);
         V3 posA = (mx + mn) * 0.5f;
-        shapeAabb(B, lB, mn, mx);
+        shapeAabb(B, st.lB, mn, mx);
         V3 posB = (mn + mx) * 0.5f;
         V3 diff = posA - posB;
         if (dot(diff, normalInB) < 0.f) normalInB *= -1.f;
         out.has = true;
         out.normal = normalInB;
-        out.point = pointOnB + positionOffset;
-        out.dist = distance;
+        out.point = st.pointOnB + st.positionOffset;
+        out.dist = st.distance;
     }
     return out;
+}
+
+RSB_HD GjkOut gjkPairDetector(EpaWork* wk, const ConvexShape& A, const Xf& trA, const ConvexShape& B, const Xf& trB,
+                              float maxDist2) {
+    GjkState st;
+    gjkIterate(A, trA, B, trB, maxDist2, st);
+    if (st.needEpa && gjkPenetrate(wk, A, B, st)) {
+        GjkOut out;
+        out.has = false;
+        out.overflow = true;
+        return out;
+    }
+    return gjkFinish(A, B, st, maxDist2);
 }
 
 // ------------------------------------------------------------------ ray vs convex

@@ -11,7 +11,10 @@
 //   heavy rays . the queued rays: meshes, planes, other bodies (castRay)
 //   bodies ..... respawns, vehicle update, gravity, predicted motion, broadphase pairs, plane
 //                contacts; queues the other contact pairs and the arenas that have any
-//   contacts ... one queued pair per thread: box-mesh, sphere-mesh, box-sphere, box-box
+//   find ....... queued mesh pairs: the triangles whose boxes overlap (candidates, in walk order)
+//   triangles .. one candidate per thread: box-triangle and box-sphere GJK; box-box pairs
+//   deep ....... the candidates whose GJK needs the penetration solver
+//   combine .... one pair per thread: its candidates' contacts into the manifold, in walk order
 //   islands .... the queued arenas: contact callbacks, islands, solver (solveIslands)
 //   finish ..... integration, post-tick updates, boost pads, goal and tick counters
 //
@@ -49,7 +52,10 @@ constexpr int NUM_DYN_PAIRS = MAX_BODIES * (MAX_BODIES - 1) / 2;
 RSB_HD int dynPair(int lo, int hi) { return lo * (2 * MAX_BODIES - lo - 1) / 2 + (hi - lo - 1); }
 
 // Queue counters.
-enum : int { QC_RAY = 0, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_WORDS };
+enum : int {
+    QC_RAY = 0, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_TRI, QC_DEEP, QC_COMBINE,
+    QC_WORDS
+};
 constexpr int NUM_TASK_TYPES = 4;  // QC_CARMESH .. QC_CARCAR
 // The most pairs of each type that an arena can have, and contact blocks (MAX_BLOCKS manifolds
 // hold contacts in one tick; more are dropped, as in the one-thread tick).
@@ -81,6 +87,25 @@ enum : uint32_t {
     PR_WORLD = 2u   // ... and the car-world callback saw it
 };
 
+// One triangle (tri < 0: the ball) that a queued pair's boxes overlap; a pair's candidates form
+// a list in the order in which the reference visits them.
+struct Candidate {
+    uint32_t res;   // the pair's place in the task and result arrays
+    int32_t tri;
+    uint32_t next;  // NO_CANDIDATE at the end
+};
+constexpr uint32_t NO_CANDIDATE = ~0u;
+// What GJK found for a candidate; between the triangles and the deep phase, its state.
+struct CandidateOut {
+    uint32_t flags;  // CO_*
+    float normal[3], point[3], dist;
+};
+enum : uint32_t { CO_HAS = 1u, CO_VALID = 2u };
+// Candidates per arena that the batch has room for.  Pairs that find none left are taken
+// triangle by triangle on one thread (the deep queue holds them as DEEP_PAIR | result).
+constexpr int CAP_CANDIDATES = 64;
+constexpr uint32_t DEEP_PAIR = 1u << 31;
+
 struct StepTemp {
     // wheel rays, [4][MAX_CARS][N]: object hit (-1 none), fraction, normal (3 planes)
     int32_t* rayObj;
@@ -98,6 +123,12 @@ struct StepTemp {
     MPoint* blocks;      // [MAX_BLOCKS * N][MAX_POINTS]
     uint32_t blockCap;
     uint32_t* solveQ;    // [N]
+    uint32_t* first;     // first candidate of each pair, as results
+    Candidate* cand;     // [candCap]
+    CandidateOut* out;   // [candCap]
+    uint32_t candCap;
+    uint32_t* deepQ;     // [CAP_RESULTS * N + candCap]
+    uint32_t* combineQ;  // [CAP_RESULTS * N]
 };
 
 // Static-test counters of one thread (rsb_stats).
@@ -938,7 +969,7 @@ RSB_HD void pairBody(const EngineView& D, int a, int b, Body& o) {
     o.noResp = b > 0 && (carWord(D, a, b - 1, RSB_PW(CarP, flags)) & CF_NO_RESPONSE) ? 1 : 0;
 }
 
-// One queued pair; `res` is its place in the task and result arrays.
+// A whole mesh pair on one thread; `res` is its place in the task and result arrays.
 RSB_HD void carMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, EpaWork* epa, PhaseStats& st) {
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, b = k.o1 - OBJ_BALL;
@@ -963,21 +994,201 @@ RSB_HD void ballMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, 
     st.nMissed += W.nMissed;
     storePair(D, T, a, W, m, res);
 }
-// Car pairs keep their points as added: the islands phase runs the callbacks on them before
-// refreshContactPoints.
-RSB_HD void carBallPhase(const EngineView& D, const StepTemp& T, uint32_t res, EpaWork* epa) {
+
+// Finds a pair's candidates: the triangles whose leaves and boxes overlap the body's box, or for
+// a car and the ball the ball itself.  A mesh pair without any is finished here.
+RSB_HD void findPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, b = k.o1 - OBJ_BALL;
-    PairWorldT<PairBodies> W;
-    pairWorldInit(D, W, epa, 0u);
-    W.b.i0 = 0;
-    pairBody(D, a, 0, W.b.v0);
-    pairBody(D, a, b, W.b.v1);
+    uint32_t first = NO_CANDIDATE, last = NO_CANDIDATE;
+    bool full = false;
+    auto add = [&](int tri) {
+        const uint32_t c = phaseAtomicAdd(&T.count[QC_TRI], 1u);
+        if (c >= T.candCap) {
+            full = true;
+            return false;
+        }
+        T.cand[c] = Candidate{res, tri, NO_CANDIDATE};
+        if (last == NO_CANDIDATE) first = c;
+        else T.cand[last].next = c;
+        last = c;
+        return true;
+    };
+    if (k.o0 == OBJ_BALL) {
+        add(-1);
+    } else {
+        V3 amn, amx;
+        const Xf xf = bodyXf(D, a, b);
+        if (b == 0) ballAabb(D.P, xf, amn, amx);
+        else carBoxAabb(D.P.car, carChildXf(D.P.car, xf), amn, amx);
+        bvhQueryAabb(D.S, k.o0, amn, amx, [&](int tri) {
+            V3 v[3];
+            triVerts(D.S, k.o0, tri, v);
+            return triAabbOverlap(v, amn, amx) ? add(tri) : true;
+        });
+    }
+    if (full) {
+        T.deepQ[phaseAtomicAdd(&T.count[QC_DEEP], 1u)] = DEEP_PAIR | res;
+        // its candidates still in the queue are worked on for nothing
+        return;
+    }
+    if (first == NO_CANDIDATE) {
+        T.results[res] = PairResult{0, 0u, 0u, {0.f, 0.f, 0.f}};
+        return;
+    }
+    T.first[res] = first;
+    T.combineQ[phaseAtomicAdd(&T.count[QC_COMBINE], 1u)] = res;
+}
+
+// The two shapes of a box candidate.
+struct CandidateShapes {
+    ConvexShape box, other;
+    Xf boxXf, otherXf;
+    float maxDist2;
+};
+RSB_HD bool candidateShapes(const EngineView& D, const StepTemp& T, const Candidate& c, CandidateShapes& o, int& a) {
+    const PairTask k = T.tasks[c.res];
+    const CarParams& C = D.P.car;
+    a = (int)k.a;
+    const int b = k.o1 - OBJ_BALL;
+    if (b == 0) return false;  // the ball's triangles are tested by the combine phase
+    o.box = carBoxShape(C);
+    o.boxXf = carChildXf(C, bodyXf(D, a, b));
+    if (c.tri < 0) {
+        o.other = makeSphere(D.P.ballRadius);
+        o.otherXf = bodyXf(D, a, 0);
+        o.maxDist2 = sq((C.boxMargin + D.P.ballMargin) + fmin_(C.cbt, D.P.ballCbt));
+        return true;
+    }
+    V3 v[3];
+    triVerts(D.S, k.o0, c.tri, v);
+    o.other = makeTri(v, 0.f);
+    o.otherXf = xfIdentity();
+    o.maxDist2 = boxMeshMaxDist2(C, C.cbt);
+    return true;
+}
+RSB_HD void storeCandidate(CandidateOut& o, uint32_t flags, V3 n, V3 p, float d) {
+    o.flags = flags;
+    o.normal[0] = n.x; o.normal[1] = n.y; o.normal[2] = n.z;
+    o.point[0] = p.x; o.point[1] = p.y; o.point[2] = p.z;
+    o.dist = d;
+}
+
+RSB_HD void trianglePhase(const EngineView& D, const StepTemp& T, uint32_t i) {
+    const Candidate c = T.cand[i];
+    CandidateShapes s;
+    int a;
+    if (!candidateShapes(D, T, c, s, a)) return;
+    T.out[i].flags = 0;
+    if (c.tri >= 0 && !boxTriNear(D.P.car, s.box, s.boxXf, D.P.car.cbt, s.other.v)) return;
+    GjkState g;
+    gjkIterate(s.box, s.boxXf, s.other, s.otherXf, s.maxDist2, g);
+    if (g.needEpa) {
+        storeCandidate(T.out[i], g.isValid ? CO_VALID : 0u, g.normalInB, g.pointOnB, g.distance);
+        T.deepQ[phaseAtomicAdd(&T.count[QC_DEEP], 1u)] = i;
+        return;
+    }
+    const GjkOut o = gjkFinish(s.box, s.other, g, s.maxDist2);
+    if (o.has) storeCandidate(T.out[i], CO_HAS, o.normal, o.point, o.dist);
+}
+
+RSB_HD void deepPhase(const EngineView& D, const StepTemp& T, uint32_t e, EpaWork* epa, PhaseStats& st) {
+    if (e & DEEP_PAIR) {
+        const uint32_t res = e & ~DEEP_PAIR;
+        const PairTask k = T.tasks[res];
+        if (k.o1 == OBJ_BALL) {
+            ballMeshPhase(D, T, res, st);
+        } else if (k.o0 == OBJ_BALL) {
+            PairWorldT<PairBodies> W;
+            pairWorldInit(D, W, epa, 0u);
+            W.b.i0 = 0;
+            pairBody(D, (int)k.a, 0, W.b.v0);
+            pairBody(D, (int)k.a, k.o1 - OBJ_BALL, W.b.v1);
+            Manifold m;
+            pairManifold(m, k.o1, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt));
+            carBallContact(W, k.o1 - OBJ_CAR0, carChildXf(D.P.car, W.b.v1.xf), m);
+            storePair(D, T, (int)k.a, W, m, res);
+        } else {
+            carMeshPhase(D, T, res, epa, st);
+        }
+        return;
+    }
+    CandidateOut& o = T.out[e];
+    CandidateShapes s;
+    int a;
+    candidateShapes(D, T, T.cand[e], s, a);
+    GjkState g;
+    gjkFrames(s.boxXf, s.otherXf, g);
+    g.isValid = (o.flags & CO_VALID) != 0;
+    g.normalInB = V3{o.normal[0], o.normal[1], o.normal[2]};
+    g.pointOnB = V3{o.point[0], o.point[1], o.point[2]};
+    g.distance = o.dist;
+    o.flags = 0;
+    if (gjkPenetrate(epa, s.box, s.other, g)) {
+        phaseAtomicOr(arenaStatus(D, a), WS_EPA_OVERFLOW);
+        return;
+    }
+    const GjkOut r = gjkFinish(s.box, s.other, g, s.maxDist2);
+    if (r.has) storeCandidate(o, CO_HAS, r.normal, r.point, r.dist);
+}
+
+// A pair's contacts in the order of its candidates.  Pairs of two bodies keep their points as
+// added: the islands phase runs the callbacks on them before refreshContactPoints.
+RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, PhaseStats& st) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a, b = k.o1 - OBJ_BALL;
+    if (k.o0 == OBJ_BALL) {
+        const CandidateOut& o = T.out[T.first[res]];
+        PairWorldT<PairBodies> W;
+        pairWorldInit(D, W, nullptr, 0u);
+        W.b.i0 = 0;
+        pairBody(D, a, 0, W.b.v0);
+        pairBody(D, a, b, W.b.v1);
+        Manifold m;
+        pairManifold(m, k.o1, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt));
+        if (o.flags & CO_HAS)
+            addContact(m, W.pool, OBJ_BALL, objRef(W, OBJ_BALL), k.o1, objRef(W, k.o1),
+                       V3{o.normal[0], o.normal[1], o.normal[2]}, V3{o.point[0], o.point[1], o.point[2]}, o.dist);
+        storePair(D, T, a, W, m, res);
+        return;
+    }
+    PairWorldT<OneBody> W;
+    pairWorldInit(D, W, nullptr, D.cull ? (D.cull[a] & (1u << b)) : 0u);
+    pairBody(D, a, b, W.b.v);
     Manifold m;
-    pairManifold(m, k.o1, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt));
-    carBallContact(W, b - 1, carChildXf(D.P.car, W.b.v1.xf), m);
+    pairManifold(m, k.o1, k.o0, b == 0 ? D.P.ballCbt : D.P.car.cbt);
+    bool found = false;
+    for (uint32_t c = T.first[res]; c != NO_CANDIDATE;) {
+        const Candidate cd = T.cand[c];
+        V3 v[3], n, p;
+        float d;
+        bool has;
+        if (b == 0) {
+            triVerts(D.S, k.o0, cd.tri, v);
+            has = ballTriContact(D.P, W.b.v.xf, m.cbt, v, p, n, d);
+        } else {
+            const CandidateOut& o = T.out[c];
+            has = (o.flags & CO_HAS) != 0;
+            if (has) {
+                triVerts(D.S, k.o0, cd.tri, v);
+                n = V3{o.normal[0], o.normal[1], o.normal[2]};
+                p = V3{o.point[0], o.point[1], o.point[2]};
+                d = o.dist;
+            }
+        }
+        if (has) {
+            found = true;
+            if (b == 0) addBallTriContact(W, k.o0, cd.tri, v, n, p, d, m);
+            else addBoxTriContact(W, k.o0, b - 1, cd.tri, v, n, p, d, m);
+        }
+        c = cd.next;
+    }
+    cullCheck(W, b, found);
+    if (m.n) refreshContactPoints(m, W.b.v.xf, xfIdentity());
+    st.nMissed += W.nMissed;
     storePair(D, T, a, W, m, res);
 }
+
 RSB_HD void carCarPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, ba = k.o0 - OBJ_BALL, bb = k.o1 - OBJ_BALL;

@@ -423,51 +423,63 @@ RSB_HD bool sphereTriCollide(const V3* v, V3 center, float radius, float cbt, V3
     return false;
 }
 
+// One triangle that overlaps the ball's AABB: the early out on the two sides of its plane
+// (btConvexConcaveCollisionAlgorithm.cpp:100-137), then btSphereTriangleCollisionAlgorithm.
+RSB_HD bool ballTriContact(const WorldParams& P, const Xf& ballXf, float cbt, const V3* v, V3& point, V3& normal,
+                           float& depth) {
+    const M3 invB = inverse(ballXf.b);
+    V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
+    float thr = cbt + 0.f;
+    for (int side = 0; side < 2; side++) {
+        V3 lp = sphereSupport(invB * tn, P.ballMargin);
+        V3 wp = xfPoint(ballXf, lp);
+        float dist = dot(tn, v[0]) - dot(tn, wp);
+        if (dist > thr) return false;
+        tn *= -1.f;
+    }
+    return sphereTriCollide(v, ballXf.o, P.ballRadius, cbt, point, normal, depth);
+}
+
+// Adds one triangle's contact with the ball to its manifold.
+template <class WT>
+RSB_HD void addBallTriContact(WT& W, int mesh, int tri, const V3* v, V3 normal, V3 point, float depth, Manifold& man) {
+    ObjRef rMesh = objRef(W, mesh), rBall = objRef(W, OBJ_BALL);
+    int idx = addContact(man, W.pool, mesh, rMesh, OBJ_BALL, rBall, normal, point, depth);
+    if (idx >= 0) {
+        MPoint& cp = man.pt[idx];
+        cp.index1 = tri;
+        cp.special = 1;  // ball + world (Arena.cpp:264-271)
+        adjustInternalEdge(cp, v, W.S->triInfo[W.S->meshes[mesh].triOff + tri]);
+    }
+}
+
 // Ball vs one arena mesh: btConvexConcaveCollisionAlgorithm (swapped: the pair is
-// (mesh, ball)) -> per triangle early-out + btSphereTriangleCollisionAlgorithm.
+// (mesh, ball)), triangle by triangle.
 template <class WT>
 RSB_HD void collideBallMesh(WT& W, int mesh, Manifold& man) {
     const WorldParams& P = *W.P;
     const Body& ball = W.b[0];
-    ObjRef rMesh = objRef(W, mesh), rBall = objRef(W, OBJ_BALL);
     bool found = false;
     if (!cullSkip(W, 0)) {
     V3 amn, amx;
     ballAabb(P, ball.xf, amn, amx);  // convexInTriangleSpace == ball transform (mesh at identity)
-    M3 invB = inverse(ball.xf.b);
     // no triangle of this mesh near the query box: the walk below could not report one
     if ((occMask(*W.S, amn - V3{kOccTol, kOccTol, kOccTol}, amx + V3{kOccTol, kOccTol, kOccTol}) >> mesh) & 1u)
     bvhQueryAabb(*W.S, mesh, amn, amx, [&](int tri) {
         V3 v[3];
         triVerts(*W.S, mesh, tri, v);
         if (!triAabbOverlap(v, amn, amx)) return true;
-        // convex-concave early out (btConvexConcaveCollisionAlgorithm.cpp:100-137)
-        V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
-        float thr = man.cbt + 0.f;
-        for (int side = 0; side < 2; side++) {
-            V3 lp = sphereSupport(invB * tn, P.ballMargin);
-            V3 wp = xfPoint(ball.xf, lp);
-            float dist = dot(tn, v[0]) - dot(tn, wp);
-            if (dist > thr) return true;
-            tn *= -1.f;
-        }
         V3 point, normal;
         float depth;
-        if (sphereTriCollide(v, ball.xf.o, P.ballRadius, man.cbt, point, normal, depth)) {
+        if (ballTriContact(P, ball.xf, man.cbt, v, point, normal, depth)) {
             found = true;
-            int idx = addContact(man, W.pool, mesh, rMesh, OBJ_BALL, rBall, normal, point, depth);
-            if (idx >= 0) {
-                MPoint& cp = man.pt[idx];
-                cp.index1 = tri;
-                cp.special = 1;  // ball + world (Arena.cpp:264-271)
-                adjustInternalEdge(cp, v, W.S->triInfo[W.S->meshes[mesh].triOff + tri]);
-            }
+            addBallTriContact(W, mesh, tri, v, normal, point, depth, man);
         }
         return true;
     });
     }
     cullCheck(W, 0, found);
-    if (man.n) refreshContactPoints(man, rBall.xf, rMesh.xf);
+    if (man.n) refreshContactPoints(man, W.b[0].xf, xfIdentity());
 }
 
 // Ball vs static plane: btConvexPlaneCollisionAlgorithm (swapped pair (plane, ball))
@@ -640,20 +652,50 @@ RSB_HD bool boxTriFar(const Xf& x, V3 he, const V3* v, float limit) {
     return false;
 }
 
+// Whether a triangle that overlaps the box's AABB goes to GJK: the early out on the two sides of
+// its plane (btConvexConcaveCollisionAlgorithm.cpp:100-137), and a reject of triangles
+// separated well beyond the contact distance, for which GJK would find no contact.
+RSB_HD bool boxTriNear(const CarParams& C, const ConvexShape& box, const Xf& childXf, float cbt, const V3* v) {
+    const M3 invB = inverse(childXf.b);
+    V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
+    for (int side = 0; side < 2; side++) {
+        V3 lp = supportVirtual(box, invB * tn);
+        V3 wp = xfPoint(childXf, lp);
+        float dist = dot(tn, v[0]) - dot(tn, wp);
+        if (dist > cbt + 0.f) return false;
+        tn *= -1.f;
+    }
+    return !boxTriFar(childXf, box.he, v, (C.boxMargin + 0.f) + cbt + 0.02f);
+}
+
+// Adds one triangle's contact with car ci's box to its manifold, with the car-world callback and
+// the internal-edge adjustment.
+template <class WT>
+RSB_HD void addBoxTriContact(WT& W, int mesh, int ci, int tri, const V3* v, V3 normal, V3 point, float dist,
+                             Manifold& man) {
+    int carObj = OBJ_CAR0 + ci;
+    ObjRef rMesh = objRef(W, mesh), rCar = objRef(W, carObj);
+    int idx = addContact(man, W.pool, mesh, rMesh, carObj, rCar, normal, point, dist);
+    if (idx >= 0 && carResponds(W, ci)) {
+        MPoint& cp = man.pt[idx];
+        cp.index1 = tri;
+        onCarWorld(W, ci, cp);
+        adjustInternalEdge(cp, v, W.S->triInfo[W.S->meshes[mesh].triOff + tri]);
+    }
+}
+
+RSB_HD float boxMeshMaxDist2(const CarParams& C, float cbt) { return sq((C.boxMargin + 0.f) + cbt); }
+
 // Car box vs one arena mesh: the compound's child algorithm is btConvexConcaveCollisionAlgorithm
 // (btConvexConcaveCollisionAlgorithm.cpp:60-250), each overlapping triangle through
 // btConvexConvexAlgorithm's GJK (btConvexConvexAlgorithm.cpp:268-590).
 template <class WT>
 RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold& man) {
     const CarParams& C = W.P->car;
-    int carObj = OBJ_CAR0 + ci;
-    ObjRef rMesh = objRef(W, mesh), rCar = objRef(W, carObj);
     ConvexShape box = carBoxShape(C);
     V3 amn, amx;
     carBoxAabb(C, childXf, amn, amx);
-    M3 invB = inverse(childXf.b);
-    float maxDist2 = sq((C.boxMargin + 0.f) + man.cbt);
-    bool responds = carResponds(W, ci);
+    float maxDist2 = boxMeshMaxDist2(C, man.cbt);
     bool found = false;
     if (!cullSkip(W, 1 + ci) &&
         ((occMask(*W.S, amn - V3{kOccTol, kOccTol, kOccTol}, amx + V3{kOccTol, kOccTol, kOccTol}) >> mesh) & 1u)) {
@@ -661,34 +703,19 @@ RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold&
         V3 v[3];
         triVerts(*W.S, mesh, tri, v);
         if (!triAabbOverlap(v, amn, amx)) return true;
-        V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
-        for (int side = 0; side < 2; side++) {
-            V3 lp = supportVirtual(box, invB * tn);
-            V3 wp = xfPoint(childXf, lp);
-            float dist = dot(tn, v[0]) - dot(tn, wp);
-            if (dist > man.cbt + 0.f) return true;
-            tn *= -1.f;
-        }
-        // separated well beyond the contact distance: GJK would find no contact
-        if (boxTriFar(childXf, box.he, v, (C.boxMargin + 0.f) + man.cbt + 0.02f)) return true;
+        if (!boxTriNear(C, box, childXf, man.cbt, v)) return true;
         ConvexShape triS = makeTri(v, 0.f);
         GjkOut g = gjkPairDetector(W.epa, box, childXf, triS, xfIdentity(), maxDist2);
         if (g.overflow) W.status |= WS_EPA_OVERFLOW;
         if (g.has) {
             found = true;
-            int idx = addContact(man, W.pool, mesh, rMesh, carObj, rCar, g.normal, g.point, g.dist);
-            if (idx >= 0 && responds) {
-                MPoint& cp = man.pt[idx];
-                cp.index1 = tri;
-                onCarWorld(W, ci, cp);
-                adjustInternalEdge(cp, v, W.S->triInfo[W.S->meshes[mesh].triOff + tri]);
-            }
+            addBoxTriContact(W, mesh, ci, tri, v, g.normal, g.point, g.dist, man);
         }
         return true;
     });
     }
     cullCheck(W, 1 + ci, found);
-    if (man.n) refreshContactPoints(man, rCar.xf, rMesh.xf);
+    if (man.n) refreshContactPoints(man, W.b[1 + ci].xf, xfIdentity());
 }
 
 // Car box vs a static plane: btConvexPlaneCollisionAlgorithm owning its manifold

@@ -191,17 +191,17 @@ static rsb_status cudaFail(rsb_handle* h, const char* what, cudaError_t e) {
 // size.
 typedef void (*StepFn)(EngineView, StepTemp);
 struct StepVariant {
-    StepFn ray, contact, solve;
+    StepFn ray, triangle, solve;
     int minBlocks;
     bool persistent;
 };
 static const StepVariant kStepVariants[] = {
-    {heavyRayKernel<1>, contactKernel<1>, solveKernel<1>, 1, false},
-    {heavyRayKernel<3>, contactKernel<3>, solveKernel<3>, 3, false},
-    {heavyRayKernel<4>, contactKernel<4>, solveKernel<4>, 4, false},
-    {heavyRayKernel<1>, contactKernel<1>, solveKernel<1>, 1, true},
-    {heavyRayKernel<3>, contactKernel<3>, solveKernel<3>, 3, true},
-    {heavyRayKernel<4>, contactKernel<4>, solveKernel<4>, 4, true}};
+    {heavyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, false},
+    {heavyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, false},
+    {heavyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, false},
+    {heavyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, true},
+    {heavyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, true},
+    {heavyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, true}};
 constexpr int kNumStepVariants = sizeof(kStepVariants) / sizeof(kStepVariants[0]);
 static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
@@ -461,6 +461,7 @@ static bool allocStep(rsb_handle* h) {
         off += count * sizeof(*p);
     };
     T.blockCap = (uint32_t)(MAX_BLOCKS * N);
+    T.candCap = (uint32_t)(CAP_CANDIDATES * N);
     for (int pass = 0; pass < 2; pass++) {
         off = 0;
         place(T.rayObj, R);
@@ -476,6 +477,11 @@ static bool allocStep(rsb_handle* h) {
         place(T.results, (size_t)CAP_RESULTS * N);
         place(T.blocks, (size_t)T.blockCap * MAX_POINTS);
         place(T.solveQ, N);
+        place(T.first, (size_t)CAP_RESULTS * N);
+        place(T.cand, T.candCap);
+        place(T.out, T.candCap);
+        place(T.deepQ, (size_t)CAP_RESULTS * N + T.candCap);
+        place(T.combineQ, (size_t)CAP_RESULTS * N);
         if (pass == 0 && cudaMalloc((void**)&h->dStep, off) != cudaSuccess) return false;
     }
     T.count = h->dWork;
@@ -630,9 +636,10 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
         // make the per-thread stack limit cover the largest (the default limit is 1 KB), and give
         // the L1 its largest share in those that use no shared memory to speak of
         size_t need = 0;
-        std::vector<const void*> fns{(const void*)predictBallKernel};
+        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)deepKernel,
+                                     (const void*)combineKernel};
         for (const StepVariant& v : kStepVariants)
-            for (StepFn f : {v.ray, v.contact, v.solve}) fns.push_back((const void*)f);
+            for (StepFn f : {v.ray, v.triangle, v.solve}) fns.push_back((const void*)f);
         for (const void* f : fns) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, f) != cudaSuccess)
@@ -735,7 +742,9 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
         return (int)g;
     };
     const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars);
-    const int contactGrid = grid(sv.contact, (int64_t)h->numCars + h->N);
+    const int pairGrid = grid(findKernel, (int64_t)h->numCars + h->N);
+    const int triGrid = grid(sv.triangle, (int64_t)h->numCars + h->N);
+    const int deepGrid = grid(deepKernel, h->N / 8), combineGrid = grid(combineKernel, h->numCars / 2 + h->N);
     const int solveGrid = grid(sv.solve, h->N);
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
@@ -744,7 +753,10 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
             sv.ray<<<rayGrid, block, 0, st>>>(D, T);
         }
         bodyKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
-        sv.contact<<<contactGrid, block, 0, st>>>(D, T);
+        findKernel<<<pairGrid, block, 0, st>>>(D, T);
+        sv.triangle<<<triGrid, block, 0, st>>>(D, T);
+        deepKernel<<<deepGrid, block, 0, st>>>(D, T);
+        combineKernel<<<combineGrid, block, 0, st>>>(D, T);
         sv.solve<<<solveGrid, block, 0, st>>>(D, T);
         finishKernel<<<groups, bodyThreads, 0, st>>>(D, T);
     }

@@ -136,32 +136,53 @@ __global__ void __launch_bounds__(BODY_THREADS) bodyKernel(const __grid_constant
     blockStats(D, st);
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) contactKernel(const __grid_constant__ EngineView D,
-                                                           const __grid_constant__ StepTemp T) {
-    EpaWork epa;
-    PhaseStats st{0, 0, 0, 0};
-    uint32_t n[NUM_TASK_TYPES], tiles = 0;
-    for (int k = 0; k < NUM_TASK_TYPES; k++) {
-        n[k] = T.count[QC_CARMESH + k];
-        tiles += (n[k] + 31u) / 32u;
-    }
-    // a warp takes 32 pairs of one type
+// Warps over the items of several queues, 32 of one queue at a time: fn(queue, item).
+template <int NQ, class F>
+RSB_D void forTiles(const uint32_t* n, F&& fn) {
+    uint32_t tiles = 0;
+    for (int k = 0; k < NQ; k++) tiles += (n[k] + 31u) / 32u;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
         uint32_t q = tile;
-        int type = 0;
-        while (q >= (n[type] + 31u) / 32u) q -= (n[type++] + 31u) / 32u;
+        int k = 0;
+        while (q >= (n[k] + 31u) / 32u) q -= (n[k++] + 31u) / 32u;
         const uint32_t i = q * 32u + (threadIdx.x & 31u);
-        if (i >= n[type]) continue;
-        const uint32_t res = (uint32_t)resultBase(QC_CARMESH + type) * (uint32_t)D.N + i;
-        switch (QC_CARMESH + type) {
-            case QC_CARMESH: carMeshPhase(D, T, res, &epa, st); break;
-            case QC_BALLMESH: ballMeshPhase(D, T, res, st); break;
-            case QC_CARBALL: carBallPhase(D, T, res, &epa); break;
-            default: carCarPhase(D, T, res); break;
-        }
+        if (i < n[k]) fn(k, i);
     }
+}
+
+__global__ void __launch_bounds__(128) findKernel(const __grid_constant__ EngineView D,
+                                                  const __grid_constant__ StepTemp T) {
+    const uint32_t n[3] = {T.count[QC_CARMESH], T.count[QC_BALLMESH], T.count[QC_CARBALL]};
+    forTiles<3>(n, [&](int k, uint32_t i) {
+        findPhase(D, T, (uint32_t)resultBase(QC_CARMESH + k) * (uint32_t)D.N + i);
+    });
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constant__ EngineView D,
+                                                            const __grid_constant__ StepTemp T) {
+    const uint32_t n[2] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR]};
+    forTiles<2>(n, [&](int k, uint32_t i) {
+        if (k == 0) trianglePhase(D, T, i);
+        else carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
+    });
+}
+
+__global__ void __launch_bounds__(128) deepKernel(const __grid_constant__ EngineView D,
+                                                  const __grid_constant__ StepTemp T) {
+    EpaWork epa;
+    PhaseStats st{0, 0, 0, 0};
+    const uint32_t n[1] = {T.count[QC_DEEP]};
+    forTiles<1>(n, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
+    blockStats(D, st);
+}
+
+__global__ void __launch_bounds__(128) combineKernel(const __grid_constant__ EngineView D,
+                                                     const __grid_constant__ StepTemp T) {
+    PhaseStats st{0, 0, 0, 0};
+    const uint32_t n[1] = {T.count[QC_COMBINE]};
+    forTiles<1>(n, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
     blockStats(D, st);
 }
 

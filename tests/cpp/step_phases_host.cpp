@@ -8,9 +8,11 @@
 
 extern "C" {
 
-// `ticks` ticks of the handle's arenas through the phases.  cull: a body mask per arena, or null.
+// `ticks` ticks of the handle's arenas through the phases.  cull: a body mask per arena, or null;
+// cand_cap: room for triangle candidates (-1: as the engine has).
 // Returns the number of items that went through each queue in counts[QC_WORDS].
-int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int64_t* counts, uint64_t* stats) {
+int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32_t cand_cap, int64_t* counts,
+                             uint64_t* stats) {
     const size_t N = h->N, B = MAX_BODIES * N, R = (size_t)4 * MAX_CARS * N;
     EngineView D;
     D.S = h->S.view;
@@ -50,6 +52,15 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int64
     T.blocks = blocks.data();
     T.blockCap = (uint32_t)(MAX_BLOCKS * N);
     T.solveQ = solveQ.data();
+    T.candCap = cand_cap < 0 ? (uint32_t)(CAP_CANDIDATES * N) : (uint32_t)cand_cap;
+    std::vector<uint32_t> first(CAP_RESULTS * N), deepQ(CAP_RESULTS * N + T.candCap), combineQ(CAP_RESULTS * N);
+    std::vector<Candidate> cand(T.candCap);
+    std::vector<CandidateOut> candOut(T.candCap);
+    T.first = first.data();
+    T.cand = cand.data();
+    T.out = candOut.data();
+    T.deepQ = deepQ.data();
+    T.combineQ = combineQ.data();
     std::unique_ptr<EpaWork> epa(new EpaWork());
     std::unique_ptr<BodyShared> sh(new BodyShared());
     std::unique_ptr<FinishShared> fs(new FinishShared());
@@ -124,12 +135,13 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int64
             const int type = QC_CARMESH + k;
             for (uint32_t i = T.count[type]; i-- > 0;) {
                 const uint32_t res = (uint32_t)resultBase(type) * (uint32_t)D.N + i;
-                if (type == QC_CARMESH) carMeshPhase(D, T, res, epa.get(), st);
-                else if (type == QC_BALLMESH) ballMeshPhase(D, T, res, st);
-                else if (type == QC_CARBALL) carBallPhase(D, T, res, epa.get());
-                else carCarPhase(D, T, res);
+                if (type == QC_CARCAR) carCarPhase(D, T, res);
+                else findPhase(D, T, res);
             }
         }
+        for (uint32_t i = std::min(T.count[QC_TRI], T.candCap); i-- > 0;) trianglePhase(D, T, i);
+        for (uint32_t i = T.count[QC_DEEP]; i-- > 0;) deepPhase(D, T, T.deepQ[i], epa.get(), st);
+        for (uint32_t i = T.count[QC_COMBINE]; i-- > 0;) combinePhase(D, T, T.combineQ[i], st);
         for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], st);
         // finish
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {

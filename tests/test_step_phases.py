@@ -18,7 +18,8 @@ from gpu_util import random_balls, random_cars, random_controls
 from host_util import ARENA_BUILD
 
 SRC = os.path.join(ROOT, "tests", "cpp", "step_phases_host.cpp")
-QUEUES = ("rays", "car-mesh", "ball-mesh", "car-ball", "car-car", "planes", "blocks", "islands")
+QUEUES = ("rays", "car-mesh", "ball-mesh", "car-ball", "car-car", "planes", "blocks", "islands", "triangles", "deep",
+          "combine")
 
 
 @pytest.fixture(scope="module")
@@ -36,7 +37,7 @@ def host(pkg, tmp_path_factory):
     lib = pkg.rsb.load_library(out)
     lib.rsb_host_records_differ.restype = C.c_int64
     lib.rsb_host_records_differ.argtypes = [C.c_void_p, C.c_void_p]
-    lib.rsb_host_step_phases.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.rsb_host_step_phases.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
     return lib, cases._arena()
 
 
@@ -77,7 +78,7 @@ def start(rsb, b, kind, seed):
     return cars, balls
 
 
-def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=None):
+def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=None, cand_cap=-1):
     rsb, (lib, arena) = pkg.rsb, host
     x, y = (rsb.Batch(lib, n, team_sizes=teams, meshes_path=arena, seed=seed) for _ in range(2))
     cars, balls = start(rsb, x, kind, seed)
@@ -96,8 +97,8 @@ def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=No
             if b.num_cars:
                 b.set_controls(ctl)
         x.step(ticks)
-        st = lib.rsb_host_step_phases(y._h, ticks, mask.ctypes.data if cull else None, counts.ctypes.data,
-                                      stats.ctypes.data)
+        st = lib.rsb_host_step_phases(y._h, ticks, mask.ctypes.data if cull else None, cand_cap,
+                                      counts.ctypes.data, stats.ctypes.data)
         assert st == 0
         d = lib.rsb_host_records_differ(x._h, y._h)
         assert d == -1, f"step {k}: plane {('ball', 'car', 'pad', 'arena')[d >> 40]}, word {(d & ((1 << 40) - 1)) // n}"
@@ -113,7 +114,7 @@ def test_phases_match_the_one_thread_tick(pkg, host, kind, ticks):
         seen = {q: seen[q] + got[q] for q in QUEUES}
     assert seen["rays"] and seen["planes"] and seen["islands"]
     if kind == "walls":
-        assert seen["car-mesh"] and seen["ball-mesh"]
+        assert seen["car-mesh"] and seen["ball-mesh"] and seen["triangles"] and seen["deep"] and seen["combine"]
     if kind in ("heap", "stack"):
         assert seen["car-car"]
     if kind == "heap":
@@ -123,6 +124,14 @@ def test_phases_match_the_one_thread_tick(pkg, host, kind, ticks):
 @pytest.mark.parametrize("n", [1, 31, 32, 33])
 def test_batch_sizes_around_a_block(pkg, host, n):
     compare(pkg, host, n, np.array([3, 2, 1] * 11, np.int32)[:n], "heap", 31, 8, 12)
+
+
+@pytest.mark.parametrize("cand_cap", [0, 3, 40])
+def test_more_triangles_than_there_is_room_for(pkg, host, cand_cap):
+    """Pairs that find the candidate list full are taken on one thread, with the same results."""
+    for kind in ("walls", "heap"):
+        got = compare(pkg, host, 64, np.full(64, 3, np.int32), kind, 71, 8, 12, cand_cap=cand_cap)
+        assert got["triangles"] > cand_cap
 
 
 def test_empty_arenas(pkg, host):
