@@ -52,9 +52,22 @@ struct SubSimplexResult {
     RSB_HD bool isValid() const { return bc[0] >= 0.f && bc[1] >= 0.f && bc[2] >= 0.f && bc[3] >= 0.f; }
 };
 
+// Element i of a small array by selection: with every index a compile-time constant the array
+// stays in registers (an array indexed at run time lives in thread-local memory).
+template <class T>
+RSB_HD T pickOf4(const T* a, int i) {
+    return i == 0 ? a[0] : (i == 1 ? a[1] : (i == 2 ? a[2] : a[3]));
+}
+template <class T>
+RSB_HD void putOf4(T* a, int i, const T& v) {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k == i) a[k] = v;
+}
+
 struct VoronoiSimplex {
     int n;
-    V3 W[5], P[5], Q[5];
+    V3 W[4], P[4], Q[4];  // a fifth vertex (n = 5 ends the query as invalid) is not kept
     V3 lastW;
     bool needsUpdate, cachedValid;
     V3 cP1, cP2, cV;
@@ -69,9 +82,9 @@ struct VoronoiSimplex {
     }
     RSB_HD void removeVertex(int i) {
         n--;
-        W[i] = W[n];
-        P[i] = P[n];
-        Q[i] = Q[n];
+        W[i] = pickOf4(W, n);
+        P[i] = pickOf4(P, n);
+        Q[i] = pickOf4(Q, n);
     }
     RSB_HD void reduce(uint32_t used) {
         if (n >= 4 && !(used & 8)) removeVertex(3);
@@ -82,15 +95,16 @@ struct VoronoiSimplex {
     RSB_HD void addVertex(V3 w, V3 p, V3 q) {
         lastW = w;
         needsUpdate = true;
-        W[n] = w;
-        P[n] = p;
-        Q[n] = q;
+        putOf4(W, n, w);
+        putOf4(P, n, p);
+        putOf4(Q, n, q);
         n++;
     }
     RSB_HD bool inSimplex(V3 w) const {
         bool found = false;
-        for (int i = 0; i < n; i++)
-            if (length2(w - W[i]) <= 0.0001f) { found = true; break; }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (i < n && length2(w - W[i]) <= 0.0001f) found = true;
         if (w == lastW) return true;
         return found;
     }

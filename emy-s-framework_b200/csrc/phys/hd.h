@@ -13,10 +13,12 @@
 #define RSB_HD __host__ __device__ __forceinline__
 #define RSB_D __device__ __forceinline__
 #define RSB_CONST __constant__
+#define RSB_HD_COLD inline __host__ __device__ __noinline__
 #else
 #define RSB_HD inline
 #define RSB_D inline
 #define RSB_CONST
+#define RSB_HD_COLD inline
 #endif
 
 #include <math.h>

@@ -176,6 +176,70 @@ RSB_HD bool rayVsMeshesVox(const ArenaStatic& S, uint32_t meshes, V3 src, V3 dst
     return rayVsMeshesVoxSerial(S, meshes, src, dst, tol, hit, cand);
 }
 
+// The same closest hit without the sorted list: of the candidates that the segment hits inside
+// their leaves' boxes the one with the smallest fraction, the first in key order among equal
+// ones, is the hit that testing them in key order keeps.  The triangle test comes first, since
+// most candidates fail it.  Returns false, with `hit` untouched, when the segment leaves the grid.
+RSB_HD bool rayVsMeshesNearest(const ArenaStatic& S, uint32_t meshes, V3 src, V3 dst, float tol, RayHit& hit) {
+    const V3 mn = vmin(src, dst) - V3{tol, tol, tol}, mx = vmax(src, dst) + V3{tol, tol, tol};
+    const float f = S.occInvCell;
+    const int x0 = (int)floorf((mn.x - S.occMin.x) * f), x1 = (int)floorf((mx.x - S.occMin.x) * f);
+    const int y0 = (int)floorf((mn.y - S.occMin.y) * f), y1 = (int)floorf((mx.y - S.occMin.y) * f);
+    const int z0 = (int)floorf((mn.z - S.occMin.z) * f), z1 = (int)floorf((mx.z - S.occMin.z) * f);
+    if (!(x0 >= 0 && y0 >= 0 && z0 >= 0 && x1 < S.occX && y1 < S.occY && z1 < S.occZ)) return false;
+    uint32_t bestKey = 0;
+    float best = hit.fraction;
+    bool flip = false;
+    for (int x = x0; x <= x1; x++)
+        for (int y = y0; y <= y1; y++) {
+            // the lists of a column of voxels lie one after another
+            const int v = (x * S.occY + y) * S.occZ;
+            for (uint32_t i = S.voxOff[v + z0], e = S.voxOff[v + z1 + 1]; i < e; i++) {
+                const uint32_t key = S.voxList[i];
+                const int m = (int)(key >> 22);
+                if (!((meshes >> m) & 1u)) continue;
+                V3 t[3];
+                triVerts(S, m, (int)(key & 0x3FFu), t);
+                const V3 n = cross(t[1] - t[0], t[2] - t[0]);
+                const float dist = dot(t[0], n);
+                const float da = dot(n, src) - dist, db = dot(n, dst) - dist;
+                if (da * db >= 0.f) continue;
+                const float distance = da / (da - db);
+                if (!(distance < best || (distance == best && key < bestKey))) continue;
+                const float edgeTol = length2(n) * -0.0001f;
+                const V3 point = src * (1.f - distance) + dst * distance;
+                const V3 v0p = t[0] - point, v1p = t[1] - point, v2p = t[2] - point;
+                if (!(dot(cross(v0p, v1p), n) >= edgeTol && dot(cross(v1p, v2p), n) >= edgeTol &&
+                      dot(cross(v2p, v0p), n) >= edgeTol))
+                    continue;
+                // the leaf's own tests (bvhQueryRay)
+                const MeshDesc& md = S.meshes[m];
+                const BvhNode nd = S.nodes[md.nodeOff + (int)((key >> 10) & 0xFFFu)];
+                const RaySetup R = raySetup(src, dst);
+                uint16_t qmn[3], qmx[3];
+                bvhQuantizeClamp(md, R.rmn, 0, qmn);
+                bvhQuantizeClamp(md, R.rmx, 1, qmx);
+                if (!qOverlap(qmn, qmx, nd.qmin, nd.qmax)) continue;
+                V3 bounds[2];
+                bounds[0] = bvhUnquantize(md, nd.qmin);
+                bounds[1] = bvhUnquantize(md, nd.qmax);
+                float param = 1.f;
+                if (!rayAabb2(src, R.inv, R.sign, bounds, param, 0.f, R.lambdaMax)) continue;
+                best = distance;
+                bestKey = key;
+                flip = da <= 0.f;
+                hit.obj = m;
+                hit.normal = n;
+            }
+        }
+    if (hit.obj >= 0) {
+        const V3 n = normalized(hit.normal);
+        hit.normal = flip ? -n : n;
+        hit.fraction = best;
+    }
+    return true;
+}
+
 RSB_HD void rayVsPlane(const ArenaStatic& S, int plane, V3 fromW, V3 toW, RayHit& hit) {
     V3 origin = S.planeOrigin[plane - MAX_MESHES];
     V3 n = S.planeNormal[plane - MAX_MESHES];

@@ -53,7 +53,7 @@ RSB_HD int dynPair(int lo, int hi) { return lo * (2 * MAX_BODIES - lo - 1) / 2 +
 
 // Queue counters.
 enum : int {
-    QC_RAY = 0, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_TRI, QC_DEEP, QC_COMBINE,
+    QC_RAY = 0, QC_BODYRAY, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_TRI, QC_DEEP, QC_COMBINE,
     QC_WORDS
 };
 constexpr int NUM_TASK_TYPES = 4;  // QC_CARMESH .. QC_CARCAR
@@ -117,7 +117,7 @@ struct StepTemp {
     float* cache;        // velocity impulse caches: 3 planes of [MAX_BODIES][N]
     uint32_t* dynRes;    // result of each dynamic pair: [NUM_DYN_PAIRS][N]
     uint32_t* count;     // QC_WORDS counters
-    uint32_t* rayQ;      // [4 * MAX_CARS * N]
+    uint32_t* rayQ;      // rays near meshes [4 * MAX_CARS * N], then as many places for the others
     PairTask* tasks;     // per type, [cap * N], at resultBase(type) * N
     PairResult* results;
     MPoint* blocks;      // [MAX_BLOCKS * N][MAX_POINTS]
@@ -360,26 +360,40 @@ RSB_HD bool rayCar(const EngineView& D, int a, int s, Xf& xf, bool& culled) {
     return true;
 }
 
-// Wheel w of car s: casts the ray if only planes can be near, else returns true (queue it).
-// `near(i, j, k)`: whether a body other than the car is registered around that cell.
+// What the ray phase leaves in rayObj of a queued ray: the meshes near it (16 bits), the bodies
+// registered around its cell (7 bits), or RAY_ANY for one that castRay takes as a whole.
+constexpr int RAY_BODIES_SHIFT = MAX_MESHES;
+constexpr uint32_t RAY_ANY = 1u << 30;
+enum RayClass : int { RAY_DONE = 0, RAY_MESHES, RAY_BODIES };
+
+// Wheel w of car s: casts the ray if only planes can be near, else says which queue it goes to.
+// `near(i, j, k)`: the bodies registered around that cell, the car itself among them.
 template <class NearF>
-RSB_HD bool rayPhase(const EngineView& D, const StepTemp& T, int a, int s, int w, const Xf& xf, bool culled,
-                     NearF&& near, PhaseStats& st) {
+RSB_HD RayClass rayPhase(const EngineView& D, const StepTemp& T, int a, int s, int w, const Xf& xf, bool culled,
+                         NearF&& near, PhaseStats& st) {
     const ArenaStatic& S = D.S;
     Body cb;
     WheelTick wt;
     V3 from, to;
     cb.xf = xf;
     wheelSegment(D.P.car, cb, wt, w, from, to);
-    if (culled || !(dist2(from, to) < S.bp.cellSize * S.bp.cellSize)) return true;
+    const size_t r = rayIdx(D, a, s, w);
+    if (culled || !(dist2(from, to) < S.bp.cellSize * S.bp.cellSize)) {
+        T.rayObj[r] = (int32_t)RAY_ANY;
+        return RAY_BODIES;
+    }
     int i, j, k;
     bpCellIndices(S.bp, from, i, j, k);
     uint32_t mask = S.bpCells[i * S.bp.cellsY * S.bp.cellsZ + j * S.bp.cellsZ + k];
-    if (near(i, j, k)) return true;
-    const uint32_t kMeshBits = (1u << MAX_MESHES) - 1u;
-    if (mask & kMeshBits) {
+    const uint32_t bodies = near(i, j, k), kMeshBits = (1u << MAX_MESHES) - 1u;
+    uint32_t meshes = mask & kMeshBits;
+    if (meshes) {
         const V3 tolv{kOccTol, kOccTol, kOccTol};
-        if (mask & kMeshBits & occMask(S, vmin(from, to) - tolv, vmax(from, to) + tolv)) return true;
+        meshes &= occMask(S, vmin(from, to) - tolv, vmax(from, to) + tolv);
+    }
+    if (meshes || (bodies & ~(2u << s))) {
+        T.rayObj[r] = (int32_t)(meshes | (bodies << RAY_BODIES_SHIFT));
+        return meshes ? RAY_MESHES : RAY_BODIES;
     }
     RayHit hit;
     hit.fraction = 1.f;
@@ -390,21 +404,14 @@ RSB_HD bool rayPhase(const EngineView& D, const StepTemp& T, int a, int s, int w
         st.nStatic++;
         rayVsPlane(S, MAX_MESHES + lowestBit(mask), from, to, hit);
     }
-    storeRay(D, T, rayIdx(D, a, s, w), hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
-    return false;
+    storeRay(D, T, r, hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
+    return RAY_DONE;
 }
 
-// A queued ray: castRay over everything around it.
-RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
-    const int a = (int)(r % (uint32_t)D.N), q = (int)(r / (uint32_t)D.N), s = q % MAX_CARS, w = q / MAX_CARS;
-    Xf xf;
-    bool culled;
-    if (!rayCar(D, a, s, xf, culled)) return;  // never queued
-    Body cb;
-    WheelTick wt;
-    V3 from, to;
-    cb.xf = xf;
-    wheelSegment(D.P.car, cb, wt, w, from, to);
+// A ray of any kind, by castRay itself: culled bodies, and segments that are longer than a
+// broadphase cell or not finite.
+RSB_HD_COLD int anyRay(const EngineView& D, int a, int s, bool culled, V3 from, V3 to, V3& hn, float& frac,
+                       PhaseStats& st) {
     RayWorld W;
     W.S = &D.S;
     W.P = &D.P;
@@ -422,14 +429,98 @@ RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, Ph
                    j = (int)bodyWord(D, a, e, RSB_PW(CarP, cj));
                    k = (int)bodyWord(D, a, e, RSB_PW(CarP, ck));
                });
-    V3 hp, hn = v3zero();
-    float frac = 1.f;
+    V3 hp;
     const int obj = castRay(W, from, to, OBJ_CAR0 + s, hp, hn, frac);
-    storeRay(D, T, r, obj, frac, hn);
     st.nStatic += W.nStatic;
     st.nCulled += W.nCulled;
     st.nMissed += W.nMissed;
     if (W.cullMissed) phaseAtomicOr(arenaStatus(D, a), W.cullMissed);
+    return obj;
+}
+
+// Bodies of `cand` in registration order, one call after another: a proxy whose stamp equals
+// the one just visited is passed over (the broadphase's rule).  -1 at the end.
+struct RegWalk {
+    uint32_t cand, last;
+    bool first;
+    template <class StampF>
+    RSB_HD int next(StampF&& stamp) {
+        while (cand) {
+            int pick = -1;
+            uint32_t ps = 0;
+            for (uint32_t m = cand; m; m &= m - 1u) {
+                const int e = lowestBit(m);
+                const uint32_t s = stamp(e);
+                if (pick < 0 || s < ps) {
+                    pick = e;
+                    ps = s;
+                }
+            }
+            cand &= ~(1u << pick);
+            if (!first && ps <= last) continue;
+            first = false;
+            last = ps;
+            return pick;
+        }
+        return -1;
+    }
+};
+
+// A queued ray: meshes, then planes, then bodies in registration order, as castRay tests them.
+RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
+    const int a = (int)(r % (uint32_t)D.N), q = (int)(r / (uint32_t)D.N), s = q % MAX_CARS, w = q / MAX_CARS;
+    const ArenaStatic& S = D.S;
+    Xf xf;
+    bool culled;
+    if (!rayCar(D, a, s, xf, culled)) return;  // never queued
+    Body cb;
+    WheelTick wt;
+    V3 from, to;
+    cb.xf = xf;
+    wheelSegment(D.P.car, cb, wt, w, from, to);
+    const uint32_t code = (uint32_t)T.rayObj[r], meshes = code & ((1u << MAX_MESHES) - 1u);
+    RayHit hit;
+    hit.fraction = 1.f;
+    hit.obj = -1;
+    hit.normal = v3zero();
+    bool any = code == RAY_ANY;
+    if (!any && meshes) any = !rayVsMeshesNearest(S, meshes, from, to, kOccTol, hit);
+    if (any) {
+        V3 hn = v3zero();
+        float frac = 1.f;
+        const int obj = anyRay(D, a, s, culled, from, to, hn, frac, st);
+        storeRay(D, T, r, obj, frac, hn);
+        return;
+    }
+    st.nStatic += (uint32_t)bitCount(meshes);
+    int i, j, k;
+    bpCellIndices(S.bp, from, i, j, k);
+    for (uint32_t m = S.bpCells[i * S.bp.cellsY * S.bp.cellsZ + j * S.bp.cellsZ + k] >> MAX_MESHES; m; m &= m - 1u) {
+        if (hit.fraction == 0.f) break;
+        st.nStatic++;
+        rayVsPlane(S, MAX_MESHES + lowestBit(m), from, to, hit);
+    }
+    RegWalk walk{code >> RAY_BODIES_SHIFT, 0u, true};
+    if (walk.cand & ~(2u << s)) {
+        const RayBodies bodies{&D, a, s, arenaTickCount(D, a)};
+        while (true) {
+            const int b = walk.next([&](int e) { return bodyWord(D, a, e, RSB_PW(CarP, regStamp)); });
+            if (b < 0) break;
+            if (b == 1 + s) continue;
+            const Xf bx = bodies[b].xf;
+            const ConvexShape sh = b == 0 ? makeSphere(D.P.ballRadius) : carBoxShape(D.P.car);
+            float frac;
+            V3 n;
+            if (subsimplexCast(from, to, sh, b == 0 ? bx : carChildXf(D.P.car, bx), frac, n) && length2(n) > 0.0001f &&
+                frac < hit.fraction) {
+                hit.fraction = frac;
+                hit.obj = OBJ_BALL + b;
+                hit.normal = normalized(n);
+            }
+        }
+        if (hit.obj >= OBJ_BALL && bodies[hit.obj - OBJ_BALL].noResp) hit.obj = -1;
+    }
+    storeRay(D, T, r, hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
 }
 
 // ------------------------------------------------------------------ bodies
@@ -716,30 +807,15 @@ RSB_HD void bodyPick(const EngineView& D, BodyThread& t, BodyShared& sh) {
             const int i = sh.cell[e][0][la], j = sh.cell[e][1][la], k = sh.cell[e][2][la];
             return ci >= i - 1 && ci <= i + 1 && cj >= j - 1 && cj <= j + 1 && ck >= k - 1 && ck <= k + 1;
         };
-        uint32_t cand = 0;
+        uint32_t cand = 0, n = 0;
         for (int e = 0; e < t.nb; e++) cand |= near(e) ? 1u << e : 0u;
-        // in registration order; a proxy whose stamp equals the one just visited is passed over
         if (cand & (cand - 1u)) {
-            uint32_t last = 0, n = 0;
-            bool first = true;
-            while (cand) {
-                int pick = -1;
-                uint32_t ps = 0;
-                for (int e = 0; e < t.nb; e++) {
-                    if (!((cand >> e) & 1u)) continue;
-                    const uint32_t st = sh.stamp[e][la];
-                    if (pick < 0 || st < ps) {
-                        pick = e;
-                        ps = st;
-                    }
-                }
-                cand &= ~(1u << pick);
-                if (!first && ps <= last) continue;
-                first = false;
-                last = ps;
-                if (pick == t.b) continue;
-                if (aabbOverlap(b.bpMin, b.bpMax, sharedV3(sh.box[pick], 0, la), sharedV3(sh.box[pick], 3, la)))
-                    t.dyn |= (uint32_t)pick << (3 * n++);
+            RegWalk walk{cand, 0u, true};
+            while (true) {
+                const int e = walk.next([&](int x) { return sh.stamp[x][la]; });
+                if (e < 0) break;
+                if (e != t.b && aabbOverlap(b.bpMin, b.bpMax, sharedV3(sh.box[e], 0, la), sharedV3(sh.box[e], 3, la)))
+                    t.dyn |= (uint32_t)e << (3 * n++);
             }
             t.dyn |= n << 24;
         }

@@ -207,6 +207,13 @@ static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
 // Resident warps per SM of a persistent launch (0 = as many as fit).
 static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
+// Warps per SM of the wide queue grids.  Few items per warp finish sooner, but a thread's local
+// memory shares its cache lines with its warp's other lanes, so the kernels that use much of it
+// lose by spreading.  Measured with 4 / 8 / 16 / 32 / 64, us per tick, 3v3 x 65,536 after 17 env
+// steps: heavy rays 180 / 125 / 111 / 104 / 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles
+// 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 / 61 / 74), find 202 with 32 items to every warp and 107
+// with 64, deep 214 and 141, combine 113 and 102 (16), islands 234 and 885 (64).
+constexpr int kRayWarps = 16, kFindWarps = 64, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
 
 // xorshift32 draw in [0, 1] and range of the reference's state ring (CudaEnvSet.cpp:608-617)
@@ -472,7 +479,7 @@ static bool allocStep(rsb_handle* h) {
         place(T.box, 6 * B);
         place(T.cache, 3 * B);
         place(T.dynRes, (size_t)NUM_DYN_PAIRS * N);
-        place(T.rayQ, R);
+        place(T.rayQ, 2 * R);
         place(T.tasks, (size_t)CAP_RESULTS * N);
         place(T.results, (size_t)CAP_RESULTS * N);
         place(T.blocks, (size_t)T.blockCap * MAX_POINTS);
@@ -730,22 +737,25 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     const StepVariant& sv = kStepVariants[v];
     const StepTemp& T = h->step;
     const int block = kStepBlocks[b], groups = (h->N + PHASE_ARENAS - 1) / PHASE_ARENAS;
-    // blocks of a queue kernel for about `items` items
-    auto grid = [&](StepFn f, int64_t items) -> int {
-        int64_t g = std::max<int64_t>(1, (items + block - 1) / block);
+    // A queue kernel's items are counted on the device only.  The wide grid gives each of up to
+    // `items` items a warp of its own, to `warpsPerSm` warps per SM in all; the persistent one is
+    // as large as fits at once (or as the residency asks).
+    auto grid = [&](StepFn f, int64_t items, int warpsPerSm) -> int {
+        const int warps = block / 32;
+        int64_t g = std::min<int64_t>(items, (int64_t)warpsPerSm * h->smCount);
         if (sv.persistent) {
             int perSm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, f, block, 0) != cudaSuccess) perSm = 1;
-            if (kStepResidency[residency] > 0) perSm = std::min(perSm, std::max(1, kStepResidency[residency] * 32 / block));
-            g = std::min<int64_t>(g, (int64_t)std::max(1, perSm) * h->smCount);
+            if (kStepResidency[residency] > 0) perSm = std::min(perSm, std::max(1, kStepResidency[residency] / warps));
+            g = std::min<int64_t>(g, (int64_t)std::max(1, perSm) * h->smCount * warps);
         }
-        return (int)g;
+        return (int)std::max<int64_t>(1, (g + warps - 1) / warps);
     };
-    const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars);
-    const int pairGrid = grid(findKernel, (int64_t)h->numCars + h->N);
-    const int triGrid = grid(sv.triangle, (int64_t)h->numCars + h->N);
-    const int deepGrid = grid(deepKernel, h->N / 8), combineGrid = grid(combineKernel, h->numCars / 2 + h->N);
-    const int solveGrid = grid(sv.solve, h->N);
+    const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars, kRayWarps);
+    const int pairGrid = grid(findKernel, 2 * ((int64_t)h->numCars + h->N), kFindWarps);
+    const int triGrid = grid(sv.triangle, 4 * ((int64_t)h->numCars + h->N), kTriangleWarps);
+    const int deepGrid = grid(deepKernel, h->numCars + h->N, kDeepWarps), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
+    const int solveGrid = grid(sv.solve, h->N, kSolveWarps);
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
         if (h->maxCars > 0) {

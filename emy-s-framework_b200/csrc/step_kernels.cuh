@@ -40,8 +40,31 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
     return base + incl - n;
 }
 
+// Items of several queues, fn(queue, item), spread over the grid's warps: a warp takes as few
+// items at a time as it takes to give every warp some, and never items of two queues at once.
+// The items' paths differ, so few items spread wide finish in the time of the longest one, and
+// 32 to a warp only pays once the queues fill the GPU.
+template <int NQ, class F>
+RSB_D void forItems(const uint32_t* n, F&& fn) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31u;
+    uint32_t total = 0, tiles = 0;
+    for (int k = 0; k < NQ; k++) total += n[k];
+    const uint32_t width = min(32u, (total + warps - 1u) / warps);
+    if (width == 0) return;
+    for (int k = 0; k < NQ; k++) tiles += (n[k] + width - 1u) / width;
+    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
+        uint32_t q = tile;
+        int k = 0;
+        while (q >= (n[k] + width - 1u) / width) q -= (n[k++] + width - 1u) / width;
+        const uint32_t i = q * width + lane;
+        if (lane < width && i < n[k]) fn(k, i);
+    }
+}
+
 constexpr int BODY_THREADS = MAX_BODIES * PHASE_ARENAS;
 constexpr int CAR_THREADS = MAX_CARS * PHASE_ARENAS;
+
+RSB_D size_t rayPlaces(const EngineView& D) { return (size_t)4 * MAX_CARS * D.N; }
 
 __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__ EngineView D,
                                                          const __grid_constant__ StepTemp T) {
@@ -59,18 +82,19 @@ __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__
     bool culled = false;
     const bool live = 1 + s < nb && rayCar(D, a, s, xf, culled);
     auto near = [&](int i, int j, int k) {
-        bool n = false;
+        uint32_t n = 0;
         for (int b = 0; b < nb; b++) {
-            if (b == 1 + s) continue;
             const int ci = cell[b][0][lane], cj = cell[b][1][lane], ck = cell[b][2][lane];
-            n |= i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1;
+            if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) n |= 1u << b;
         }
         return n;
     };
     for (int w = 0; w < 4; w++) {
-        const bool heavy = live && rayPhase(D, T, a, s, w, xf, culled, near, st);
-        const uint32_t at = queueAlloc(&T.count[QC_RAY], heavy ? 1u : 0u);
-        if (heavy) T.rayQ[at] = (uint32_t)rayIdx(D, a, s, w);
+        const RayClass c = live ? rayPhase(D, T, a, s, w, xf, culled, near, st) : RAY_DONE;
+        const uint32_t m = queueAlloc(&T.count[QC_RAY], c == RAY_MESHES ? 1u : 0u);
+        const uint32_t o = queueAlloc(&T.count[QC_BODYRAY], c == RAY_BODIES ? 1u : 0u);
+        if (c == RAY_MESHES) T.rayQ[m] = (uint32_t)rayIdx(D, a, s, w);
+        else if (c == RAY_BODIES) T.rayQ[rayPlaces(D) + o] = (uint32_t)rayIdx(D, a, s, w);
     }
     blockStats(D, st);
 }
@@ -78,10 +102,9 @@ __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) heavyRayKernel(const __grid_constant__ EngineView D,
                                                             const __grid_constant__ StepTemp T) {
-    const uint32_t n = T.count[QC_RAY];
+    const uint32_t n[2] = {T.count[QC_RAY], T.count[QC_BODYRAY]};
     PhaseStats st{0, 0, 0, 0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        heavyRayPhase(D, T, T.rayQ[i], st);
+    forItems<2>(n, [&](int q, uint32_t i) { heavyRayPhase(D, T, T.rayQ[q * rayPlaces(D) + i], st); });
     blockStats(D, st);
 }
 
@@ -97,7 +120,7 @@ __global__ void __launch_bounds__(BODY_THREADS) bodyKernel(const __grid_constant
     t.finished = true;
     t.deps = 0;
     const bool valid = t.b < t.nb;
-    if (blockIdx.x == 0 && threadIdx.x == 0) T.count[QC_RAY] = 0;  // the queued rays are cast
+    if (blockIdx.x == 0 && threadIdx.x == 0) T.count[QC_RAY] = T.count[QC_BODYRAY] = 0;  // the queued rays are cast
     if (threadIdx.x < PHASE_ARENAS) sh.done[lane] = sh.need[lane] = 0;
     if (valid) bodyLoad(D, T, t, sh);
     __syncthreads();
@@ -136,25 +159,10 @@ __global__ void __launch_bounds__(BODY_THREADS) bodyKernel(const __grid_constant
     blockStats(D, st);
 }
 
-// Warps over the items of several queues, 32 of one queue at a time: fn(queue, item).
-template <int NQ, class F>
-RSB_D void forTiles(const uint32_t* n, F&& fn) {
-    uint32_t tiles = 0;
-    for (int k = 0; k < NQ; k++) tiles += (n[k] + 31u) / 32u;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
-        uint32_t q = tile;
-        int k = 0;
-        while (q >= (n[k] + 31u) / 32u) q -= (n[k++] + 31u) / 32u;
-        const uint32_t i = q * 32u + (threadIdx.x & 31u);
-        if (i < n[k]) fn(k, i);
-    }
-}
-
 __global__ void __launch_bounds__(128) findKernel(const __grid_constant__ EngineView D,
                                                   const __grid_constant__ StepTemp T) {
     const uint32_t n[3] = {T.count[QC_CARMESH], T.count[QC_BALLMESH], T.count[QC_CARBALL]};
-    forTiles<3>(n, [&](int k, uint32_t i) {
+    forItems<3>(n, [&](int k, uint32_t i) {
         findPhase(D, T, (uint32_t)resultBase(QC_CARMESH + k) * (uint32_t)D.N + i);
     });
 }
@@ -163,7 +171,7 @@ template <int MINB>
 __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constant__ EngineView D,
                                                             const __grid_constant__ StepTemp T) {
     const uint32_t n[2] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR]};
-    forTiles<2>(n, [&](int k, uint32_t i) {
+    forItems<2>(n, [&](int k, uint32_t i) {
         if (k == 0) trianglePhase(D, T, i);
         else carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
     });
@@ -174,7 +182,7 @@ __global__ void __launch_bounds__(128) deepKernel(const __grid_constant__ Engine
     EpaWork epa;
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[1] = {T.count[QC_DEEP]};
-    forTiles<1>(n, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
+    forItems<1>(n, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
     blockStats(D, st);
 }
 
@@ -182,17 +190,16 @@ __global__ void __launch_bounds__(128) combineKernel(const __grid_constant__ Eng
                                                      const __grid_constant__ StepTemp T) {
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[1] = {T.count[QC_COMBINE]};
-    forTiles<1>(n, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
+    forItems<1>(n, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
     blockStats(D, st);
 }
 
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) solveKernel(const __grid_constant__ EngineView D,
                                                          const __grid_constant__ StepTemp T) {
-    const uint32_t n = T.count[QC_SOLVE];
+    const uint32_t n[1] = {T.count[QC_SOLVE]};
     PhaseStats st{0, 0, 0, 0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        solvePhase(D, T, (int)T.solveQ[i], st);
+    forItems<1>(n, [&](int, uint32_t i) { solvePhase(D, T, (int)T.solveQ[i], st); });
     blockStats(D, st);
 }
 
@@ -206,7 +213,7 @@ __global__ void __launch_bounds__(BODY_THREADS) finishKernel(const __grid_consta
     t.a = blockIdx.x * PHASE_ARENAS + lane;
     t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
     const bool valid = t.b < t.nb, pads = t.nb > 1;
-    if (blockIdx.x == 0 && threadIdx.x < QC_WORDS && threadIdx.x != QC_RAY) T.count[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x >= QC_CARMESH && threadIdx.x < QC_WORDS) T.count[threadIdx.x] = 0;
     if (pads)
         for (int p = warp; p < NUM_PADS; p += warps) padLoad(D, t.a, lane, p, sh);
     if (warp > 0) sh.picked[warp - 1][lane] = 0;

@@ -32,7 +32,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     D.work = nullptr;
     std::vector<int32_t> rayObj(R);
     std::vector<float> rayFrac(R), rayN(3 * R), force(6 * B), box(6 * B), cache(3 * B);
-    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(R), solveQ(N);
+    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(2 * R), solveQ(N);
     std::vector<PairTask> tasks(CAP_RESULTS * N);
     std::vector<PairResult> results(CAP_RESULTS * N);
     std::vector<MPoint> blocks(MAX_BLOCKS * N * MAX_POINTS);
@@ -75,19 +75,24 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
                 bool culled;
                 if (!rayCar(D, a, s, xf, culled)) continue;
                 auto near = [&](int i, int j, int k) {
+                    uint32_t n = 0;
                     for (int b = 0; b < arenaBodies(D, a); b++) {
-                        if (b == 1 + s) continue;
                         const int w = (int)(offsetof(CarP, ci) / 4);
                         const int ci = (int)bodyWord(D, a, b, w), cj = (int)bodyWord(D, a, b, w + 1), ck = (int)bodyWord(D, a, b, w + 2);
-                        if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) return true;
+                        if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) n |= 1u << b;
                     }
-                    return false;
+                    return n;
                 };
-                for (int w = 0; w < 4; w++)
-                    if (rayPhase(D, T, a, s, w, xf, culled, near, st)) T.rayQ[T.count[QC_RAY]++] = (uint32_t)rayIdx(D, a, s, w);
+                for (int w = 0; w < 4; w++) {
+                    const RayClass c = rayPhase(D, T, a, s, w, xf, culled, near, st);
+                    if (c == RAY_MESHES) T.rayQ[T.count[QC_RAY]++] = (uint32_t)rayIdx(D, a, s, w);
+                    else if (c == RAY_BODIES) T.rayQ[R + T.count[QC_BODYRAY]++] = (uint32_t)rayIdx(D, a, s, w);
+                }
             }
-        counts[QC_RAY] += T.count[QC_RAY];
-        while (T.count[QC_RAY] > 0) heavyRayPhase(D, T, T.rayQ[--T.count[QC_RAY]], st);
+        for (int k = QC_RAY; k <= QC_BODYRAY; k++) {
+            counts[k] += T.count[k];
+            while (T.count[k] > 0) heavyRayPhase(D, T, T.rayQ[(k == QC_RAY ? 0 : R) + --T.count[k]], st);
+        }
         // bodies
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {
             auto each = [&](auto&& fn) {

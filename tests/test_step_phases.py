@@ -18,8 +18,8 @@ from gpu_util import random_balls, random_cars, random_controls
 from host_util import ARENA_BUILD
 
 SRC = os.path.join(ROOT, "tests", "cpp", "step_phases_host.cpp")
-QUEUES = ("rays", "car-mesh", "ball-mesh", "car-ball", "car-car", "planes", "blocks", "islands", "triangles", "deep",
-          "combine")
+QUEUES = ("mesh rays", "body rays", "car-mesh", "ball-mesh", "car-ball", "car-car", "planes", "blocks", "islands",
+          "triangles", "deep", "combine")
 
 
 @pytest.fixture(scope="module")
@@ -112,7 +112,7 @@ def test_phases_match_the_one_thread_tick(pkg, host, kind, ticks):
     for seed in (11, 12):
         got = compare(pkg, host, len(teams), teams, kind, seed, ticks, 160 // ticks)
         seen = {q: seen[q] + got[q] for q in QUEUES}
-    assert seen["rays"] and seen["planes"] and seen["islands"]
+    assert seen["mesh rays"] and seen["body rays"] and seen["planes"] and seen["islands"]
     if kind == "walls":
         assert seen["car-mesh"] and seen["ball-mesh"] and seen["triangles"] and seen["deep"] and seen["combine"]
     if kind in ("heap", "stack"):
