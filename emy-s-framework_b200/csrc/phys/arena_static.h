@@ -170,15 +170,15 @@ RSB_HD void bvhQueryAabb(const ArenaStatic& S, int mesh, V3 aabbMin, V3 aabbMax,
 
 // btRayAabb2 (btAabbUtil2.h)
 RSB_HD bool rayAabb2(V3 src, V3 invDir, const unsigned* sign, const V3* bounds, float& tmin, float lmin, float lmax) {
-    float txmin = (bounds[sign[0]].x - src.x) * invDir.x;
-    float txmax = (bounds[1 - sign[0]].x - src.x) * invDir.x;
-    float tymin = (bounds[sign[1]].y - src.y) * invDir.y;
-    float tymax = (bounds[1 - sign[1]].y - src.y) * invDir.y;
+    float txmin = ((sign[0] ? bounds[1].x : bounds[0].x) - src.x) * invDir.x;
+    float txmax = ((sign[0] ? bounds[0].x : bounds[1].x) - src.x) * invDir.x;
+    float tymin = ((sign[1] ? bounds[1].y : bounds[0].y) - src.y) * invDir.y;
+    float tymax = ((sign[1] ? bounds[0].y : bounds[1].y) - src.y) * invDir.y;
     if ((txmin > tymax) || (tymin > txmax)) return false;
     if (tymin > txmin) txmin = tymin;
     if (tymax < txmax) txmax = tymax;
-    float tzmin = (bounds[sign[2]].z - src.z) * invDir.z;
-    float tzmax = (bounds[1 - sign[2]].z - src.z) * invDir.z;
+    float tzmin = ((sign[2] ? bounds[1].z : bounds[0].z) - src.z) * invDir.z;
+    float tzmax = ((sign[2] ? bounds[0].z : bounds[1].z) - src.z) * invDir.z;
     if ((txmin > tzmax) || (tzmin > txmax)) return false;
     if (tzmin > txmin) txmin = tzmin;
     if (tzmax < txmax) txmax = tzmax;

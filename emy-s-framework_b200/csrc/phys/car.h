@@ -231,6 +231,7 @@ RSB_HD void calcFrictionImpulses(WT& W, int ci, float timeStep) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     float frictionScale = C.mass / 3.f;
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         WheelTick& w = c.w[i];
         if (w.ground >= 0) {
@@ -277,6 +278,7 @@ RSB_HD void updateSuspension(WT& W, int ci, float dt) {
     const CarParams& C = W.P->car;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         WheelTick& w = c.w[i];
         if (w.inContact) {
@@ -289,6 +291,7 @@ RSB_HD void updateSuspension(WT& W, int ci, float dt) {
             w.susForce = 0;
         }
     }
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         WheelTick& w = c.w[i];
         if (w.susForce != 0) {
@@ -306,6 +309,7 @@ RSB_HD void applyFrictionImpulses(WT& W, int ci, float dt) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     V3 up = chassisUp(cb);
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         WheelTick& w = c.w[i];
         if (!isZero(w.impulse)) {
@@ -322,6 +326,7 @@ template <class WT>
 RSB_HD V3 upwardsDirFromWheels(const WT& W, int ci) {
     const CarSim& c = W.c[ci];
     V3 sum = v3zero();
+#pragma unroll
     for (int i = 0; i < 4; i++)
         if (c.w[i].inContact) sum = sum + c.w[i].contactNormal;
     if (sum == v3zero()) return chassisUp(W.b[1 + ci]);
@@ -361,6 +366,7 @@ RSB_HD void carSetSpawnState(WT& W, int ci, V3 posUu, const M3& rot, float boost
     c.ballHitTick = c.ballHitExtraTick = ~0ull;
     c.ballHitRelPos = c.ballHitBallPos = c.ballHitExtraVel = v3zero();
     c.rotMat = rot;
+#pragma unroll
     for (int k = 0; k < 5; k++) c.lastCtl[k] = 0.f;
     c.lastCtlBits = 0;
 }
@@ -394,6 +400,7 @@ RSB_HD void updateWheels(WT& W, int ci, float dt, int numContact, float fwdSpeed
     CarSim& c = W.c[ci];
     float absFwd = fabsf(fwdSpeedUu);
     bool worldContact = false;
+#pragma unroll
     for (int i = 0; i < 4; i++) worldContact |= c.w[i].withWorld != 0;
     bool handbrake = (c.ctlBits & 4u) != 0, boostIn = (c.ctlBits & 2u) != 0;
     if (handbrake) c.handbrakeVal += POWERSLIDE_RISE_RATE * dt;
@@ -431,6 +438,7 @@ RSB_HD void updateWheels(WT& W, int ci, float dt, int numContact, float fwdSpeed
         steerAngle *= c.ctl[1];
         c.steerAngle = steerAngle;
     }
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         WheelTick& w = c.w[i];
         if (w.ground >= 0) {
@@ -707,6 +715,7 @@ RSB_HD bool carPreTickStatus(WT& W, int ci, uint32_t respawnPick) {
     const float dt = W.P->dt;
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
+#pragma unroll
     for (int k = 0; k < 5; k++) c.ctl[k] = clampf(c.ctl[k], -1, 1);
     if (cflag(c, CF_DEMOED)) {
         c.demoRespawnTimer = fmax_(c.demoRespawnTimer - dt, 0);
@@ -732,6 +741,7 @@ RSB_HD void carDrive(WT& W, int ci) {
     bool jumpPressed = jump && !lastJump;
     int numContact = 0;
     c.flags &= ~(0xFu * CF_WHEEL0);
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         if (c.w[i].inContact) c.flags |= CF_WHEEL0 << i;
         numContact += c.w[i].inContact ? 1 : 0;
@@ -759,7 +769,9 @@ RSB_HD void carPreTick(WT& W, int ci, uint32_t respawnPick) {
     Body& cb = W.b[1 + ci];
     CarSim& c = W.c[ci];
     // btVehicleRL::updateVehicleFirst
+#pragma unroll
     for (int i = 0; i < 4; i++) wheelTransform(W.P->car, cb, c.w[i], i, i < 2 ? c.steerAngle : 0.f);
+#pragma unroll
     for (int i = 0; i < 4; i++) wheelRayCast(W, ci, i);
     carDrive(W, ci);
 }
@@ -784,6 +796,7 @@ RSB_HD void carPostTick(WT& W, int ci) {
         else c.supersonicTime = 0;
     }
     if (c.carContactCooldown > 0) c.carContactCooldown = fmax_(c.carContactCooldown - dt, 0);
+#pragma unroll
     for (int k = 0; k < 5; k++) c.lastCtl[k] = c.ctl[k];
     c.lastCtlBits = c.ctlBits;
     // _FinishPhysicsTick

@@ -87,15 +87,29 @@ struct Curve {
 RSB_HD float curveOut(const Curve& c, float input, float def = 1.f) {
     if (c.n == 0) return def;
     if (input <= c.x[0]) return c.y[0];
-    for (int i = 1; i < c.n; i++) {
-        if (c.x[i] > input) {
-            float range = c.x[i] - c.x[i - 1];
-            float vdiff = c.y[i] - c.y[i - 1];
-            float f = (input - c.x[i - 1]) / range;
-            return c.y[i - 1] + vdiff * f;
+    // the first segment that ends above the input, by selection; then one interpolation
+    float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
+    bool in = false;
+#pragma unroll
+    for (int i = 5; i >= 1; i--)
+        if (i < c.n && c.x[i] > input) {
+            x0 = c.x[i - 1];
+            x1 = c.x[i];
+            y0 = c.y[i - 1];
+            y1 = c.y[i];
+            in = true;
         }
+    if (in) {
+        float range = x1 - x0;
+        float vdiff = y1 - y0;
+        float f = (input - x0) / range;
+        return y0 + vdiff * f;
     }
-    return c.y[c.n - 1];
+    float last = c.y[0];
+#pragma unroll
+    for (int i = 1; i < 6; i++)
+        if (i < c.n) last = c.y[i];
+    return last;
 }
 
 // Curves are produced by value (functions usable from host and device code):

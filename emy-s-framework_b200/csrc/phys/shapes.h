@@ -73,7 +73,8 @@ RSB_HD float fsels(float a, float b, float c) { return a >= 0.f ? b : c; }
 
 RSB_HD V3 triSupport(const ConvexShape& s, V3 dir) {
     V3 dots = V3{dot(dir, s.v[0]), dot(dir, s.v[1]), dot(dir, s.v[2])};
-    return s.v[maxAxis(dots)];
+    const int k = maxAxis(dots);  // by selection: an indexed array would live in local memory
+    return k == 0 ? s.v[0] : (k == 1 ? s.v[1] : s.v[2]);
 }
 
 RSB_HD V3 supportNoMargin(const ConvexShape& s, V3 dir) {
@@ -115,6 +116,7 @@ RSB_HD void shapeAabb(const ConvexShape& s, const Xf& t, V3& mn, V3& mx) {
         mn = t.o - e;
         mx = t.o + e;
     } else {
+#pragma unroll
         for (int i = 0; i < 3; i++) {
             V3 vec = v3zero();
             vec[i] = 1.f;

@@ -9,10 +9,11 @@
 //
 //   rays ....... every wheel ray of every car: the planes here, the rest into the ray queue
 //   heavy rays . the queued rays: meshes, planes, other bodies (castRay)
-//   bodies ..... respawns, vehicle update, gravity, predicted motion, broadphase pairs, plane
-//                contacts; queues the other contact pairs and the arenas that have any
+//   drive ...... respawns and the vehicle update of every car
+//   pairs ...... predicted motion of every body, broadphase pairs; queues the pairs that can be in
+//                contact and the arenas that have any
 //   find ....... queued mesh pairs: the triangles whose boxes overlap (candidates, in walk order)
-//   triangles .. one candidate per thread: box-triangle and box-sphere GJK; box-box pairs
+//   triangles .. one candidate per thread: box-triangle and box-sphere GJK; box-box and plane pairs
 //   deep ....... the candidates whose GJK needs the penetration solver
 //   combine .... one pair per thread: its candidates' contacts into the manifold, in walk order
 //   islands .... the queued arenas: contact callbacks, islands, solver (solveIslands)
@@ -36,8 +37,8 @@ enum : int {
     BI_MANI,        // static pairs that have a manifold (20 bits)
     BI_TASKS,       // meshes with a queued contact pair (16 bits) | planes with a contact << 16
     BI_MESHRES,     // result of the first queued mesh pair (the others follow)
-    BI_PLANERES,    // results of the plane contacts (4 words)
-    BI_DYN = BI_PLANERES + NUM_PLANES,  // dynamic pairs in visiting order, 3 bits each, count << 24
+    BI_PLANERES,    // result of the first plane contact (the others follow)
+    BI_DYN,         // dynamic pairs in visiting order, 3 bits each, count << 24
     BI_DYNMANI,     // bodies of higher index with which this body has a manifold (7 bits)
     BI_WORDS
 };
@@ -525,17 +526,20 @@ RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, Ph
 
 // ------------------------------------------------------------------ bodies
 
-// What the threads of one arena's bodies exchange during the bodies phase, one column per arena.
+// What the threads of one arena's cars exchange during the drive phase, one column per arena.
 constexpr int PHASE_ARENAS = 32;
-struct BodyShared {
+struct DriveShared {
     float pre[MAX_CARS][6][PHASE_ARENAS];   // linear and angular velocity before the car's pre-tick
     float post[MAX_CARS][6][PHASE_ARENAS];  // ... and after it
+    uint32_t done[PHASE_ARENAS];            // cars whose pre-tick is finished
+};
+// ... and the threads of its bodies during the pairs phase.
+struct PairShared {
     float box[MAX_BODIES][6][PHASE_ARENAS];
     int32_t cell[MAX_BODIES][3][PHASE_ARENAS];
     uint32_t stamp[MAX_BODIES][PHASE_ARENAS];
     uint32_t pick[MAX_BODIES][PHASE_ARENAS];  // BI_DYN word of each body
     uint32_t live[MAX_BODIES][PHASE_ARENAS];  // 1: active (objActive)
-    uint32_t done[PHASE_ARENAS];              // cars whose pre-tick is finished
     uint32_t need[PHASE_ARENAS];              // the arena has contacts or dynamic pairs to solve
 };
 
@@ -559,7 +563,7 @@ struct CarWorld {
     OneBody b;
     OneCar c;
     const EngineView* D;
-    const BodyShared* sh;
+    const DriveShared* sh;
     int a, la, ci;
 };
 
@@ -594,13 +598,12 @@ RSB_HD GroundRef groundRef(const CarWorld& W, int o) {
     return g;
 }
 
-// One body's thread of the bodies phase.
-struct BodyThread {
-    int a, la, b, nb;   // b < nb when there is such a body
-    bool live;          // a car whose vehicle update runs (not demoed)
+// One car's thread of the drive phase.
+struct DriveThread {
+    int a, la, s;
+    bool live;          // the vehicle update runs (the car is not demoed)
     bool respawned, finished;
     uint32_t deps;      // cars whose finished pre-tick this one waits for
-    uint32_t dyn;       // BI_DYN word
     CarWorld W;
 };
 
@@ -609,41 +612,28 @@ RSB_HD void publishVel(float (*v)[PHASE_ARENAS], int la, const Body& b) {
     v[3][la] = b.ang.x; v[4][la] = b.ang.y; v[5][la] = b.ang.z;
 }
 
-// Loads the body; a car runs its status update.  Nothing is written to the records before
-// every thread of the arena has published what others read.
-RSB_HD void bodyLoad(const EngineView& D, const StepTemp& T, BodyThread& t, BodyShared& sh) {
+// Loads the car, runs its status update and takes up its rays' results.  Nothing is written to
+// the records before every thread of the arena has published what others read.
+RSB_HD void driveLoad(const EngineView& D, const StepTemp& T, DriveThread& t, DriveShared& sh) {
     CarWorld& W = t.W;
     Body& b = W.b.v;
     CarSim& c = W.c.v;
+    const int a = t.a, s = t.s;
     W.S = &D.S;
     W.P = &D.P;
     W.D = &D;
     W.sh = &sh;
-    W.a = t.a;
+    W.a = a;
     W.la = t.la;
-    W.ci = t.b - 1;
-    W.tick = arenaTickCount(D, t.a);
+    W.ci = s;
+    W.tick = arenaTickCount(D, a);
     W.cull = 0;
-    t.live = t.respawned = false;
-    t.finished = true;
     t.deps = 0;
-    t.dyn = 0;
-    const int a = t.a, s = t.b - 1;
-    bodyConstants(D, t.b, b);
-    b.xf = bodyXf(D, a, t.b);
-    b.lin = bodyV3(D, a, t.b, RSB_PW(CarP, lin));
-    b.ang = bodyV3(D, a, t.b, RSB_PW(CarP, ang));
-    b.cell = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cell));
-    b.ci = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ci));
-    b.cj = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cj));
-    b.ck = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ck));
-    b.regStamp = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, regStamp));
+    bodyConstants(D, 1 + s, b);
+    b.xf = bodyXf(D, a, 1 + s);
+    b.lin = bodyV3(D, a, 1 + s, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, 1 + s, RSB_PW(CarP, ang));
     updateInertia(b);
-    if (t.b == 0) {
-        // ball zero-velocity sleeping (Arena.cpp:721-727)
-        b.act = (length2(b.lin) == 0.f && length2(b.ang) == 0.f) ? ACT_SLEEPING : ACT_ACTIVE;
-        return;
-    }
     publishVel(sh.pre[s], t.la, b);
     c.flags = carWord(D, a, s, RSB_PW(CarP, flags));
     c.team = (c.flags & CF_TEAM_ORANGE) ? 1 : 0;
@@ -660,17 +650,20 @@ RSB_HD void bodyLoad(const EngineView& D, const StepTemp& T, BodyThread& t, Body
     c.demoRespawnTimer = carFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer));
     c.flipRelTorque = carV3(D, a, s, RSB_PW(CarP, flipRelTorque));
     c.worldContactNormal = carV3(D, a, s, RSB_PW(CarP, worldContactNormal));
+#pragma unroll
     for (int r = 0; r < 3; r++) c.rotMat.r[r] = carV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r);
     c.lastCtlBits = carWord(D, a, s, RSB_PW(CarP, lastCtlBits));
     c.steerAngle = carFloat(D, a, s, RSB_PW(CarP, steerAngle));
     c.engineForce = carFloat(D, a, s, RSB_PW(CarP, engineForce));
     c.brake = carFloat(D, a, s, RSB_PW(CarP, brake));
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         c.latF[i] = carFloat(D, a, s, RSB_PW(CarP, latFriction) + i);
         c.longF[i] = carFloat(D, a, s, RSB_PW(CarP, longFriction) + i);
         c.extraPush[i] = carFloat(D, a, s, RSB_PW(CarP, extraPushback) + i);
     }
     const CtlRec& ctl = D.controls[D.carOffset[a] + s];
+#pragma unroll
     for (int k = 0; k < 5; k++) c.ctl[k] = ctl.v[k];
     c.ctlBits = (ctl.jump ? 1u : 0u) | (ctl.boost ? 2u : 0u) | (ctl.handbrake ? 4u : 0u);
     const bool wasDemoed = (c.flags & CF_DEMOED) != 0;
@@ -678,12 +671,16 @@ RSB_HD void bodyLoad(const EngineView& D, const StepTemp& T, BodyThread& t, Body
     t.respawned = wasDemoed && t.live;
     t.finished = !t.live;
     if (t.finished) publishVel(sh.post[s], t.la, b);
-    if (t.respawned && D.cull) phaseAtomicAnd(const_cast<uint32_t*>(D.cull) + a, ~(1u << t.b));
+    if (t.respawned && D.cull) phaseAtomicAnd(const_cast<uint32_t*>(D.cull) + a, ~(2u << s));
     if (!t.live) return;
-    // wheels: steering basis and the rays' results
+    // wheels: the steering basis (the same for both wheels of an axle) and the rays' results
+    wheelTransform(D.P.car, b, c.w[0], 0, c.steerAngle);
+    wheelTransform(D.P.car, b, c.w[2], 2, 0.f);
+    c.w[1].basis = c.w[0].basis;
+    c.w[3].basis = c.w[2].basis;
     const size_t rst = (size_t)4 * MAX_CARS * D.N;
+#pragma unroll
     for (int i = 0; i < 4; i++) {
-        wheelTransform(D.P.car, b, c.w[i], i, i < 2 ? c.steerAngle : 0.f);
         V3 from, to, hp = v3zero(), hn = v3zero();
         wheelSegment(D.P.car, b, c.w[i], i, from, to);
         const size_t r = rayIdx(D, a, s, i);
@@ -699,65 +696,25 @@ RSB_HD void bodyLoad(const EngineView& D, const StepTemp& T, BodyThread& t, Body
 }
 
 // The vehicle update, once the cars it stands on have finished theirs.
-RSB_HD void bodyDrive(BodyThread& t, BodyShared& sh) {
-    carDrive(t.W, t.b - 1);
-    publishVel(sh.post[t.b - 1], t.la, t.W.b.v);
+RSB_HD void driveRun(DriveThread& t, DriveShared& sh) {
+    carDrive(t.W, t.s);
+    publishVel(sh.post[t.s], t.la, t.W.b.v);
     t.finished = true;
 }
 
-// Gravity, predicted motion, broadphase box and registration; writes the record.
-RSB_HD void bodyMove(const EngineView& D, const StepTemp& T, BodyThread& t, BodyShared& sh, bool firstTick) {
+// Gravity; writes the record.
+RSB_HD void driveStore(const EngineView& D, const StepTemp& T, DriveThread& t) {
     Body& b = t.W.b.v;
-    CarSim& c = t.W.c.v;
-    const int a = t.a, s = t.b - 1, la = t.la;
-    const float dt = D.P.dt;
+    const CarSim& c = t.W.c.v;
+    const int a = t.a, s = t.s;
     if (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) b.force = b.force + b.grav;
-    b.lin = b.lin * b.linDampFactor;
-    b.ixf = t.b == 0 ? integrateTransformNoRot(b.xf, b.lin, dt) : integrateTransform(b.xf, b.lin, b.ang, dt);
-    // the box of the last tick stays when this one's is not finite
-    b.bpMin = b.bpMax = b.xf.o;
-    struct {
-        const ArenaStatic* S;
-        const WorldParams* P;
-        int nb;
-        OneBody* bp;
-        uint32_t stampBase, status;
-        struct Ref {
-            OneBody* p;
-            RSB_HD Body& operator[](int i) { return (*p)[i]; }
-        } b;
-    } M{&D.S, &D.P, t.nb, nullptr, (uint32_t)((t.W.tick + 1) * 8u), 0u, {&t.W.b}};
-    updateBodyAabb(M, t.b);
-    if (M.status) {
-        phaseAtomicOr(arenaStatus(D, a), M.status);
-        if (!firstTick) {
-            b.bpMin = tempV3(D, T.box, a, t.b, 0);
-            b.bpMax = tempV3(D, T.box, a, t.b, 3);
-        }
-    }
-    putTempV3(D, T.box, a, t.b, 0, b.bpMin);
-    putTempV3(D, T.box, a, t.b, 3, b.bpMax);
-    putTempV3(D, T.force, a, t.b, 0, b.force);
-    putTempV3(D, T.force, a, t.b, 3, b.torque);
-    const float bx[6] = {b.bpMin.x, b.bpMin.y, b.bpMin.z, b.bpMax.x, b.bpMax.y, b.bpMax.z};
-    for (int k = 0; k < 6; k++) sh.box[t.b][k][la] = bx[k];
-    sh.cell[t.b][0][la] = b.ci;
-    sh.cell[t.b][1][la] = b.cj;
-    sh.cell[t.b][2][la] = b.ck;
-    sh.stamp[t.b][la] = (uint32_t)b.regStamp;
-    sh.live[t.b][la] = (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) ? 1u : 0u;
-
-    putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
-    putBodyWord(D, a, t.b, RSB_PW(CarP, cell), (uint32_t)b.cell);
-    putBodyWord(D, a, t.b, RSB_PW(CarP, ci), (uint32_t)b.ci);
-    putBodyWord(D, a, t.b, RSB_PW(CarP, cj), (uint32_t)b.cj);
-    putBodyWord(D, a, t.b, RSB_PW(CarP, ck), (uint32_t)b.ck);
-    putBodyWord(D, a, t.b, RSB_PW(CarP, regStamp), (uint32_t)b.regStamp);
-    if (t.b == 0) return;
+    putTempV3(D, T.force, a, 1 + s, 0, b.force);
+    putTempV3(D, T.force, a, 1 + s, 3, b.torque);
     putCarWord(D, a, s, RSB_PW(CarP, flags), (c.flags & ~CF_NO_RESPONSE) | (b.noResp ? CF_NO_RESPONSE : 0u));
     putCarFloat(D, a, s, RSB_PW(CarP, demoRespawnTimer), c.demoRespawnTimer);
     if (!t.live) return;
-    putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+    putBodyV3(D, a, 1 + s, RSB_PW(CarP, lin), b.lin);
+    putBodyV3(D, a, 1 + s, RSB_PW(CarP, ang), b.ang);
     putCarFloat(D, a, s, RSB_PW(CarP, boost), c.boost);
     putCarFloat(D, a, s, RSB_PW(CarP, timeSpentBoosting), c.timeSpentBoosting);
     putCarFloat(D, a, s, RSB_PW(CarP, jumpTime), c.jumpTime);
@@ -771,6 +728,7 @@ RSB_HD void bodyMove(const EngineView& D, const StepTemp& T, BodyThread& t, Body
     putCarFloat(D, a, s, RSB_PW(CarP, steerAngle), c.steerAngle);
     putCarFloat(D, a, s, RSB_PW(CarP, engineForce), c.engineForce);
     putCarFloat(D, a, s, RSB_PW(CarP, brake), c.brake);
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         putCarFloat(D, a, s, RSB_PW(CarP, latFriction) + i, c.latF[i]);
         putCarFloat(D, a, s, RSB_PW(CarP, longFriction) + i, c.longF[i]);
@@ -778,7 +736,7 @@ RSB_HD void bodyMove(const EngineView& D, const StepTemp& T, BodyThread& t, Body
     }
     if (!t.respawned) return;
     // Car::SetState of the spawn: the rest of the record
-    putBodyXf(D, a, t.b, b.xf);
+    putBodyXf(D, a, 1 + s, b.xf);
     putCarFloat(D, a, s, RSB_PW(CarP, supersonicTime), 0.f);
     putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), 0.f);
     putCarV3(D, a, s, RSB_PW(CarP, worldContactNormal), v3zero());
@@ -793,11 +751,86 @@ RSB_HD void bodyMove(const EngineView& D, const StepTemp& T, BodyThread& t, Body
     for (int r = 0; r < 3; r++) putCarV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r, c.rotMat.r[r]);
 }
 
+// One body's thread of the pairs phase.
+struct PairThread {
+    int a, la, b, nb;   // b < nb when there is such a body
+    uint32_t dyn;       // BI_DYN word
+    OneBody body;
+};
+// The body as updateBodyAabb sees it.
+struct BoxWorld {
+    const ArenaStatic* S;
+    const WorldParams* P;
+    int nb;
+    uint32_t stampBase, status;
+    OneBody& b;
+};
+
+// Predicted motion, broadphase box and registration.
+RSB_HD void pairLoad(const EngineView& D, const StepTemp& T, PairThread& t, PairShared& sh, bool firstTick) {
+    Body& b = t.body.v;
+    const int a = t.a, la = t.la;
+    const float dt = D.P.dt;
+    bodyConstants(D, t.b, b);
+    b.xf = bodyXf(D, a, t.b);
+    b.lin = bodyV3(D, a, t.b, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, t.b, RSB_PW(CarP, ang));
+    b.cell = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cell));
+    b.ci = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ci));
+    b.cj = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, cj));
+    b.ck = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, ck));
+    b.regStamp = (int32_t)bodyWord(D, a, t.b, RSB_PW(CarP, regStamp));
+    if (t.b == 0) {
+        // ball zero-velocity sleeping (Arena.cpp:721-727)
+        b.act = (length2(b.lin) == 0.f && length2(b.ang) == 0.f) ? ACT_SLEEPING : ACT_ACTIVE;
+        if (b.act != ACT_SLEEPING) b.force = b.force + b.grav;
+        putTempV3(D, T.force, a, 0, 0, b.force);
+        putTempV3(D, T.force, a, 0, 3, b.torque);
+        b.lin = b.lin * b.linDampFactor;
+        putBodyV3(D, a, 0, RSB_PW(BallP, lin), b.lin);
+        b.ixf = integrateTransformNoRot(b.xf, b.lin, dt);
+    } else {
+        // a car without contact response is out of the simulation, and no other is
+        b.noResp = carWord(D, a, t.b - 1, RSB_PW(CarP, flags)) & CF_NO_RESPONSE ? 1 : 0;
+        b.act = b.noResp ? ACT_DISABLE_SIM : ACT_ACTIVE;
+        b.ixf = integrateTransform(b.xf, b.lin, b.ang, dt);
+    }
+    // the box of the last tick stays when this one's is not finite
+    b.bpMin = b.bpMax = b.xf.o;
+    const int32_t cell0 = b.cell, stamp0 = b.regStamp;
+    BoxWorld M{&D.S, &D.P, t.nb, (uint32_t)((arenaTickCount(D, a) + 1) * 8u), 0u, t.body};
+    updateBodyAabb(M, t.b);
+    if (M.status) {
+        phaseAtomicOr(arenaStatus(D, a), M.status);
+        if (!firstTick) {
+            b.bpMin = tempV3(D, T.box, a, t.b, 0);
+            b.bpMax = tempV3(D, T.box, a, t.b, 3);
+        }
+    }
+    putTempV3(D, T.box, a, t.b, 0, b.bpMin);
+    putTempV3(D, T.box, a, t.b, 3, b.bpMax);
+    const float bx[6] = {b.bpMin.x, b.bpMin.y, b.bpMin.z, b.bpMax.x, b.bpMax.y, b.bpMax.z};
+#pragma unroll
+    for (int k = 0; k < 6; k++) sh.box[t.b][k][la] = bx[k];
+    sh.cell[t.b][0][la] = b.ci;
+    sh.cell[t.b][1][la] = b.cj;
+    sh.cell[t.b][2][la] = b.ck;
+    sh.stamp[t.b][la] = (uint32_t)b.regStamp;
+    sh.live[t.b][la] = (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) ? 1u : 0u;
+    if (b.cell != cell0) putBodyWord(D, a, t.b, RSB_PW(CarP, cell), (uint32_t)b.cell);
+    if (b.regStamp != stamp0) {
+        putBodyWord(D, a, t.b, RSB_PW(CarP, ci), (uint32_t)b.ci);
+        putBodyWord(D, a, t.b, RSB_PW(CarP, cj), (uint32_t)b.cj);
+        putBodyWord(D, a, t.b, RSB_PW(CarP, ck), (uint32_t)b.ck);
+        putBodyWord(D, a, t.b, RSB_PW(CarP, regStamp), (uint32_t)b.regStamp);
+    }
+}
+
 RSB_HD V3 sharedV3(const float (*v)[PHASE_ARENAS], int k, int la) { return V3{v[k][la], v[k + 1][la], v[k + 2][la]}; }
 
 // The dynamic pairs of this body in visiting order (the second half of computePairs).
-RSB_HD void bodyPick(const EngineView& D, BodyThread& t, BodyShared& sh) {
-    const Body& b = t.W.b.v;
+RSB_HD void pairPick(const EngineView& D, PairThread& t, PairShared& sh) {
+    const Body& b = t.body.v;
     const BpGrid& g = D.S.bp;
     const int la = t.la;
     t.dyn = 0;
@@ -826,7 +859,7 @@ RSB_HD void bodyPick(const EngineView& D, BodyThread& t, BodyShared& sh) {
 // Contact world of one pair: at most two bodies.
 struct LocalPool {
     int32_t n;
-    uint32_t* status;
+    uint32_t* status;  // only written when more than MAX_BLOCKS manifolds share the pool; one does here
     MPoint pts[MAX_POINTS];
 };
 struct PairBodies {
@@ -841,19 +874,22 @@ struct PairWorldT {
     const WorldParams* P;
     BodiesT b;
     OneCar c;
-    LocalPool pool;
+    LocalPool* pool;  // apart, so that the points' indexing leaves the rest in registers
     uint32_t status;
     EpaWork* epa;
     uint32_t cull;
     int32_t cullAudit;
     mutable uint32_t nStatic, nCulled, nMissed, cullMissed;
 };
+template <class BodiesT>
+RSB_HD LocalPool& poolOf(PairWorldT<BodiesT>& W) { return *W.pool; }
 template <class WT>
-RSB_HD void pairWorldInit(const EngineView& D, WT& W, EpaWork* epa, uint32_t cull) {
+RSB_HD void pairWorldInit(const EngineView& D, WT& W, LocalPool& pool, EpaWork* epa, uint32_t cull) {
     W.S = &D.S;
     W.P = &D.P;
-    W.pool.n = 0;
-    W.pool.status = &W.status;
+    W.pool = &pool;
+    pool.n = 0;
+    pool.status = 0;
     W.status = 0;
     W.epa = epa;
     W.cull = cull;
@@ -893,23 +929,21 @@ RSB_HD void storePair(const EngineView& D, const StepTemp& T, int a, WT& W, cons
     if (W.status | W.cullMissed) phaseAtomicOr(arenaStatus(D, a), W.status | W.cullMissed);
 }
 
-// Static pairs: manifolds, plane contacts, queued meshes (the mesh bits are returned; the
-// caller allocates their places and stores them with bodyStaticStore).
+// Static pairs: all of them, those with a manifold, and those that can be in contact (the
+// caller allocates the queue places of these, and pairStore fills them).
 struct BodyStatics {
     uint32_t pairs, mani, meshes, planes;
-    uint32_t planeRes[NUM_PLANES];
 };
-RSB_HD BodyStatics bodyStatics(const EngineView& D, const StepTemp& T, BodyThread& t, PhaseStats& st) {
+RSB_HD BodyStatics pairStatics(const EngineView& D, PairThread& t, PhaseStats& st) {
     BodyStatics o;
     o.pairs = o.mani = o.meshes = o.planes = 0;
-    for (int p = 0; p < NUM_PLANES; p++) o.planeRes[p] = 0;
     const ArenaStatic& S = D.S;
-    const Body& b = t.W.b.v;
+    const Body& b = t.body.v;
     const CarParams& C = D.P.car;
     const bool active = b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM;
-    const uint32_t cull = D.cull ? (D.cull[t.a] & (1u << t.b)) : 0u;
+    const bool culled = D.cull && ((D.cull[t.a] >> t.b) & 1u);
     // the box the narrowphase tests: the ball's, or the hitbox at its place in the car
-    Xf childXf = t.b == 0 ? b.xf : carChildXf(C, b.xf);
+    const Xf childXf = t.b == 0 ? b.xf : carChildXf(C, b.xf);
     V3 bmn, bmx;
     if (t.b == 0) ballAabb(D.P, b.xf, bmn, bmx);
     else carBoxAabb(C, childXf, bmn, bmx);
@@ -929,13 +963,13 @@ RSB_HD BodyStatics bodyStatics(const EngineView& D, const StepTemp& T, BodyThrea
             if (!aabbOverlap(bmn, bmx, smn, smx)) continue;  // its manifold is released again
         }
         o.mani |= 1u << s;
+        // cullSkip's bookkeeping, then the rejects of the tests themselves
+        if (culled) {
+            st.nCulled++;
+            if (!D.cullAudit) continue;
+        }
+        st.nStatic++;
         if (s < MAX_MESHES) {
-            // cullSkip's bookkeeping, then the occupancy reject of the mesh walk
-            if (cull) {
-                st.nCulled++;
-                if (!D.cullAudit) continue;
-            }
-            st.nStatic++;
             if (!occKnown) {
                 const V3 tolv{kOccTol, kOccTol, kOccTol};
                 occ = occMask(S, bmn - tolv, bmx + tolv);
@@ -943,38 +977,19 @@ RSB_HD BodyStatics bodyStatics(const EngineView& D, const StepTemp& T, BodyThrea
             }
             if ((occ >> s) & 1u) o.meshes |= 1u << s;
         } else {
-            PairWorldT<OneBody> W;
-            pairWorldInit(D, W, nullptr, cull);
-            W.b.v = b;
-            Manifold m;
-            if (t.b == 0) {
-                pairManifold(m, OBJ_BALL, s, D.P.ballCbt);
-                collideBallPlane(W, s, m);
-            } else {
-                pairManifold(m, OBJ_CAR0 + t.b - 1, s, C.cbt);
-                collideBoxPlane(W, s, t.b - 1, childXf, m);
-            }
-            st.nStatic += W.nStatic;
-            st.nCulled += W.nCulled;
-            st.nMissed += W.nMissed;
-            if (m.pt) {
-                const uint32_t k = phaseAtomicAdd(&T.count[QC_PLANE], 1u);
-                const uint32_t r = (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + k;
-                o.planes |= 1u << (s - MAX_MESHES);
-                o.planeRes[s - MAX_MESHES] = r;
-                storePair(D, T, t.a, W, m, r);
-            } else if (W.cullMissed) {
-                phaseAtomicOr(arenaStatus(D, t.a), W.cullMissed);
-            }
+            V3 vip;
+            const bool near = t.b == 0 ? ballPlaneDistance(S, D.P, s, b.xf, vip) < D.P.ballCbt + 0.f
+                                       : boxPlaneDistance(S, C, s, childXf, vip) < C.cbt + 0.f;
+            if (near) o.planes |= 1u << (s - MAX_MESHES);
         }
     }
     return o;
 }
 
 // The dynamic pairs (b, hi > b) that have a manifold: bit hi.
-RSB_HD uint32_t bodyDynamics(const EngineView& D, const BodyThread& t, const BodyShared& sh) {
+RSB_HD uint32_t pairDynamics(const EngineView& D, const PairThread& t, const PairShared& sh) {
     const CarParams& C = D.P.car;
-    const Body& b = t.W.b.v;
+    const Body& b = t.body.v;
     uint32_t m = 0;
     auto picked = [&](int x, int y) {
         const uint32_t d = sh.pick[x][t.la];
@@ -985,8 +1000,6 @@ RSB_HD uint32_t bodyDynamics(const EngineView& D, const BodyThread& t, const Bod
     for (int hi = t.b + 1; hi < t.nb; hi++) {
         if (!picked(t.b, hi) && !picked(hi, t.b)) continue;
         if (!sh.live[t.b][t.la] && !sh.live[hi][t.la]) continue;
-        // the other body's transform: a car that respawned wrote its spawn to its record, which
-        // every thread of the arena has finished by now
         const Xf hx = bodyXf(D, t.a, hi);
         V3 mn, mx, mn2, mx2;
         if (t.b == 0) {
@@ -1006,11 +1019,11 @@ RSB_HD uint32_t bodyDynamics(const EngineView& D, const BodyThread& t, const Bod
 }
 
 // Stores the body's pair information and fills its queue places: `mesh0` the first of its mesh
-// pairs in their queue, `dyn0` the first of its dynamic pairs in theirs.
-RSB_HD void bodyStore(const EngineView& D, const StepTemp& T, const BodyThread& t, BodyShared& sh,
-                      const BodyStatics& o, uint32_t dynMani, uint32_t mesh0, uint32_t dyn0) {
+// pairs in their queue, `plane0` of its plane contacts, `dyn0` of its dynamic pairs.
+RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& t, PairShared& sh,
+                      const BodyStatics& o, uint32_t dynMani, uint32_t mesh0, uint32_t plane0, uint32_t dyn0) {
     const int a = t.a;
-    const Body& b = t.W.b.v;
+    const Body& b = t.body.v;
     const int meshType = t.b == 0 ? QC_BALLMESH : QC_CARMESH, dynType = t.b == 0 ? QC_CARBALL : QC_CARCAR;
     infoWord(D, T, a, t.b, BI_PAIRS) = o.pairs | ((uint32_t)b.act << BI_ACT_SHIFT) | (b.noResp ? 0u : BI_RESPONDS);
     infoWord(D, T, a, t.b, BI_DYN) = t.dyn;
@@ -1019,19 +1032,19 @@ RSB_HD void bodyStore(const EngineView& D, const StepTemp& T, const BodyThread& 
         infoWord(D, T, a, t.b, BI_TASKS) = o.meshes | (o.planes << 16);
         infoWord(D, T, a, t.b, BI_DYNMANI) = dynMani;
     }
-    const uint32_t mb = (uint32_t)resultBase(meshType) * (uint32_t)D.N + mesh0;
-    if (o.meshes) infoWord(D, T, a, t.b, BI_MESHRES) = mb;
-    uint32_t k = 0;
+    uint32_t k = (uint32_t)resultBase(meshType) * (uint32_t)D.N + mesh0;
+    if (o.meshes) infoWord(D, T, a, t.b, BI_MESHRES) = k;
     for (uint32_t m = o.meshes; m; m &= m - 1u, k++)
-        T.tasks[mb + k] = PairTask{(uint32_t)a, (uint16_t)lowestBit(m), (uint16_t)(OBJ_BALL + t.b)};
-    for (int p = 0; p < NUM_PLANES; p++)
-        if ((o.planes >> p) & 1u) infoWord(D, T, a, t.b, BI_PLANERES + p) = o.planeRes[p];
-    const uint32_t db = (uint32_t)resultBase(dynType) * (uint32_t)D.N + dyn0;
-    k = 0;
+        T.tasks[k] = PairTask{(uint32_t)a, (uint16_t)lowestBit(m), (uint16_t)(OBJ_BALL + t.b)};
+    k = (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + plane0;
+    if (o.planes) infoWord(D, T, a, t.b, BI_PLANERES) = k;
+    for (uint32_t m = o.planes; m; m &= m - 1u, k++)
+        T.tasks[k] = PairTask{(uint32_t)a, (uint16_t)(MAX_MESHES + lowestBit(m)), (uint16_t)(OBJ_BALL + t.b)};
+    k = (uint32_t)resultBase(dynType) * (uint32_t)D.N + dyn0;
     for (uint32_t m = dynMani; m; m &= m - 1u, k++) {
         const int hi = lowestBit(m);
-        T.tasks[db + k] = PairTask{(uint32_t)a, (uint16_t)(OBJ_BALL + t.b), (uint16_t)(OBJ_BALL + hi)};
-        T.dynRes[(size_t)dynPair(t.b, hi) * D.N + a] = db + k;
+        T.tasks[k] = PairTask{(uint32_t)a, (uint16_t)(OBJ_BALL + t.b), (uint16_t)(OBJ_BALL + hi)};
+        T.dynRes[(size_t)dynPair(t.b, hi) * D.N + a] = k;
     }
     // an arena without contacts and without dynamic pairs has nothing to solve
     if (o.meshes | o.planes | dynMani | t.dyn) phaseAtomicOr(&sh.need[t.la], 1u);
@@ -1050,7 +1063,8 @@ RSB_HD void carMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, E
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, b = k.o1 - OBJ_BALL;
     PairWorldT<OneBody> W;
-    pairWorldInit(D, W, epa, D.cull ? (D.cull[a] & (1u << b)) : 0u);
+    LocalPool pool;
+    pairWorldInit(D, W, pool, epa, D.cull ? (D.cull[a] & (1u << b)) : 0u);
     pairBody(D, a, b, W.b.v);
     Manifold m;
     pairManifold(m, k.o1, k.o0, D.P.car.cbt);
@@ -1062,7 +1076,8 @@ RSB_HD void ballMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, 
     const PairTask k = T.tasks[res];
     const int a = (int)k.a;
     PairWorldT<OneBody> W;
-    pairWorldInit(D, W, nullptr, D.cull ? (D.cull[a] & 1u) : 0u);
+    LocalPool pool;
+    pairWorldInit(D, W, pool, nullptr, D.cull ? (D.cull[a] & 1u) : 0u);
     pairBody(D, a, 0, W.b.v);
     Manifold m;
     pairManifold(m, OBJ_BALL, k.o0, D.P.ballCbt);
@@ -1176,7 +1191,8 @@ RSB_HD void deepPhase(const EngineView& D, const StepTemp& T, uint32_t e, EpaWor
             ballMeshPhase(D, T, res, st);
         } else if (k.o0 == OBJ_BALL) {
             PairWorldT<PairBodies> W;
-            pairWorldInit(D, W, epa, 0u);
+            LocalPool pool;
+            pairWorldInit(D, W, pool, epa, 0u);
             W.b.i0 = 0;
             pairBody(D, (int)k.a, 0, W.b.v0);
             pairBody(D, (int)k.a, k.o1 - OBJ_BALL, W.b.v1);
@@ -1216,20 +1232,22 @@ RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, P
     if (k.o0 == OBJ_BALL) {
         const CandidateOut& o = T.out[T.first[res]];
         PairWorldT<PairBodies> W;
-        pairWorldInit(D, W, nullptr, 0u);
+        LocalPool pool;
+        pairWorldInit(D, W, pool, nullptr, 0u);
         W.b.i0 = 0;
         pairBody(D, a, 0, W.b.v0);
         pairBody(D, a, b, W.b.v1);
         Manifold m;
         pairManifold(m, k.o1, OBJ_BALL, fmin_(D.P.car.cbt, D.P.ballCbt));
         if (o.flags & CO_HAS)
-            addContact(m, W.pool, OBJ_BALL, objRef(W, OBJ_BALL), k.o1, objRef(W, k.o1),
+            addContact(m, pool, OBJ_BALL, objRef(W, OBJ_BALL), k.o1, objRef(W, k.o1),
                        V3{o.normal[0], o.normal[1], o.normal[2]}, V3{o.point[0], o.point[1], o.point[2]}, o.dist);
         storePair(D, T, a, W, m, res);
         return;
     }
     PairWorldT<OneBody> W;
-    pairWorldInit(D, W, nullptr, D.cull ? (D.cull[a] & (1u << b)) : 0u);
+    LocalPool pool;
+    pairWorldInit(D, W, pool, nullptr, D.cull ? (D.cull[a] & (1u << b)) : 0u);
     pairBody(D, a, b, W.b.v);
     Manifold m;
     pairManifold(m, k.o1, k.o0, b == 0 ? D.P.ballCbt : D.P.car.cbt);
@@ -1265,11 +1283,28 @@ RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, P
     storePair(D, T, a, W, m, res);
 }
 
+// A plane pair whose test found it in contact.
+RSB_HD void planePhase(const EngineView& D, const StepTemp& T, uint32_t res, PhaseStats& st) {
+    const PairTask k = T.tasks[res];
+    const int a = (int)k.a, b = k.o1 - OBJ_BALL;
+    PairWorldT<OneBody> W;
+    LocalPool pool;
+    pairWorldInit(D, W, pool, nullptr, D.cull ? (D.cull[a] & (1u << b)) : 0u);
+    pairBody(D, a, b, W.b.v);
+    Manifold m;
+    pairManifold(m, k.o1, k.o0, b == 0 ? D.P.ballCbt : D.P.car.cbt);
+    if (b == 0) collideBallPlane(W, k.o0, m);
+    else collideBoxPlane(W, k.o0, b - 1, carChildXf(D.P.car, W.b.v.xf), m);
+    st.nMissed += W.nMissed;
+    storePair(D, T, a, W, m, res);
+}
+
 RSB_HD void carCarPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, ba = k.o0 - OBJ_BALL, bb = k.o1 - OBJ_BALL;
     PairWorldT<PairBodies> W;
-    pairWorldInit(D, W, nullptr, 0u);
+    LocalPool pool;
+    pairWorldInit(D, W, pool, nullptr, 0u);
     W.b.i0 = ba;
     pairBody(D, a, ba, W.b.v0);
     pairBody(D, a, bb, W.b.v1);
@@ -1279,7 +1314,7 @@ RSB_HD void carCarPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     carCarContacts(W, ba - 1, bb - 1, bc);
     ObjRef rA = objRef(W, k.o0), rB = objRef(W, k.o1);
     for (int c = 0; c < bc.n; c++)
-        addContact(m, W.pool, k.o0, rA, k.o1, rB, bc.c[c].normalOnB, bc.c[c].point, bc.c[c].depth);
+        addContact(m, pool, k.o0, rA, k.o1, rB, bc.c[c].normalOnB, bc.c[c].point, bc.c[c].depth);
     storePair(D, T, a, W, m, res);
 }
 
@@ -1395,7 +1430,8 @@ RSB_HD void solvePhase(const EngineView& D, const StepTemp& T, int a, PhaseStats
                 if ((tasks >> s) & 1u)
                     r = T.results + infoWord(D, T, a, i, BI_MESHRES) + bitCount(tasks & ((1u << s) - 1u));
             } else if ((tasks >> s) & 1u) {
-                r = T.results + infoWord(D, T, a, i, BI_PLANERES + s - MAX_MESHES);
+                r = T.results + infoWord(D, T, a, i, BI_PLANERES) +
+                    bitCount((tasks >> MAX_MESHES) & ((1u << (s - MAX_MESHES)) - 1u));
             }
             if (addManifold(OBJ_BALL + i, s, i == 0 ? D.P.ballCbt : D.P.car.cbt, r) && (r->flags & PR_WORLD)) {
                 // onCarWorld's state; its material is in the points already
@@ -1485,85 +1521,83 @@ RSB_HD void padLoad(const EngineView& D, int a, int la, int p, FinishShared& sh)
 }
 
 struct FinishThread {
-    int a, la, b, nb;
-    Body body;
-    CarSim c;
+    const WorldParams* P;
+    OneBody b;
+    OneCar c;
+    int a, la, body, nb;
     uint64_t tick;
     bool pads;  // the car may collide with pads
 };
 
 // Integration and post-tick of one body (integrateBodies, updateActivation, carPostTick,
-// ballFinishTick), then the pads around a car.
+// ballFinishTick).
 RSB_HD void finishBody(const EngineView& D, const StepTemp& T, FinishThread& t, FinishShared& sh) {
-    Body& b = t.body;
-    CarSim& c = t.c;
-    const int a = t.a, s = t.b - 1;
+    Body& b = t.b.v;
+    CarSim& c = t.c.v;
+    const int a = t.a, i = t.body, s = i - 1;
     const float dt = D.P.dt;
-    const uint32_t info = infoWord(D, T, a, t.b, BI_PAIRS);
+    const uint32_t info = infoWord(D, T, a, i, BI_PAIRS);
+    t.P = &D.P;
     t.tick = arenaTickCount(D, a);
     t.pads = false;
-    bodyConstants(D, t.b, b);
+    bodyConstants(D, i, b);
     b.act = (int32_t)((info & BI_ACT_MASK) >> BI_ACT_SHIFT);
-    b.xf = bodyXf(D, a, t.b);
-    b.lin = bodyV3(D, a, t.b, RSB_PW(CarP, lin));
-    b.ang = bodyV3(D, a, t.b, RSB_PW(CarP, ang));
+    b.xf = bodyXf(D, a, i);
+    b.lin = bodyV3(D, a, i, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, i, RSB_PW(CarP, ang));
     const bool moves = b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM;
     if (!(info & BI_SOLVED) && moves) {
         // an island of one body without contacts: the solver adds the external impulses only
         updateInertia(b);
-        b.force = tempV3(D, T.force, a, t.b, 0);
-        b.torque = tempV3(D, T.force, a, t.b, 3);
+        b.force = tempV3(D, T.force, a, i, 0);
+        b.torque = tempV3(D, T.force, a, i, 3);
         const V3 extF = (b.force * b.invMass) * dt, extT = tmul(b.torque, b.invIw) * dt;
         b.lin = (b.lin + v3zero()) + extF;
         b.ang = (b.ang + v3zero()) + extT;
     }
-    if (moves) b.xf = t.b == 0 ? integrateTransformNoRot(b.xf, b.lin, dt) : integrateTransform(b.xf, b.lin, b.ang, dt);
+    if (moves) b.xf = i == 0 ? integrateTransformNoRot(b.xf, b.lin, dt) : integrateTransform(b.xf, b.lin, b.ang, dt);
     if (b.act == ACT_SLEEPING) b.lin = b.ang = v3zero();
     if (moves) {
-        putBodyV3(D, a, t.b, RSB_PW(CarP, pos), b.xf.o);
-        if (t.b != 0)
-            for (int r = 0; r < 3; r++) putBodyV3(D, a, t.b, RSB_PW(CarP, rot) + 3 * r, b.xf.b.r[r]);
+        putBodyV3(D, a, i, RSB_PW(CarP, pos), b.xf.o);
+        if (i != 0)
+#pragma unroll
+            for (int r = 0; r < 3; r++) putBodyV3(D, a, i, RSB_PW(CarP, rot) + 3 * r, b.xf.b.r[r]);
     }
-    if (t.b == 0) {
-        struct {
-            const WorldParams* P;
-            OneBody b;
-        } W{&D.P, {b}};
-        ballFinishTick(W, (info & BI_CACHE) ? tempV3(D, T.cache, a, 0, 0) : v3zero());
-        putBodyV3(D, a, 0, RSB_PW(BallP, lin), W.b.v.lin);
-        putBodyV3(D, a, 0, RSB_PW(BallP, ang), W.b.v.ang);
+    if (i == 0) {
+        ballFinishTick(t, (info & BI_CACHE) ? tempV3(D, T.cache, a, 0, 0) : v3zero());
+        putBodyV3(D, a, 0, RSB_PW(BallP, lin), b.lin);
+        putBodyV3(D, a, 0, RSB_PW(BallP, ang), b.ang);
         return;
     }
     c.flags = carWord(D, a, s, RSB_PW(CarP, flags));
-    c.boost = carFloat(D, a, s, RSB_PW(CarP, boost));
     if (!(c.flags & CF_DEMOED)) {
+        const uint32_t flags0 = c.flags;
+        c.boost = carFloat(D, a, s, RSB_PW(CarP, boost));
         c.supersonicTime = carFloat(D, a, s, RSB_PW(CarP, supersonicTime));
         c.carContactCooldown = carFloat(D, a, s, RSB_PW(CarP, carContactCooldown));
+        const float supersonic0 = c.supersonicTime, cooldown0 = c.carContactCooldown;
         const CtlRec& ctl = D.controls[D.carOffset[a] + s];
+#pragma unroll
         for (int k = 0; k < 5; k++) c.ctl[k] = clampf(ctl.v[k], -1, 1);
         c.ctlBits = (ctl.jump ? 1u : 0u) | (ctl.boost ? 2u : 0u) | (ctl.handbrake ? 4u : 0u);
-        c.velCache = (info & BI_CACHE) ? tempV3(D, T.cache, a, t.b, 0) : v3zero();
-        struct {
-            const WorldParams* P;
-            OneBody b;
-            OneCar c;
-        } W{&D.P, {b}, {c}};
-        carPostTick(W, s);
-        b = W.b.v;
-        c = W.c.v;
-        putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
-        putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+        c.velCache = (info & BI_CACHE) ? tempV3(D, T.cache, a, i, 0) : v3zero();
+        carPostTick(t, s);
+        putBodyV3(D, a, i, RSB_PW(CarP, lin), b.lin);
+        putBodyV3(D, a, i, RSB_PW(CarP, ang), b.ang);
+#pragma unroll
         for (int r = 0; r < 3; r++) putCarV3(D, a, s, RSB_PW(CarP, rotMat) + 3 * r, c.rotMat.r[r]);
-        putCarWord(D, a, s, RSB_PW(CarP, flags), c.flags);
-        putCarFloat(D, a, s, RSB_PW(CarP, supersonicTime), c.supersonicTime);
-        putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), c.carContactCooldown);
+        if (c.flags != flags0) putCarWord(D, a, s, RSB_PW(CarP, flags), c.flags);
+        if (f2u(c.supersonicTime) != f2u(supersonic0)) putCarFloat(D, a, s, RSB_PW(CarP, supersonicTime), c.supersonicTime);
+        if (f2u(c.carContactCooldown) != f2u(cooldown0))
+            putCarFloat(D, a, s, RSB_PW(CarP, carContactCooldown), c.carContactCooldown);
+#pragma unroll
         for (int k = 0; k < 5; k++) putCarFloat(D, a, s, RSB_PW(CarP, lastCtl) + k, c.lastCtl[k]);
         putCarWord(D, a, s, RSB_PW(CarP, lastCtlBits), c.lastCtlBits);
         t.pads = c.boost < 100;
     } else if (moves) {
         // demoed in this tick: integrated, then left alone
-        putBodyV3(D, a, t.b, RSB_PW(CarP, lin), b.lin);
-        putBodyV3(D, a, t.b, RSB_PW(CarP, ang), b.ang);
+        putBodyV3(D, a, i, RSB_PW(CarP, lin), b.lin);
+        putBodyV3(D, a, i, RSB_PW(CarP, ang), b.ang);
     }
     const uint64_t hit = (uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitTick)) |
                          ((uint64_t)carWord(D, a, s, RSB_PW(CarP, ballHitTick) + 1) << 32);
@@ -1574,18 +1608,18 @@ RSB_HD void finishBody(const EngineView& D, const StepTemp& T, FinishThread& t, 
 // the last writer of the reference's loop over the cars in reverse creation order).
 RSB_HD void finishPads(const EngineView& D, FinishThread& t, FinishShared& sh) {
     if (!t.pads) return;
-    const V3 carPos = t.body.xf.o * kBtToUu;
+    const V3 carPos = t.b.v.xf.o * kBtToUu;
     if (carPos.z > PAD_CYL_HEIGHT + 250.f) return;
     const int ix = (int)(carPos.x / 1024.f + 4.f), iy = (int)(carPos.y / 1024.f + 5.f);
     for (int i = imax_(ix - 1, 0); i <= imin_(ix + 1, 7); i++)
         for (int j = imax_(iy - 1, 0); j <= imin_(iy + 1, 9); j++) {
             const int p = D.P.padGrid[i * 10 + j];
             if (p < 0) continue;
-            if (padCollides(D.P, p, t.body.xf, sh.prevLocked[p][t.la] == (uint32_t)t.b)) {
+            if (padCollides(D.P, p, t.b.v.xf, sh.prevLocked[p][t.la] == (uint32_t)t.body)) {
 #if defined(__CUDA_ARCH__)
-                atomicMin(&sh.locked[p][t.la], t.b - 1);
+                atomicMin(&sh.locked[p][t.la], t.body - 1);
 #else
-                sh.locked[p][t.la] = imin_(sh.locked[p][t.la], t.b - 1);
+                sh.locked[p][t.la] = imin_(sh.locked[p][t.la], t.body - 1);
 #endif
             }
         }
@@ -1615,10 +1649,10 @@ RSB_HD void finishPad(const EngineView& D, int a, int la, int p, FinishShared& s
 // The boost of the pads a car took.  The amounts are added one by one and clamped, so their
 // order does not matter: equal amounts commute, and a big pad fills the tank.
 RSB_HD void finishBoost(const EngineView& D, const FinishThread& t, const FinishShared& sh) {
-    const int s = t.b - 1;
+    const int s = t.body - 1;
     const uint32_t n = sh.picked[s][t.la];
     if (!n) return;
-    float boost = t.c.boost;
+    float boost = t.c.v.boost;
     for (uint32_t k = 0; k < (n & 0xffffu); k++) boost = fmin_(boost + PAD_BOOST_AMOUNT_SMALL, BOOST_MAX);
     for (uint32_t k = 0; k < (n >> 16); k++) boost = fmin_(boost + PAD_BOOST_AMOUNT_BIG, BOOST_MAX);
     putCarFloat(D, t.a, s, RSB_PW(CarP, boost), boost);
@@ -1627,11 +1661,8 @@ RSB_HD void finishBoost(const EngineView& D, const FinishThread& t, const Finish
 // Arena counters, by the ball's thread.
 RSB_HD void finishArena(const EngineView& D, const FinishThread& t, const FinishShared& sh) {
     const int a = t.a;
-    struct {
-        OneBody b;
-    } W{{t.body}};
-    const bool scored = ballScored(W, D.P.goalBaseY, D.P.ballRadiusUu);
-    const int side = W.b.v.xf.o.y > 0 ? 0 : 1;
+    const bool scored = ballScored(t, D.P.goalBaseY, D.P.ballRadiusUu);
+    const int side = t.b.v.xf.o.y > 0 ? 0 : 1;
     auto put = [&](int w, uint32_t v) { D.arena[(size_t)w * D.N + a] = v; };
     if (scored && (int32_t)arenaWord(D, a, RSB_PW(ArenaP, goalTeam)) < 0) put(RSB_PW(ArenaP, goalTeam), (uint32_t)side);
     put(RSB_PW(ArenaP, scored), scored ? (side == 0 ? 1u : 2u) : 0u);

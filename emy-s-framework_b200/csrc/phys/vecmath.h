@@ -227,6 +227,18 @@ RSB_HD M3 m3fromQuat(Quat q) {
               r20 * s, r21 * s, r22 * s + 1.f);
 }
 // btMatrix3x3::getRotation (SSE path)
+// One case of quatFromM3: largest diagonal element I, the next two in cyclic order J, K.
+// (Compile-time indices: a matrix indexed at run time would live in thread-local memory, with
+// whatever structure holds it.)
+template <int I, int J, int K>
+RSB_HD float quatCase(const M3& m, float* t) {
+    const float x = m.r[I][I] - m.r[J][J] - m.r[K][K] + 1.f;
+    t[3] = m.r[K][J] - m.r[J][K];
+    t[J] = m.r[J][I] + m.r[I][J];
+    t[K] = m.r[K][I] + m.r[I][K];
+    t[I] = x;
+    return x;
+}
 RSB_HD Quat quatFromM3(const M3& m) {
     float trace = m.r[0].x + m.r[1].y + m.r[2].z;
     float t[4];
@@ -237,20 +249,10 @@ RSB_HD Quat quatFromM3(const M3& m) {
         t[1] = m.r[0].z - m.r[2].x;
         t[2] = m.r[1].x - m.r[0].y;
         t[3] = x;
+    } else if (m.r[0].x < m.r[1].y) {
+        x = m.r[1].y < m.r[2].z ? quatCase<2, 0, 1>(m, t) : quatCase<1, 2, 0>(m, t);
     } else {
-        int i, j, k;
-        if (m.r[0].x < m.r[1].y) {
-            if (m.r[1].y < m.r[2].z) { i = 2; j = 0; k = 1; }
-            else { i = 1; j = 2; k = 0; }
-        } else {
-            if (m.r[0].x < m.r[2].z) { i = 2; j = 0; k = 1; }
-            else { i = 0; j = 1; k = 2; }
-        }
-        x = m.r[i][i] - m.r[j][j] - m.r[k][k] + 1.f;
-        t[3] = m.r[k][j] - m.r[j][k];
-        t[j] = m.r[j][i] + m.r[i][j];
-        t[k] = m.r[k][i] + m.r[i][k];
-        t[i] = x;
+        x = m.r[0].x < m.r[2].z ? quatCase<2, 0, 1>(m, t) : quatCase<0, 1, 2>(m, t);
     }
     float s = fsqrt(x);
     s = 0.5f / s;

@@ -79,6 +79,9 @@ struct World {
     RegOrder reg;
 };
 
+// The point pool of a world (step_phases.h has worlds that keep it apart).
+RSB_HD BlockPool& poolOf(World& W) { return W.pool; }
+
 // world status bits (per-arena status word)
 enum : uint32_t { WS_NONFINITE = 1u, WS_OVERFLOW = 2u, WS_CULL_MISS = 8u, WS_EPA_OVERFLOW = 16u };  // 4 is reserved (rsb.h)
 
@@ -444,7 +447,7 @@ RSB_HD bool ballTriContact(const WorldParams& P, const Xf& ballXf, float cbt, co
 template <class WT>
 RSB_HD void addBallTriContact(WT& W, int mesh, int tri, const V3* v, V3 normal, V3 point, float depth, Manifold& man) {
     ObjRef rMesh = objRef(W, mesh), rBall = objRef(W, OBJ_BALL);
-    int idx = addContact(man, W.pool, mesh, rMesh, OBJ_BALL, rBall, normal, point, depth);
+    int idx = addContact(man, poolOf(W), mesh, rMesh, OBJ_BALL, rBall, normal, point, depth);
     if (idx >= 0) {
         MPoint& cp = man.pt[idx];
         cp.index1 = tri;
@@ -482,25 +485,32 @@ RSB_HD void collideBallMesh(WT& W, int mesh, Manifold& man) {
     if (man.n) refreshContactPoints(man, W.b[0].xf, xfIdentity());
 }
 
+// The ball's deepest point toward a plane (in the plane's frame) and its distance.
+RSB_HD float ballPlaneDistance(const ArenaStatic& S, const WorldParams& P, int plane, const Xf& ballXf, V3& vip) {
+    const Xf planeXf{m3identity(), S.planeOrigin[plane - MAX_MESHES]};
+    V3 pn = S.planeNormal[plane - MAX_MESHES];
+    float pc = 0.f;
+    Xf planeInConvex = xfMul(xfInverse(ballXf), planeXf);
+    Xf convexInPlane = xfMul(xfInverse(planeXf), ballXf);
+    V3 vtx = sphereSupport(planeInConvex.b * (-pn), P.ballMargin);
+    vip = xfPoint(convexInPlane, vtx);
+    return dot(pn, vip) - pc;
+}
+
 // Ball vs static plane: btConvexPlaneCollisionAlgorithm (swapped pair (plane, ball))
 template <class WT>
 RSB_HD void collideBallPlane(WT& W, int plane, Manifold& man) {
-    const WorldParams& P = *W.P;
     ObjRef rPlane = objRef(W, plane), rBall = objRef(W, OBJ_BALL);
     V3 pn = W.S->planeNormal[plane - MAX_MESHES];
-    float pc = 0.f;
-    Xf planeInConvex = xfMul(xfInverse(rBall.xf), rPlane.xf);
-    Xf convexInPlane = xfMul(xfInverse(rPlane.xf), rBall.xf);
     if (!cullSkip(W, 0)) {
-        V3 vtx = sphereSupport(planeInConvex.b * (-pn), P.ballMargin);
-        V3 vip = xfPoint(convexInPlane, vtx);
-        float distance = dot(pn, vip) - pc;
+        V3 vip;
+        float distance = ballPlaneDistance(*W.S, *W.P, plane, rBall.xf, vip);
         if (distance < man.cbt + 0.f) {
             cullCheck(W, 0, true);
             V3 proj = vip - pn * distance;
             V3 world = xfPoint(rPlane.xf, proj);
             V3 nb = rPlane.xf.b * pn;
-            int idx = addContact(man, W.pool, plane, rPlane, OBJ_BALL, rBall, nb, world, distance);
+            int idx = addContact(man, poolOf(W), plane, rPlane, OBJ_BALL, rBall, nb, world, distance);
             if (idx >= 0) man.pt[idx].special = 1;
         }
     }
@@ -675,7 +685,7 @@ RSB_HD void addBoxTriContact(WT& W, int mesh, int ci, int tri, const V3* v, V3 n
                              Manifold& man) {
     int carObj = OBJ_CAR0 + ci;
     ObjRef rMesh = objRef(W, mesh), rCar = objRef(W, carObj);
-    int idx = addContact(man, W.pool, mesh, rMesh, carObj, rCar, normal, point, dist);
+    int idx = addContact(man, poolOf(W), mesh, rMesh, carObj, rCar, normal, point, dist);
     if (idx >= 0 && carResponds(W, ci)) {
         MPoint& cp = man.pt[idx];
         cp.index1 = tri;
@@ -718,26 +728,33 @@ RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold&
     if (man.n) refreshContactPoints(man, W.b[1 + ci].xf, xfIdentity());
 }
 
+// The car box's deepest point toward a plane (in the plane's frame) and its distance.
+RSB_HD float boxPlaneDistance(const ArenaStatic& S, const CarParams& C, int plane, const Xf& childXf, V3& vip) {
+    const Xf planeXf{m3identity(), S.planeOrigin[plane - MAX_MESHES]};
+    V3 pn = S.planeNormal[plane - MAX_MESHES];
+    ConvexShape box = carBoxShape(C);
+    Xf planeInConvex = xfMul(xfInverse(childXf), planeXf);
+    Xf convexInPlane = xfMul(xfInverse(planeXf), childXf);
+    V3 vtx = supportVirtual(box, planeInConvex.b * (-pn));
+    vip = xfPoint(convexInPlane, vtx);
+    return dot(pn, vip) - 0.f;
+}
+
 // Car box vs a static plane: btConvexPlaneCollisionAlgorithm owning its manifold
 template <class WT>
 RSB_HD void collideBoxPlane(WT& W, int plane, int ci, const Xf& childXf, Manifold& man) {
-    const CarParams& C = W.P->car;
     int carObj = OBJ_CAR0 + ci;
     ObjRef rPlane = objRef(W, plane), rCar = objRef(W, carObj);
-    ConvexShape box = carBoxShape(C);
     V3 pn = W.S->planeNormal[plane - MAX_MESHES];
-    Xf planeInConvex = xfMul(xfInverse(childXf), rPlane.xf);
-    Xf convexInPlane = xfMul(xfInverse(rPlane.xf), childXf);
     if (!cullSkip(W, 1 + ci)) {
-        V3 vtx = supportVirtual(box, planeInConvex.b * (-pn));
-        V3 vip = xfPoint(convexInPlane, vtx);
-        float distance = dot(pn, vip) - 0.f;
+        V3 vip;
+        float distance = boxPlaneDistance(*W.S, W.P->car, plane, childXf, vip);
         if (distance < man.cbt + 0.f) {
             cullCheck(W, 1 + ci, true);
             V3 proj = vip - pn * distance;
             V3 world = xfPoint(rPlane.xf, proj);
             V3 nb = rPlane.xf.b * pn;
-            int idx = addContact(man, W.pool, plane, rPlane, carObj, rCar, nb, world, distance);
+            int idx = addContact(man, poolOf(W), plane, rPlane, carObj, rCar, nb, world, distance);
             if (idx >= 0 && carResponds(W, ci)) onCarWorld(W, ci, man.pt[idx]);
         }
     }
@@ -777,7 +794,7 @@ RSB_HD int carBallContact(WT& W, int ci, const Xf& childXf, Manifold& man) {
     GjkOut g = gjkPairDetector(W.epa, box, childXf, sph, rBall.xf, maxDist2);
     if (g.overflow) W.status |= WS_EPA_OVERFLOW;
     if (!g.has) return -1;
-    return addContact(man, W.pool, OBJ_BALL, rBall, carObj, rCar, g.normal, g.point, g.dist);
+    return addContact(man, poolOf(W), OBJ_BALL, rBall, carObj, rCar, g.normal, g.point, g.dist);
 }
 
 // (ball, car) pair: swapped compound over a btConvexConvexAlgorithm that creates its
@@ -832,7 +849,7 @@ RSB_HD void collideCarCar(World& W, int ca, int cb) {
             carCarContacts(W, ca, cb, bc);
             bool responds = carResponds(W, ca) && carResponds(W, cb);
             for (int k = 0; k < bc.n; k++) {
-                int idx = addContact(man, W.pool, objA, rA, objB, rB, bc.c[k].normalOnB, bc.c[k].point, bc.c[k].depth);
+                int idx = addContact(man, poolOf(W), objA, rA, objB, rB, bc.c[k].normalOnB, bc.c[k].point, bc.c[k].depth);
                 if (idx >= 0 && responds) onCarCar(W, cb, ca, man.pt[idx]);
             }
             if (man.n) refreshContactPoints(man, rB.xf, rA.xf);

@@ -761,8 +761,9 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
         if (h->maxCars > 0) {
             rayKernel<<<groups, carThreads, 0, st>>>(D, T);
             sv.ray<<<rayGrid, block, 0, st>>>(D, T);
+            driveKernel<<<groups, carThreads, 0, st>>>(D, T);
         }
-        bodyKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
+        pairKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
         findKernel<<<pairGrid, block, 0, st>>>(D, T);
         sv.triangle<<<triGrid, block, 0, st>>>(D, T);
         deepKernel<<<deepGrid, block, 0, st>>>(D, T);

@@ -1,6 +1,6 @@
 // Kernels of the step: the phases of phys/step_phases.h on the device.
 //
-// A block of the ray, body and finish kernels serves 32 arenas, one warp per car or body: lanes
+// A block of the ray, drive, pair and finish kernels serves 32 arenas, one warp per car or body: lanes
 // run over arenas, so every record word is read and written coalesced, and the bodies of an
 // arena exchange what the reference's order needs through shared memory.  The queue kernels
 // (heavy rays, contacts, islands) run one queued item per thread; their counts are known on the
@@ -108,48 +108,64 @@ __global__ void __launch_bounds__(128, MINB) heavyRayKernel(const __grid_constan
     blockStats(D, st);
 }
 
-__global__ void __launch_bounds__(BODY_THREADS) bodyKernel(const __grid_constant__ EngineView D,
-                                                           const __grid_constant__ StepTemp T, bool firstTick) {
-    __shared__ BodyShared sh;
+// The car's state and its four wheels fill about 250 registers; held to 168, two blocks share an
+// SM at the price of some spills: 183 us against 265 at 3v3 x 65,536.
+__global__ void __launch_bounds__(CAR_THREADS, 2) driveKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T) {
+    __shared__ DriveShared sh;
     const int lane = threadIdx.x & 31;
-    BodyThread t;
-    t.b = threadIdx.x >> 5;
+    DriveThread t;
+    t.s = threadIdx.x >> 5;
     t.la = lane;
     t.a = blockIdx.x * PHASE_ARENAS + lane;
-    t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
     t.finished = true;
     t.deps = 0;
-    const bool valid = t.b < t.nb;
+    const bool valid = t.a < D.N && 1 + t.s < arenaBodies(D, t.a);
     if (blockIdx.x == 0 && threadIdx.x == 0) T.count[QC_RAY] = T.count[QC_BODYRAY] = 0;  // the queued rays are cast
-    if (threadIdx.x < PHASE_ARENAS) sh.done[lane] = sh.need[lane] = 0;
-    if (valid) bodyLoad(D, T, t, sh);
+    if (threadIdx.x < PHASE_ARENAS) sh.done[lane] = 0;
+    if (valid) driveLoad(D, T, t, sh);
     __syncthreads();
-    if (valid && t.b > 0 && t.finished) atomicOr(&sh.done[lane], 1u << (t.b - 1));
+    if (valid && t.finished) atomicOr(&sh.done[lane], 1u << t.s);
     __syncthreads();
     // a car waits only for cars of higher slots, so every round finishes the highest one left
     for (int round = 0; round <= MAX_CARS; round++) {
         const bool ready = !t.finished && !(t.deps & ~sh.done[lane]);
-        if (ready) bodyDrive(t, sh);
+        if (ready) driveRun(t, sh);
         const int all = __syncthreads_and(t.finished);
         if (all) break;
-        if (ready) atomicOr(&sh.done[lane], 1u << (t.b - 1));
+        if (ready) atomicOr(&sh.done[lane], 1u << t.s);
         __syncthreads();
     }
-    if (valid) bodyMove(D, T, t, sh, firstTick);
+    if (valid) driveStore(D, T, t);
+}
+
+__global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T, bool firstTick) {
+    __shared__ PairShared sh;
+    const int lane = threadIdx.x & 31;
+    PairThread t;
+    t.b = threadIdx.x >> 5;
+    t.la = lane;
+    t.a = blockIdx.x * PHASE_ARENAS + lane;
+    t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
+    const bool valid = t.b < t.nb;
+    if (threadIdx.x < PHASE_ARENAS) sh.need[lane] = 0;
+    if (valid) pairLoad(D, T, t, sh, firstTick);
     __syncthreads();
-    if (valid) bodyPick(D, t, sh);
+    if (valid) pairPick(D, t, sh);
     __syncthreads();
     PhaseStats st{0, 0, 0, 0};
     BodyStatics o;
     o.meshes = o.planes = 0;
     uint32_t dyn = 0;
     if (valid) {
-        o = bodyStatics(D, T, t, st);
-        dyn = bodyDynamics(D, t, sh);
+        o = pairStatics(D, t, st);
+        dyn = pairDynamics(D, t, sh);
     }
     const uint32_t m0 = queueAlloc(&T.count[t.b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)__popc(o.meshes));
+    const uint32_t p0 = queueAlloc(&T.count[QC_PLANE], (uint32_t)__popc(o.planes));
     const uint32_t d0 = queueAlloc(&T.count[t.b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)__popc(dyn));
-    if (valid) bodyStore(D, T, t, sh, o, dyn, m0, d0);
+    if (valid) pairStore(D, T, t, sh, o, dyn, m0, p0, d0);
     __syncthreads();
     if (threadIdx.x < PHASE_ARENAS) {
         const bool need = sh.need[lane] != 0;
@@ -170,11 +186,14 @@ __global__ void __launch_bounds__(128) findKernel(const __grid_constant__ Engine
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constant__ EngineView D,
                                                             const __grid_constant__ StepTemp T) {
-    const uint32_t n[2] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR]};
-    forItems<2>(n, [&](int k, uint32_t i) {
+    PhaseStats st{0, 0, 0, 0};
+    const uint32_t n[3] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR], T.count[QC_PLANE]};
+    forItems<3>(n, [&](int k, uint32_t i) {
         if (k == 0) trianglePhase(D, T, i);
-        else carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
+        else if (k == 1) carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
+        else planePhase(D, T, (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + i, st);
     });
+    blockStats(D, st);
 }
 
 __global__ void __launch_bounds__(128) deepKernel(const __grid_constant__ EngineView D,
@@ -208,11 +227,11 @@ __global__ void __launch_bounds__(BODY_THREADS) finishKernel(const __grid_consta
     __shared__ FinishShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     FinishThread t;
-    t.b = warp;
+    t.body = warp;
     t.la = lane;
     t.a = blockIdx.x * PHASE_ARENAS + lane;
     t.nb = t.a < D.N ? arenaBodies(D, t.a) : 0;
-    const bool valid = t.b < t.nb, pads = t.nb > 1;
+    const bool valid = t.body < t.nb, pads = t.nb > 1;
     if (blockIdx.x == 0 && threadIdx.x >= QC_CARMESH && threadIdx.x < QC_WORDS) T.count[threadIdx.x] = 0;
     if (pads)
         for (int p = warp; p < NUM_PADS; p += warps) padLoad(D, t.a, lane, p, sh);
@@ -221,14 +240,14 @@ __global__ void __launch_bounds__(BODY_THREADS) finishKernel(const __grid_consta
     __syncthreads();
     if (valid) {
         finishBody(D, T, t, sh);
-        if (t.b > 0) finishPads(D, t, sh);
+        if (t.body > 0) finishPads(D, t, sh);
     }
     __syncthreads();
     if (pads)
         for (int p = warp; p < NUM_PADS; p += warps) finishPad(D, t.a, lane, p, sh);
     __syncthreads();
     if (!valid) return;
-    if (t.b > 0) finishBoost(D, t, sh);
+    if (t.body > 0) finishBoost(D, t, sh);
     else finishArena(D, t, sh);
 }
 

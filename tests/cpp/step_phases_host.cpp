@@ -62,9 +62,11 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     T.deepQ = deepQ.data();
     T.combineQ = combineQ.data();
     std::unique_ptr<EpaWork> epa(new EpaWork());
-    std::unique_ptr<BodyShared> sh(new BodyShared());
+    std::unique_ptr<DriveShared> ds(new DriveShared());
+    std::unique_ptr<PairShared> sh(new PairShared());
     std::unique_ptr<FinishShared> fs(new FinishShared());
-    std::vector<BodyThread> bt(MAX_BODIES * PHASE_ARENAS);
+    std::vector<DriveThread> dt(MAX_CARS * PHASE_ARENAS);
+    std::vector<PairThread> bt(MAX_BODIES * PHASE_ARENAS);
     std::vector<FinishThread> ft(MAX_BODIES * PHASE_ARENAS);
     PhaseStats st{0, 0, 0, 0};
     for (int tick = 0; tick < ticks; tick++) {
@@ -93,44 +95,59 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
             counts[k] += T.count[k];
             while (T.count[k] > 0) heavyRayPhase(D, T, T.rayQ[(k == QC_RAY ? 0 : R) + --T.count[k]], st);
         }
-        // bodies
+        // cars
+        for (int g = 0; g < h->N; g += PHASE_ARENAS) {
+            auto each = [&](auto&& fn) {
+                for (int s = MAX_CARS - 1; s >= 0; s--)
+                    for (int la = 0; la < PHASE_ARENAS && g + la < h->N; la++)
+                        if (1 + s < arenaBodies(D, g + la)) fn(dt[s * PHASE_ARENAS + la], s, la);
+            };
+            std::memset(ds->done, 0, sizeof ds->done);
+            each([&](DriveThread& t, int s, int la) {
+                t.s = s;
+                t.la = la;
+                t.a = g + la;
+                driveLoad(D, T, t, *ds);
+                if (t.finished) ds->done[la] |= 1u << s;
+            });
+            for (bool all = false; !all;) {
+                std::vector<DriveThread*> ran;
+                all = true;
+                each([&](DriveThread& t, int, int la) {
+                    if (!t.finished && !(t.deps & ~ds->done[la])) {
+                        driveRun(t, *ds);
+                        ran.push_back(&t);
+                    }
+                });
+                for (DriveThread* t : ran) ds->done[t->la] |= 1u << t->s;
+                each([&](DriveThread& t, int, int) { all &= t.finished; });
+                if (!all && ran.empty()) return -1;
+            }
+            each([&](DriveThread& t, int, int) { driveStore(D, T, t); });
+        }
+        // pairs
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {
             auto each = [&](auto&& fn) {
                 for (int b = MAX_BODIES - 1; b >= 0; b--)
                     for (int la = 0; la < PHASE_ARENAS && g + la < h->N; la++)
                         if (b < arenaBodies(D, g + la)) fn(bt[b * PHASE_ARENAS + la], b, la);
             };
-            std::memset(sh->done, 0, sizeof sh->done);
             std::memset(sh->need, 0, sizeof sh->need);
-            each([&](BodyThread& t, int b, int la) {
+            each([&](PairThread& t, int b, int la) {
                 t.b = b;
                 t.la = la;
                 t.a = g + la;
                 t.nb = arenaBodies(D, t.a);
-                bodyLoad(D, T, t, *sh);
-                if (b > 0 && t.finished) sh->done[la] |= 1u << (b - 1);
+                pairLoad(D, T, t, *sh, tick == 0);
             });
-            for (bool all = false; !all;) {
-                std::vector<BodyThread*> ran;
-                all = true;
-                each([&](BodyThread& t, int, int la) {
-                    if (!t.finished && !(t.deps & ~sh->done[la])) {
-                        bodyDrive(t, *sh);
-                        ran.push_back(&t);
-                    }
-                });
-                for (BodyThread* t : ran) sh->done[t->la] |= 1u << (t->b - 1);
-                each([&](BodyThread& t, int, int) { all &= t.finished; });
-                if (!all && ran.empty()) return -1;
-            }
-            each([&](BodyThread& t, int, int) { bodyMove(D, T, t, *sh, tick == 0); });
-            each([&](BodyThread& t, int, int) { bodyPick(D, t, *sh); });
-            each([&](BodyThread& t, int b, int) {
-                const BodyStatics o = bodyStatics(D, T, t, st);
-                const uint32_t dyn = bodyDynamics(D, t, *sh);
+            each([&](PairThread& t, int, int) { pairPick(D, t, *sh); });
+            each([&](PairThread& t, int b, int) {
+                const BodyStatics o = pairStatics(D, t, st);
+                const uint32_t dyn = pairDynamics(D, t, *sh);
                 const uint32_t m0 = phaseAtomicAdd(&T.count[b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)bitCount(o.meshes));
+                const uint32_t p0 = phaseAtomicAdd(&T.count[QC_PLANE], (uint32_t)bitCount(o.planes));
                 const uint32_t d0 = phaseAtomicAdd(&T.count[b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)bitCount(dyn));
-                bodyStore(D, T, t, *sh, o, dyn, m0, d0);
+                pairStore(D, T, t, *sh, o, dyn, m0, p0, d0);
             });
             for (int la = 0; la < PHASE_ARENAS; la++)
                 if (sh->need[la]) T.solveQ[T.count[QC_SOLVE]++] = (uint32_t)(g + la);
@@ -145,6 +162,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
             }
         }
         for (uint32_t i = std::min(T.count[QC_TRI], T.candCap); i-- > 0;) trianglePhase(D, T, i);
+        for (uint32_t i = T.count[QC_PLANE]; i-- > 0;) planePhase(D, T, (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + i, st);
         for (uint32_t i = T.count[QC_DEEP]; i-- > 0;) deepPhase(D, T, T.deepQ[i], epa.get(), st);
         for (uint32_t i = T.count[QC_COMBINE]; i-- > 0;) combinePhase(D, T, T.combineQ[i], st);
         for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], st);
@@ -164,7 +182,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
             std::memset(fs->picked, 0, sizeof fs->picked);
             std::memset(fs->touched, 0, sizeof fs->touched);
             each([&](FinishThread& t, int b, int la) {
-                t.b = b;
+                t.body = b;
                 t.la = la;
                 t.a = g + la;
                 t.nb = arenaBodies(D, t.a);
