@@ -16,7 +16,8 @@
 //   triangles .. one candidate per thread: box-triangle and box-sphere GJK; box-box and plane pairs
 //   deep ....... the candidates whose GJK needs the penetration solver
 //   combine .... one pair per thread: its candidates' contacts into the manifold, in walk order
-//   islands .... the queued arenas: contact callbacks, islands, solver (solveIslands)
+//   islands .... bodies whose contacts are all with static objects, one per thread; the arenas
+//                with pairs of bodies: contact callbacks, islands, solver (solveIslands)
 //   finish ..... integration, post-tick updates, boost pads, goal and tick counters
 //
 // Between the phases a tick lives in the persistent records (state.h) and in StepTemp.  What
@@ -54,7 +55,7 @@ RSB_HD int dynPair(int lo, int hi) { return lo * (2 * MAX_BODIES - lo - 1) / 2 +
 
 // Queue counters.
 enum : int {
-    QC_RAY = 0, QC_BODYRAY, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_TRI, QC_DEEP, QC_COMBINE,
+    QC_RAY = 0, QC_BODYRAY, QC_CARMESH, QC_BALLMESH, QC_CARBALL, QC_CARCAR, QC_PLANE, QC_BLOCK, QC_SOLVE, QC_BODY, QC_TRI, QC_DEEP, QC_COMBINE,
     QC_WORDS
 };
 constexpr int NUM_TASK_TYPES = 4;  // QC_CARMESH .. QC_CARCAR
@@ -123,13 +124,15 @@ struct StepTemp {
     PairResult* results;
     MPoint* blocks;      // [MAX_BLOCKS * N][MAX_POINTS]
     uint32_t blockCap;
-    uint32_t* solveQ;    // [N]
+    uint32_t* solveQ;    // arenas with pairs of bodies [N]
+    uint32_t* bodyQ;     // bodies with contacts in the others, b * N + a [MAX_BODIES * N]
     uint32_t* first;     // first candidate of each pair, as results
     Candidate* cand;     // [candCap]
     CandidateOut* out;   // [candCap]
     uint32_t candCap;
     uint32_t* deepQ;     // [CAP_RESULTS * N + candCap]
     uint32_t* combineQ;  // [CAP_RESULTS * N]
+    uint32_t sms;        // multiprocessors of the device
 };
 
 // Static-test counters of one thread (rsb_stats).
@@ -540,7 +543,7 @@ struct PairShared {
     uint32_t stamp[MAX_BODIES][PHASE_ARENAS];
     uint32_t pick[MAX_BODIES][PHASE_ARENAS];  // BI_DYN word of each body
     uint32_t live[MAX_BODIES][PHASE_ARENAS];  // 1: active (objActive)
-    uint32_t need[PHASE_ARENAS];              // the arena has contacts or dynamic pairs to solve
+    uint32_t need[PHASE_ARENAS];              // PN_* sums over the arena's bodies
 };
 
 struct OneBody {
@@ -596,6 +599,16 @@ RSB_HD GroundRef groundRef(const CarWorld& W, int o) {
         g.invMass = W.P->car.invMass;
     }
     return g;
+}
+
+// Sums over an arena's bodies: pairs that can be in contact (8 bits), static pairs (8 bits), and
+// whether any pair of bodies exists.  Without such pairs every island is one body, solved by
+// itself, unless the arena's contacts might not fit its pools, whose limits run over all bodies.
+constexpr uint32_t PN_PAIR = 1u << 8, PN_DYN = 1u << 24;
+constexpr int BODY_MAX_TASKS = 14;  // MAX_BLOCKS blocks, and MAX_CONTACT_ROWS rows with the special rows
+RSB_HD bool arenaHasContacts(uint32_t need) { return (need & 255u) != 0 || need >= PN_DYN; }
+RSB_HD bool arenaByBodies(uint32_t need) {
+    return need < PN_DYN && (need & 255u) <= (uint32_t)BODY_MAX_TASKS && ((need >> 8) & 255u) <= (uint32_t)MAX_PAIRS;
 }
 
 // One car's thread of the drive phase.
@@ -1020,8 +1033,8 @@ RSB_HD uint32_t pairDynamics(const EngineView& D, const PairThread& t, const Pai
 
 // Stores the body's pair information and fills its queue places: `mesh0` the first of its mesh
 // pairs in their queue, `plane0` of its plane contacts, `dyn0` of its dynamic pairs.
-RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& t, PairShared& sh,
-                      const BodyStatics& o, uint32_t dynMani, uint32_t mesh0, uint32_t plane0, uint32_t dyn0) {
+RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& t, const BodyStatics& o,
+                      uint32_t dynMani, uint32_t mesh0, uint32_t plane0, uint32_t dyn0) {
     const int a = t.a;
     const Body& b = t.body.v;
     const int meshType = t.b == 0 ? QC_BALLMESH : QC_CARMESH, dynType = t.b == 0 ? QC_CARBALL : QC_CARCAR;
@@ -1046,8 +1059,12 @@ RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& 
         T.tasks[k] = PairTask{(uint32_t)a, (uint16_t)(OBJ_BALL + t.b), (uint16_t)(OBJ_BALL + hi)};
         T.dynRes[(size_t)dynPair(t.b, hi) * D.N + a] = k;
     }
-    // an arena without contacts and without dynamic pairs has nothing to solve
-    if (o.meshes | o.planes | dynMani | t.dyn) phaseAtomicOr(&sh.need[t.la], 1u);
+}
+
+RSB_HD void pairNeed(const PairThread& t, const BodyStatics& o, PairShared& sh) {
+    const uint32_t v = (uint32_t)bitCount(o.meshes) + (uint32_t)bitCount(o.planes) +
+                       PN_PAIR * (uint32_t)bitCount(o.pairs) + (t.dyn ? PN_DYN : 0u);
+    if (v) phaseAtomicAdd(&sh.need[t.la], v);
 }
 
 // ------------------------------------------------------------------ contacts
@@ -1316,6 +1333,266 @@ RSB_HD void carCarPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     for (int c = 0; c < bc.n; c++)
         addContact(m, pool, k.o0, rA, k.o1, rB, bc.c[c].normalOnB, bc.c[c].point, bc.c[c].depth);
     storePair(D, T, a, W, m, res);
+}
+
+// ------------------------------------------------------------------ islands of one body
+
+// Rows of a body against the fixed body: the general rows (SRow) without the fixed side, whose
+// vectors are zero, and without the constants (cfm = 0 * jacInv, limits).
+struct ContactRow1 {
+    V3 n, rc, ang;
+    float rhs, rhsPen, jacInv, friction, applied, push;
+    int32_t special;
+};
+struct FrictionRow1 {
+    V3 n, rc, ang;
+    float rhs, jacInv, applied;
+    int32_t contact;
+};
+constexpr int MAX_ROWS1 = BODY_MAX_TASKS * MAX_POINTS + 1;
+
+// setupContactConstraint and convertContactInner's friction row for one contact of the body.
+struct Solver1 {
+    V3 lin, ang, extF, extT;   // the solver body's velocities and external impulses
+    V3 dLin, dAng, push, turn;
+    V3 invMassV;
+    int nc, nf;
+    ContactRow1 c[MAX_ROWS1];
+    FrictionRow1 f[MAX_ROWS1];
+};
+RSB_HD void addRows1(Solver1& S, const Body& b, V3 normal, float dist, float fric, float rest, V3 rel, float dt,
+                     int special) {
+    ContactRow1& r = S.c[S.nc];
+    const float invDt = 1.f / dt;
+    const V3 torqueAxis = cross(rel, normal);
+    const V3 angA = b.invIw * torqueAxis;
+    const float denom0 = b.invMass + dot(normal, cross(angA, rel));
+    const float jacInv = 1.f / (denom0 + 0.f + 0.f);
+    const V3 vel = b.lin + cross(b.ang, rel);
+    const float relVel = dot(normal, vel - v3zero());
+    float restitution = restitutionCurve(relVel, rest);
+    if (restitution <= 0.f) restitution = 0.f;
+    const float v1 = dot(normal, S.lin + S.extF) + dot(torqueAxis, S.ang + S.extT);
+    const float rel1 = v1 + 0.f;
+    const float velErr = restitution - rel1;
+    const float penetration = dist + 0.f;
+    const float posErr = (penetration > 0) ? 0.f : -penetration * kErp2 * invDt;
+    r.n = normal;
+    r.rc = torqueAxis;
+    r.ang = angA;
+    r.rhsPen = posErr * jacInv;
+    r.rhs = velErr * jacInv;
+    r.jacInv = jacInv;
+    r.friction = fric;
+    r.applied = r.push = 0.f;
+    r.special = special;
+    // friction along the lateral velocity
+    const V3 v = (S.lin + S.extF + cross(S.ang + S.extT, rel)) - v3zero();
+    const float rv = dot(normal, v);
+    V3 lat = v - normal * rv;
+    const float latRel = length2(lat);
+    if (latRel > kEpsilon) {
+        lat *= 1.f / fsqrt(latRel);
+    } else {
+        V3 lat2;
+        planeSpace1(normal, lat, lat2);
+    }
+    FrictionRow1& fr = S.f[S.nf];
+    fr.n = lat;
+    fr.rc = cross(rel, lat);
+    fr.ang = b.invIw * fr.rc;
+    const float d0 = b.invMass + dot(lat, cross(fr.ang, rel));
+    fr.jacInv = 1.f / (d0 + 0.f);
+    const float fv1 = dot(lat, S.lin + S.extF) + dot(fr.rc, S.ang);
+    const float fvelErr = 0.f - (fv1 + 0.f);
+    fr.rhs = 0.f + fvelErr * fr.jacInv;
+    fr.applied = 0.f;
+    fr.contact = S.nc;
+    S.nc++;
+    S.nf++;
+}
+
+// resolveSingleConstraintRow* against the fixed body; returns the impulse.
+RSB_HD float solveRow1(Solver1& S, V3 n, V3 rc, V3 ang, float rhs, float cfm, float jacInv, float lo, float hi,
+                       bool generic, float& applied) {
+    const float applied0 = applied;
+    float delta = rhs - applied0 * cfm;
+    const float d1 = dot_simd(n, S.dLin) + dot_simd(rc, S.dAng);
+    delta = delta - d1 * jacInv;
+    delta = delta - 0.f * jacInv;
+    const float sum = applied0 + delta;
+    const bool lowerLess = sum < lo;
+    delta = lowerLess ? (lo - applied0) : delta;
+    applied = lowerLess ? lo : sum;
+    if (generic) {
+        const bool upperLess = sum < hi;
+        delta = upperLess ? delta : (hi - applied0);
+        applied = upperLess ? applied : hi;
+    }
+    S.dLin = S.dLin + (n * S.invMassV) * delta;
+    S.dAng = S.dAng + ang * delta;
+    return delta;
+}
+RSB_HD void iterate1(Solver1& S) {
+    for (int it = 0; it < kNumIterations; it++) {
+        bool any = false;
+        for (int j = 0; j < S.nc; j++) {
+            ContactRow1& c = S.c[j];
+            if (c.rhsPen == 0.f) continue;
+            const float applied0 = c.push;
+            float delta = c.rhsPen - applied0 * (0.f * c.jacInv);
+            const float d1 = dot_simd(c.n, S.push) + dot_simd(c.rc, S.turn);
+            delta = delta - d1 * c.jacInv;
+            delta = delta - 0.f * c.jacInv;
+            const float sum = applied0 + delta;
+            const bool lowerLess = sum < 0.f;
+            delta = lowerLess ? (0.f - applied0) : delta;
+            c.push = lowerLess ? 0.f : sum;
+            S.push = S.push + (c.n * S.invMassV) * delta;
+            S.turn = S.turn + c.ang * delta;
+            any |= delta != 0.f;
+        }
+        if (!any) break;
+    }
+    for (int it = 0; it < kNumIterations; it++) {
+        for (int j = 0; j < S.nc; j++) {
+            ContactRow1& c = S.c[j];
+            if (c.special) continue;
+            solveRow1(S, c.n, c.rc, c.ang, c.rhs, 0.f * c.jacInv, c.jacInv, 0.f, 1e10f, false, c.applied);
+        }
+        for (int j = 0; j < S.nf; j++) {
+            FrictionRow1& fr = S.f[j];
+            const ContactRow1& c = S.c[fr.contact];
+            const float total = c.applied;
+            if (total > 0.f)
+                solveRow1(S, fr.n, fr.rc, fr.ang, fr.rhs, 0.f, fr.jacInv, -(c.friction * total), c.friction * total, true,
+                          fr.applied);
+        }
+    }
+}
+
+// The place of body i's k-th manifold (in dispatch order) among its island's manifolds in the
+// order solveIslands takes them: its unstable sort of the arena's manifolds by island, here one
+// island per body, permutes manifolds of one island too.
+struct ManifoldOrder {
+    int32_t key[MAX_MANIFOLDS], idx[MAX_MANIFOLDS];
+    int n;
+};
+RSB_HD void manifoldOrder(const EngineView& D, const StepTemp& T, int a, int nb, ManifoldOrder& o) {
+    o.n = 0;
+    for (int i = 0; i < nb; i++) {
+        const uint32_t p = infoWord(D, T, a, i, BI_PAIRS);
+        const uint32_t act = (p & BI_ACT_MASK) >> BI_ACT_SHIFT;
+        // manifolds of sleeping and of non-responding bodies are not in the list
+        if (!(p & ((1u << NUM_STATICS) - 1u)) || act == ACT_SLEEPING || !(p & BI_RESPONDS)) continue;
+        const int cnt = bitCount(infoWord(D, T, a, i, BI_MANI));
+        for (int k = 0; k < cnt; k++) {
+            o.key[o.n] = i;
+            o.idx[o.n] = k;
+            o.n++;
+        }
+    }
+    uint32_t status = 0;
+    if (o.n > 1) quickSortKV(o.key, o.idx, 0, o.n - 1, status);
+}
+
+// Callbacks and solver of one body that touches static objects only.
+RSB_HD void bodyPhase(const EngineView& D, const StepTemp& T, uint32_t e, PhaseStats& st) {
+    const int a = (int)(e % (uint32_t)D.N), i = (int)(e / (uint32_t)D.N);
+    const float dt = D.P.dt;
+    const uint32_t info = infoWord(D, T, a, i, BI_PAIRS), mani = infoWord(D, T, a, i, BI_MANI),
+                   tasks = infoWord(D, T, a, i, BI_TASKS);
+    // the results of the body's manifolds, in dispatch order
+    const uint32_t mesh0 = (tasks & ((1u << MAX_MESHES) - 1u)) ? infoWord(D, T, a, i, BI_MESHRES) : 0u;
+    const uint32_t plane0 = (tasks >> MAX_MESHES) ? infoWord(D, T, a, i, BI_PLANERES) : 0u;
+    auto resultOf = [&](int s) -> const PairResult& {
+        return s < MAX_MESHES
+                   ? T.results[mesh0 + bitCount(tasks & ((1u << s) - 1u))]
+                   : T.results[plane0 + bitCount((tasks >> MAX_MESHES) & ((1u << (s - MAX_MESHES)) - 1u))];
+    };
+    uint32_t with = 0;  // manifolds that hold points
+    bool world = false;
+    V3 worldNormal = v3zero();
+    for (uint32_t m = tasks; m; m &= m - 1u) {
+        const int s = lowestBit(m);
+        const PairResult& r = resultOf(s);
+        if (r.n > 0) with |= 1u << s;
+        if (r.flags & PR_WORLD) {
+            world = true;
+            worldNormal = V3{r.normal[0], r.normal[1], r.normal[2]};
+        }
+    }
+    if (world) {
+        // onCarWorld's state; its material is in the points already
+        putCarV3(D, a, i - 1, RSB_PW(CarP, worldContactNormal), worldNormal);
+        putCarWord(D, a, i - 1, RSB_PW(CarP, flags), carWord(D, a, i - 1, RSB_PW(CarP, flags)) | CF_WORLD_CONTACT);
+    }
+    if (!with) return;  // the finish phase adds the external impulses
+    Body b;
+    bodyConstants(D, i, b);
+    b.xf = bodyXf(D, a, i);
+    b.lin = bodyV3(D, a, i, RSB_PW(CarP, lin));
+    b.ang = bodyV3(D, a, i, RSB_PW(CarP, ang));
+    updateInertia(b);
+    Solver1 S;
+    S.lin = b.lin;
+    S.ang = b.ang;
+    S.extF = (tempV3(D, T.force, a, i, 0) * b.invMass) * dt;
+    S.extT = tmul(tempV3(D, T.force, a, i, 3), b.invIw) * dt;
+    S.dLin = S.dAng = S.push = S.turn = v3zero();
+    S.invMassV = V3{b.invMass, b.invMass, b.invMass};
+    S.nc = S.nf = 0;
+    int spCount = 0;
+    float spFric = 0.f, spRest = 0.f, spDist = 0.f;
+    V3 spNormal = v3zero();
+    auto addManifold = [&](int s) {
+        const PairResult& r = resultOf(s);
+        const MPoint* pt = T.blocks + (size_t)MAX_POINTS * r.block;
+        for (int j = 0; j < r.n; j++) {
+            const MPoint& cp = pt[j];
+            const V3 rel = cp.posA - b.xf.o, normal = cp.normal;
+            if (cp.special) {
+                spCount++;
+                spFric = cp.fric;
+                spRest = cp.rest;
+                spNormal = spNormal + normal;
+                spDist = spDist + length(rel);
+            }
+            addRows1(S, b, normal, cp.dist, cp.fric, cp.rest, rel, dt, cp.special);
+        }
+    };
+    if (!(with & (with - 1u))) {
+        addManifold(lowestBit(with));
+    } else {
+        ManifoldOrder o;
+        manifoldOrder(D, T, a, arenaBodies(D, a), o);
+        for (int k = 0; k < o.n; k++) {
+            if (o.key[k] != i) continue;
+            uint32_t m = mani;
+            for (int q = 0; q < o.idx[k]; q++) m &= m - 1u;
+            const int s = lowestBit(m);
+            if ((with >> s) & 1u) addManifold(s);
+        }
+    }
+    if (spCount > 0) {
+        // convertContactSpecial
+        const float distance = spDist / (float)spCount;
+        const V3 normal = bdiv(spNormal, (float)spCount);
+        addRows1(S, b, normal, distance, spFric, spRest, normal * -distance, dt, 0);
+    }
+    st.nRows += (uint32_t)(S.nc + S.nf);
+    iterate1(S);
+    // writeBackBodies
+    S.lin = S.lin + S.dLin;
+    S.ang = S.ang + S.dAng;
+    if (S.push.x != 0.f || S.push.y != 0 || S.push.z != 0 || S.turn.x != 0.f || S.turn.y != 0 || S.turn.z != 0) {
+        if (i == 0) b.xf = integrateTransformNoRot(b.xf, S.push, dt);
+        else b.xf = integrateTransform(b.xf, S.push, S.turn * kSplitTurnErp, dt);
+        putBodyXf(D, a, i, b.xf);
+    }
+    putBodyV3(D, a, i, RSB_PW(CarP, lin), S.lin + S.extF);
+    putBodyV3(D, a, i, RSB_PW(CarP, ang), S.ang + S.extT);
+    infoWord(D, T, a, i, BI_PAIRS) = info | BI_SOLVED;
 }
 
 // ------------------------------------------------------------------ islands

@@ -207,13 +207,6 @@ static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
 // Resident warps per SM of a persistent launch (0 = as many as fit).
 static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
-// Warps per SM of the wide queue grids.  Few items per warp finish sooner, but a thread's local
-// memory shares its cache lines with its warp's other lanes, so the kernels that use much of it
-// lose by spreading.  Measured with 4 / 8 / 16 / 32 / 64, us per tick, 3v3 x 65,536 after 17 env
-// steps: heavy rays 180 / 125 / 111 / 104 / 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles
-// 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 / 61 / 74), find 202 with 32 items to every warp and 107
-// with 64, deep 214 and 141, combine 113 and 102 (16), islands 234 and 885 (64).
-constexpr int kRayWarps = 16, kFindWarps = 64, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
 
 // xorshift32 draw in [0, 1] and range of the reference's state ring (CudaEnvSet.cpp:608-617)
@@ -484,6 +477,7 @@ static bool allocStep(rsb_handle* h) {
         place(T.results, (size_t)CAP_RESULTS * N);
         place(T.blocks, (size_t)T.blockCap * MAX_POINTS);
         place(T.solveQ, N);
+        place(T.bodyQ, B);
         place(T.first, (size_t)CAP_RESULTS * N);
         place(T.cand, T.candCap);
         place(T.out, T.candCap);
@@ -492,6 +486,7 @@ static bool allocStep(rsb_handle* h) {
         if (pass == 0 && cudaMalloc((void**)&h->dStep, off) != cudaSuccess) return false;
     }
     T.count = h->dWork;
+    T.sms = (uint32_t)h->smCount;
     return true;
 }
 
@@ -675,7 +670,7 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
         !dalloc(h->dRewards, (size_t)h->numCars * 4) || !dalloc(h->dTerminals, N) ||
         !dalloc(h->dResetIdx, N * 4) || !dalloc(h->dCull, N * 4) ||
         !dalloc(h->dCounters, 4 * sizeof(unsigned long long)) || !dalloc(h->dWork, QC_WORDS * sizeof(unsigned int)) ||
-        !allocStep(h) || cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
+        cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess || !allocStep(h))
         return fail(nullptr, RSB_ERR_NOMEM, "device allocation failed");
     cudaMemcpy(h->dTeamSize, h->teamSize.data(), N * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(h->dCarOffset, h->carOffset.data(), (N + 1) * 4, cudaMemcpyHostToDevice);
@@ -737,12 +732,12 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     const StepVariant& sv = kStepVariants[v];
     const StepTemp& T = h->step;
     const int block = kStepBlocks[b], groups = (h->N + PHASE_ARENAS - 1) / PHASE_ARENAS;
-    // A queue kernel's items are counted on the device only.  The wide grid gives each of up to
-    // `items` items a warp of its own, to `warpsPerSm` warps per SM in all; the persistent one is
-    // as large as fits at once (or as the residency asks).
+    // A queue kernel's items are counted on the device only; `items` is about how many there may
+    // be.  The wide grid has a warp for every 32 of them, or for each up to the kernel's spread;
+    // the persistent one is as large as fits at once (or as the residency asks).
     auto grid = [&](StepFn f, int64_t items, int warpsPerSm) -> int {
         const int warps = block / 32;
-        int64_t g = std::min<int64_t>(items, (int64_t)warpsPerSm * h->smCount);
+        int64_t g = std::min<int64_t>(items, std::max<int64_t>((int64_t)warpsPerSm * h->smCount, (items + 31) / 32));
         if (sv.persistent) {
             int perSm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, f, block, 0) != cudaSuccess) perSm = 1;
@@ -755,7 +750,7 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     const int pairGrid = grid(findKernel, 2 * ((int64_t)h->numCars + h->N), kFindWarps);
     const int triGrid = grid(sv.triangle, 4 * ((int64_t)h->numCars + h->N), kTriangleWarps);
     const int deepGrid = grid(deepKernel, h->numCars + h->N, kDeepWarps), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
-    const int solveGrid = grid(sv.solve, h->N, kSolveWarps);
+    const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kSolveWarps);
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
         if (h->maxCars > 0) {

@@ -40,16 +40,24 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
     return base + incl - n;
 }
 
-// Items of several queues, fn(queue, item), spread over the grid's warps: a warp takes as few
-// items at a time as it takes to give every warp some, and never items of two queues at once.
-// The items' paths differ, so few items spread wide finish in the time of the longest one, and
-// 32 to a warp only pays once the queues fill the GPU.
+// Warps per SM that a queue kernel spreads its items over before a warp takes more than one of
+// them, up to 32.  Items' paths differ, so few items spread wide finish in the time of the longest
+// one; but a thread's local memory shares its cache lines with its warp's other lanes, so the
+// kernels that use much of it lose by spreading when the queues are long.  Measured with 4 / 8 /
+// 16 / 32 / 64, us per tick, 3v3 x 65,536 after 17 env steps: heavy rays 180 / 125 / 111 / 104 /
+// 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 /
+// 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113
+// and 102 (16), whole-arena islands 234 and 886 (64).
+constexpr int kRayWarps = 16, kFindWarps = 64, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
+
+// Items of several queues, fn(queue, item): a warp takes `width` items of one queue at a time,
+// as few as it takes to give each of `spread` warps some.
 template <int NQ, class F>
-RSB_D void forItems(const uint32_t* n, F&& fn) {
+RSB_D void forItems(const uint32_t* n, uint32_t spread, F&& fn) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31u;
     uint32_t total = 0, tiles = 0;
     for (int k = 0; k < NQ; k++) total += n[k];
-    const uint32_t width = min(32u, (total + warps - 1u) / warps);
+    const uint32_t width = min(32u, (total + spread - 1u) / spread);
     if (width == 0) return;
     for (int k = 0; k < NQ; k++) tiles += (n[k] + width - 1u) / width;
     for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
@@ -104,7 +112,7 @@ __global__ void __launch_bounds__(128, MINB) heavyRayKernel(const __grid_constan
                                                             const __grid_constant__ StepTemp T) {
     const uint32_t n[2] = {T.count[QC_RAY], T.count[QC_BODYRAY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<2>(n, [&](int q, uint32_t i) { heavyRayPhase(D, T, T.rayQ[q * rayPlaces(D) + i], st); });
+    forItems<2>(n, kRayWarps * T.sms, [&](int q, uint32_t i) { heavyRayPhase(D, T, T.rayQ[q * rayPlaces(D) + i], st); });
     blockStats(D, st);
 }
 
@@ -165,12 +173,19 @@ __global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant
     const uint32_t m0 = queueAlloc(&T.count[t.b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)__popc(o.meshes));
     const uint32_t p0 = queueAlloc(&T.count[QC_PLANE], (uint32_t)__popc(o.planes));
     const uint32_t d0 = queueAlloc(&T.count[t.b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)__popc(dyn));
-    if (valid) pairStore(D, T, t, sh, o, dyn, m0, p0, d0);
+    if (valid) {
+        pairStore(D, T, t, o, dyn, m0, p0, d0);
+        pairNeed(t, o, sh);
+    }
     __syncthreads();
+    const uint32_t need = sh.need[lane];
+    const bool alone = valid && (o.meshes | o.planes) && arenaByBodies(need);
+    const uint32_t at = queueAlloc(&T.count[QC_BODY], alone ? 1u : 0u);
+    if (alone) T.bodyQ[at] = (uint32_t)bodyIdx(D, t.a, t.b);
     if (threadIdx.x < PHASE_ARENAS) {
-        const bool need = sh.need[lane] != 0;
-        const uint32_t at = queueAlloc(&T.count[QC_SOLVE], need ? 1u : 0u);
-        if (need) T.solveQ[at] = (uint32_t)t.a;
+        const bool whole = arenaHasContacts(need) && !arenaByBodies(need);
+        const uint32_t as = queueAlloc(&T.count[QC_SOLVE], whole ? 1u : 0u);
+        if (whole) T.solveQ[as] = (uint32_t)t.a;
     }
     blockStats(D, st);
 }
@@ -178,7 +193,7 @@ __global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant
 __global__ void __launch_bounds__(128) findKernel(const __grid_constant__ EngineView D,
                                                   const __grid_constant__ StepTemp T) {
     const uint32_t n[3] = {T.count[QC_CARMESH], T.count[QC_BALLMESH], T.count[QC_CARBALL]};
-    forItems<3>(n, [&](int k, uint32_t i) {
+    forItems<3>(n, kFindWarps * T.sms, [&](int k, uint32_t i) {
         findPhase(D, T, (uint32_t)resultBase(QC_CARMESH + k) * (uint32_t)D.N + i);
     });
 }
@@ -188,7 +203,7 @@ __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constan
                                                             const __grid_constant__ StepTemp T) {
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[3] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR], T.count[QC_PLANE]};
-    forItems<3>(n, [&](int k, uint32_t i) {
+    forItems<3>(n, kTriangleWarps * T.sms, [&](int k, uint32_t i) {
         if (k == 0) trianglePhase(D, T, i);
         else if (k == 1) carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
         else planePhase(D, T, (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + i, st);
@@ -201,7 +216,7 @@ __global__ void __launch_bounds__(128) deepKernel(const __grid_constant__ Engine
     EpaWork epa;
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[1] = {T.count[QC_DEEP]};
-    forItems<1>(n, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
+    forItems<1>(n, kDeepWarps * T.sms, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
     blockStats(D, st);
 }
 
@@ -209,16 +224,19 @@ __global__ void __launch_bounds__(128) combineKernel(const __grid_constant__ Eng
                                                      const __grid_constant__ StepTemp T) {
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[1] = {T.count[QC_COMBINE]};
-    forItems<1>(n, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
+    forItems<1>(n, kCombineWarps * T.sms, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
     blockStats(D, st);
 }
 
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) solveKernel(const __grid_constant__ EngineView D,
                                                          const __grid_constant__ StepTemp T) {
-    const uint32_t n[1] = {T.count[QC_SOLVE]};
+    const uint32_t n[2] = {T.count[QC_SOLVE], T.count[QC_BODY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<1>(n, [&](int, uint32_t i) { solvePhase(D, T, (int)T.solveQ[i], st); });
+    forItems<2>(n, kSolveWarps * T.sms, [&](int k, uint32_t i) {
+        if (k == 0) solvePhase(D, T, (int)T.solveQ[i], st);
+        else bodyPhase(D, T, T.bodyQ[i], st);
+    });
     blockStats(D, st);
 }
 

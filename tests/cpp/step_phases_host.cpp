@@ -9,9 +9,11 @@
 extern "C" {
 
 // `ticks` ticks of the handle's arenas through the phases.  cull: a body mask per arena, or null;
-// cand_cap: room for triangle candidates (-1: as the engine has).
+// cand_cap: room for triangle candidates (-1: as the engine has); by_bodies 0: every arena with
+// contacts is solved as a whole.
 // Returns the number of items that went through each queue in counts[QC_WORDS].
-int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32_t cand_cap, int64_t* counts,
+int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32_t cand_cap, int32_t by_bodies,
+                             int64_t* counts,
                              uint64_t* stats) {
     const size_t N = h->N, B = MAX_BODIES * N, R = (size_t)4 * MAX_CARS * N;
     EngineView D;
@@ -32,7 +34,8 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     D.work = nullptr;
     std::vector<int32_t> rayObj(R);
     std::vector<float> rayFrac(R), rayN(3 * R), force(6 * B), box(6 * B), cache(3 * B);
-    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(2 * R), solveQ(N);
+    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(2 * R), solveQ(N), bodyQ(B),
+        statics(MAX_BODIES * PHASE_ARENAS);
     std::vector<PairTask> tasks(CAP_RESULTS * N);
     std::vector<PairResult> results(CAP_RESULTS * N);
     std::vector<MPoint> blocks(MAX_BLOCKS * N * MAX_POINTS);
@@ -52,6 +55,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     T.blocks = blocks.data();
     T.blockCap = (uint32_t)(MAX_BLOCKS * N);
     T.solveQ = solveQ.data();
+    T.bodyQ = bodyQ.data();
     T.candCap = cand_cap < 0 ? (uint32_t)(CAP_CANDIDATES * N) : (uint32_t)cand_cap;
     std::vector<uint32_t> first(CAP_RESULTS * N), deepQ(CAP_RESULTS * N + T.candCap), combineQ(CAP_RESULTS * N);
     std::vector<Candidate> cand(T.candCap);
@@ -61,6 +65,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     T.out = candOut.data();
     T.deepQ = deepQ.data();
     T.combineQ = combineQ.data();
+    T.sms = 1;
     std::unique_ptr<EpaWork> epa(new EpaWork());
     std::unique_ptr<DriveShared> ds(new DriveShared());
     std::unique_ptr<PairShared> sh(new PairShared());
@@ -147,10 +152,17 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
                 const uint32_t m0 = phaseAtomicAdd(&T.count[b == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)bitCount(o.meshes));
                 const uint32_t p0 = phaseAtomicAdd(&T.count[QC_PLANE], (uint32_t)bitCount(o.planes));
                 const uint32_t d0 = phaseAtomicAdd(&T.count[b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)bitCount(dyn));
-                pairStore(D, T, t, *sh, o, dyn, m0, p0, d0);
+                pairStore(D, T, t, o, dyn, m0, p0, d0);
+                pairNeed(t, o, *sh);
+                statics[b * PHASE_ARENAS + t.la] = o.meshes | o.planes;
+            });
+            each([&](PairThread& t, int b, int la) {
+                if (statics[b * PHASE_ARENAS + la] && arenaByBodies(sh->need[la]) && by_bodies)
+                    T.bodyQ[T.count[QC_BODY]++] = (uint32_t)bodyIdx(D, t.a, b);
             });
             for (int la = 0; la < PHASE_ARENAS; la++)
-                if (sh->need[la]) T.solveQ[T.count[QC_SOLVE]++] = (uint32_t)(g + la);
+                if (arenaHasContacts(sh->need[la]) && !(arenaByBodies(sh->need[la]) && by_bodies))
+                    T.solveQ[T.count[QC_SOLVE]++] = (uint32_t)(g + la);
         }
         // contacts, islands
         for (int k = 0; k < NUM_TASK_TYPES; k++) {
@@ -166,6 +178,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
         for (uint32_t i = T.count[QC_DEEP]; i-- > 0;) deepPhase(D, T, T.deepQ[i], epa.get(), st);
         for (uint32_t i = T.count[QC_COMBINE]; i-- > 0;) combinePhase(D, T, T.combineQ[i], st);
         for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], st);
+        for (uint32_t i = T.count[QC_BODY]; i-- > 0;) bodyPhase(D, T, T.bodyQ[i], st);
         // finish
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {
             auto each = [&](auto&& fn) {

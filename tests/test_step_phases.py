@@ -19,7 +19,7 @@ from host_util import ARENA_BUILD
 
 SRC = os.path.join(ROOT, "tests", "cpp", "step_phases_host.cpp")
 QUEUES = ("mesh rays", "body rays", "car-mesh", "ball-mesh", "car-ball", "car-car", "planes", "blocks", "islands",
-          "triangles", "deep", "combine")
+          "bodies", "triangles", "deep", "combine")
 
 
 @pytest.fixture(scope="module")
@@ -37,7 +37,7 @@ def host(pkg, tmp_path_factory):
     lib = pkg.rsb.load_library(out)
     lib.rsb_host_records_differ.restype = C.c_int64
     lib.rsb_host_records_differ.argtypes = [C.c_void_p, C.c_void_p]
-    lib.rsb_host_step_phases.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
+    lib.rsb_host_step_phases.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]
     return lib, cases._arena()
 
 
@@ -78,7 +78,7 @@ def start(rsb, b, kind, seed):
     return cars, balls
 
 
-def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=None, cand_cap=-1):
+def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=None, cand_cap=-1, by_bodies=1):
     rsb, (lib, arena) = pkg.rsb, host
     x, y = (rsb.Batch(lib, n, team_sizes=teams, meshes_path=arena, seed=seed) for _ in range(2))
     cars, balls = start(rsb, x, kind, seed)
@@ -97,12 +97,12 @@ def compare(pkg, host, n, teams, kind, seed, ticks, steps, cull=False, mutate=No
             if b.num_cars:
                 b.set_controls(ctl)
         x.step(ticks)
-        st = lib.rsb_host_step_phases(y._h, ticks, mask.ctypes.data if cull else None, cand_cap,
+        st = lib.rsb_host_step_phases(y._h, ticks, mask.ctypes.data if cull else None, cand_cap, by_bodies,
                                       counts.ctypes.data, stats.ctypes.data)
         assert st == 0
         d = lib.rsb_host_records_differ(x._h, y._h)
         assert d == -1, f"step {k}: plane {('ball', 'car', 'pad', 'arena')[d >> 40]}, word {(d & ((1 << 40) - 1)) // n}"
-    return dict(zip(QUEUES, counts.tolist()))
+    return dict(zip(QUEUES, counts.tolist()), rows=int(stats[3]))
 
 
 @pytest.mark.parametrize("kind,ticks", [("field", 8), ("walls", 8), ("heap", 3), ("heap", 8), ("stack", 1), ("stack", 8)])
@@ -112,7 +112,7 @@ def test_phases_match_the_one_thread_tick(pkg, host, kind, ticks):
     for seed in (11, 12):
         got = compare(pkg, host, len(teams), teams, kind, seed, ticks, 160 // ticks)
         seen = {q: seen[q] + got[q] for q in QUEUES}
-    assert seen["mesh rays"] and seen["body rays"] and seen["planes"] and seen["islands"]
+    assert seen["mesh rays"] and seen["body rays"] and seen["planes"] and seen["islands"] and seen["bodies"]
     if kind == "walls":
         assert seen["car-mesh"] and seen["ball-mesh"] and seen["triangles"] and seen["deep"] and seen["combine"]
     if kind in ("heap", "stack"):
@@ -132,6 +132,15 @@ def test_more_triangles_than_there_is_room_for(pkg, host, cand_cap):
     for kind in ("walls", "heap"):
         got = compare(pkg, host, 64, np.full(64, 3, np.int32), kind, 71, 8, 12, cand_cap=cand_cap)
         assert got["triangles"] > cand_cap
+
+
+def test_islands_of_one_body_against_the_whole_solver(pkg, host):
+    """Solver rows counted and records equal whether bodies that touch static objects only are
+    solved by themselves or with their arena."""
+    for kind in ("walls", "field"):
+        got = [compare(pkg, host, 64, np.full(64, 3, np.int32), kind, 81, 8, 12, by_bodies=k) for k in (0, 1)]
+        assert got[0]["bodies"] == 0 and got[1]["bodies"] > 0
+        assert got[0]["rows"] == got[1]["rows"] > 0
 
 
 def test_empty_arenas(pkg, host):
