@@ -363,6 +363,26 @@ bool buildArenaStatic(const std::string& folder, ArenaStaticHost& out) {
     }
     out.triInfo.assign(out.triVerts.size() / 3, TriEdgeInfo{kTwoPi, kTwoPi, kTwoPi, 0});
 
+    // the leaves of each subtree, and what the queries test first of each triangle
+    for (int mi = 0; mi < S.numMeshes; mi++) {
+        const MeshDesc& d = S.meshes[mi];
+        for (int k = 0; k < d.subCount; k++) {
+            const BvhSubtree& st = out.subs[(size_t)d.subOff + k];
+            SubtreeLeaves l{(int32_t)out.leaves.size(), 0};
+            for (int n = st.root; n < st.root + st.size; n++) {
+                const BvhNode& nd = out.nodes[(size_t)d.nodeOff + n];
+                if (nd.data < 0) continue;
+                out.leaves.push_back(nd);
+                l.count++;
+            }
+            out.subLeaves.push_back(l);
+        }
+    }
+    for (size_t t = 0; t < out.triVerts.size() / 3; t++) out.triData.push_back(triDataOf(&out.triVerts[3 * t]));
+    S.triData = out.triData.data();
+    S.subLeaves = out.subLeaves.data();
+    S.leaves = out.leaves.data();
+
     // temporary host view for the BVH queries below
     S.nodes = out.nodes.data();
     S.subs = out.subs.data();

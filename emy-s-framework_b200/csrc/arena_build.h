@@ -11,6 +11,9 @@ struct ArenaStaticHost {
     std::vector<BvhNode> nodes;
     std::vector<BvhSubtree> subs;
     std::vector<V3> triVerts;
+    std::vector<TriData> triData;
+    std::vector<SubtreeLeaves> subLeaves;
+    std::vector<BvhNode> leaves;
     std::vector<TriEdgeInfo> triInfo;
     std::vector<uint32_t> bpCells;
     std::vector<uint16_t> occ;

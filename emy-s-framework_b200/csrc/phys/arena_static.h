@@ -61,10 +61,43 @@ struct BpGrid {
     int cellsX, cellsY, cellsZ;
 };
 
+// What the queries test first of a triangle, worked out once: its normal v10 x v20 with the
+// plane's offset (rayTriangle), the unit normal with its offset (the two-sided early outs of
+// the convex-concave algorithm), and its AABB.  Each value is the one the query would compute.
+struct alignas(16) TriData {
+    V3 n;
+    float dist;
+    V3 unit;
+    float unitDist;
+    V3 lo;
+    float pad0;
+    V3 hi;
+    float pad1;
+};
+RSB_HD TriData triDataOf(const V3* v) {
+    TriData t;
+    t.n = cross(v[1] - v[0], v[2] - v[0]);
+    t.dist = dot(v[0], t.n);
+    t.unit = normalized(t.n);
+    t.unitDist = dot(t.unit, v[0]);
+    t.lo = V3{fmin_(fmin_(v[0].x, v[1].x), v[2].x), fmin_(fmin_(v[0].y, v[1].y), v[2].y), fmin_(fmin_(v[0].z, v[1].z), v[2].z)};
+    t.hi = V3{fmax_(fmax_(v[0].x, v[1].x), v[2].x), fmax_(fmax_(v[0].y, v[1].y), v[2].y), fmax_(fmax_(v[0].z, v[1].z), v[2].z)};
+    t.pad0 = t.pad1 = 0.f;
+    return t;
+}
+
+// The leaves of one BVH subtree, in node order.
+struct SubtreeLeaves {
+    int32_t off, count;
+};
+
 struct ArenaStatic {
     const BvhNode* nodes;
     const BvhSubtree* subs;
     const V3* triVerts;        // 3 per triangle, Bullet units
+    const TriData* triData;    // per triangle
+    const SubtreeLeaves* subLeaves;  // per subtree, into leaves
+    const BvhNode* leaves;     // leaf nodes, subtree after subtree
     const TriEdgeInfo* triInfo;
     const uint32_t* bpCells;   // bit s set: static object s registered in the cell
     // Mesh occupancy grid (Bullet units): bit m of voxel v set when some triangle of mesh
@@ -219,6 +252,31 @@ RSB_HD void bvhQueryRay(const ArenaStatic& S, int mesh, V3 src, V3 dst, F&& fn) 
         if (rayOv || leaf) cur++;
         else cur += -n.data;
     }
+}
+
+// The same leaves as bvhQueryAabb, in the same order, without the walk: a leaf whose box overlaps
+// the query has ancestors that do, so each subtree's leaves are tested by themselves.
+template <class F>
+RSB_HD void bvhQueryLeaves(const ArenaStatic& S, int mesh, V3 aabbMin, V3 aabbMax, F&& fn) {
+    const MeshDesc& m = S.meshes[mesh];
+    uint16_t qmn[3], qmx[3];
+    bvhQuantizeClamp(m, aabbMin, 0, qmn);
+    bvhQuantizeClamp(m, aabbMax, 1, qmx);
+    for (int s = 0; s < m.subCount; s++) {
+        const BvhSubtree& st = S.subs[m.subOff + s];
+        if (!qOverlap(qmn, qmx, st.qmin, st.qmax)) continue;
+        const SubtreeLeaves l = S.subLeaves[m.subOff + s];
+        for (int k = 0; k < l.count; k++) {
+            const BvhNode& n = S.leaves[l.off + k];
+            if (qOverlap(qmn, qmx, n.qmin, n.qmax) && !fn(n.data)) return;
+        }
+    }
+}
+
+RSB_HD const TriData& triData(const ArenaStatic& S, int mesh, int tri) { return S.triData[S.meshes[mesh].triOff + tri]; }
+// triAabbOverlap on the stored box.
+RSB_HD bool triBoxOverlap(const TriData& t, V3 mn, V3 mx) {
+    return !(t.lo.x > mx.x || t.hi.x < mn.x || t.lo.z > mx.z || t.hi.z < mn.z || t.lo.y > mx.y || t.hi.y < mn.y);
 }
 
 RSB_HD void triVerts(const ArenaStatic& S, int mesh, int tri, V3* v) {

@@ -198,14 +198,16 @@ RSB_HD bool rayVsMeshesNearest(const ArenaStatic& S, uint32_t meshes, V3 src, V3
                 const uint32_t key = S.voxList[i];
                 const int m = (int)(key >> 22);
                 if (!((meshes >> m) & 1u)) continue;
-                V3 t[3];
-                triVerts(S, m, (int)(key & 0x3FFu), t);
-                const V3 n = cross(t[1] - t[0], t[2] - t[0]);
-                const float dist = dot(t[0], n);
+                const int tri = (int)(key & 0x3FFu);
+                const TriData& td = triData(S, m, tri);
+                const V3 n = td.n;
+                const float dist = td.dist;
                 const float da = dot(n, src) - dist, db = dot(n, dst) - dist;
                 if (da * db >= 0.f) continue;
                 const float distance = da / (da - db);
                 if (!(distance < best || (distance == best && key < bestKey))) continue;
+                V3 t[3];
+                triVerts(S, m, tri, t);
                 const float edgeTol = length2(n) * -0.0001f;
                 const V3 point = src * (1.f - distance) + dst * distance;
                 const V3 v0p = t[0] - point, v1p = t[1] - point, v2p = t[2] - point;

@@ -12,7 +12,8 @@
 //   drive ...... respawns and the vehicle update of every car
 //   pairs ...... predicted motion of every body, broadphase pairs; queues the pairs that can be in
 //                contact and the arenas that have any
-//   find ....... queued mesh pairs: the triangles whose boxes overlap (candidates, in walk order)
+//   find ....... queued mesh pairs: the triangles whose boxes and planes the body's box meets
+//                (candidates, in walk order)
 //   triangles .. one candidate per thread: box-triangle and box-sphere GJK; box-box and plane pairs
 //   deep ....... the candidates whose GJK needs the penetration solver
 //   combine .... one pair per thread: its candidates' contacts into the manifold, in walk order
@@ -89,23 +90,22 @@ enum : uint32_t {
     PR_WORLD = 2u   // ... and the car-world callback saw it
 };
 
-// One triangle (tri < 0: the ball) that a queued pair's boxes overlap; a pair's candidates form
-// a list in the order in which the reference visits them.
+// One triangle (tri < 0: the ball) that a queued pair may touch; a pair's candidates lie one
+// after another in the order in which the reference visits them.
 struct Candidate {
     uint32_t res;   // the pair's place in the task and result arrays
     int32_t tri;
-    uint32_t next;  // NO_CANDIDATE at the end
 };
-constexpr uint32_t NO_CANDIDATE = ~0u;
 // What GJK found for a candidate; between the triangles and the deep phase, its state.
 struct CandidateOut {
     uint32_t flags;  // CO_*
     float normal[3], point[3], dist;
 };
 enum : uint32_t { CO_HAS = 1u, CO_VALID = 2u };
-// Candidates per arena that the batch has room for.  Pairs that find none left are taken
-// triangle by triangle on one thread (the deep queue holds them as DEEP_PAIR | result).
-constexpr int CAP_CANDIDATES = 64;
+// Candidates per arena that the batch has room for, and per pair.  Pairs with more of them, and
+// pairs that find no room left, are taken triangle by triangle on one thread (the deep queue
+// holds them as DEEP_PAIR | result).
+constexpr int CAP_CANDIDATES = 64, PAIR_CANDIDATES = 32;
 constexpr uint32_t DEEP_PAIR = 1u << 31;
 
 struct StepTemp {
@@ -126,7 +126,7 @@ struct StepTemp {
     uint32_t blockCap;
     uint32_t* solveQ;    // arenas with pairs of bodies [N]
     uint32_t* bodyQ;     // bodies with contacts in the others, b * N + a [MAX_BODIES * N]
-    uint32_t* first;     // first candidate of each pair, as results
+    uint32_t* first;     // first candidate of each pair and their number << 26, as results
     Candidate* cand;     // [candCap]
     CandidateOut* out;   // [candCap]
     uint32_t candCap;
@@ -1103,49 +1103,71 @@ RSB_HD void ballMeshPhase(const EngineView& D, const StepTemp& T, uint32_t res, 
     storePair(D, T, a, W, m, res);
 }
 
-// Finds a pair's candidates: the triangles whose leaves and boxes overlap the body's box, or for
-// a car and the ball the ball itself.  A mesh pair without any is finished here.
+// What a mesh pair's body tests triangles with.
+struct FindBody {
+    Xf xf;      // the ball's transform, the hitbox's otherwise
+    M3 invB;
+    V3 amn, amx;
+    bool ball;
+};
+RSB_HD void findBody(const EngineView& D, int a, int b, FindBody& f) {
+    f.ball = b == 0;
+    f.xf = bodyXf(D, a, b);
+    if (f.ball) {
+        ballAabb(D.P, f.xf, f.amn, f.amx);
+    } else {
+        f.xf = carChildXf(D.P.car, f.xf);
+        carBoxAabb(D.P.car, f.xf, f.amn, f.amx);
+    }
+    f.invB = inverse(f.xf.b);
+}
+RSB_HD bool findTest(const EngineView& D, const FindBody& f, const TriData& t) {
+    if (!triBoxOverlap(t, f.amn, f.amx)) return false;
+    return f.ball ? ballTriPlanes(D.P, f.xf, f.invB, D.P.ballCbt, t.unit, t.unitDist)
+                  : boxTriPlanes(carBoxShape(D.P.car), f.xf, f.invB, D.P.car.cbt, t.unit, t.unitDist);
+}
+// A pair whose n candidates begin at `first`: nothing to combine, too many, or to combine (the
+// return value; the caller queues the pair).
+constexpr int CANDIDATE_SHIFT = 26;
+RSB_HD bool findStore(const StepTemp& T, uint32_t res, uint32_t first, uint32_t n) {
+    if (n == 0) {
+        T.results[res] = PairResult{0, 0u, 0u, {0.f, 0.f, 0.f}};
+        return false;
+    }
+    if (n > (uint32_t)PAIR_CANDIDATES || first + n > T.candCap || first >= (1u << CANDIDATE_SHIFT)) {
+        T.deepQ[phaseAtomicAdd(&T.count[QC_DEEP], 1u)] = DEEP_PAIR | res;
+        return false;
+    }
+    T.first[res] = first | (n << CANDIDATE_SHIFT);
+    return true;
+}
+RSB_HD void putCandidate(const StepTemp& T, uint32_t at, uint32_t res, int tri) {
+    if (at < T.candCap) T.cand[at] = Candidate{res, tri};
+}
+
+// A pair on one thread.
 RSB_HD void findPhase(const EngineView& D, const StepTemp& T, uint32_t res) {
     const PairTask k = T.tasks[res];
-    const int a = (int)k.a, b = k.o1 - OBJ_BALL;
-    uint32_t first = NO_CANDIDATE, last = NO_CANDIDATE;
-    bool full = false;
-    auto add = [&](int tri) {
-        const uint32_t c = phaseAtomicAdd(&T.count[QC_TRI], 1u);
-        if (c >= T.candCap) {
-            full = true;
-            return false;
-        }
-        T.cand[c] = Candidate{res, tri, NO_CANDIDATE};
-        if (last == NO_CANDIDATE) first = c;
-        else T.cand[last].next = c;
-        last = c;
-        return true;
-    };
+    uint32_t n = 0, first = 0;
     if (k.o0 == OBJ_BALL) {
-        add(-1);
+        first = phaseAtomicAdd(&T.count[QC_TRI], 1u);
+        n = 1;
+        putCandidate(T, first, res, -1);
     } else {
-        V3 amn, amx;
-        const Xf xf = bodyXf(D, a, b);
-        if (b == 0) ballAabb(D.P, xf, amn, amx);
-        else carBoxAabb(D.P.car, carChildXf(D.P.car, xf), amn, amx);
-        bvhQueryAabb(D.S, k.o0, amn, amx, [&](int tri) {
-            V3 v[3];
-            triVerts(D.S, k.o0, tri, v);
-            return triAabbOverlap(v, amn, amx) ? add(tri) : true;
+        int16_t tri[PAIR_CANDIDATES];
+        FindBody f;
+        findBody(D, (int)k.a, k.o1 - OBJ_BALL, f);
+        bvhQueryLeaves(D.S, k.o0, f.amn, f.amx, [&](int t) {
+            if (!findTest(D, f, triData(D.S, k.o0, t))) return true;
+            if (n < (uint32_t)PAIR_CANDIDATES) tri[n] = (int16_t)t;
+            return ++n <= (uint32_t)PAIR_CANDIDATES;
         });
+        if (n > 0 && n <= (uint32_t)PAIR_CANDIDATES) {
+            first = phaseAtomicAdd(&T.count[QC_TRI], n);
+            for (uint32_t i = 0; i < n; i++) putCandidate(T, first + i, res, tri[i]);
+        }
     }
-    if (full) {
-        T.deepQ[phaseAtomicAdd(&T.count[QC_DEEP], 1u)] = DEEP_PAIR | res;
-        // its candidates still in the queue are worked on for nothing
-        return;
-    }
-    if (first == NO_CANDIDATE) {
-        T.results[res] = PairResult{0, 0u, 0u, {0.f, 0.f, 0.f}};
-        return;
-    }
-    T.first[res] = first;
-    T.combineQ[phaseAtomicAdd(&T.count[QC_COMBINE], 1u)] = res;
+    if (findStore(T, res, first, n)) T.combineQ[phaseAtomicAdd(&T.count[QC_COMBINE], 1u)] = res;
 }
 
 // The two shapes of a box candidate.
@@ -1188,7 +1210,7 @@ RSB_HD void trianglePhase(const EngineView& D, const StepTemp& T, uint32_t i) {
     int a;
     if (!candidateShapes(D, T, c, s, a)) return;
     T.out[i].flags = 0;
-    if (c.tri >= 0 && !boxTriNear(D.P.car, s.box, s.boxXf, D.P.car.cbt, s.other.v)) return;
+    if (c.tri >= 0 && boxTriApart(D.P.car, s.box, s.boxXf, D.P.car.cbt, s.other.v)) return;
     GjkState g;
     gjkIterate(s.box, s.boxXf, s.other, s.otherXf, s.maxDist2, g);
     if (g.needEpa) {
@@ -1247,7 +1269,7 @@ RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, P
     const PairTask k = T.tasks[res];
     const int a = (int)k.a, b = k.o1 - OBJ_BALL;
     if (k.o0 == OBJ_BALL) {
-        const CandidateOut& o = T.out[T.first[res]];
+        const CandidateOut& o = T.out[T.first[res] & ((1u << CANDIDATE_SHIFT) - 1u)];
         PairWorldT<PairBodies> W;
         LocalPool pool;
         pairWorldInit(D, W, pool, nullptr, 0u);
@@ -1269,14 +1291,15 @@ RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, P
     Manifold m;
     pairManifold(m, k.o1, k.o0, b == 0 ? D.P.ballCbt : D.P.car.cbt);
     bool found = false;
-    for (uint32_t c = T.first[res]; c != NO_CANDIDATE;) {
+    const uint32_t f = T.first[res], c0 = f & ((1u << CANDIDATE_SHIFT) - 1u);
+    for (uint32_t c = c0; c < c0 + (f >> CANDIDATE_SHIFT); c++) {
         const Candidate cd = T.cand[c];
         V3 v[3], n, p;
         float d;
         bool has;
         if (b == 0) {
             triVerts(D.S, k.o0, cd.tri, v);
-            has = ballTriContact(D.P, W.b.v.xf, m.cbt, v, p, n, d);
+            has = sphereTriCollide(v, W.b.v.xf.o, D.P.ballRadius, m.cbt, p, n, d);
         } else {
             const CandidateOut& o = T.out[c];
             has = (o.flags & CO_HAS) != 0;
@@ -1292,7 +1315,6 @@ RSB_HD void combinePhase(const EngineView& D, const StepTemp& T, uint32_t res, P
             if (b == 0) addBallTriContact(W, k.o0, cd.tri, v, n, p, d, m);
             else addBoxTriContact(W, k.o0, b - 1, cd.tri, v, n, p, d, m);
         }
-        c = cd.next;
     }
     cullCheck(W, b, found);
     if (m.n) refreshContactPoints(m, W.b.v.xf, xfIdentity());

@@ -426,21 +426,19 @@ RSB_HD bool sphereTriCollide(const V3* v, V3 center, float radius, float cbt, V3
     return false;
 }
 
-// One triangle that overlaps the ball's AABB: the early out on the two sides of its plane
-// (btConvexConcaveCollisionAlgorithm.cpp:100-137), then btSphereTriangleCollisionAlgorithm.
-RSB_HD bool ballTriContact(const WorldParams& P, const Xf& ballXf, float cbt, const V3* v, V3& point, V3& normal,
-                           float& depth) {
-    const M3 invB = inverse(ballXf.b);
-    V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
+// The early out on the two sides of a triangle's plane for the ball
+// (btConvexConcaveCollisionAlgorithm.cpp:100-137).
+RSB_HD bool ballTriPlanes(const WorldParams& P, const Xf& ballXf, const M3& invB, float cbt, V3 unit, float unitDist) {
     float thr = cbt + 0.f;
     for (int side = 0; side < 2; side++) {
-        V3 lp = sphereSupport(invB * tn, P.ballMargin);
+        V3 lp = sphereSupport(invB * unit, P.ballMargin);
         V3 wp = xfPoint(ballXf, lp);
-        float dist = dot(tn, v[0]) - dot(tn, wp);
+        float dist = unitDist - dot(unit, wp);
         if (dist > thr) return false;
-        tn *= -1.f;
+        unit *= -1.f;
+        unitDist *= -1.f;
     }
-    return sphereTriCollide(v, ballXf.o, P.ballRadius, cbt, point, normal, depth);
+    return true;
 }
 
 // Adds one triangle's contact with the ball to its manifold.
@@ -466,6 +464,7 @@ RSB_HD void collideBallMesh(WT& W, int mesh, Manifold& man) {
     if (!cullSkip(W, 0)) {
     V3 amn, amx;
     ballAabb(P, ball.xf, amn, amx);  // convexInTriangleSpace == ball transform (mesh at identity)
+    const M3 invB = inverse(ball.xf.b);
     // no triangle of this mesh near the query box: the walk below could not report one
     if ((occMask(*W.S, amn - V3{kOccTol, kOccTol, kOccTol}, amx + V3{kOccTol, kOccTol, kOccTol}) >> mesh) & 1u)
     bvhQueryAabb(*W.S, mesh, amn, amx, [&](int tri) {
@@ -474,7 +473,9 @@ RSB_HD void collideBallMesh(WT& W, int mesh, Manifold& man) {
         if (!triAabbOverlap(v, amn, amx)) return true;
         V3 point, normal;
         float depth;
-        if (ballTriContact(P, ball.xf, man.cbt, v, point, normal, depth)) {
+        const TriData& td = triData(*W.S, mesh, tri);
+        if (ballTriPlanes(P, ball.xf, invB, man.cbt, td.unit, td.unitDist) &&
+            sphereTriCollide(v, ball.xf.o, P.ballRadius, man.cbt, point, normal, depth)) {
             found = true;
             addBallTriContact(W, mesh, tri, v, normal, point, depth, man);
         }
@@ -662,20 +663,22 @@ RSB_HD bool boxTriFar(const Xf& x, V3 he, const V3* v, float limit) {
     return false;
 }
 
-// Whether a triangle that overlaps the box's AABB goes to GJK: the early out on the two sides of
-// its plane (btConvexConcaveCollisionAlgorithm.cpp:100-137), and a reject of triangles
-// separated well beyond the contact distance, for which GJK would find no contact.
-RSB_HD bool boxTriNear(const CarParams& C, const ConvexShape& box, const Xf& childXf, float cbt, const V3* v) {
-    const M3 invB = inverse(childXf.b);
-    V3 tn = normalized(cross(v[1] - v[0], v[2] - v[0]));
+// The early out on the two sides of a triangle's plane (btConvexConcaveCollisionAlgorithm.cpp:
+// 100-137) for the car box: unit normal and its offset, invB the inverse of the box's basis.
+RSB_HD bool boxTriPlanes(const ConvexShape& box, const Xf& childXf, const M3& invB, float cbt, V3 unit, float unitDist) {
     for (int side = 0; side < 2; side++) {
-        V3 lp = supportVirtual(box, invB * tn);
+        V3 lp = supportVirtual(box, invB * unit);
         V3 wp = xfPoint(childXf, lp);
-        float dist = dot(tn, v[0]) - dot(tn, wp);
+        float dist = unitDist - dot(unit, wp);
         if (dist > cbt + 0.f) return false;
-        tn *= -1.f;
+        unit *= -1.f;
+        unitDist *= -1.f;
     }
-    return !boxTriFar(childXf, box.he, v, (C.boxMargin + 0.f) + cbt + 0.02f);
+    return true;
+}
+// A triangle separated well beyond the contact distance: GJK would find no contact.
+RSB_HD bool boxTriApart(const CarParams& C, const ConvexShape& box, const Xf& childXf, float cbt, const V3* v) {
+    return boxTriFar(childXf, box.he, v, (C.boxMargin + 0.f) + cbt + 0.02f);
 }
 
 // Adds one triangle's contact with car ci's box to its manifold, with the car-world callback and
@@ -706,6 +709,7 @@ RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold&
     V3 amn, amx;
     carBoxAabb(C, childXf, amn, amx);
     float maxDist2 = boxMeshMaxDist2(C, man.cbt);
+    const M3 invB = inverse(childXf.b);
     bool found = false;
     if (!cullSkip(W, 1 + ci) &&
         ((occMask(*W.S, amn - V3{kOccTol, kOccTol, kOccTol}, amx + V3{kOccTol, kOccTol, kOccTol}) >> mesh) & 1u)) {
@@ -713,7 +717,9 @@ RSB_HD void collideBoxMesh(WT& W, int mesh, int ci, const Xf& childXf, Manifold&
         V3 v[3];
         triVerts(*W.S, mesh, tri, v);
         if (!triAabbOverlap(v, amn, amx)) return true;
-        if (!boxTriNear(C, box, childXf, man.cbt, v)) return true;
+        const TriData& td = triData(*W.S, mesh, tri);
+        if (!boxTriPlanes(box, childXf, invB, man.cbt, td.unit, td.unitDist)) return true;
+        if (boxTriApart(C, box, childXf, man.cbt, v)) return true;
         ConvexShape triS = makeTri(v, 0.f);
         GjkOut g = gjkPairDetector(W.epa, box, childXf, triS, xfIdentity(), maxDist2);
         if (g.overflow) W.status |= WS_EPA_OVERFLOW;

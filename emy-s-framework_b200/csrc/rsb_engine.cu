@@ -43,6 +43,9 @@ struct DevStatic {
     BvhNode* nodes = nullptr;
     BvhSubtree* subs = nullptr;
     V3* triVerts = nullptr;
+    TriData* triData = nullptr;
+    SubtreeLeaves* subLeaves = nullptr;
+    BvhNode* leaves = nullptr;
     TriEdgeInfo* triInfo = nullptr;
     uint32_t* bpCells = nullptr;
     uint16_t* occ = nullptr;
@@ -208,6 +211,14 @@ constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
 // Resident warps per SM of a persistent launch (0 = as many as fit).
 static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
+
+// Fills the triangles' query data (TriData) on the device.
+__global__ void triDataKernel(const V3* verts, int n, TriData* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const V3 v[3] = {verts[3 * t], verts[3 * t + 1], verts[3 * t + 2]};
+    out[t] = triDataOf(v);
+}
 
 // xorshift32 draw in [0, 1] and range of the reference's state ring (CudaEnvSet.cpp:608-617)
 RSB_HD float ringRand01(uint32_t& rng) {
@@ -613,7 +624,8 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
                 if (cudaMalloc((void**)&dst, bytes ? bytes : 4) != cudaSuccess) return false;
                 return cudaMemcpy(dst, v.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
             };
-            if (!up(D->nodes, H->nodes) || !up(D->subs, H->subs) || !up(D->triVerts, H->triVerts) ||
+            if (!up(D->nodes, H->nodes) || !up(D->subs, H->subs) || !up(D->subLeaves, H->subLeaves) || !up(D->leaves, H->leaves) ||
+                !up(D->triData, H->triData) || !up(D->triVerts, H->triVerts) ||
                 !up(D->triInfo, H->triInfo) || !up(D->bpCells, H->bpCells) || !up(D->occ, H->occ) ||
                 !up(D->voxOff, H->voxOff) || !up(D->voxList, H->voxList) || !up(D->occDist, H->occDist))
                 return fail(nullptr, RSB_ERR_CUDA, "uploading arena meshes failed");
@@ -627,6 +639,14 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
             if (cudaMemcpyToSymbol(g_rsqrtTable, c.rsqrtTable, sizeof(c.rsqrtTable)) != cudaSuccess)
                 return fail(nullptr, RSB_ERR_CUDA, "uploading the rsqrt estimate table failed");
             c.rsqrtDevices.insert(h->device);
+            D->view.triData = D->triData;
+            D->view.subLeaves = D->subLeaves;
+            D->view.leaves = D->leaves;
+            // the triangles' unit normals as the kernels would compute them, with that table
+            const int nTri = (int)H->triData.size();
+            triDataKernel<<<(nTri + 127) / 128, 128>>>(D->triVerts, nTri, D->triData);
+            if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+                return fail(nullptr, RSB_ERR_CUDA, "preparing the arena triangles failed");
             c.dev[key] = D;
             h->stat = D;
         }
@@ -747,7 +767,8 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
         return (int)std::max<int64_t>(1, (g + warps - 1) / warps);
     };
     const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars, kRayWarps);
-    const int pairGrid = grid(findKernel, 2 * ((int64_t)h->numCars + h->N), kFindWarps);
+    // four pairs to a warp
+    const int pairGrid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)h->numCars + h->N) / 16, 16 * (int64_t)h->smCount));
     const int triGrid = grid(sv.triangle, 4 * ((int64_t)h->numCars + h->N), kTriangleWarps);
     const int deepGrid = grid(deepKernel, h->numCars + h->N, kDeepWarps), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
     const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kSolveWarps);
@@ -759,7 +780,7 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
             driveKernel<<<groups, carThreads, 0, st>>>(D, T);
         }
         pairKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
-        findKernel<<<pairGrid, block, 0, st>>>(D, T);
+        findKernel<<<pairGrid, FIND_THREADS, 0, st>>>(D, T);
         sv.triangle<<<triGrid, block, 0, st>>>(D, T);
         deepKernel<<<deepGrid, block, 0, st>>>(D, T);
         combineKernel<<<combineGrid, block, 0, st>>>(D, T);

@@ -46,9 +46,9 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
 // kernels that use much of it lose by spreading when the queues are long.  Measured with 4 / 8 /
 // 16 / 32 / 64, us per tick, 3v3 x 65,536 after 17 env steps: heavy rays 180 / 125 / 111 / 104 /
 // 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 /
-// 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113
-// and 102 (16), whole-arena islands 234 and 886 (64).
-constexpr int kRayWarps = 16, kFindWarps = 64, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
+// 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113 and 102, whole-arena
+// islands 234 and 886 (64).
+constexpr int kRayWarps = 16, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
 
 // Items of several queues, fn(queue, item): a warp takes `width` items of one queue at a time,
 // as few as it takes to give each of `spread` warps some.
@@ -190,12 +190,91 @@ __global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant
     blockStats(D, st);
 }
 
-__global__ void __launch_bounds__(128) findKernel(const __grid_constant__ EngineView D,
-                                                  const __grid_constant__ StepTemp T) {
-    const uint32_t n[3] = {T.count[QC_CARMESH], T.count[QC_BALLMESH], T.count[QC_CARBALL]};
-    forItems<3>(n, kFindWarps * T.sms, [&](int k, uint32_t i) {
-        findPhase(D, T, (uint32_t)resultBase(QC_CARMESH + k) * (uint32_t)D.N + i);
-    });
+// The candidates of mesh pairs, eight lanes to a pair: the subtrees' headers and then the leaves of
+// those that overlap, eight at a time, so that the loads of a pair do not wait for one another as
+// those of a walk do.  The four pairs of a warp step together (their lanes meet in the ballots).
+constexpr int FIND_LANES = 8, FIND_GROUPS = 32 / FIND_LANES, FIND_HEADERS = 64;
+constexpr int FIND_THREADS = 128;
+__global__ void __launch_bounds__(FIND_THREADS) findKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T) {
+    __shared__ int16_t list[FIND_THREADS / FIND_LANES][PAIR_CANDIDATES];
+    const uint32_t nCar = T.count[QC_CARMESH], total = nCar + T.count[QC_BALLMESH], nBall = T.count[QC_CARBALL];
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), warps = gridDim.x * (blockDim.x >> 5);
+    const int lane = threadIdx.x & 31, g = lane / FIND_LANES, l = lane % FIND_LANES;
+    const uint32_t groupBits = (1u << FIND_LANES) - 1u, all = 0xffffffffu;
+    int16_t* mine = list[threadIdx.x / FIND_LANES];
+    const ArenaStatic& S = D.S;
+    for (uint32_t p0 = warp * FIND_GROUPS; p0 < total; p0 += warps * FIND_GROUPS) {
+        const uint32_t p = p0 + g;
+        bool has = p < total;
+        uint32_t res = 0, n = 0;
+        int mesh = 0, subCount = 0, subOff = 0;
+        FindBody f;
+        uint16_t qmn[3], qmx[3];
+        if (has) {
+            res = p < nCar ? (uint32_t)resultBase(QC_CARMESH) * (uint32_t)D.N + p
+                           : (uint32_t)resultBase(QC_BALLMESH) * (uint32_t)D.N + (p - nCar);
+            const PairTask k = T.tasks[res];
+            mesh = k.o0;
+            findBody(D, (int)k.a, k.o1 - OBJ_BALL, f);
+            const MeshDesc& m = S.meshes[mesh];
+            bvhQuantizeClamp(m, f.amn, 0, qmn);
+            bvhQuantizeClamp(m, f.amx, 1, qmx);
+            subCount = m.subCount;
+            subOff = m.subOff;
+        }
+        if (has && subCount > FIND_HEADERS) {
+            // more subtrees than a group's mask holds
+            if (l == 0) findPhase(D, T, res);
+            has = false;
+            subCount = 0;
+        }
+        unsigned long long mask = 0;
+        const int rounds = (__reduce_max_sync(all, subCount) + FIND_LANES - 1) / FIND_LANES;
+        for (int r = 0; r < rounds; r++) {
+            const int h = r * FIND_LANES + l;
+            bool ov = false;
+            if (h < subCount) {
+                const BvhSubtree& st = S.subs[subOff + h];
+                ov = qOverlap(qmn, qmx, st.qmin, st.qmax);
+            }
+            const uint32_t bal = __ballot_sync(all, ov);
+            mask |= (unsigned long long)((bal >> (g * FIND_LANES)) & groupBits) << (r * FIND_LANES);
+        }
+        int pos = 0, end = 0;
+        while (__any_sync(all, mask != 0 || pos < end)) {
+            if (pos >= end && mask) {
+                const SubtreeLeaves sl = S.subLeaves[subOff + __ffsll((long long)mask) - 1];
+                mask &= mask - 1ull;
+                pos = sl.off;
+                end = sl.off + sl.count;
+            }
+            bool ok = pos + l < end;
+            int tri = 0;
+            if (ok) {
+                const BvhNode nd = S.leaves[pos + l];
+                tri = nd.data;
+                ok = qOverlap(qmn, qmx, nd.qmin, nd.qmax) && findTest(D, f, triData(S, mesh, tri));
+            }
+            const uint32_t bits = (__ballot_sync(all, ok) >> (g * FIND_LANES)) & groupBits;
+            const uint32_t at = n + (uint32_t)__popc(bits & ((1u << l) - 1u));
+            if (ok && at < (uint32_t)PAIR_CANDIDATES) mine[at] = (int16_t)tri;
+            n += (uint32_t)__popc(bits);
+            pos += FIND_LANES;
+        }
+        __syncwarp();
+        // places for the warp's candidates, then its pairs' places in the queues
+        const uint32_t cnt = has && l == 0 && n <= (uint32_t)PAIR_CANDIDATES ? n : 0u;
+        const uint32_t first = __shfl_sync(all, queueAlloc(&T.count[QC_TRI], cnt), g * FIND_LANES);
+        if (has && n <= (uint32_t)PAIR_CANDIDATES)
+            for (uint32_t i = l; i < n; i += FIND_LANES) putCandidate(T, first + i, res, mine[i]);
+        const bool combine = has && l == 0 && findStore(T, res, first, n);
+        const uint32_t at = queueAlloc(&T.count[QC_COMBINE], combine ? 1u : 0u);
+        if (combine) T.combineQ[at] = res;
+        __syncwarp();
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nBall; i += gridDim.x * blockDim.x)
+        findPhase(D, T, (uint32_t)resultBase(QC_CARBALL) * (uint32_t)D.N + i);
 }
 
 template <int MINB>
