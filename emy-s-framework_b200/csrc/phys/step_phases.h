@@ -8,7 +8,8 @@
 // of it instead of the few that 32 arenas happen to have at the same time.
 //
 //   rays ....... every wheel ray of every car: the planes here, the rest into the ray queue
-//   heavy rays . the queued rays: meshes, planes, other bodies (castRay)
+//   mesh rays .. the queued rays near meshes: meshes, planes
+//   body rays .. the queued rays near other bodies: what the mesh rays left, then the bodies
 //   drive ...... respawns and the vehicle update of every car
 //   pairs ...... predicted motion of every body, broadphase pairs; queues the pairs that can be in
 //                contact and the arenas that have any
@@ -49,6 +50,8 @@ constexpr uint32_t BI_ACT_MASK = 7u << BI_ACT_SHIFT;
 constexpr uint32_t BI_SOLVED = 1u << 24;    // velocities and transform were written by the islands phase
 constexpr uint32_t BI_CACHE = 1u << 25;     // the body's velocity cache holds an impulse
 constexpr uint32_t BI_RESPONDS = 1u << 26;  // contact response on (cars)
+constexpr uint32_t BI_ALONE = 1u << 27;     // every island of the arena is one body
+constexpr uint32_t BI_CONTACT = 1u << 28;   // a contact of the body was found (and its place in bodyQ taken)
 
 // Dynamic pairs (lo < hi) of seven bodies.
 constexpr int NUM_DYN_PAIRS = MAX_BODIES * (MAX_BODIES - 1) / 2;
@@ -149,11 +152,13 @@ RSB_HD uint32_t phaseAtomicAdd(uint32_t* p, uint32_t v) {
     return o;
 #endif
 }
-RSB_HD void phaseAtomicOr(uint32_t* p, uint32_t v) {
+RSB_HD uint32_t phaseAtomicOr(uint32_t* p, uint32_t v) {
 #if defined(__CUDA_ARCH__)
-    atomicOr(p, v);
+    return atomicOr(p, v);
 #else
+    const uint32_t o = *p;
     *p |= v;
+    return o;
 #endif
 }
 RSB_HD void phaseAtomicAnd(uint32_t* p, uint32_t v) {
@@ -470,33 +475,8 @@ struct RegWalk {
     }
 };
 
-// A queued ray: meshes, then planes, then bodies in registration order, as castRay tests them.
-RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
-    const int a = (int)(r % (uint32_t)D.N), q = (int)(r / (uint32_t)D.N), s = q % MAX_CARS, w = q / MAX_CARS;
-    const ArenaStatic& S = D.S;
-    Xf xf;
-    bool culled;
-    if (!rayCar(D, a, s, xf, culled)) return;  // never queued
-    Body cb;
-    WheelTick wt;
-    V3 from, to;
-    cb.xf = xf;
-    wheelSegment(D.P.car, cb, wt, w, from, to);
-    const uint32_t code = (uint32_t)T.rayObj[r], meshes = code & ((1u << MAX_MESHES) - 1u);
-    RayHit hit;
-    hit.fraction = 1.f;
-    hit.obj = -1;
-    hit.normal = v3zero();
-    bool any = code == RAY_ANY;
-    if (!any && meshes) any = !rayVsMeshesNearest(S, meshes, from, to, kOccTol, hit);
-    if (any) {
-        V3 hn = v3zero();
-        float frac = 1.f;
-        const int obj = anyRay(D, a, s, culled, from, to, hn, frac, st);
-        storeRay(D, T, r, obj, frac, hn);
-        return;
-    }
-    st.nStatic += (uint32_t)bitCount(meshes);
+// The planes registered in the cell of a ray's start, in their order.
+RSB_HD void rayPlanes(const ArenaStatic& S, V3 from, V3 to, RayHit& hit, PhaseStats& st) {
     int i, j, k;
     bpCellIndices(S.bp, from, i, j, k);
     for (uint32_t m = S.bpCells[i * S.bp.cellsY * S.bp.cellsZ + j * S.bp.cellsZ + k] >> MAX_MESHES; m; m &= m - 1u) {
@@ -504,26 +484,94 @@ RSB_HD void heavyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, Ph
         st.nStatic++;
         rayVsPlane(S, MAX_MESHES + lowestBit(m), from, to, hit);
     }
-    RegWalk walk{code >> RAY_BODIES_SHIFT, 0u, true};
-    if (walk.cand & ~(2u << s)) {
-        const RayBodies bodies{&D, a, s, arenaTickCount(D, a)};
-        while (true) {
-            const int b = walk.next([&](int e) { return bodyWord(D, a, e, RSB_PW(CarP, regStamp)); });
-            if (b < 0) break;
-            if (b == 1 + s) continue;
-            const Xf bx = bodies[b].xf;
-            const ConvexShape sh = b == 0 ? makeSphere(D.P.ballRadius) : carBoxShape(D.P.car);
-            float frac;
-            V3 n;
-            if (subsimplexCast(from, to, sh, b == 0 ? bx : carChildXf(D.P.car, bx), frac, n) && length2(n) > 0.0001f &&
-                frac < hit.fraction) {
-                hit.fraction = frac;
-                hit.obj = OBJ_BALL + b;
-                hit.normal = normalized(n);
-            }
-        }
-        if (hit.obj >= OBJ_BALL && bodies[hit.obj - OBJ_BALL].noResp) hit.obj = -1;
+}
+struct RayItem {
+    int a, s;
+    V3 from, to;
+};
+RSB_HD bool rayItem(const EngineView& D, uint32_t r, RayItem& o, bool& culled) {
+    const int q = (int)(r / (uint32_t)D.N), w = q / MAX_CARS;
+    o.a = (int)(r % (uint32_t)D.N);
+    o.s = q % MAX_CARS;
+    Xf xf;
+    if (!rayCar(D, o.a, o.s, xf, culled)) return false;  // never queued
+    Body cb;
+    WheelTick wt;
+    cb.xf = xf;
+    wheelSegment(D.P.car, cb, wt, w, o.from, o.to);
+    return true;
+}
+
+// A queued ray near meshes: these, then the planes.  Returns true when it goes on to the body
+// queue: with what was hit so far (RAY_PART), or as a whole.
+constexpr uint32_t RAY_PART = 1u << 29;
+RSB_HD bool meshRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
+    RayItem q;
+    bool culled;
+    if (!rayItem(D, r, q, culled)) return false;
+    const uint32_t code = (uint32_t)T.rayObj[r], meshes = code & ((1u << MAX_MESHES) - 1u);
+    RayHit hit;
+    hit.fraction = 1.f;
+    hit.obj = -1;
+    hit.normal = v3zero();
+    if (!rayVsMeshesNearest(D.S, meshes, q.from, q.to, kOccTol, hit)) {
+        T.rayObj[r] = (int32_t)RAY_ANY;
+        return true;
     }
+    st.nStatic += (uint32_t)bitCount(meshes);
+    rayPlanes(D.S, q.from, q.to, hit, st);
+    if ((code >> RAY_BODIES_SHIFT) & ~(2u << q.s)) {
+        storeRay(D, T, r, 0, hit.fraction, hit.normal);
+        T.rayObj[r] = (int32_t)(RAY_PART | (uint32_t)(hit.obj & 31) | (code >> RAY_BODIES_SHIFT << RAY_BODIES_SHIFT));
+        return true;
+    }
+    storeRay(D, T, r, hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
+    return false;
+}
+
+// A queued ray near other bodies, these in registration order, as castRay tests them.
+RSB_HD void bodyRayPhase(const EngineView& D, const StepTemp& T, uint32_t r, PhaseStats& st) {
+    RayItem q;
+    bool culled;
+    if (!rayItem(D, r, q, culled)) return;
+    const uint32_t code = (uint32_t)T.rayObj[r];
+    if (code == RAY_ANY) {
+        V3 hn = v3zero();
+        float frac = 1.f;
+        const int obj = anyRay(D, q.a, q.s, culled, q.from, q.to, hn, frac, st);
+        storeRay(D, T, r, obj, frac, hn);
+        return;
+    }
+    RayHit hit;
+    hit.fraction = 1.f;
+    hit.obj = -1;
+    hit.normal = v3zero();
+    if (code & RAY_PART) {
+        const size_t rst = (size_t)4 * MAX_CARS * D.N;
+        if ((code & 31u) != 31u) hit.obj = (int)(code & 31u);
+        hit.fraction = T.rayFrac[r];
+        hit.normal = V3{T.rayN[r], T.rayN[r + rst], T.rayN[r + 2 * rst]};
+    } else {
+        rayPlanes(D.S, q.from, q.to, hit, st);
+    }
+    RegWalk walk{(code >> RAY_BODIES_SHIFT) & ((1u << MAX_BODIES) - 1u), 0u, true};
+    const RayBodies bodies{&D, q.a, q.s, arenaTickCount(D, q.a)};
+    while (true) {
+        const int b = walk.next([&](int e) { return bodyWord(D, q.a, e, RSB_PW(CarP, regStamp)); });
+        if (b < 0) break;
+        if (b == 1 + q.s) continue;
+        const Xf bx = bodies[b].xf;
+        const ConvexShape sh = b == 0 ? makeSphere(D.P.ballRadius) : carBoxShape(D.P.car);
+        float frac;
+        V3 n;
+        if (subsimplexCast(q.from, q.to, sh, b == 0 ? bx : carChildXf(D.P.car, bx), frac, n) && length2(n) > 0.0001f &&
+            frac < hit.fraction) {
+            hit.fraction = frac;
+            hit.obj = OBJ_BALL + b;
+            hit.normal = normalized(n);
+        }
+    }
+    if (hit.obj >= OBJ_BALL && bodies[hit.obj - OBJ_BALL].noResp) hit.obj = -1;
     storeRay(D, T, r, hit.obj, hit.fraction, hit.obj >= 0 ? normalized(hit.normal) : hit.normal);
 }
 
@@ -940,6 +988,11 @@ RSB_HD void storePair(const EngineView& D, const StepTemp& T, int a, WT& W, cons
     }
     T.results[res] = r;
     if (W.status | W.cullMissed) phaseAtomicOr(arenaStatus(D, a), W.status | W.cullMissed);
+    // the first contact of a body that is an island by itself queues the body
+    const int b = imax_(m.o0, m.o1) - OBJ_BALL;
+    if (r.flags && !(infoWord(D, T, a, b, BI_PAIRS) & BI_CONTACT) && (infoWord(D, T, a, b, BI_PAIRS) & BI_ALONE) &&
+        !(phaseAtomicOr(&infoWord(D, T, a, b, BI_PAIRS), BI_CONTACT) & BI_CONTACT))
+        T.bodyQ[phaseAtomicAdd(&T.count[QC_BODY], 1u)] = (uint32_t)bodyIdx(D, a, b);
 }
 
 // Static pairs: all of them, those with a manifold, and those that can be in contact (the
@@ -1038,7 +1091,6 @@ RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& 
     const int a = t.a;
     const Body& b = t.body.v;
     const int meshType = t.b == 0 ? QC_BALLMESH : QC_CARMESH, dynType = t.b == 0 ? QC_CARBALL : QC_CARCAR;
-    infoWord(D, T, a, t.b, BI_PAIRS) = o.pairs | ((uint32_t)b.act << BI_ACT_SHIFT) | (b.noResp ? 0u : BI_RESPONDS);
     infoWord(D, T, a, t.b, BI_DYN) = t.dyn;
     if (o.pairs | t.dyn | dynMani) {
         infoWord(D, T, a, t.b, BI_MANI) = o.mani;
@@ -1059,6 +1111,14 @@ RSB_HD void pairStore(const EngineView& D, const StepTemp& T, const PairThread& 
         T.tasks[k] = PairTask{(uint32_t)a, (uint16_t)(OBJ_BALL + t.b), (uint16_t)(OBJ_BALL + hi)};
         T.dynRes[(size_t)dynPair(t.b, hi) * D.N + a] = k;
     }
+}
+
+// The body's first word, once the sums over the arena's bodies are known.
+RSB_HD void pairStoreHead(const EngineView& D, const StepTemp& T, const PairThread& t, const BodyStatics& o,
+                          uint32_t need) {
+    const Body& b = t.body.v;
+    infoWord(D, T, t.a, t.b, BI_PAIRS) = o.pairs | ((uint32_t)b.act << BI_ACT_SHIFT) | (b.noResp ? 0u : BI_RESPONDS) |
+                                         (arenaByBodies(need) ? BI_ALONE : 0u);
 }
 
 RSB_HD void pairNeed(const PairThread& t, const BodyStatics& o, PairShared& sh) {

@@ -199,12 +199,12 @@ struct StepVariant {
     bool persistent;
 };
 static const StepVariant kStepVariants[] = {
-    {heavyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, false},
-    {heavyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, false},
-    {heavyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, false},
-    {heavyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, true},
-    {heavyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, true},
-    {heavyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, true}};
+    {bodyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, false},
+    {bodyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, false},
+    {bodyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, false},
+    {bodyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, true},
+    {bodyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, true},
+    {bodyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, true}};
 constexpr int kNumStepVariants = sizeof(kStepVariants) / sizeof(kStepVariants[0]);
 static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
@@ -658,7 +658,7 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
         // make the per-thread stack limit cover the largest (the default limit is 1 KB), and give
         // the L1 its largest share in those that use no shared memory to speak of
         size_t need = 0;
-        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)deepKernel,
+        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)meshRayKernel,
                                      (const void*)combineKernel};
         for (const StepVariant& v : kStepVariants)
             for (StepFn f : {v.ray, v.triangle, v.solve}) fns.push_back((const void*)f);
@@ -766,23 +766,25 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
         }
         return (int)std::max<int64_t>(1, (g + warps - 1) / warps);
     };
-    const int rayGrid = grid(sv.ray, 4 * (int64_t)h->numCars, kRayWarps);
+    const int meshRayGrid = (int)std::max<int64_t>(1, std::min<int64_t>((4 * (int64_t)h->numCars + 31) / 32, 32 * (int64_t)h->smCount));
+    const int rayGrid = grid(sv.ray, 2 * (int64_t)h->numCars, kBodyRayWarps);
     // four pairs to a warp
     const int pairGrid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)h->numCars + h->N) / 16, 16 * (int64_t)h->smCount));
     const int triGrid = grid(sv.triangle, 4 * ((int64_t)h->numCars + h->N), kTriangleWarps);
-    const int deepGrid = grid(deepKernel, h->numCars + h->N, kDeepWarps), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
+    const int deepGrid = (int)std::min<int64_t>(h->numCars + h->N, 16 * (int64_t)h->smCount), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
     const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kSolveWarps);
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
         if (h->maxCars > 0) {
             rayKernel<<<groups, carThreads, 0, st>>>(D, T);
+            meshRayKernel<<<meshRayGrid, MESHRAY_THREADS, 0, st>>>(D, T);
             sv.ray<<<rayGrid, block, 0, st>>>(D, T);
             driveKernel<<<groups, carThreads, 0, st>>>(D, T);
         }
         pairKernel<<<groups, bodyThreads, 0, st>>>(D, T, t == 0);
         findKernel<<<pairGrid, FIND_THREADS, 0, st>>>(D, T);
         sv.triangle<<<triGrid, block, 0, st>>>(D, T);
-        deepKernel<<<deepGrid, block, 0, st>>>(D, T);
+        deepKernel<<<deepGrid, 32, 0, st>>>(D, T);
         combineKernel<<<combineGrid, block, 0, st>>>(D, T);
         sv.solve<<<solveGrid, block, 0, st>>>(D, T);
         finishKernel<<<groups, bodyThreads, 0, st>>>(D, T);

@@ -48,7 +48,7 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
 // 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 /
 // 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113 and 102, whole-arena
 // islands 234 and 886 (64).
-constexpr int kRayWarps = 16, kTriangleWarps = 12, kDeepWarps = 16, kCombineWarps = 16, kSolveWarps = 4;
+constexpr int kMeshRayWarps = 32, kBodyRayWarps = 16, kTriangleWarps = 12, kCombineWarps = 16, kSolveWarps = 4;
 
 // Items of several queues, fn(queue, item): a warp takes `width` items of one queue at a time,
 // as few as it takes to give each of `spread` warps some.
@@ -107,12 +107,26 @@ __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__
     blockStats(D, st);
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) heavyRayKernel(const __grid_constant__ EngineView D,
-                                                            const __grid_constant__ StepTemp T) {
-    const uint32_t n[2] = {T.count[QC_RAY], T.count[QC_BODYRAY]};
+// Rays near meshes: few registers, so that many warps wait for triangles at once (in one kernel
+// with the convex casts, at 232 registers, 295 us per tick at 3v3 x 65,536).
+constexpr int MESHRAY_THREADS = 128;
+__global__ void __launch_bounds__(MESHRAY_THREADS) meshRayKernel(const __grid_constant__ EngineView D,
+                                                                 const __grid_constant__ StepTemp T) {
+    const uint32_t n[1] = {T.count[QC_RAY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<2>(n, kRayWarps * T.sms, [&](int q, uint32_t i) { heavyRayPhase(D, T, T.rayQ[q * rayPlaces(D) + i], st); });
+    forItems<1>(n, kMeshRayWarps * T.sms, [&](int, uint32_t i) {
+        const uint32_t r = T.rayQ[i];
+        if (meshRayPhase(D, T, r, st)) T.rayQ[rayPlaces(D) + atomicAdd(&T.count[QC_BODYRAY], 1u)] = r;
+    });
+    blockStats(D, st);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) bodyRayKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T) {
+    const uint32_t n[1] = {T.count[QC_BODYRAY]};
+    PhaseStats st{0, 0, 0, 0};
+    forItems<1>(n, kBodyRayWarps * T.sms, [&](int, uint32_t i) { bodyRayPhase(D, T, T.rayQ[rayPlaces(D) + i], st); });
     blockStats(D, st);
 }
 
@@ -179,9 +193,7 @@ __global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant
     }
     __syncthreads();
     const uint32_t need = sh.need[lane];
-    const bool alone = valid && (o.meshes | o.planes) && arenaByBodies(need);
-    const uint32_t at = queueAlloc(&T.count[QC_BODY], alone ? 1u : 0u);
-    if (alone) T.bodyQ[at] = (uint32_t)bodyIdx(D, t.a, t.b);
+    if (valid) pairStoreHead(D, T, t, o, need);
     if (threadIdx.x < PHASE_ARENAS) {
         const bool whole = arenaHasContacts(need) && !arenaByBodies(need);
         const uint32_t as = queueAlloc(&T.count[QC_SOLVE], whole ? 1u : 0u);
@@ -290,12 +302,18 @@ __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constan
     blockStats(D, st);
 }
 
-__global__ void __launch_bounds__(128) deepKernel(const __grid_constant__ EngineView D,
-                                                  const __grid_constant__ StepTemp T) {
-    EpaWork epa;
+// The penetration solver, one item to a warp with the solver's 12 KB of faces and support points
+// in shared memory.  The items are few (about one in forty arenas) and each is a serial chain
+// through that memory; as thread-local memory every word of it took a sector of its own, since
+// one lane was active, and a tick waited 140 us for the longest item at 3v3 x 65,536.
+__global__ void __launch_bounds__(32) deepKernel(const __grid_constant__ EngineView D,
+                                                 const __grid_constant__ StepTemp T) {
+    __shared__ EpaWork epa;
     PhaseStats st{0, 0, 0, 0};
-    const uint32_t n[1] = {T.count[QC_DEEP]};
-    forItems<1>(n, kDeepWarps * T.sms, [&](int, uint32_t i) { deepPhase(D, T, T.deepQ[i], &epa, st); });
+    const uint32_t n = T.count[QC_DEEP];
+    if (threadIdx.x == 0)
+        for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) deepPhase(D, T, T.deepQ[i], &epa, st);
+    __syncwarp();
     blockStats(D, st);
 }
 

@@ -34,8 +34,8 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     D.work = nullptr;
     std::vector<int32_t> rayObj(R);
     std::vector<float> rayFrac(R), rayN(3 * R), force(6 * B), box(6 * B), cache(3 * B);
-    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(2 * R), solveQ(N), bodyQ(B),
-        statics(MAX_BODIES * PHASE_ARENAS);
+    std::vector<uint32_t> info(BI_WORDS * B, 0xdeadbeefu), dynRes(NUM_DYN_PAIRS * N), count(QC_WORDS, 0u), rayQ(2 * R), solveQ(N), bodyQ(B);
+    std::vector<BodyStatics> statics(MAX_BODIES * PHASE_ARENAS);
     std::vector<PairTask> tasks(CAP_RESULTS * N);
     std::vector<PairResult> results(CAP_RESULTS * N);
     std::vector<MPoint> blocks(MAX_BLOCKS * N * MAX_POINTS);
@@ -96,10 +96,13 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
                     else if (c == RAY_BODIES) T.rayQ[R + T.count[QC_BODYRAY]++] = (uint32_t)rayIdx(D, a, s, w);
                 }
             }
-        for (int k = QC_RAY; k <= QC_BODYRAY; k++) {
-            counts[k] += T.count[k];
-            while (T.count[k] > 0) heavyRayPhase(D, T, T.rayQ[(k == QC_RAY ? 0 : R) + --T.count[k]], st);
+        counts[QC_RAY] += T.count[QC_RAY];
+        while (T.count[QC_RAY] > 0) {
+            const uint32_t r = T.rayQ[--T.count[QC_RAY]];
+            if (meshRayPhase(D, T, r, st)) T.rayQ[R + T.count[QC_BODYRAY]++] = r;
         }
+        counts[QC_BODYRAY] += T.count[QC_BODYRAY];
+        while (T.count[QC_BODYRAY] > 0) bodyRayPhase(D, T, T.rayQ[R + --T.count[QC_BODYRAY]], st);
         // cars
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {
             auto each = [&](auto&& fn) {
@@ -154,11 +157,10 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
                 const uint32_t d0 = phaseAtomicAdd(&T.count[b == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)bitCount(dyn));
                 pairStore(D, T, t, o, dyn, m0, p0, d0);
                 pairNeed(t, o, *sh);
-                statics[b * PHASE_ARENAS + t.la] = o.meshes | o.planes;
+                statics[b * PHASE_ARENAS + t.la] = o;
             });
             each([&](PairThread& t, int b, int la) {
-                if (statics[b * PHASE_ARENAS + la] && arenaByBodies(sh->need[la]) && by_bodies)
-                    T.bodyQ[T.count[QC_BODY]++] = (uint32_t)bodyIdx(D, t.a, b);
+                pairStoreHead(D, T, t, statics[b * PHASE_ARENAS + la], by_bodies ? sh->need[la] : sh->need[la] | PN_DYN);
             });
             for (int la = 0; la < PHASE_ARENAS; la++)
                 if (arenaHasContacts(sh->need[la]) && !(arenaByBodies(sh->need[la]) && by_bodies))
