@@ -600,6 +600,17 @@ bool buildArenaStatic(const std::string& folder, ArenaStaticHost& out) {
                     }
         }
         S.occ = out.occ.data();
+        // the four voxels from each on, one axis after another
+        out.occAhead = out.occ;
+        const int dims[3] = {S.occX, S.occY, S.occZ}, step[3] = {S.occY * S.occZ, S.occZ, 1};
+        for (int axis = 0; axis < 3; axis++) {
+            const std::vector<uint16_t> from = out.occAhead;
+            for (size_t v = 0; v < nv; v++) {
+                const int at = (int)(v / step[axis]) % dims[axis];
+                for (int k = 1; k < 4 && at + k < dims[axis]; k++) out.occAhead[v] |= from[v + (size_t)k * step[axis]];
+            }
+        }
+        S.occAhead = out.occAhead.data();
         // per-voxel triangle lists, each sorted by (mesh, BVH leaf): the order in which the
         // meshes' BVH walks would report them
         std::sort(lists.begin(), lists.end());

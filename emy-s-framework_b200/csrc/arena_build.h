@@ -16,7 +16,7 @@ struct ArenaStaticHost {
     std::vector<BvhNode> leaves;
     std::vector<TriEdgeInfo> triInfo;
     std::vector<uint32_t> bpCells;
-    std::vector<uint16_t> occ;
+    std::vector<uint16_t> occ, occAhead;
     std::vector<uint32_t> voxOff, voxList;
     std::vector<uint16_t> occDist;
     ArenaStatic view;  // pointers into the vectors above (host addresses)

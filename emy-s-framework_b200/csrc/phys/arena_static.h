@@ -106,6 +106,9 @@ struct ArenaStatic {
     // region holds no triangle there, so its queries confined to the region cannot find
     // anything and are skipped.
     const uint16_t* occ;
+    // Per voxel, the bits of the 4 x 4 x 4 voxels from it on: zero says that a box of at most
+    // four voxels a side that starts there meets no mesh.
+    const uint16_t* occAhead;
     // Per voxel (CSR: voxOff[v] .. voxOff[v + 1] into voxList), the mesh triangles marked in
     // it as voxKey(mesh, BVH leaf node, triangle), sorted: the order the meshes' BVH walks
     // visit them.
@@ -140,6 +143,8 @@ RSB_HD uint32_t occMask(const ArenaStatic& S, V3 mn, V3 mx) {
     int y0 = (int)floorf((mn.y - S.occMin.y) * f), y1 = (int)floorf((mx.y - S.occMin.y) * f);
     int z0 = (int)floorf((mn.z - S.occMin.z) * f), z1 = (int)floorf((mx.z - S.occMin.z) * f);
     if (!(x0 >= 0 && y0 >= 0 && z0 >= 0 && x1 < S.occX && y1 < S.occY && z1 < S.occZ)) return 0xffffffffu;
+    // most boxes are far from every mesh, which one voxel's word says
+    if (x1 - x0 < 4 && y1 - y0 < 4 && z1 - z0 < 4 && !S.occAhead[(x0 * S.occY + y0) * S.occZ + z0]) return 0;
     uint32_t m = 0;
     for (int x = x0; x <= x1; x++)
         for (int y = y0; y <= y1; y++)

@@ -274,6 +274,25 @@ RSB_HD Xf respawnXf(const EngineView& D, int a, int s, uint32_t flags, uint64_t 
     return Xf{rot, pos * kUuToBt};
 }
 
+// A broadphase cell's indices in one word (they are below 256, as every registration is in the
+// grid), and whether two cells are neighbours or the same (inRegNeighbourhood).
+RSB_HD uint32_t cellWord(int i, int j, int k) { return (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16); }
+RSB_HD bool cellsNear(uint32_t p, uint32_t q) {
+#if defined(__CUDA_ARCH__)
+    return (__vabsdiffu4(p, q) & 0x00fefefeu) == 0;
+#else
+    for (int s = 0; s < 24; s += 8) {
+        const int d = (int)((p >> s) & 255u) - (int)((q >> s) & 255u);
+        if (d < -1 || d > 1) return false;
+    }
+    return true;
+#endif
+}
+RSB_HD uint32_t bodyCellWord(const EngineView& D, int a, int b) {
+    return cellWord((int)bodyWord(D, a, b, RSB_PW(CarP, ci)), (int)bodyWord(D, a, b, RSB_PW(CarP, cj)),
+                    (int)bodyWord(D, a, b, RSB_PW(CarP, ck)));
+}
+
 // ------------------------------------------------------------------ wheel rays
 
 // What castRay reads of the world, for the rays of car `viewer`, from the records as the last
@@ -376,7 +395,7 @@ constexpr uint32_t RAY_ANY = 1u << 30;
 enum RayClass : int { RAY_DONE = 0, RAY_MESHES, RAY_BODIES };
 
 // Wheel w of car s: casts the ray if only planes can be near, else says which queue it goes to.
-// `near(i, j, k)`: the bodies registered around that cell, the car itself among them.
+// `near(cell)`: the bodies registered around that cell, the car itself among them.
 template <class NearF>
 RSB_HD RayClass rayPhase(const EngineView& D, const StepTemp& T, int a, int s, int w, const Xf& xf, bool culled,
                          NearF&& near, PhaseStats& st) {
@@ -394,7 +413,7 @@ RSB_HD RayClass rayPhase(const EngineView& D, const StepTemp& T, int a, int s, i
     int i, j, k;
     bpCellIndices(S.bp, from, i, j, k);
     uint32_t mask = S.bpCells[i * S.bp.cellsY * S.bp.cellsZ + j * S.bp.cellsZ + k];
-    const uint32_t bodies = near(i, j, k), kMeshBits = (1u << MAX_MESHES) - 1u;
+    const uint32_t bodies = near(cellWord(i, j, k)), kMeshBits = (1u << MAX_MESHES) - 1u;
     uint32_t meshes = mask & kMeshBits;
     if (meshes) {
         const V3 tolv{kOccTol, kOccTol, kOccTol};
@@ -587,7 +606,7 @@ struct DriveShared {
 // ... and the threads of its bodies during the pairs phase.
 struct PairShared {
     float box[MAX_BODIES][6][PHASE_ARENAS];
-    int32_t cell[MAX_BODIES][3][PHASE_ARENAS];
+    uint32_t cell[MAX_BODIES][PHASE_ARENAS];  // cellWord of the registration
     uint32_t stamp[MAX_BODIES][PHASE_ARENAS];
     uint32_t pick[MAX_BODIES][PHASE_ARENAS];  // BI_DYN word of each body
     uint32_t live[MAX_BODIES][PHASE_ARENAS];  // 1: active (objActive)
@@ -873,9 +892,7 @@ RSB_HD void pairLoad(const EngineView& D, const StepTemp& T, PairThread& t, Pair
     const float bx[6] = {b.bpMin.x, b.bpMin.y, b.bpMin.z, b.bpMax.x, b.bpMax.y, b.bpMax.z};
 #pragma unroll
     for (int k = 0; k < 6; k++) sh.box[t.b][k][la] = bx[k];
-    sh.cell[t.b][0][la] = b.ci;
-    sh.cell[t.b][1][la] = b.cj;
-    sh.cell[t.b][2][la] = b.ck;
+    sh.cell[t.b][la] = cellWord(b.ci, b.cj, b.ck);
     sh.stamp[t.b][la] = (uint32_t)b.regStamp;
     sh.live[t.b][la] = (b.act != ACT_SLEEPING && b.act != ACT_DISABLE_SIM) ? 1u : 0u;
     if (b.cell != cell0) putBodyWord(D, a, t.b, RSB_PW(CarP, cell), (uint32_t)b.cell);
@@ -896,13 +913,9 @@ RSB_HD void pairPick(const EngineView& D, PairThread& t, PairShared& sh) {
     const int la = t.la;
     t.dyn = 0;
     if (t.nb > 1) {
-        const int ci = b.cell / (g.cellsY * g.cellsZ), cj = (b.cell / g.cellsZ) % g.cellsY, ck = b.cell % g.cellsZ;
-        auto near = [&](int e) {
-            const int i = sh.cell[e][0][la], j = sh.cell[e][1][la], k = sh.cell[e][2][la];
-            return ci >= i - 1 && ci <= i + 1 && cj >= j - 1 && cj <= j + 1 && ck >= k - 1 && ck <= k + 1;
-        };
+        const uint32_t own = cellWord(b.cell / (g.cellsY * g.cellsZ), (b.cell / g.cellsZ) % g.cellsY, b.cell % g.cellsZ);
         uint32_t cand = 0, n = 0;
-        for (int e = 0; e < t.nb; e++) cand |= near(e) ? 1u << e : 0u;
+        for (int e = 0; e < t.nb; e++) cand |= cellsNear(own, sh.cell[e][la]) ? 1u << e : 0u;
         if (cand & (cand - 1u)) {
             RegWalk walk{cand, 0u, true};
             while (true) {

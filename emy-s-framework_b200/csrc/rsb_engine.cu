@@ -48,7 +48,7 @@ struct DevStatic {
     BvhNode* leaves = nullptr;
     TriEdgeInfo* triInfo = nullptr;
     uint32_t* bpCells = nullptr;
-    uint16_t* occ = nullptr;
+    uint16_t *occ = nullptr, *occAhead = nullptr;
     uint32_t* voxOff = nullptr;
     uint32_t* voxList = nullptr;
     uint16_t* occDist = nullptr;
@@ -626,7 +626,7 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
             };
             if (!up(D->nodes, H->nodes) || !up(D->subs, H->subs) || !up(D->subLeaves, H->subLeaves) || !up(D->leaves, H->leaves) ||
                 !up(D->triData, H->triData) || !up(D->triVerts, H->triVerts) ||
-                !up(D->triInfo, H->triInfo) || !up(D->bpCells, H->bpCells) || !up(D->occ, H->occ) ||
+                !up(D->triInfo, H->triInfo) || !up(D->bpCells, H->bpCells) || !up(D->occ, H->occ) || !up(D->occAhead, H->occAhead) ||
                 !up(D->voxOff, H->voxOff) || !up(D->voxList, H->voxList) || !up(D->occDist, H->occDist))
                 return fail(nullptr, RSB_ERR_CUDA, "uploading arena meshes failed");
             D->view = deviceView(*H, D->nodes, D->subs, D->triVerts, D->triInfo, D->bpCells, D->occ, D->voxOff,
@@ -639,6 +639,7 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
             if (cudaMemcpyToSymbol(g_rsqrtTable, c.rsqrtTable, sizeof(c.rsqrtTable)) != cudaSuccess)
                 return fail(nullptr, RSB_ERR_CUDA, "uploading the rsqrt estimate table failed");
             c.rsqrtDevices.insert(h->device);
+            D->view.occAhead = D->occAhead;
             D->view.triData = D->triData;
             D->view.subLeaves = D->subLeaves;
             D->view.leaves = D->leaves;
@@ -770,9 +771,9 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     const int rayGrid = grid(sv.ray, 2 * (int64_t)h->numCars, kBodyRayWarps);
     // four pairs to a warp
     const int pairGrid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)h->numCars + h->N) / 16, 16 * (int64_t)h->smCount));
-    const int triGrid = grid(sv.triangle, 4 * ((int64_t)h->numCars + h->N), kTriangleWarps);
+    const int triGrid = grid(sv.triangle, (int64_t)h->numCars + h->N, kTriangleWarps + kPairWarps);
     const int deepGrid = (int)std::min<int64_t>(h->numCars + h->N, 16 * (int64_t)h->smCount), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
-    const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kSolveWarps);
+    const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kWholeWarps + kBodyWarps);
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
         if (h->maxCars > 0) {

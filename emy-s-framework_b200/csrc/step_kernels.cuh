@@ -48,24 +48,32 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
 // 149 (2v2 x 8,192: 49 / 42 / 52 / 61 / 83), triangles 116 / 79 / 64 / 95 / 145 (44 / 33 / 46 /
 // 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113 and 102, whole-arena
 // islands 234 and 886 (64).
-constexpr int kMeshRayWarps = 32, kBodyRayWarps = 16, kTriangleWarps = 12, kCombineWarps = 16, kSolveWarps = 4;
+constexpr int kMeshRayWarps = 32, kBodyRayWarps = 16, kTriangleWarps = 12, kPairWarps = 12, kCombineWarps = 16,
+              kWholeWarps = 16, kBodyWarps = 8;
 
-// Items of several queues, fn(queue, item): a warp takes `width` items of one queue at a time,
-// as few as it takes to give each of `spread` warps some.
+// Items of several queues, fn(queue, item): a warp takes items of one queue at a time, as few as
+// it takes to give each of spread[queue] warps some.
 template <int NQ, class F>
-RSB_D void forItems(const uint32_t* n, uint32_t spread, F&& fn) {
+RSB_D void forItems(const uint32_t (&n)[NQ], const uint32_t (&spread)[NQ], F&& fn) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31u;
-    uint32_t total = 0, tiles = 0;
-    for (int k = 0; k < NQ; k++) total += n[k];
-    const uint32_t width = min(32u, (total + spread - 1u) / spread);
-    if (width == 0) return;
-    for (int k = 0; k < NQ; k++) tiles += (n[k] + width - 1u) / width;
-    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
+    uint32_t width[NQ], tiles[NQ], total = 0;
+#pragma unroll
+    for (int k = 0; k < NQ; k++) {
+        width[k] = max(1u, min(32u, (n[k] + spread[k] - 1u) / spread[k]));
+        tiles[k] = (n[k] + width[k] - 1u) / width[k];
+        total += tiles[k];
+    }
+    for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < total; tile += warps) {
         uint32_t q = tile;
-        int k = 0;
-        while (q >= (n[k] + width - 1u) / width) q -= (n[k++] + width - 1u) / width;
-        const uint32_t i = q * width + lane;
-        if (lane < width && i < n[k]) fn(k, i);
+#pragma unroll
+        for (int k = 0; k < NQ; k++) {
+            if (q < tiles[k]) {
+                const uint32_t i = q * width[k] + lane;
+                if (lane < width[k] && i < n[k]) fn(k, i);
+                break;
+            }
+            q -= tiles[k];
+        }
     }
 }
 
@@ -76,25 +84,20 @@ RSB_D size_t rayPlaces(const EngineView& D) { return (size_t)4 * MAX_CARS * D.N;
 
 __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__ EngineView D,
                                                          const __grid_constant__ StepTemp T) {
-    __shared__ int32_t cell[MAX_BODIES][3][PHASE_ARENAS];
+    __shared__ uint32_t cell[MAX_BODIES][PHASE_ARENAS];
     const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
     const int a = blockIdx.x * PHASE_ARENAS + lane;
     const int nb = a < D.N ? arenaBodies(D, a) : 0;
     for (int b = s; b < MAX_BODIES; b += blockDim.x >> 5)
-        if (b < nb)
-            for (int k = 0; k < 3; k++)
-                cell[b][k][lane] = (int32_t)bodyWord(D, a, b, (int)(offsetof(CarP, ci) / 4) + k);
+        if (b < nb) cell[b][lane] = bodyCellWord(D, a, b);
     __syncthreads();
     PhaseStats st{0, 0, 0, 0};
     Xf xf;
     bool culled = false;
     const bool live = 1 + s < nb && rayCar(D, a, s, xf, culled);
-    auto near = [&](int i, int j, int k) {
+    auto near = [&](uint32_t at) {
         uint32_t n = 0;
-        for (int b = 0; b < nb; b++) {
-            const int ci = cell[b][0][lane], cj = cell[b][1][lane], ck = cell[b][2][lane];
-            if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) n |= 1u << b;
-        }
+        for (int b = 0; b < nb; b++) n |= cellsNear(at, cell[b][lane]) ? 1u << b : 0u;
         return n;
     };
     for (int w = 0; w < 4; w++) {
@@ -114,7 +117,8 @@ __global__ void __launch_bounds__(MESHRAY_THREADS) meshRayKernel(const __grid_co
                                                                  const __grid_constant__ StepTemp T) {
     const uint32_t n[1] = {T.count[QC_RAY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<1>(n, kMeshRayWarps * T.sms, [&](int, uint32_t i) {
+    const uint32_t w[1] = {kMeshRayWarps * T.sms};
+    forItems(n, w, [&](int, uint32_t i) {
         const uint32_t r = T.rayQ[i];
         if (meshRayPhase(D, T, r, st)) T.rayQ[rayPlaces(D) + atomicAdd(&T.count[QC_BODYRAY], 1u)] = r;
     });
@@ -126,7 +130,8 @@ __global__ void __launch_bounds__(128, MINB) bodyRayKernel(const __grid_constant
                                                            const __grid_constant__ StepTemp T) {
     const uint32_t n[1] = {T.count[QC_BODYRAY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<1>(n, kBodyRayWarps * T.sms, [&](int, uint32_t i) { bodyRayPhase(D, T, T.rayQ[rayPlaces(D) + i], st); });
+    const uint32_t w[1] = {kBodyRayWarps * T.sms};
+    forItems(n, w, [&](int, uint32_t i) { bodyRayPhase(D, T, T.rayQ[rayPlaces(D) + i], st); });
     blockStats(D, st);
 }
 
@@ -294,7 +299,8 @@ __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constan
                                                             const __grid_constant__ StepTemp T) {
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[3] = {min(T.count[QC_TRI], T.candCap), T.count[QC_CARCAR], T.count[QC_PLANE]};
-    forItems<3>(n, kTriangleWarps * T.sms, [&](int k, uint32_t i) {
+    const uint32_t w[3] = {kTriangleWarps * T.sms, kPairWarps * T.sms, kPairWarps * T.sms};
+    forItems(n, w, [&](int k, uint32_t i) {
         if (k == 0) trianglePhase(D, T, i);
         else if (k == 1) carCarPhase(D, T, (uint32_t)resultBase(QC_CARCAR) * (uint32_t)D.N + i);
         else planePhase(D, T, (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + i, st);
@@ -321,7 +327,8 @@ __global__ void __launch_bounds__(128) combineKernel(const __grid_constant__ Eng
                                                      const __grid_constant__ StepTemp T) {
     PhaseStats st{0, 0, 0, 0};
     const uint32_t n[1] = {T.count[QC_COMBINE]};
-    forItems<1>(n, kCombineWarps * T.sms, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
+    const uint32_t w[1] = {kCombineWarps * T.sms};
+    forItems(n, w, [&](int, uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
     blockStats(D, st);
 }
 
@@ -330,7 +337,8 @@ __global__ void __launch_bounds__(128, MINB) solveKernel(const __grid_constant__
                                                          const __grid_constant__ StepTemp T) {
     const uint32_t n[2] = {T.count[QC_SOLVE], T.count[QC_BODY]};
     PhaseStats st{0, 0, 0, 0};
-    forItems<2>(n, kSolveWarps * T.sms, [&](int k, uint32_t i) {
+    const uint32_t w[2] = {kWholeWarps * T.sms, kBodyWarps * T.sms};
+    forItems(n, w, [&](int k, uint32_t i) {
         if (k == 0) solvePhase(D, T, (int)T.solveQ[i], st);
         else bodyPhase(D, T, T.bodyQ[i], st);
     });

@@ -81,13 +81,9 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
                 Xf xf;
                 bool culled;
                 if (!rayCar(D, a, s, xf, culled)) continue;
-                auto near = [&](int i, int j, int k) {
+                auto near = [&](uint32_t at) {
                     uint32_t n = 0;
-                    for (int b = 0; b < arenaBodies(D, a); b++) {
-                        const int w = (int)(offsetof(CarP, ci) / 4);
-                        const int ci = (int)bodyWord(D, a, b, w), cj = (int)bodyWord(D, a, b, w + 1), ck = (int)bodyWord(D, a, b, w + 2);
-                        if (i >= ci - 1 && i <= ci + 1 && j >= cj - 1 && j <= cj + 1 && k >= ck - 1 && k <= ck + 1) n |= 1u << b;
-                    }
+                    for (int b = 0; b < arenaBodies(D, a); b++) n |= cellsNear(at, bodyCellWord(D, a, b)) ? 1u << b : 0u;
                     return n;
                 };
                 for (int w = 0; w < 4; w++) {
