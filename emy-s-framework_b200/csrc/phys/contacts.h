@@ -182,138 +182,64 @@ RSB_HD bool clampNormal(V3 edge, V3 triNormalOrg, V3 localNormal, float correcte
 }
 
 // The mesh's collision object is at the identity transform, so mesh-local and world
-// coordinates coincide (the reference's basis products with the identity are exact).
+// coordinates coincide (the reference's basis products with the identity are exact).  The
+// reference tests its three edges in turn but acts only on the nearest one with an angle, the
+// first of those equally near, so that edge alone is worked on here.
 RSB_HD void adjustInternalEdge(MPoint& cp, const V3* v, const TriEdgeInfo& info) {
     if (!(info.flags & TRI_INFO_PRESENT)) return;
     const float kMaxEdgeAngle = kTwoPi, kConvexEps = 0.f, kEdgeDist = 0.1f;
     const float frontFacing = 1.f;  // normalAdjustFlags == 0
-    V3 v0 = v[0], v1 = v[1], v2 = v[2];
+    const V3 v0 = v[0], v1 = v[1], v2 = v[2];
     V3 triNormal = normalized(cross(v1 - v0, v2 - v0));
-    V3 nearest;
-    nearestPointInLineSegment(cp.localB, v0, v1, nearest);
-    V3 contact = cp.localB;
-    bool isNearEdge = false;
-    int numConcave = 0;
+    const V3 contact = cp.localB;
     V3 localNormal = normalized(cp.normal);
     int best = -1;
     float bestDist = kLargeFloat;
-    if (fabsf(info.a01) < kMaxEdgeAngle) {
+    auto edgeDistance = [&](V3 a, V3 b) {
         V3 nr;
-        nearestPointInLineSegment(cp.localB, v0, v1, nr);
-        float len = length(contact - nr);
+        nearestPointInLineSegment(contact, a, b, nr);
+        return length(contact - nr);
+    };
+    if (fabsf(info.a01) < kMaxEdgeAngle) {
+        float len = edgeDistance(v0, v1);
         if (len < bestDist) { best = 0; bestDist = len; }
     }
     if (fabsf(info.a12) < kMaxEdgeAngle) {
-        V3 nr;
-        nearestPointInLineSegment(cp.localB, v1, v2, nr);
-        float len = length(contact - nr);
+        float len = edgeDistance(v1, v2);
         if (len < bestDist) { best = 1; bestDist = len; }
     }
     if (fabsf(info.a20) < kMaxEdgeAngle) {
-        V3 nr;
-        nearestPointInLineSegment(cp.localB, v2, v0, nr);
-        float len = length(contact - nr);
+        float len = edgeDistance(v2, v0);
         if (len < bestDist) { best = 2; bestDist = len; }
     }
-    // edge v0-v1 (uses the outer `localNormal`, normalised)
-    if (fabsf(info.a01) < kMaxEdgeAngle) {
-        float len = length(contact - nearest);
-        if (len < kEdgeDist && best == 0) {
-            V3 edge = v0 - v1;
-            isNearEdge = true;
-            if (info.a01 == 0.f) {
-                numConcave++;
-            } else {
-                bool isConvex = (info.flags & TRI_INFO_V0V1_CONVEX) != 0;
-                float swapFactor = isConvex ? 1.f : -1.f;
-                V3 nA = triNormal * swapFactor;
-                V3 cnB = quatRotate(qaxisAngle(edge, info.a01), triNormal);
-                if (info.flags & TRI_INFO_V0V1_SWAP_NORMALB) cnB *= -1.f;
-                V3 nB = cnB * swapFactor;
-                float ndA = dot(localNormal, nA), ndB = dot(localNormal, nB);
-                bool back = (ndA < kConvexEps) && (ndB < kConvexEps);
-                if (back) {
-                    numConcave++;
-                } else {
-                    V3 clamped;
-                    if (clampNormal(edge, triNormal * swapFactor, localNormal, info.a01, clamped)) {
-                        if (dot(clamped, triNormal * frontFacing) > 0) {
-                            cp.normal = clamped;
-                            cp.posB = cp.posA - cp.normal * cp.dist;
-                            cp.localB = cp.posB;
-                        }
-                    }
+    if (best < 0 || !(bestDist < kEdgeDist)) return;
+    const V3 edge = best == 0 ? v0 - v1 : (best == 1 ? v1 - v2 : v2 - v0);
+    const float angle = best == 0 ? info.a01 : (best == 1 ? info.a12 : info.a20);
+    const int32_t convexFlag = best == 0 ? TRI_INFO_V0V1_CONVEX : (best == 1 ? TRI_INFO_V1V2_CONVEX : TRI_INFO_V2V0_CONVEX);
+    const int32_t swapFlag =
+        best == 0 ? TRI_INFO_V0V1_SWAP_NORMALB : (best == 1 ? TRI_INFO_V1V2_SWAP_NORMALB : TRI_INFO_V2V0_SWAP_NORMALB);
+    bool concave = angle == 0.f;
+    if (!concave) {
+        float swapFactor = (info.flags & convexFlag) ? 1.f : -1.f;
+        V3 nA = triNormal * swapFactor;
+        V3 cnB = quatRotate(qaxisAngle(edge, angle), triNormal);
+        if (info.flags & swapFlag) cnB *= -1.f;
+        V3 nB = cnB * swapFactor;
+        float ndA = dot(localNormal, nA), ndB = dot(localNormal, nB);
+        concave = (ndA < kConvexEps) && (ndB < kConvexEps);
+        if (!concave) {
+            // the first edge clamps the normalised normal, the others the normal as it is
+            V3 clamped;
+            if (clampNormal(edge, triNormal * swapFactor, best == 0 ? localNormal : cp.normal, angle, clamped)) {
+                if (dot(clamped, triNormal * frontFacing) > 0) {
+                    cp.normal = clamped;
+                    cp.posB = cp.posA - cp.normal * cp.dist;
+                    cp.localB = cp.posB;
                 }
             }
         }
     }
-    nearestPointInLineSegment(contact, v1, v2, nearest);
-    if (fabsf(info.a12) < kMaxEdgeAngle) {
-        float len = length(contact - nearest);
-        if (len < kEdgeDist && best == 1) {
-            isNearEdge = true;
-            V3 edge = v1 - v2;
-            if (info.a12 == 0.f) {
-                numConcave++;
-            } else {
-                bool isConvex = (info.flags & TRI_INFO_V1V2_CONVEX) != 0;
-                float swapFactor = isConvex ? 1.f : -1.f;
-                V3 nA = triNormal * swapFactor;
-                V3 cnB = quatRotate(qaxisAngle(edge, info.a12), triNormal);
-                if (info.flags & TRI_INFO_V1V2_SWAP_NORMALB) cnB *= -1.f;
-                V3 nB = cnB * swapFactor;
-                float ndA = dot(localNormal, nA), ndB = dot(localNormal, nB);
-                bool back = (ndA < kConvexEps) && (ndB < kConvexEps);
-                if (back) {
-                    numConcave++;
-                } else {
-                    V3 ln = cp.normal;  // recomputed without normalisation, as the reference does
-                    V3 clamped;
-                    if (clampNormal(edge, triNormal * swapFactor, ln, info.a12, clamped)) {
-                        if (dot(clamped, triNormal * frontFacing) > 0) {
-                            cp.normal = clamped;
-                            cp.posB = cp.posA - cp.normal * cp.dist;
-                            cp.localB = cp.posB;
-                        }
-                    }
-                }
-            }
-        }
-    }
-    nearestPointInLineSegment(contact, v2, v0, nearest);
-    if (fabsf(info.a20) < kMaxEdgeAngle) {
-        float len = length(contact - nearest);
-        if (len < kEdgeDist && best == 2) {
-            isNearEdge = true;
-            V3 edge = v2 - v0;
-            if (info.a20 == 0.f) {
-                numConcave++;
-            } else {
-                bool isConvex = (info.flags & TRI_INFO_V2V0_CONVEX) != 0;
-                float swapFactor = isConvex ? 1.f : -1.f;
-                V3 nA = triNormal * swapFactor;
-                V3 cnB = quatRotate(qaxisAngle(edge, info.a20), triNormal);
-                if (info.flags & TRI_INFO_V2V0_SWAP_NORMALB) cnB *= -1.f;
-                V3 nB = cnB * swapFactor;
-                float ndA = dot(localNormal, nA), ndB = dot(localNormal, nB);
-                bool back = (ndA < kConvexEps) && (ndB < kConvexEps);
-                if (back) {
-                    numConcave++;
-                } else {
-                    V3 ln = cp.normal;
-                    V3 clamped;
-                    if (clampNormal(edge, triNormal * swapFactor, ln, info.a20, clamped)) {
-                        if (dot(clamped, triNormal * frontFacing) > 0) {
-                            cp.normal = clamped;
-                            cp.posB = cp.posA - cp.normal * cp.dist;
-                            cp.localB = cp.posB;
-                        }
-                    }
-                }
-            }
-        }
-    }
-    if (isNearEdge && numConcave > 0) {
+    if (concave) {
         V3 newNormal = triNormal * frontFacing;
         float d = dot(newNormal, localNormal);
         if (d < 0) return;

@@ -177,48 +177,31 @@ struct VoronoiSimplex {
         }
         if (!oABC && !oACD && !oADB && !oBDC) return false;
         float best = 3.402823466e+38f;
-        if (oABC) {
-            closestPtTri(p, a, b, c, t);
+        // the faces ABC, ACD, ADB, BDC in turn, by selection: one copy of the code
+#pragma unroll 1
+        for (int f = 0; f < 4; f++) {
+            if (!(f == 0 ? oABC : (f == 1 ? oACD : (f == 2 ? oADB : oBDC)))) continue;
+            const V3 x = f == 3 ? b : a, y = f == 0 ? b : (f == 1 ? c : d), z = f == 0 ? c : (f == 1 ? d : (f == 2 ? b : c));
+            closestPtTri(p, x, y, z, t);
             V3 q = t.closest;
             float sq = dot(q - p, q - p);
             if (sq < best) {
                 best = sq;
                 fin.closest = q;
-                fin.used = t.used & 7;
-                fin.setBC(t.bc[0], t.bc[1], t.bc[2], 0);
-            }
-        }
-        if (oACD) {
-            closestPtTri(p, a, c, d, t);
-            V3 q = t.closest;
-            float sq = dot(q - p, q - p);
-            if (sq < best) {
-                best = sq;
-                fin.closest = q;
-                fin.used = (t.used & 1) | ((t.used & 2) ? 4u : 0u) | ((t.used & 4) ? 8u : 0u);
-                fin.setBC(t.bc[0], 0, t.bc[1], t.bc[2]);
-            }
-        }
-        if (oADB) {
-            closestPtTri(p, a, d, b, t);
-            V3 q = t.closest;
-            float sq = dot(q - p, q - p);
-            if (sq < best) {
-                best = sq;
-                fin.closest = q;
-                fin.used = (t.used & 1) | ((t.used & 4) ? 2u : 0u) | ((t.used & 2) ? 8u : 0u);
-                fin.setBC(t.bc[0], t.bc[2], 0, t.bc[1]);
-            }
-        }
-        if (oBDC) {
-            closestPtTri(p, b, d, c, t);
-            V3 q = t.closest;
-            float sq = dot(q - p, q - p);
-            if (sq < best) {
-                best = sq;
-                fin.closest = q;
-                fin.used = ((t.used & 1) ? 2u : 0u) | ((t.used & 4) ? 4u : 0u) | ((t.used & 2) ? 8u : 0u);
-                fin.setBC(0, t.bc[0], t.bc[2], t.bc[1]);
+                const uint32_t u0 = t.used & 1u, u1 = (t.used >> 1) & 1u, u2 = (t.used >> 2) & 1u;
+                if (f == 0) {
+                    fin.used = t.used & 7;
+                    fin.setBC(t.bc[0], t.bc[1], t.bc[2], 0);
+                } else if (f == 1) {
+                    fin.used = u0 | (u1 << 2) | (u2 << 3);
+                    fin.setBC(t.bc[0], 0, t.bc[1], t.bc[2]);
+                } else if (f == 2) {
+                    fin.used = u0 | (u2 << 1) | (u1 << 3);
+                    fin.setBC(t.bc[0], t.bc[2], 0, t.bc[1]);
+                } else {
+                    fin.used = (u0 << 1) | (u2 << 2) | (u1 << 3);
+                    fin.setBC(0, t.bc[0], t.bc[2], t.bc[1]);
+                }
             }
         }
         return true;

@@ -188,8 +188,9 @@ RSB_HD void sbVelNoDelta(const SBody& s, V3 relPos, V3& v) {
     else v = v3zero();
 }
 
-// convertContactInner (without rolling friction: every combined rolling friction is 0)
-RSB_HD bool addFrictionFor(Solver& S, int contactRow, int sA, int sB, const Body* b0, const Body* b1,
+// The friction row of convertContactInner (without rolling friction: every combined rolling
+// friction is 0) for contact row `contactRow`.
+RSB_HD void frictionRowFor(SRow& fr, Solver& S, int contactRow, int sA, int sB, const Body* b0, const Body* b1,
                            V3 normal, float fric, V3 relPos1, V3 relPos2) {
     V3 vel1, vel2;
     sbVelNoDelta(S.sb[sA], relPos1, vel1);
@@ -204,12 +205,8 @@ RSB_HD bool addFrictionFor(Solver& S, int contactRow, int sA, int sB, const Body
         V3 lat2;
         planeSpace1(normal, lat1, lat2);
     }
-    if (S.nf >= MAX_FRICTION_ROWS) return false;
-    SRow& fr = S.f[S.nf];
     fr.fIdx = (int16_t)contactRow;
     setupFrictionRow(fr, S, sA, sB, b0, b1, lat1, fric, relPos1, relPos2);
-    S.nf++;
-    return true;
 }
 
 RSB_HD void applyImpulseDelta(SBody& s, V3 lin, V3 ang, float imp) {
@@ -289,23 +286,20 @@ RSB_HD void solverIterate(Solver& S) {
     }
 }
 
-// writeBackBodies with split-impulse position correction
-RSB_HD void solverWriteBack(Solver& S, Body* bodies, const int* noRot, float dt) {
-    for (int i = 0; i < S.nsb; i++) {
-        SBody& s = S.sb[i];
-        if (s.body < 0) continue;
-        Body& b = bodies[s.body];
-        s.lin = s.lin + s.dLin;
-        s.ang = s.ang + s.dAng;
-        if (s.push.x != 0.f || s.push.y != 0 || s.push.z != 0 || s.turn.x != 0.f || s.turn.y != 0 || s.turn.z != 0) {
-            if (noRot[s.body]) s.xf = integrateTransformNoRot(s.xf, s.push, dt);
-            else s.xf = integrateTransform(s.xf, s.push, s.turn * kSplitTurnErp, dt);
-        }
-        b.lin = s.lin + s.extF;
-        b.ang = s.ang + s.extT;
-        b.xf = s.xf;
-        b.solverId = -1;
+// writeBackBodies with split-impulse position correction, for one solver body
+RSB_HD void solverWriteBack(SBody& s, Body* bodies, const int* noRot, float dt) {
+    if (s.body < 0) return;
+    Body& b = bodies[s.body];
+    s.lin = s.lin + s.dLin;
+    s.ang = s.ang + s.dAng;
+    if (s.push.x != 0.f || s.push.y != 0 || s.push.z != 0 || s.turn.x != 0.f || s.turn.y != 0 || s.turn.z != 0) {
+        if (noRot[s.body]) s.xf = integrateTransformNoRot(s.xf, s.push, dt);
+        else s.xf = integrateTransform(s.xf, s.push, s.turn * kSplitTurnErp, dt);
     }
+    b.lin = s.lin + s.extF;
+    b.ang = s.ang + s.extT;
+    b.xf = s.xf;
+    b.solverId = -1;
 }
 
 }  // namespace rsb

@@ -1730,33 +1730,18 @@ RSB_HD void loadContactCar(const EngineView& D, int a, int s, CarSim& c, V3 velC
     c.velCache = velCache;
 }
 
-// Callbacks, islands and solver of one arena.
-RSB_HD void solvePhase(const EngineView& D, const StepTemp& T, int a, PhaseStats& st) {
+// One arena's solver as its lanes share it.
+struct SolveShared {
     SolveWorld W;
-    W.S = &D.S;
-    W.P = &D.P;
-    W.nb = arenaBodies(D, a);
-    W.status = 0;
-    W.nRows = 0;
-    W.tick = arenaTickCount(D, a);
-    W.ballVelCache = v3zero();
-    W.np = W.nm = 0;
-    uint32_t actBits[MAX_BODIES], cached = 0, dynDone = 0;
-    for (int i = 0; i < W.nb; i++) {
-        Body& b = W.b[i];
-        bodyConstants(D, i, b);
-        const uint32_t p = infoWord(D, T, a, i, BI_PAIRS);
-        actBits[i] = p;
-        b.act = (int32_t)((p & BI_ACT_MASK) >> BI_ACT_SHIFT);
-        b.noResp = i > 0 && !(p & BI_RESPONDS) ? 1 : 0;
-        b.xf = bodyXf(D, a, i);
-        b.lin = bodyV3(D, a, i, RSB_PW(CarP, lin));
-        b.ang = bodyV3(D, a, i, RSB_PW(CarP, ang));
-        b.force = tempV3(D, T.force, a, i, 0);
-        b.torque = tempV3(D, T.force, a, i, 3);
-        updateInertia(b);
-        W.noRot[i] = i == 0 ? 1 : 0;
-    }
+    IslandWork I;
+    uint32_t actBits[MAX_BODIES], cached;
+};
+
+// Pairs, manifolds and contact callbacks of one arena, in dispatch order.
+RSB_HD void solveCallbacks(const EngineView& D, const StepTemp& T, int a, SolveShared& sh) {
+    SolveWorld& W = sh.W;
+    const uint32_t* actBits = sh.actBits;
+    uint32_t cached = 0, dynDone = 0;
     int blocks = 0;
     auto addPairTo = [&](int lo, int hi) -> bool {
         if (W.np >= MAX_PAIRS) {
@@ -1864,18 +1849,60 @@ RSB_HD void solvePhase(const EngineView& D, const StepTemp& T, int a, PhaseStats
             }
         }
     }
-    solveIslands(W);
-    for (int i = 0; i < W.nb; i++) {
+    sh.cached = cached;
+}
+
+// Callbacks, islands and solver of one arena.
+template <class LanesT>
+RSB_HD void solvePhase(const EngineView& D, const StepTemp& T, int a, SolveShared& sh, const LanesT& L, PhaseStats& st) {
+    SolveWorld& W = sh.W;
+    if (L.lane == 0) {
+        W.S = &D.S;
+        W.P = &D.P;
+        W.nb = arenaBodies(D, a);
+        W.status = 0;
+        W.nRows = 0;
+        W.tick = arenaTickCount(D, a);
+        W.ballVelCache = v3zero();
+        W.np = W.nm = 0;
+    }
+    const int nb = arenaBodies(D, a);
+    for (int i = L.lane; i < nb; i += L.count) {
+        Body& b = W.b[i];
+        bodyConstants(D, i, b);
+        const uint32_t p = infoWord(D, T, a, i, BI_PAIRS);
+        sh.actBits[i] = p;
+        b.act = (int32_t)((p & BI_ACT_MASK) >> BI_ACT_SHIFT);
+        b.noResp = i > 0 && !(p & BI_RESPONDS) ? 1 : 0;
+        b.xf = bodyXf(D, a, i);
+        b.lin = bodyV3(D, a, i, RSB_PW(CarP, lin));
+        b.ang = bodyV3(D, a, i, RSB_PW(CarP, ang));
+        b.force = tempV3(D, T.force, a, i, 0);
+        b.torque = tempV3(D, T.force, a, i, 3);
+        updateInertia(b);
+        W.noRot[i] = i == 0 ? 1 : 0;
+    }
+    L.sync();
+    if (L.lane == 0) {
+        solveCallbacks(D, T, a, sh);
+        islandLists(W, sh.I);
+    }
+    L.sync();
+    solveLists(W, sh.I, L);
+    for (int i = L.lane; i < nb; i += L.count) {
         const Body& b = W.b[i];
         putBodyXf(D, a, i, b.xf);
         putBodyV3(D, a, i, RSB_PW(CarP, lin), b.lin);
         putBodyV3(D, a, i, RSB_PW(CarP, ang), b.ang);
-        infoWord(D, T, a, i, BI_PAIRS) = (actBits[i] & ~BI_ACT_MASK) | ((uint32_t)b.act << BI_ACT_SHIFT) | BI_SOLVED |
-                                         ((cached >> i) & 1u ? BI_CACHE : 0u);
+        infoWord(D, T, a, i, BI_PAIRS) = (sh.actBits[i] & ~BI_ACT_MASK) | ((uint32_t)b.act << BI_ACT_SHIFT) | BI_SOLVED |
+                                         ((sh.cached >> i) & 1u ? BI_CACHE : 0u);
     }
-    if (cached & 1u) putTempV3(D, T.cache, a, 0, 0, W.ballVelCache);
-    st.nRows += W.nRows;
-    if (W.status) phaseAtomicOr(arenaStatus(D, a), W.status);
+    if (L.lane == 0) {
+        if (sh.cached & 1u) putTempV3(D, T.cache, a, 0, 0, W.ballVelCache);
+        st.nRows += W.nRows;
+        if (W.status) phaseAtomicOr(arenaStatus(D, a), W.status);
+    }
+    L.sync();
 }
 
 // ------------------------------------------------------------------ finish

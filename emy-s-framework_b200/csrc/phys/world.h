@@ -1066,10 +1066,18 @@ RSB_HD void quickSortKV(int* key, int* val, int lo, int hi, uint32_t& status) {
     }
 }
 
-// btSimulationIslandManager + InplaceSolverIslandCallback + btSequentialImpulseConstraintSolver
+// What one batched solveGroup takes: bodies and manifolds in island order, then the solver.
+struct IslandWork {
+    int bodyList[MAX_BODIES], nbl;
+    int manList[MAX_MANIFOLDS], nml;
+    int8_t rowMan[MAX_CONTACT_ROWS], rowPt[MAX_CONTACT_ROWS];  // manifold and point of each contact row
+    float spLen[MAX_CONTACT_ROWS][2];                          // arm lengths of a special contact's sides
+    Solver Sv;
+};
+
+// btSimulationIslandManager: the islands' bodies and manifolds in solving order
 template <class WT>
-RSB_HD void solveIslands(WT& W) {
-    const float dt = W.P->dt;
+RSB_HD void islandLists(WT& W, IslandWork& I) {
     UnionFind uf;
     uf.reset(W.nb);
     for (int i = 0; i < W.nb; i++) W.b[i].islandTag = i;
@@ -1132,8 +1140,9 @@ RSB_HD void solveIslands(WT& W) {
     if (nim > 1) quickSortKV(mkey, midx, 0, nim - 1, W.status);
 
     // processIslands -> one batched solveGroup
-    int bodyList[MAX_BODIES], nbl = 0;
-    int manList[MAX_MANIFOLDS], nml = 0;
+    int* bodyList = I.bodyList;
+    int* manList = I.manList;
+    int nbl = 0, nml = 0;
     int sm = 0;
     for (int s = 0; s < W.nb;) {
         int island = eid[s];
@@ -1159,76 +1168,115 @@ RSB_HD void solveIslands(WT& W) {
         s = e;
     }
 
-    // ---- solveGroup
-    Solver Sv;
-    Sv.nsb = 0;
-    Sv.fixedId = -1;
-    Sv.nc = 0;
-    Sv.nf = 0;
-    for (int i = 0; i < W.nb; i++) W.b[i].solverId = -1;
-    for (int k = 0; k < nbl; k++) solverBodyOf(Sv, W.b, OBJ_BALL + bodyList[k], dt);
-    for (int k = 0; k < nml; k++) {
-        Manifold& m = W.m[manList[k]];
-        int sA = solverBodyOf(Sv, W.b, m.o0, dt);
-        int sB = solverBodyOf(Sv, W.b, m.o1, dt);
+    I.nbl = nbl;
+    I.nml = nml;
+}
+
+// The lanes that share one arena's solver: all of a warp, or (host) one.
+struct OneLane {
+    int lane = 0, count = 1;
+    RSB_HD void sync() const {}
+};
+
+// btSequentialImpulseConstraintSolver over the lists: rows are set up a lane each (they read the
+// solver bodies and write themselves), what runs in order runs on lane 0.
+template <class WT, class LanesT>
+RSB_HD void solveLists(WT& W, IslandWork& I, const LanesT& L) {
+    const float dt = W.P->dt;
+    Solver& Sv = I.Sv;
+    if (L.lane == 0) {
+        Sv.nsb = 0;
+        Sv.fixedId = -1;
+        Sv.nc = 0;
+        for (int i = 0; i < W.nb; i++) W.b[i].solverId = -1;
+        for (int k = 0; k < I.nbl; k++) solverBodyOf(Sv, W.b, OBJ_BALL + I.bodyList[k], dt);
+        for (int k = 0; k < I.nml; k++) {
+            const Manifold& m = W.m[I.manList[k]];
+            solverBodyOf(Sv, W.b, m.o0, dt);
+            solverBodyOf(Sv, W.b, m.o1, dt);
+            for (int j = 0; j < m.n; j++) {
+                if (Sv.nc >= MAX_CONTACT_ROWS) { W.status |= 2u; break; }
+                I.rowMan[Sv.nc] = (int8_t)I.manList[k];
+                I.rowPt[Sv.nc] = (int8_t)j;
+                Sv.nc++;
+            }
+        }
+        Sv.nf = Sv.nc;
+    }
+    L.sync();
+    auto solverId = [&](int o) { return objIsStatic(o) ? Sv.fixedId : W.b[o - OBJ_BALL].solverId; };
+    for (int row = L.lane; row < Sv.nc; row += L.count) {
+        const Manifold& m = W.m[I.rowMan[row]];
+        const MPoint& cp = m.pt[I.rowPt[row]];
+        const int sA = solverId(m.o0), sB = solverId(m.o1);
         const Body* rb0 = objIsStatic(m.o0) ? nullptr : &W.b[m.o0 - OBJ_BALL];
         const Body* rb1 = objIsStatic(m.o1) ? nullptr : &W.b[m.o1 - OBJ_BALL];
-        if (!rb0 && !rb1) continue;
         ObjRef r0 = objRef(W, m.o0), r1 = objRef(W, m.o1);
-        for (int j = 0; j < m.n; j++) {
-            MPoint& cp = m.pt[j];
-            if (Sv.nc >= MAX_CONTACT_ROWS) { W.status |= 2u; break; }
-            int row = Sv.nc++;
-            SRow& r = Sv.c[row];
-            V3 rel1 = cp.posA - r0.xf.o;
-            V3 rel2 = cp.posB - r1.xf.o;
-            setupContactRow(r, Sv, sA, sB, rb0, rb1, cp.normal, cp.dist, cp.fric, cp.rest, rel1, rel2, dt, cp.special);
-            r.fIdx = (int16_t)Sv.nf;
-            if (cp.special) {
-                for (int side = 0; side < 2; side++) {
-                    int o = side ? m.o1 : m.o0;
-                    if (objIsStatic(o)) continue;
-                    Body& sb = W.b[o - OBJ_BALL];
-                    sb.spCount++;
-                    sb.spFric = cp.fric;
-                    sb.spRest = cp.rest;
-                    sb.spNormal = sb.spNormal + cp.normal;
-                    sb.spDist = sb.spDist + length(side ? rel2 : rel1);
-                }
+        V3 rel1 = cp.posA - r0.xf.o;
+        V3 rel2 = cp.posB - r1.xf.o;
+        SRow& r = Sv.c[row];
+        setupContactRow(r, Sv, sA, sB, rb0, rb1, cp.normal, cp.dist, cp.fric, cp.rest, rel1, rel2, dt, cp.special);
+        r.fIdx = (int16_t)row;
+        if (cp.special) {
+            I.spLen[row][0] = length(rel1);
+            I.spLen[row][1] = length(rel2);
+        }
+        frictionRowFor(Sv.f[row], Sv, row, sA, sB, rb0, rb1, cp.normal, cp.fric, rel1, rel2);
+    }
+    L.sync();
+    if (L.lane == 0) {
+        for (int row = 0; row < Sv.nc; row++) {
+            if (!Sv.c[row].special) continue;
+            const Manifold& m = W.m[I.rowMan[row]];
+            const MPoint& cp = m.pt[I.rowPt[row]];
+            for (int side = 0; side < 2; side++) {
+                int o = side ? m.o1 : m.o0;
+                if (objIsStatic(o)) continue;
+                Body& sb = W.b[o - OBJ_BALL];
+                sb.spCount++;
+                sb.spFric = cp.fric;
+                sb.spRest = cp.rest;
+                sb.spNormal = sb.spNormal + cp.normal;
+                sb.spDist = sb.spDist + I.spLen[row][side];
             }
-            if (!addFrictionFor(Sv, row, sA, sB, rb0, rb1, cp.normal, cp.fric, rel1, rel2)) { W.status |= 2u; break; }
         }
+        // convertContactSpecial, per body in island order
+        for (int k = 0; k < I.nbl; k++) {
+            Body& b = W.b[I.bodyList[k]];
+            if (b.spCount <= 0) continue;
+            float distance = b.spDist / (float)b.spCount;
+            V3 normal = bdiv(b.spNormal, (float)b.spCount);
+            int sA = solverBodyOf(Sv, W.b, OBJ_BALL + I.bodyList[k], dt);
+            int sB = solverBodyOf(Sv, W.b, 0, dt);
+            if (Sv.nc < MAX_CONTACT_ROWS) {
+                int row = Sv.nc++;
+                Sv.nf = Sv.nc;
+                V3 rel1 = normal * -distance;
+                V3 rel2 = v3zero();
+                SRow& r = Sv.c[row];
+                setupContactRow(r, Sv, sA, sB, &b, nullptr, normal, distance, b.spFric, b.spRest, rel1, rel2, dt, 0);
+                r.fIdx = (int16_t)row;
+                frictionRowFor(Sv.f[row], Sv, row, sA, sB, &b, nullptr, normal, b.spFric, rel1, rel2);
+            } else {
+                W.status |= 2u;
+            }
+            b.spCount = 0;
+            b.spFric = b.spRest = b.spDist = 0.f;
+            b.spNormal = v3zero();
+        }
+        W.nRows += (uint32_t)(Sv.nc + Sv.nf);
+        solverIterate(Sv);
     }
-    // convertContactSpecial, per body in island order
-    for (int k = 0; k < nbl; k++) {
-        Body& b = W.b[bodyList[k]];
-        if (b.spCount <= 0) continue;
-        float distance = b.spDist / (float)b.spCount;
-        V3 normal = bdiv(b.spNormal, (float)b.spCount);
-        int sA = solverBodyOf(Sv, W.b, OBJ_BALL + bodyList[k], dt);
-        if (Sv.fixedId < 0) {
-            Sv.fixedId = Sv.nsb++;
-            sbInitFixed(Sv.sb[Sv.fixedId]);
-        }
-        int sB = Sv.fixedId;
-        if (Sv.nc < MAX_CONTACT_ROWS) {
-            int row = Sv.nc++;
-            SRow& r = Sv.c[row];
-            V3 rel1 = normal * -distance;
-            V3 rel2 = v3zero();
-            setupContactRow(r, Sv, sA, sB, &b, nullptr, normal, distance, b.spFric, b.spRest, rel1, rel2, dt, 0);
-            r.fIdx = (int16_t)Sv.nf;
-            if (!addFrictionFor(Sv, row, sA, sB, &b, nullptr, normal, b.spFric, rel1, rel2)) W.status |= 2u;
-        } else {
-            W.status |= 2u;
-        }
-        b.spCount = 0;
-        b.spFric = b.spRest = b.spDist = 0.f;
-        b.spNormal = v3zero();
-    }
-    W.nRows += (uint32_t)(Sv.nc + Sv.nf);
-    solverIterate(Sv);
-    solverWriteBack(Sv, W.b, W.noRot, dt);
+    L.sync();
+    for (int i = L.lane; i < Sv.nsb; i += L.count) solverWriteBack(Sv.sb[i], W.b, W.noRot, dt);
+    L.sync();
+}
+
+template <class WT>
+RSB_HD void solveIslands(WT& W) {
+    IslandWork I;
+    islandLists(W, I);
+    solveLists(W, I, OneLane{});
 }
 
 // ------------------------------------------------------------------ integration

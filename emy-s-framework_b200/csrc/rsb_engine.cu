@@ -194,17 +194,17 @@ static rsb_status cudaFail(rsb_handle* h, const char* what, cudaError_t e) {
 // size.
 typedef void (*StepFn)(EngineView, StepTemp);
 struct StepVariant {
-    StepFn ray, triangle, solve;
+    StepFn ray, triangle;
     int minBlocks;
     bool persistent;
 };
 static const StepVariant kStepVariants[] = {
-    {bodyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, false},
-    {bodyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, false},
-    {bodyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, false},
-    {bodyRayKernel<1>, triangleKernel<1>, solveKernel<1>, 1, true},
-    {bodyRayKernel<3>, triangleKernel<3>, solveKernel<3>, 3, true},
-    {bodyRayKernel<4>, triangleKernel<4>, solveKernel<4>, 4, true}};
+    {bodyRayKernel<1>, triangleKernel<1>, 1, false},
+    {bodyRayKernel<3>, triangleKernel<3>, 3, false},
+    {bodyRayKernel<4>, triangleKernel<4>, 4, false},
+    {bodyRayKernel<1>, triangleKernel<1>, 1, true},
+    {bodyRayKernel<3>, triangleKernel<3>, 3, true},
+    {bodyRayKernel<4>, triangleKernel<4>, 4, true}};
 constexpr int kNumStepVariants = sizeof(kStepVariants) / sizeof(kStepVariants[0]);
 static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
@@ -659,10 +659,10 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
         // make the per-thread stack limit cover the largest (the default limit is 1 KB), and give
         // the L1 its largest share in those that use no shared memory to speak of
         size_t need = 0;
-        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)meshRayKernel,
+        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)meshRayKernel, (const void*)solveBodyKernel,
                                      (const void*)combineKernel};
         for (const StepVariant& v : kStepVariants)
-            for (StepFn f : {v.ray, v.triangle, v.solve}) fns.push_back((const void*)f);
+            for (StepFn f : {v.ray, v.triangle}) fns.push_back((const void*)f);
         for (const void* f : fns) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, f) != cudaSuccess)
@@ -773,7 +773,8 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     const int pairGrid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)h->numCars + h->N) / 16, 16 * (int64_t)h->smCount));
     const int triGrid = grid(sv.triangle, (int64_t)h->numCars + h->N, kTriangleWarps + kPairWarps);
     const int deepGrid = (int)std::min<int64_t>(h->numCars + h->N, 16 * (int64_t)h->smCount), combineGrid = grid(combineKernel, 2 * ((int64_t)h->numCars + h->N), kCombineWarps);
-    const int solveGrid = grid(sv.solve, 2 * (int64_t)h->N, kWholeWarps + kBodyWarps);
+    const int solveGrid = (int)std::min<int64_t>(h->N, 9 * (int64_t)h->smCount);  // as many as fit at once
+    const int solveBodyGrid = (int)std::max<int64_t>(1, std::min<int64_t>((h->numCars + h->N + 1) / 2, 16 * (int64_t)h->smCount));
     const int carThreads = PHASE_ARENAS * h->maxCars, bodyThreads = PHASE_ARENAS * (1 + h->maxCars);
     for (int t = 0; t < ticks; t++) {
         if (h->maxCars > 0) {
@@ -787,7 +788,8 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
         sv.triangle<<<triGrid, block, 0, st>>>(D, T);
         deepKernel<<<deepGrid, 32, 0, st>>>(D, T);
         combineKernel<<<combineGrid, block, 0, st>>>(D, T);
-        sv.solve<<<solveGrid, block, 0, st>>>(D, T);
+        solveKernel<<<solveGrid, 32, 0, st>>>(D, T);
+        solveBodyKernel<<<solveBodyGrid, SOLVEBODY_THREADS, 0, st>>>(D, T);
         finishKernel<<<groups, bodyThreads, 0, st>>>(D, T);
     }
     return cudaGetLastError();

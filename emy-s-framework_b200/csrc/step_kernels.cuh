@@ -49,7 +49,7 @@ RSB_D uint32_t queueAlloc(uint32_t* counter, uint32_t n) {
 // 61 / 74); find 202 with 32 items to every warp and 107 with 64, deep 214 and 141, combine 113 and 102, whole-arena
 // islands 234 and 886 (64).
 constexpr int kMeshRayWarps = 32, kBodyRayWarps = 16, kTriangleWarps = 12, kPairWarps = 12, kCombineWarps = 16,
-              kWholeWarps = 16, kBodyWarps = 8;
+              kBodyWarps = 8;
 
 // Items of several queues, fn(queue, item): a warp takes items of one queue at a time, as few as
 // it takes to give each of spread[queue] warps some.
@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(CAR_THREADS) rayKernel(const __grid_constant__
         for (int b = 0; b < nb; b++) n |= cellsNear(at, cell[b][lane]) ? 1u << b : 0u;
         return n;
     };
+#pragma unroll 1
     for (int w = 0; w < 4; w++) {
         const RayClass c = live ? rayPhase(D, T, a, s, w, xf, culled, near, st) : RAY_DONE;
         const uint32_t m = queueAlloc(&T.count[QC_RAY], c == RAY_MESHES ? 1u : 0u);
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(128, MINB) triangleKernel(const __grid_constan
 // in shared memory.  The items are few (about one in forty arenas) and each is a serial chain
 // through that memory; as thread-local memory every word of it took a sector of its own, since
 // one lane was active, and a tick waited 140 us for the longest item at 3v3 x 65,536.
-__global__ void __launch_bounds__(32) deepKernel(const __grid_constant__ EngineView D,
+__global__ void __launch_bounds__(32, 1) deepKernel(const __grid_constant__ EngineView D,
                                                  const __grid_constant__ StepTemp T) {
     __shared__ EpaWork epa;
     PhaseStats st{0, 0, 0, 0};
@@ -332,16 +333,29 @@ __global__ void __launch_bounds__(128) combineKernel(const __grid_constant__ Eng
     blockStats(D, st);
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) solveKernel(const __grid_constant__ EngineView D,
-                                                         const __grid_constant__ StepTemp T) {
-    const uint32_t n[2] = {T.count[QC_SOLVE], T.count[QC_BODY]};
+struct WarpLanes {
+    int lane = (int)(threadIdx.x & 31), count = 32;
+    RSB_D void sync() const { __syncwarp(); }
+};
+
+// Arenas with pairs of bodies, one to a warp with its solver in shared memory: bodies are loaded
+// and rows set up a lane each, the iterations run on one.  These arenas are few (one in fifty),
+// and a tick waits for the one with the most rows.
+__global__ void __launch_bounds__(32, 1) solveKernel(const __grid_constant__ EngineView D,
+                                                     const __grid_constant__ StepTemp T) {
+    __shared__ SolveShared sh;
+    const uint32_t n = T.count[QC_SOLVE];
     PhaseStats st{0, 0, 0, 0};
-    const uint32_t w[2] = {kWholeWarps * T.sms, kBodyWarps * T.sms};
-    forItems(n, w, [&](int k, uint32_t i) {
-        if (k == 0) solvePhase(D, T, (int)T.solveQ[i], st);
-        else bodyPhase(D, T, T.bodyQ[i], st);
-    });
+    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) solvePhase(D, T, (int)T.solveQ[i], sh, WarpLanes{}, st);
+    blockStats(D, st);
+}
+
+constexpr int SOLVEBODY_THREADS = 64;
+__global__ void __launch_bounds__(SOLVEBODY_THREADS) solveBodyKernel(const __grid_constant__ EngineView D,
+                                                                     const __grid_constant__ StepTemp T) {
+    const uint32_t n[1] = {T.count[QC_BODY]}, w[1] = {kBodyWarps * T.sms};
+    PhaseStats st{0, 0, 0, 0};
+    forItems(n, w, [&](int, uint32_t i) { bodyPhase(D, T, T.bodyQ[i], st); });
     blockStats(D, st);
 }
 

@@ -69,6 +69,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     std::unique_ptr<EpaWork> epa(new EpaWork());
     std::unique_ptr<DriveShared> ds(new DriveShared());
     std::unique_ptr<PairShared> sh(new PairShared());
+    std::unique_ptr<SolveShared> ss(new SolveShared());
     std::unique_ptr<FinishShared> fs(new FinishShared());
     std::vector<DriveThread> dt(MAX_CARS * PHASE_ARENAS);
     std::vector<PairThread> bt(MAX_BODIES * PHASE_ARENAS);
@@ -175,7 +176,7 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
         for (uint32_t i = T.count[QC_PLANE]; i-- > 0;) planePhase(D, T, (uint32_t)resultBase(QC_PLANE) * (uint32_t)D.N + i, st);
         for (uint32_t i = T.count[QC_DEEP]; i-- > 0;) deepPhase(D, T, T.deepQ[i], epa.get(), st);
         for (uint32_t i = T.count[QC_COMBINE]; i-- > 0;) combinePhase(D, T, T.combineQ[i], st);
-        for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], st);
+        for (uint32_t i = T.count[QC_SOLVE]; i-- > 0;) solvePhase(D, T, (int)T.solveQ[i], *ss, OneLane{}, st);
         for (uint32_t i = T.count[QC_BODY]; i-- > 0;) bodyPhase(D, T, T.bodyQ[i], st);
         // finish
         for (int g = 0; g < h->N; g += PHASE_ARENAS) {
