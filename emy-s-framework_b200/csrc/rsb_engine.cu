@@ -135,6 +135,7 @@ struct rsb_handle {
     std::shared_ptr<ArenaStaticHost> host;
     // launch configuration of the step's queue kernels (indices into kStepVariants / kStepBlocks)
     int stepVariant = 0, stepBlock = 1, stepResidency = 0;
+    bool stepPinned = false;        // set by rsb_set_step_config or rsb_autotune
     uint32_t* dScratch = nullptr;   // the autotuner's copy of the arena records
     unsigned int* dWork = nullptr;  // queue counters of the step phases (zero between ticks)
     StepTemp step{};                // what the phases of a tick hand on (one allocation, dStep)
@@ -210,6 +211,13 @@ static const int kStepBlocks[] = {32, 64, 128};
 constexpr int kNumStepBlocks = sizeof(kStepBlocks) / sizeof(kStepBlocks[0]);
 // Resident warps per SM of a persistent launch (0 = as many as fit).
 static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
+// Blocks of the one-kernel step: about this many share a batch, so that several small batches run
+// side by side (a block takes a multiprocessor).  us per env step of 2v2 x 250, three batches in
+// turn / one alone: 575 / 1651 with 32 blocks, 568 / 1455 with 63, 764 / 1211 with 125, 1236 /
+// 1892 with 250; a kernel per phase 742 / 1955.  3v3 x 1,023, 4 ticks: 496 / 1365
+// with 64 blocks, 783 / 1147 with 128, 551 / 1387 with a kernel per phase, which is the faster one
+// once 64 blocks of 32 arenas are full.
+constexpr int kStepBlockGrid = 64;
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
 
 // Fills the triangles' query data (TriData) on the device.
@@ -670,6 +678,9 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
             need = std::max(need, ((fa.localSizeBytes + 4096) + 1023) / 1024 * 1024);
             cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
         }
+        if (cudaFuncSetAttribute(stepBlockKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockShared)) !=
+            cudaSuccess)
+            return fail(nullptr, RSB_ERR_CUDA, "shared memory of the step kernel");
         size_t cur = 0;
         cudaDeviceGetLimit(&cur, cudaLimitStackSize);
         if (cur < need && cudaDeviceSetLimit(cudaLimitStackSize, need) != cudaSuccess)
@@ -747,11 +758,18 @@ rsb_status rsb_obs_stride(const rsb_handle* h, int32_t* stride) {
     return RSB_OK;
 }
 
-// Launches `ticks` ticks on stream st, the queue kernels as variant v with block size index b.
+// Launches `ticks` ticks on stream st: the kernels of each phase, the queue kernels as variant v
+// with block size index b, or (v = -1) one kernel for all.
 static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, int ticks, cudaStream_t st,
                               int residency = 0) {
-    const StepVariant& sv = kStepVariants[v];
     const StepTemp& T = h->step;
+    if (v < 0) {
+        const int perBlock = (h->N + kStepBlockGrid - 1) / kStepBlockGrid;
+        stepBlockKernel<<<(h->N + perBlock - 1) / perBlock, BLOCK_THREADS, sizeof(BlockShared), st>>>(D, T, ticks, perBlock,
+                                                                                                     h->maxCars);
+        return cudaGetLastError();
+    }
+    const StepVariant& sv = kStepVariants[v];
     const int block = kStepBlocks[b], groups = (h->N + PHASE_ARENAS - 1) / PHASE_ARENAS;
     // A queue kernel's items are counted on the device only; `items` is about how many there may
     // be.  The wide grid has a warp for every 32 of them, or for each up to the kernel's spread;
@@ -795,6 +813,12 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
     return cudaGetLastError();
 }
 
+// The default launch: one kernel while its blocks hold the batch, a kernel per phase beyond; a
+// configuration that was set or tuned is taken as it is.
+static int stepVariantFor(const rsb_handle* h) {
+    return !h->stepPinned && h->N <= kStepBlockGrid * PHASE_ARENAS ? -1 : h->stepVariant;
+}
+
 rsb_status rsb_step(rsb_handle* h, int32_t ticks, void* stream) {
     if (!h || ticks < 0) return fail(h, RSB_ERR_INVALID, "bad tick count");
     if (ticks == 0) return RSB_OK;
@@ -812,7 +836,7 @@ rsb_status rsb_step(rsb_handle* h, int32_t ticks, void* stream) {
         RSB_CUDA(cudaGetLastError());
         D.cull = h->dCull;
     }
-    RSB_CUDA(launchStep(h, D, h->stepVariant, h->stepBlock, ticks, st, h->stepResidency));
+    RSB_CUDA(launchStep(h, D, stepVariantFor(h), h->stepBlock, ticks, st, h->stepResidency));
     h->stats.ticks_simulated += (uint64_t)h->N * ticks;
     return RSB_OK;
 }
@@ -870,8 +894,15 @@ rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32
     rsb_status st = RSB_OK;
     // every (variant, block) with all warp slots filled; the residency caps on the persistent
     // variant with the largest register budget, at 32 and 64 threads per block
+    // and, first and unreported, the default launch where it is none of them: it stays unless a
+    // candidate is faster
     struct Cand { int v, b, r; };
     std::vector<Cand> cands;
+    const bool pinned = h->stepPinned;
+    h->stepPinned = false;
+    const bool block = stepVariantFor(h) < 0;
+    h->stepPinned = pinned;
+    if (block) cands.push_back({-1, 0, 0});
     for (int v = 0; v < kNumStepVariants; v++)
         for (int b = 0; b < kNumStepBlocks; b++) cands.push_back({v, b, 0});
     for (int v = 0; v < kNumStepVariants; v++)
@@ -903,6 +934,11 @@ rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32
                 ms = std::min(ms, t);
             }
             if (st != RSB_OK) break;
+            if (v < 0) {
+                best = ms;
+                bestV = v;
+                continue;
+            }
             if (out && n < cap)
                 out[n] = rsb_tune_entry{kStepVariants[v].minBlocks, kStepBlocks[b], ms,
                                         kStepVariants[v].persistent ? 1 : 0, kStepResidency[c.r]};
@@ -913,7 +949,8 @@ rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st != RSB_OK) return st;
-    h->stepVariant = bestV;
+    h->stepPinned = bestV >= 0;
+    h->stepVariant = std::max(0, bestV);
     h->stepBlock = bestB;
     h->stepResidency = bestR;
     if (count) *count = n;
@@ -934,6 +971,7 @@ rsb_status rsb_set_step_config(rsb_handle* h, const rsb_tune_entry* cfg) {
                 h->stepVariant = v;
                 h->stepBlock = b;
                 h->stepResidency = r;
+                h->stepPinned = true;
                 return RSB_OK;
             }
     return fail(h, RSB_ERR_INVALID, "rsb_set_step_config: no such launch configuration");

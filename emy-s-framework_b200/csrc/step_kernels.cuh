@@ -212,15 +212,13 @@ __global__ void __launch_bounds__(BODY_THREADS) pairKernel(const __grid_constant
 // those that overlap, eight at a time, so that the loads of a pair do not wait for one another as
 // those of a walk do.  The four pairs of a warp step together (their lanes meet in the ballots).
 constexpr int FIND_LANES = 8, FIND_GROUPS = 32 / FIND_LANES, FIND_HEADERS = 64;
-constexpr int FIND_THREADS = 128;
-__global__ void __launch_bounds__(FIND_THREADS) findKernel(const __grid_constant__ EngineView D,
-                                                           const __grid_constant__ StepTemp T) {
-    __shared__ int16_t list[FIND_THREADS / FIND_LANES][PAIR_CANDIDATES];
-    const uint32_t nCar = T.count[QC_CARMESH], total = nCar + T.count[QC_BALLMESH], nBall = T.count[QC_CARBALL];
-    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), warps = gridDim.x * (blockDim.x >> 5);
+// `list`: PAIR_CANDIDATES places for each of the warp's groups.  The pairs are nCar car pairs from
+// place car0 of their queue on, then those of the ball up to `total`, from ball0 on.
+RSB_D void findPairs(const EngineView& D, const StepTemp& T, int16_t (*list)[PAIR_CANDIDATES], uint32_t car0,
+                     uint32_t nCar, uint32_t ball0, uint32_t total, uint32_t warp, uint32_t warps) {
     const int lane = threadIdx.x & 31, g = lane / FIND_LANES, l = lane % FIND_LANES;
     const uint32_t groupBits = (1u << FIND_LANES) - 1u, all = 0xffffffffu;
-    int16_t* mine = list[threadIdx.x / FIND_LANES];
+    int16_t* mine = list[g];
     const ArenaStatic& S = D.S;
     for (uint32_t p0 = warp * FIND_GROUPS; p0 < total; p0 += warps * FIND_GROUPS) {
         const uint32_t p = p0 + g;
@@ -230,8 +228,8 @@ __global__ void __launch_bounds__(FIND_THREADS) findKernel(const __grid_constant
         FindBody f;
         uint16_t qmn[3], qmx[3];
         if (has) {
-            res = p < nCar ? (uint32_t)resultBase(QC_CARMESH) * (uint32_t)D.N + p
-                           : (uint32_t)resultBase(QC_BALLMESH) * (uint32_t)D.N + (p - nCar);
+            res = p < nCar ? (uint32_t)resultBase(QC_CARMESH) * (uint32_t)D.N + car0 + p
+                           : (uint32_t)resultBase(QC_BALLMESH) * (uint32_t)D.N + ball0 + (p - nCar);
             const PairTask k = T.tasks[res];
             mesh = k.o0;
             findBody(D, (int)k.a, k.o1 - OBJ_BALL, f);
@@ -291,6 +289,15 @@ __global__ void __launch_bounds__(FIND_THREADS) findKernel(const __grid_constant
         if (combine) T.combineQ[at] = res;
         __syncwarp();
     }
+}
+
+constexpr int FIND_THREADS = 128;
+__global__ void __launch_bounds__(FIND_THREADS) findKernel(const __grid_constant__ EngineView D,
+                                                           const __grid_constant__ StepTemp T) {
+    __shared__ int16_t list[FIND_THREADS / FIND_LANES][PAIR_CANDIDATES];
+    const uint32_t nCar = T.count[QC_CARMESH], total = nCar + T.count[QC_BALLMESH], nBall = T.count[QC_CARBALL];
+    const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    findPairs(D, T, list + warp * FIND_GROUPS, 0u, nCar, 0u, total, blockIdx.x * warps + warp, gridDim.x * warps);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nBall; i += gridDim.x * blockDim.x)
         findPhase(D, T, (uint32_t)resultBase(QC_CARBALL) * (uint32_t)D.N + i);
 }
@@ -386,6 +393,214 @@ __global__ void __launch_bounds__(BODY_THREADS) finishKernel(const __grid_consta
     if (!valid) return;
     if (t.body > 0) finishBoost(D, t, sh);
     else finishArena(D, t, sh);
+}
+
+// ------------------------------------------------------------------ small batches
+
+// All phases of all ticks in one launch, for batches that do not fill the GPU: a block owns up to
+// 32 arenas and runs the phases in turn with barriers between them, its queues in its arenas'
+// share of the batch's.  Arenas are independent, so nothing crosses blocks.  What a batch of this
+// size waits for otherwise is twelve launches a tick, each with a handful of items to it.
+constexpr int BLOCK_WARPS = 8, BLOCK_THREADS = 32 * BLOCK_WARPS;
+static_assert(MAX_BODIES * PHASE_ARENAS <= BLOCK_THREADS, "one thread per body");
+struct BlockShared {
+    union {
+        PairShared pair;
+        DriveShared drive;
+        FinishShared finish;
+        int16_t list[BLOCK_WARPS * FIND_GROUPS][PAIR_CANDIDATES];
+        EpaWork epa[BLOCK_WARPS];
+        SolveShared solve[BLOCK_WARPS];
+    };
+    RSB_D BlockShared() {}
+};
+
+__global__ void __launch_bounds__(BLOCK_THREADS, 1) stepBlockKernel(const __grid_constant__ EngineView D,
+                                                                    const __grid_constant__ StepTemp T0, int ticks,
+                                                                    int perBlock, int maxCars) {
+    extern __shared__ __align__(16) unsigned char blockSmem[];
+    BlockShared& sh = *reinterpret_cast<BlockShared*>(blockSmem);
+    __shared__ uint32_t count[QC_WORDS], base[QC_WORDS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int a0 = blockIdx.x * perBlock, n = min(perBlock, D.N - a0);
+    const size_t rays = rayPlaces(D);
+    // this block's share of every queue
+    StepTemp T = T0;
+    T.count = count;
+    T.candCap = (uint32_t)(CAP_CANDIDATES * (a0 + n));
+    T.blockCap = (uint32_t)(MAX_BLOCKS * (a0 + n));
+    if (tid == 0) {
+        base[QC_RAY] = base[QC_BODYRAY] = (uint32_t)(4 * MAX_CARS * a0);
+        base[QC_CARMESH] = (uint32_t)(CAP_CARMESH * a0);
+        base[QC_BALLMESH] = (uint32_t)(CAP_BALLMESH * a0);
+        base[QC_CARBALL] = (uint32_t)(CAP_CARBALL * a0);
+        base[QC_CARCAR] = (uint32_t)(CAP_CARCAR * a0);
+        base[QC_PLANE] = (uint32_t)(CAP_PLANE * a0);
+        base[QC_BLOCK] = (uint32_t)(MAX_BLOCKS * a0);
+        base[QC_SOLVE] = (uint32_t)a0;
+        base[QC_BODY] = (uint32_t)(MAX_BODIES * a0);
+        base[QC_TRI] = (uint32_t)(CAP_CANDIDATES * a0);
+        base[QC_DEEP] = (uint32_t)((CAP_RESULTS + CAP_CANDIDATES) * a0);
+        base[QC_COMBINE] = (uint32_t)(CAP_RESULTS * a0);
+    }
+    __syncthreads();
+    if (tid < QC_WORDS) count[tid] = base[tid];
+    __syncthreads();
+    // items go to warps in turn, so that few items have a warp each
+    const int first = lane * BLOCK_WARPS + warp;
+    auto each = [&](int items, auto&& fn) {
+        for (int i = first; i < items; i += BLOCK_THREADS) fn(i);
+    };
+    auto queue = [&](int q, auto&& fn) {
+        const uint32_t b = base[q], e = count[q];
+        for (uint32_t i = b + first; i < e; i += BLOCK_THREADS) fn(i);
+    };
+    auto place = [&](int q, uint32_t res0) { return (uint32_t)resultBase(q) * (uint32_t)D.N + res0; };
+    PhaseStats st{0, 0, 0, 0};
+    const int bodies = 1 + maxCars;
+    // this thread's car and body
+    const int la = first % n, slot = first / n, a = a0 + la;
+    const int nb = arenaBodies(D, a);
+    const bool hasCar = slot < maxCars && 1 + slot < nb, hasBody = slot < bodies && slot < nb;
+#pragma unroll 1
+    for (int tick = 0; tick < ticks; tick++) {
+        // rays
+        if (hasBody) sh.pair.cell[slot][la] = bodyCellWord(D, a, slot);
+        __syncthreads();
+        each(4 * maxCars * n, [&](int i) {
+            const int l = i % n, q = i / n, s = q % maxCars, w = q / maxCars, ar = a0 + l, nbr = arenaBodies(D, ar);
+            Xf xf;
+            bool culled;
+            if (1 + s >= nbr || !rayCar(D, ar, s, xf, culled)) return;
+            const RayClass c = rayPhase(D, T, ar, s, w, xf, culled, [&](uint32_t at) {
+                uint32_t m = 0;
+                for (int b = 0; b < nbr; b++) m |= cellsNear(at, sh.pair.cell[b][l]) ? 1u << b : 0u;
+                return m;
+            }, st);
+            if (c == RAY_MESHES) T.rayQ[atomicAdd(&count[QC_RAY], 1u)] = (uint32_t)rayIdx(D, ar, s, w);
+            else if (c == RAY_BODIES) T.rayQ[rays + atomicAdd(&count[QC_BODYRAY], 1u)] = (uint32_t)rayIdx(D, ar, s, w);
+        });
+        __syncthreads();
+        queue(QC_RAY, [&](uint32_t i) {
+            const uint32_t r = T.rayQ[i];
+            if (meshRayPhase(D, T, r, st)) T.rayQ[rays + atomicAdd(&count[QC_BODYRAY], 1u)] = r;
+        });
+        __syncthreads();
+        queue(QC_BODYRAY, [&](uint32_t i) { bodyRayPhase(D, T, T.rayQ[rays + i], st); });
+        __syncthreads();
+        // cars
+        if (maxCars > 0) {
+            DriveShared& ds = sh.drive;
+            DriveThread t;
+            t.s = slot;
+            t.la = la;
+            t.a = a;
+            t.finished = true;
+            t.deps = 0;
+            if (tid < PHASE_ARENAS) ds.done[tid] = 0;
+            if (hasCar) driveLoad(D, T, t, ds);
+            __syncthreads();
+            if (hasCar && t.finished) atomicOr(&ds.done[la], 1u << slot);
+            __syncthreads();
+            for (int round = 0; round <= MAX_CARS; round++) {
+                const bool ready = !t.finished && !(t.deps & ~ds.done[la]);
+                if (ready) driveRun(t, ds);
+                const int all = __syncthreads_and(t.finished);
+                if (all) break;
+                if (ready) atomicOr(&ds.done[la], 1u << slot);
+                __syncthreads();
+            }
+            if (hasCar) driveStore(D, T, t);
+            __syncthreads();
+        }
+        // pairs
+        {
+            PairShared& ps = sh.pair;
+            PairThread t;
+            t.b = slot;
+            t.la = la;
+            t.a = a;
+            t.nb = nb;
+            if (tid < PHASE_ARENAS) ps.need[tid] = 0;
+            if (hasBody) pairLoad(D, T, t, ps, tick == 0);
+            __syncthreads();
+            if (hasBody) pairPick(D, t, ps);
+            __syncthreads();
+            BodyStatics o;
+            if (hasBody) {
+                o = pairStatics(D, t, st);
+                const uint32_t dyn = pairDynamics(D, t, ps);
+                const uint32_t m0 = atomicAdd(&count[slot == 0 ? QC_BALLMESH : QC_CARMESH], (uint32_t)__popc(o.meshes));
+                const uint32_t p0 = atomicAdd(&count[QC_PLANE], (uint32_t)__popc(o.planes));
+                const uint32_t d0 = atomicAdd(&count[slot == 0 ? QC_CARBALL : QC_CARCAR], (uint32_t)__popc(dyn));
+                pairStore(D, T, t, o, dyn, m0, p0, d0);
+                pairNeed(t, o, ps);
+            }
+            __syncthreads();
+            if (hasBody) {
+                const uint32_t need = ps.need[la];
+                pairStoreHead(D, T, t, o, need);
+                if (slot == 0 && arenaHasContacts(need) && !arenaByBodies(need))
+                    T.solveQ[atomicAdd(&count[QC_SOLVE], 1u)] = (uint32_t)a;
+            }
+            __syncthreads();
+        }
+        // contacts
+        {
+            const uint32_t c0 = base[QC_CARMESH], b0 = base[QC_BALLMESH], nCar = count[QC_CARMESH] - c0;
+            findPairs(D, T, sh.list + warp * FIND_GROUPS, c0, nCar, b0, nCar + count[QC_BALLMESH] - b0, (uint32_t)warp,
+                      (uint32_t)BLOCK_WARPS);
+            queue(QC_CARBALL, [&](uint32_t i) { findPhase(D, T, place(QC_CARBALL, i)); });
+        }
+        __syncthreads();
+        if (tid == 0) count[QC_TRI] = min(count[QC_TRI], T.candCap);
+        __syncthreads();
+        queue(QC_TRI, [&](uint32_t i) { trianglePhase(D, T, i); });
+        queue(QC_CARCAR, [&](uint32_t i) { carCarPhase(D, T, place(QC_CARCAR, i)); });
+        queue(QC_PLANE, [&](uint32_t i) { planePhase(D, T, place(QC_PLANE, i), st); });
+        __syncthreads();
+        for (uint32_t i = base[QC_DEEP] + warp, e = count[QC_DEEP]; i < e; i += BLOCK_WARPS)
+            if (lane == 0) deepPhase(D, T, T.deepQ[i], &sh.epa[warp], st);
+        __syncthreads();
+        queue(QC_COMBINE, [&](uint32_t i) { combinePhase(D, T, T.combineQ[i], st); });
+        __syncthreads();
+        // islands
+        for (uint32_t i = base[QC_SOLVE] + warp, e = count[QC_SOLVE]; i < e; i += BLOCK_WARPS)
+            solvePhase(D, T, (int)T.solveQ[i], sh.solve[warp], WarpLanes{}, st);
+        queue(QC_BODY, [&](uint32_t i) { bodyPhase(D, T, T.bodyQ[i], st); });
+        __syncthreads();
+        // finish
+        {
+            FinishShared& fs = sh.finish;
+            FinishThread t;
+            t.body = slot;
+            t.la = la;
+            t.a = a;
+            t.nb = nb;
+            if (tid < QC_WORDS) count[tid] = base[tid];
+            each(NUM_PADS * n, [&](int i) {
+                if (arenaBodies(D, a0 + i % n) > 1) padLoad(D, a0 + i % n, i % n, i / n, fs);
+            });
+            if (hasCar) fs.picked[slot][la] = 0;
+            if (slot == 0) fs.touched[la] = 0;
+            __syncthreads();
+            if (hasBody) {
+                finishBody(D, T, t, fs);
+                if (slot > 0) finishPads(D, t, fs);
+            }
+            __syncthreads();
+            each(NUM_PADS * n, [&](int i) {
+                if (arenaBodies(D, a0 + i % n) > 1) finishPad(D, a0 + i % n, i % n, i / n, fs);
+            });
+            __syncthreads();
+            if (hasBody) {
+                if (slot > 0) finishBoost(D, t, fs);
+                else finishArena(D, t, fs);
+            }
+            __syncthreads();
+        }
+    }
+    blockStats(D, st);
 }
 
 }  // namespace rsb
