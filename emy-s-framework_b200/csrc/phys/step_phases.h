@@ -1446,18 +1446,19 @@ struct FrictionRow1 {
 };
 constexpr int MAX_ROWS1 = BODY_MAX_TASKS * MAX_POINTS + 1;
 
-// setupContactConstraint and convertContactInner's friction row for one contact of the body.
-struct Solver1 {
+struct Solver1State {
     V3 lin, ang, extF, extT;   // the solver body's velocities and external impulses
     V3 dLin, dAng, push, turn;
     V3 invMassV;
+};
+struct Solver1 : Solver1State {
     int nc, nf;
     ContactRow1 c[MAX_ROWS1];
     FrictionRow1 f[MAX_ROWS1];
 };
-RSB_HD void addRows1(Solver1& S, const Body& b, V3 normal, float dist, float fric, float rest, V3 rel, float dt,
-                     int special) {
-    ContactRow1& r = S.c[S.nc];
+// setupContactConstraint and convertContactInner's friction row for one contact of the body.
+RSB_HD void makeRows1(const Solver1State& S, const Body& b, V3 normal, float dist, float fric, float rest, V3 rel, float dt,
+                      int special, ContactRow1& r, FrictionRow1& fr) {
     const float invDt = 1.f / dt;
     const V3 torqueAxis = cross(rel, normal);
     const V3 angA = b.invIw * torqueAxis;
@@ -1492,7 +1493,6 @@ RSB_HD void addRows1(Solver1& S, const Body& b, V3 normal, float dist, float fri
         V3 lat2;
         planeSpace1(normal, lat, lat2);
     }
-    FrictionRow1& fr = S.f[S.nf];
     fr.n = lat;
     fr.rc = cross(rel, lat);
     fr.ang = b.invIw * fr.rc;
@@ -1502,13 +1502,17 @@ RSB_HD void addRows1(Solver1& S, const Body& b, V3 normal, float dist, float fri
     const float fvelErr = 0.f - (fv1 + 0.f);
     fr.rhs = 0.f + fvelErr * fr.jacInv;
     fr.applied = 0.f;
-    fr.contact = S.nc;
+}
+RSB_HD void addRows1(Solver1& S, const Body& b, V3 normal, float dist, float fric, float rest, V3 rel, float dt,
+                     int special) {
+    makeRows1(S, b, normal, dist, fric, rest, rel, dt, special, S.c[S.nc], S.f[S.nf]);
+    S.f[S.nf].contact = S.nc;
     S.nc++;
     S.nf++;
 }
 
 // resolveSingleConstraintRow* against the fixed body; returns the impulse.
-RSB_HD float solveRow1(Solver1& S, V3 n, V3 rc, V3 ang, float rhs, float cfm, float jacInv, float lo, float hi,
+RSB_HD float solveRow1(Solver1State& S, V3 n, V3 rc, V3 ang, float rhs, float cfm, float jacInv, float lo, float hi,
                        bool generic, float& applied) {
     const float applied0 = applied;
     float delta = rhs - applied0 * cfm;
@@ -1528,25 +1532,27 @@ RSB_HD float solveRow1(Solver1& S, V3 n, V3 rc, V3 ang, float rhs, float cfm, fl
     S.dAng = S.dAng + ang * delta;
     return delta;
 }
+// One pass of the split impulse's row; whether it changed anything.
+template <class RowT>
+RSB_HD bool pushRow1(Solver1State& S, RowT& c) {
+    if (c.rhsPen == 0.f) return false;
+    const float applied0 = c.push;
+    float delta = c.rhsPen - applied0 * (0.f * c.jacInv);
+    const float d1 = dot_simd(c.n, S.push) + dot_simd(c.rc, S.turn);
+    delta = delta - d1 * c.jacInv;
+    delta = delta - 0.f * c.jacInv;
+    const float sum = applied0 + delta;
+    const bool lowerLess = sum < 0.f;
+    delta = lowerLess ? (0.f - applied0) : delta;
+    c.push = lowerLess ? 0.f : sum;
+    S.push = S.push + (c.n * S.invMassV) * delta;
+    S.turn = S.turn + c.ang * delta;
+    return delta != 0.f;
+}
 RSB_HD void iterate1(Solver1& S) {
     for (int it = 0; it < kNumIterations; it++) {
         bool any = false;
-        for (int j = 0; j < S.nc; j++) {
-            ContactRow1& c = S.c[j];
-            if (c.rhsPen == 0.f) continue;
-            const float applied0 = c.push;
-            float delta = c.rhsPen - applied0 * (0.f * c.jacInv);
-            const float d1 = dot_simd(c.n, S.push) + dot_simd(c.rc, S.turn);
-            delta = delta - d1 * c.jacInv;
-            delta = delta - 0.f * c.jacInv;
-            const float sum = applied0 + delta;
-            const bool lowerLess = sum < 0.f;
-            delta = lowerLess ? (0.f - applied0) : delta;
-            c.push = lowerLess ? 0.f : sum;
-            S.push = S.push + (c.n * S.invMassV) * delta;
-            S.turn = S.turn + c.ang * delta;
-            any |= delta != 0.f;
-        }
+        for (int j = 0; j < S.nc; j++) any |= pushRow1(S, S.c[j]);
         if (!any) break;
     }
     for (int it = 0; it < kNumIterations; it++) {

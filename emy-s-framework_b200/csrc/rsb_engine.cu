@@ -21,6 +21,7 @@
 #include "engine_host.h"
 #include "env_kernels.cuh"
 #include "step_kernels.cuh"
+#include "phys/ball_phase.h"
 #include "culler.cuh"
 #include "vanta.cuh"
 
@@ -350,44 +351,134 @@ struct PredSlices {
     int32_t n;
 };
 
+// A ball's triangle list (ball_phase.h) by the whole warp: headers and leaves 32 at a time, in the
+// order of ballListMake.  Returns its length, BALL_LIST_OVER when it does not fit, and in clear how
+// far its triangles are from `at`.
+__device__ __noinline__ int warpBallList(const EngineView& D, V3 at, V3 mn, V3 mx, uint16_t* list, float& clear) {
+    const ArenaStatic& S = D.S;
+    const int lane = threadIdx.x & 31;
+    const uint32_t all = 0xffffffffu, below = (1u << lane) - 1u;
+    int n = 0;
+    float near = 1e30f;
+    for (int m = 0; m < S.numMeshes; m++) {
+        const MeshDesc& md = S.meshes[m];
+        if (!aabbOverlap(mn, mx, md.shapeMin, md.shapeMax)) continue;
+        uint16_t qmn[3], qmx[3];
+        bvhQuantizeClamp(md, mn, 0, qmn);
+        bvhQuantizeClamp(md, mx, 1, qmx);
+        for (int h0 = 0; h0 < md.subCount; h0 += 32) {
+            const int h = h0 + lane;
+            bool ov = false;
+            if (h < md.subCount) {
+                const BvhSubtree& st = S.subs[md.subOff + h];
+                ov = qOverlap(qmn, qmx, st.qmin, st.qmax);
+            }
+            for (uint32_t subs = __ballot_sync(all, ov); subs; subs &= subs - 1u) {
+                const SubtreeLeaves sl = S.subLeaves[md.subOff + h0 + __ffs((int)subs) - 1];
+                for (int k0 = 0; k0 < sl.count; k0 += 32) {
+                    bool ok = k0 + lane < sl.count;
+                    int tri = 0;
+                    if (ok) {
+                        const BvhNode nd = S.leaves[sl.off + k0 + lane];
+                        tri = nd.data;
+                        const TriData& td = triData(S, m, tri);
+                        ok = qOverlap(qmn, qmx, nd.qmin, nd.qmax) && triBoxOverlap(td, mn, mx);
+                        if (ok) near = fmin_(near, triBoxDistance(td, at));
+                    }
+                    const uint32_t bits = __ballot_sync(all, ok);
+                    const int place = n + __popc(bits & below);
+                    if (ok && place < BALL_LIST) list[place] = ballListKey(m, tri);
+                    n += __popc(bits);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    clear = __uint_as_float(__reduce_min_sync(all, __float_as_uint(near)));  // not negative: ordered as words
+    return n <= BALL_LIST ? n : BALL_LIST_OVER;
+}
+
 // BallPredTracker::ForceUpdateAllPred (BallPredTracker.cpp:80-88) for every arena at once: the
 // arena's ball passes through Ball::GetState / Ball::SetState into a world of its own with no
 // cars, which steps one tick at a time (Arena::Step of a ball-only arena); out[a * n + k] is the
-// ball after s.t[k] ticks.  The arena's own records are only read.  At most 128 registers a
-// thread, so that 4 blocks share an SM and 65,536 arenas run in one wave (103 ms against 116 ms
-// at 168 registers for 3v3 x 65,536 x 360 ticks; identical results).
-__global__ void __launch_bounds__(128, 4) predictBallKernel(EngineView D, PredSlices s, rsb_ball_state* out) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= D.N) return;
-    ArenaSim A;
-    EpaWork epa;
-    World& W = A.W;
-    W.epa = &epa;
-    W.S = &D.S;
-    W.P = &D.P;
-    A.teamSize = A.numCars = 0;
-    W.nc = 0;
-    W.nb = 1;
-    W.status = 0;
-    W.noRot[0] = 1;
+// ball after s.t[k] ticks.  The arena's own records are only read.
+//
+// One thread per ball, its state in registers: a rollout is a serial chain of ticks, so the time is
+// that of the slowest chain.  What a tick does with the meshes is the warp's work: it makes a ball's
+// triangle list when the ball needs a new one, and tests the triangles of a list 32 at a time, so
+// that the ball's own thread sees only those that it touches.  A list that does not fit is made
+// again each tick for the ball's own box.  What bounds a tick is a chain of dependent instructions,
+// and contacts, which differ from ball to ball: 14,000 cycles for a tick of a warp in which a ball
+// touches something, 3,000 for one in which all fly.  A warp still takes a full 32 balls from
+// PRED_WARPS * SMs * 32 balls on: narrower warps spread the contacts, but each holds its own lines
+// of local memory and of code.  16,384 balls, 360 ticks, three such calls side by side, with 2, 4,
+// 8, 16, 32 and 64 warps per SM: 5.7, 6.0, 7.4, 9.5, 12.1 and 17.0 ms each; 1,024 balls with 2, 4
+// and 8: 1.1, 1.3 and 1.7 ms.  One thread per ball on the general tick, whose arena lies in local
+// memory, took 17.0 ms; this takes 5.1 ms.
+constexpr int PRED_THREADS = 64, PRED_WARPS = 2;
+__global__ void __launch_bounds__(PRED_THREADS) predictBallKernel(const __grid_constant__ EngineView D, PredSlices s,
+                                                                  rsb_ball_state* out, int width) {
+    __shared__ uint16_t lists[PRED_THREADS][BALL_LIST], hits[PRED_THREADS][BALL_LIST];
+    const uint32_t all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp0 = threadIdx.x & ~31;
+    const int tile = blockIdx.x * (PRED_THREADS / 32) + (threadIdx.x >> 5);
+    const int64_t a = (int64_t)tile * width + lane;
+    const bool live = lane < width && a < D.N;
     BallP p;
-    loadPlanes(p, D.ball, a, D.N);
-    applyBallState(p, ballStateOf(p));
-    ballBodyOf(D, p, W.b[0]);
-    A.tickCount = 0;
-    A.status = 0;
-    A.goalTeam = -1;
-    A.touchedMask = 0;
-    A.rngKey = 0;
-    W.cull = 0;
-    W.cullAudit = 0;
-    W.nStatic = W.nCulled = W.nMissed = 0;
-    W.cullMissed = 0;
-    W.nRows = 0;
+    BallSim b;
+    BallContacts C;
+    BallRows R;
+    if (live) {
+        loadPlanes(p, D.ball, (int)a, D.N);
+        applyBallState(p, ballStateOf(p));
+        ballSimInit(D, p, b);
+    }
+    auto shuffled = [&](V3 v, int j) {
+        return V3{__shfl_sync(all, v.x, j), __shfl_sync(all, v.y, j), __shfl_sync(all, v.z, j)};
+    };
     int t = 0;
     for (int k = 0; k < s.n; k++) {
-        for (; t < s.t[k]; t++) arenaTick(A);
-        out[(size_t)a * s.n + k] = ballStateOf(ballRecordOf(W.b[0]));
+        for (; t < s.t[k]; t++) {
+            for (uint32_t need = __ballot_sync(all, live && ballTickPairs(D, b)); need; need &= need - 1u) {
+                const int j = __ffs((int)need) - 1;
+                const V3 at = shuffled(b.listAt, j);
+                V3 mn, mx;
+                ballListBox(D.P, at, mn, mx);
+                float clear;
+                const int n = warpBallList(D, at, mn, mx, lists[warp0 + j], clear);
+                if (lane == j) {
+                    b.listN = n;
+                    b.listClear = clear;
+                }
+            }
+            int found = 0;
+            for (uint32_t read = __ballot_sync(all, live && ballReadsList(D.P, b)); read; read &= read - 1u) {
+                const int j = __ffs((int)read) - 1, listN = __shfl_sync(all, b.listN, j);
+                Xf xf = b.xf;
+                xf.o = shuffled(b.xf.o, j);
+                for (int r = 0; r < 3; r++) xf.b.r[r] = shuffled(b.xf.b.r[r], j);
+                BallBox box;
+                ballBoxOf(D.P, xf, box);
+                int n = 0;
+                if (listN == BALL_LIST_OVER) {
+                    float clear;
+                    n = warpBallList(D, xf.o, box.mn, box.mx, hits[warp0 + j], clear);
+                } else {
+                    for (int k0 = 0; k0 < listN; k0 += 32) {
+                        const uint16_t key = k0 + lane < listN ? lists[warp0 + j][k0 + lane] : (uint16_t)0;
+                        const uint32_t bits = __ballot_sync(
+                            all, k0 + lane < listN && ballNear(D, xf, box, key >> 10, key & 1023));
+                        if (bits >> lane & 1u) hits[warp0 + j][n + __popc(bits & ((1u << lane) - 1u))] = key;
+                        n += __popc(bits);
+                    }
+                    __syncwarp();
+                }
+                if (lane == j) found = n;
+            }
+            if (live) ballTickSolve(D, b, hits[threadIdx.x], found, C, R);
+            __syncwarp();
+        }
+        if (live) out[(size_t)a * s.n + k] = ballStateOf(ballSimRecord(p, b));
     }
 }
 
@@ -510,6 +601,14 @@ static bool allocStep(rsb_handle* h) {
 }
 
 static cudaStream_t pick(rsb_handle* h, void* s) { return s ? (cudaStream_t)s : h->stream; }
+
+static cudaError_t launchPredict(rsb_handle* h, const PredSlices& s, rsb_ball_state* out, cudaStream_t st) {
+    const int spread = PRED_WARPS * h->smCount;
+    const int width = std::min(32, (h->N + spread - 1) / spread), tiles = (h->N + width - 1) / width;
+    predictBallKernel<<<(tiles + PRED_THREADS / 32 - 1) / (PRED_THREADS / 32), PRED_THREADS, 0, st>>>(devView(h), s, out,
+                                                                                                     width);
+    return cudaGetLastError();
+}
 
 // ------------------------------------------------------------------ C ABI
 
@@ -864,8 +963,7 @@ rsb_status rsb_predict_ball(rsb_handle* h, const int32_t* slice_ticks, int32_t n
         h->predCap = cap;
     }
     cudaStream_t st = pick(h, stream);
-    predictBallKernel<<<(h->N + 127) / 128, 128, 0, st>>>(devView(h), s, h->dPred);
-    RSB_CUDA(cudaGetLastError());
+    RSB_CUDA(launchPredict(h, s, h->dPred, st));
     if (out) {
         RSB_CUDA(cudaMemcpyAsync(out, h->dPred, need * sizeof(rsb_ball_state), cudaMemcpyDeviceToHost, st));
         RSB_CUDA(cudaStreamSynchronize(st));
@@ -1957,8 +2055,7 @@ rsb_status rsb_build_vanta_obs(rsb_handle* h, void* stream) {
         ps.t[0] = 120;
         ps.t[1] = 240;
         ps.t[2] = 360;
-        predictBallKernel<<<(h->N + 127) / 128, 128, 0, st>>>(devView(h), ps, h->dVantaPred);
-        RSB_CUDA(cudaGetLastError());
+        RSB_CUDA(launchPredict(h, ps, h->dVantaPred, st));
         V.pred = h->dVantaPred;
     }
     const EnvView E = envView(h);

@@ -4,6 +4,7 @@
 // thread per body, queues taken from the back so that nothing depends on their order.
 #include "host_engine.cpp"
 
+#include "phys/ball_phase.h"
 #include "phys/step_phases.h"
 
 extern "C" {
@@ -217,6 +218,79 @@ int32_t rsb_host_step_phases(rsb_handle* h, int32_t ticks, uint32_t* cull, int32
     stats[2] += st.nMissed;
     stats[3] += st.nRows;
     return RSB_OK;
+}
+
+// `ticks` ticks of every arena's ball in a world without cars, by arenaTick (ref) and by the
+// ball's own tick: the number of (arena, tick) pairs whose records differ, and in seen[] how many
+// ticks had a list made, contacts, more than one manifold with contacts, and an overflowed list.
+int64_t rsb_host_ball_ticks_differ(rsb_handle* h, int32_t ticks, int64_t* seen) {
+    EngineView D;
+    std::memset(&D, 0, sizeof D);
+    D.S = h->S.view;
+    D.P = h->P;
+    D.N = h->N;
+    std::unique_ptr<ArenaSim> A(new ArenaSim());
+    std::unique_ptr<EpaWork> epa(new EpaWork());
+    std::unique_ptr<BallContacts> C(new BallContacts());
+    std::unique_ptr<BallRows> R(new BallRows());
+    int64_t bad = 0;
+    for (int a = 0; a < h->N; a++) {
+        World& W = A->W;
+        W.epa = epa.get();
+        W.S = &D.S;
+        W.P = &D.P;
+        A->teamSize = A->numCars = 0;
+        W.nc = 0;
+        W.nb = 1;
+        W.status = 0;
+        W.noRot[0] = 1;
+        BallP p;
+        loadPlanes(p, h->ball.data(), a, h->N);
+        applyBallState(p, ballStateOf(p));
+        ballBodyOf(D, p, W.b[0]);
+        BallSim s;
+        ballSimInit(D, p, s);
+        A->tickCount = 0;
+        A->status = 0;
+        A->goalTeam = -1;
+        A->touchedMask = 0;
+        A->rngKey = 0;
+        W.cull = 0;
+        W.cullAudit = 0;
+        W.nStatic = W.nCulled = W.nMissed = 0;
+        W.cullMissed = 0;
+        W.nRows = 0;
+        uint16_t list[BALL_LIST], hits[BALL_LIST];
+        BallBox box;
+        for (int t = 0; t < ticks; t++) {
+            arenaTick(*A);
+            if (ballTickPairs(D, s)) {
+                ballListMake(D, s, list);
+                seen[0]++;
+                seen[3] += s.listN == BALL_LIST_OVER;
+            }
+            C->blocks = 0;
+            ballBoxOf(D.P, s.xf, box);
+            // every other tick the triangles that pass the first tests only, as the kernel takes them
+            int n = s.listN;
+            if (t & 1) {
+                n = ballReadsList(D.P, s) ? s.listN : 0;
+                const int all = n;
+                if (n > 0) n = 0;
+                for (int k = 0; k < all; k++)
+                    if (ballNear(D, s.xf, box, list[k] >> 10, list[k] & 1023)) hits[n++] = list[k];
+            }
+            ballTickSolve(D, s, t & 1 ? hits : list, n, *C, *R);
+            seen[1] += C->blocks > 0;
+            seen[2] += C->blocks > 1;
+            const rsb_ball_state x = ballStateOf(ballRecordOf(W.b[0])), y = ballStateOf(ballSimRecord(p, s));
+            if (std::memcmp(&x, &y, sizeof x) != 0) {
+                bad++;
+                break;
+            }
+        }
+    }
+    return bad;
 }
 
 // The first word at which the records of two handles differ, as plane * 2^40 + index, or -1.

@@ -37,6 +37,8 @@ def host(pkg, tmp_path_factory):
     lib = pkg.rsb.load_library(out)
     lib.rsb_host_records_differ.restype = C.c_int64
     lib.rsb_host_records_differ.argtypes = [C.c_void_p, C.c_void_p]
+    lib.rsb_host_ball_ticks_differ.restype = C.c_int64
+    lib.rsb_host_ball_ticks_differ.argtypes = [C.c_void_p, C.c_int32, C.c_void_p]
     lib.rsb_host_step_phases.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]
     return lib, cases._arena()
 
@@ -161,3 +163,27 @@ def test_states_that_are_not_finite(pkg, host, value):
         balls["vel"]["z"][2] = value
 
     compare(pkg, host, 7, np.full(7, 2, np.int32), "heap", 61, 2, 3, mutate=mutate)
+
+
+@pytest.mark.parametrize("kind", ["field", "walls", "still", "notfinite"])
+def test_ball_alone_matches_the_ball_only_arena(pkg, host, kind):
+    """The ball prediction's own tick against the ball-only arena, every tick of 360, byte by byte:
+    flight, floor and ceiling, ramps, corners, goals, resting balls and balls that are not finite."""
+    rsb, (lib, arena) = pkg.rsb, host
+    b = rsb.Batch(lib, 256, team_size=1, meshes_path=arena)
+    _, balls = start(rsb, b, "walls" if kind == "walls" else "field", 91)
+    if kind == "still":
+        for f in ("vel", "ang_vel"):
+            for c in "xyz":
+                balls[f][c][::2] = 0
+        balls["pos"]["z"] = 93.15
+    if kind == "notfinite":
+        for i, v in enumerate((np.nan, np.inf, 3e7, 1e30)):
+            balls["vel"]["xyz"[i % 3]][i] = v
+            balls["pos"]["xyz"[i % 3]][8 + i] = v
+    b.set_balls(balls)
+    seen = np.zeros(4, np.int64)
+    assert lib.rsb_host_ball_ticks_differ(b._h, 360, seen.ctypes.data) == 0
+    assert seen[0] and seen[1]
+    if kind == "walls":
+        assert seen[2]
