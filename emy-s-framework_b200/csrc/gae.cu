@@ -7,19 +7,13 @@
 // (GAECuda.cu:120-129).  Compiled with --fmad=false, so each multiply and add rounds as the
 // reference's --fmad=false build does.
 //
-// Layout of the work (three launches, no host round trip):
-//   gaeSummaryKernel  one block per 4,096-element chunk: truncations in the chunk and the
-//                     position of its last nonzero terminal;
-//   gaeScanKernel     one block: exclusive prefix (truncations before each chunk, last
-//                     terminal before each chunk);
-//   gaeSegmentKernel  one block per chunk: stages the chunk's rewards, values and terminals in
-//                     shared memory with coalesced loads, lists the segments that END in the
-//                     chunk, runs each one on its own thread (a segment that began in an earlier
-//                     chunk walks on into global memory), and writes the chunk's results back
-//                     with coalesced stores.  Every element is written by the thread of the
-//                     segment that contains it and by no other.  Per-block sums of |r/std| and
-//                     |clip(r/std)| go to a scratch row; the last block to finish (a ticket
-//                     counter, no waiting) adds them in block order and writes rewClipPortion.
+// Layout of the work (two launches, no host round trip):
+//   gaeSummaryKernel  truncations in each 4,096-element chunk (left out when there are none);
+//   gaeScanKernel     their exclusive prefix, for buffers of more than kGaeDirect chunks; in
+//                     smaller ones each block adds up the counts before its own;
+//   gaeSegmentKernel  one block per chunk, for the segments that END in it: see there.
+// The last block to finish (a ticket counter, no waiting) adds the blocks' sums of |r/std| and
+// of what clipping took of it in block order and writes rewClipPortion.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -38,25 +32,21 @@ namespace {
 constexpr int kGaeThreads = 256;
 constexpr int kGaePerThread = 16;
 constexpr int kGaeChunk = kGaeThreads * kGaePerThread;  // elements per block
-constexpr int kPosBits = 13;                             // chunk-relative position field of a segment entry
-constexpr int kPosMask = (1 << kPosBits) - 1;
 constexpr int8_t kTermNormal = 1;
 constexpr int8_t kTermTruncated = 2;
 // largest T: chunk arithmetic stays inside int32
 constexpr int32_t kGaeMaxT = INT32_MAX - 2 * kGaeChunk;
 
-// Shared memory of gaeSegmentKernel.  The float rows are padded by one word per 32 elements,
-// so that lanes walking segments whose lengths are multiples of 32 (one trajectory of a
-// 32-step rollout per lane) fall into different banks.
+// Shared rows are padded by one word per 32 elements, so that lanes walking segments whose lengths
+// are multiples of 32 (one trajectory of a 32-step rollout per lane) fall into different banks.
 constexpr int kPadded = kGaeChunk + kGaeChunk / 32;
 __host__ __device__ constexpr int padIdx(int i) { return i + (i >> 5); }
-constexpr size_t kSmemRew = sizeof(float) * kPadded;        // rewards, then advantages
-constexpr size_t kSmemRet = sizeof(float) * kPadded;        // returns
-constexpr size_t kSmemVal = sizeof(float) * (kPadded + 4);  // values + the one after the chunk
-constexpr size_t kSmemSeg = sizeof(int) * (kGaeChunk + 4);  // segment ends
-constexpr size_t kSmemTerm = kGaeChunk;                     // terminals (16-byte aligned)
-constexpr size_t kSmemSegment = kSmemRew + kSmemRet + kSmemVal + kSmemSeg + kSmemTerm;
-static_assert((kSmemRew + kSmemRet + kSmemVal + kSmemSeg) % 16 == 0, "terminal row must be 16-byte aligned");
+constexpr int kGaeWords = kGaeChunk / 32;
+constexpr int kGaeHalo = 4 * kGaeThreads;
+// Up to this many chunks (16.8 million elements) a block adds up the counts of the chunks before
+// its own, at most 16 loads a thread beside those of its elements; a scan of its own costs a launch
+// and a single block's pass, 4 us at 3,072 chunks.
+constexpr int kGaeDirect = 4096;
 
 struct GaeArgs {
     const float* rews;
@@ -71,7 +61,8 @@ struct GaeArgs {
     int T;
     int nChunks;
     float gamma, lambda, returnStd, clipRange;
-    const int2* pre;
+    const int* count;  // truncations of each chunk, or before each chunk (counted)
+    bool counted;
     float2* part;
     unsigned* ticket;
 };
@@ -82,336 +73,344 @@ __device__ __forceinline__ int warpSum(int v) {
     return v;
 }
 
-__device__ __forceinline__ int warpMax(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
+__device__ __forceinline__ int warpMax(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
-// Truncations and the last nonzero terminal of each chunk.  Thread t reads bytes
-// [16 t, 16 t + 16) of its chunk, as one 16-byte load when the row is 16-byte aligned.
+// Truncations of each chunk.  Thread t reads bytes [16 t, 16 t + 16) of its chunk, as one 16-byte
+// load when the row is 16-byte aligned.  The first block clears the ticket.
 template <bool kVec>
 __global__ void __launch_bounds__(kGaeThreads) gaeSummaryKernel(const int8_t* __restrict__ term, int T,
-                                                                int2* __restrict__ sum) {
+                                                                int* __restrict__ count, unsigned* ticket) {
     const int base = blockIdx.x * kGaeChunk;
     const int len = min(kGaeChunk, T - base);
     const int j0 = threadIdx.x * kGaePerThread;
-    int tr = 0, last = -1;
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
+    int tr = 0;
     if (kVec && j0 + kGaePerThread <= len) {
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(term + base + j0));
         const unsigned words[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int k = 0; k < kGaePerThread; ++k) {
-            const int8_t t = (int8_t)(words[k >> 2] >> (8 * (k & 3)));
-            tr += t == kTermTruncated;
-            if (t != 0) last = base + j0 + k;
-        }
+        for (int k = 0; k < kGaePerThread; ++k) tr += (int8_t)(words[k >> 2] >> (8 * (k & 3))) == kTermTruncated;
     } else {
-        for (int k = 0; k < kGaePerThread && j0 + k < len; ++k) {
-            const int8_t t = __ldg(term + base + j0 + k);
-            tr += t == kTermTruncated;
-            if (t != 0) last = base + j0 + k;
-        }
+        for (int k = 0; k < kGaePerThread && j0 + k < len; ++k) tr += __ldg(term + base + j0 + k) == kTermTruncated;
     }
-    tr = warpSum(tr);
-    last = warpMax(last);
-    __shared__ int sTr[kGaeThreads / 32], sLast[kGaeThreads / 32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-        sTr[warp] = tr;
-        sLast[warp] = last;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int a = 0, m = -1;
-        for (int w = 0; w < kGaeThreads / 32; ++w) {
-            a += sTr[w];
-            m = max(m, sLast[w]);
-        }
-        sum[blockIdx.x] = make_int2(a, m);
-    }
+    tr = __syncthreads_count(tr & 1) + 2 * __syncthreads_count(tr >> 1 & 1) + 4 * __syncthreads_count(tr >> 2 & 1) +
+         8 * __syncthreads_count(tr >> 3 & 1) + 16 * __syncthreads_count(tr >> 4 & 1);
+    if (threadIdx.x == 0) count[blockIdx.x] = tr;
 }
 
-// Exclusive prefix over chunks: truncations before the chunk, last terminal before it (-1).
-__global__ void __launch_bounds__(1024) gaeScanKernel(const int2* __restrict__ sum, int n, int2* __restrict__ pre) {
-    __shared__ int wSum[32], wMax[32];
-    __shared__ int carrySum, carryMax;
+// Exclusive prefix over chunks, in place: truncations before the chunk.
+__global__ void __launch_bounds__(1024) gaeScanKernel(int* __restrict__ count, int n) {
+    __shared__ int wSum[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        carrySum = 0;
-        carryMax = -1;
-    }
-    __syncthreads();
+    int carry = 0;
     for (int base = 0; base < n; base += 1024) {
         const int i = base + (int)threadIdx.x;
-        const int2 v = i < n ? sum[i] : make_int2(0, -1);
-        int s = v.x, m = v.y;
+        const int v = i < n ? count[i] : 0;
+        int s = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int s2 = __shfl_up_sync(0xffffffffu, s, o);
-            const int m2 = __shfl_up_sync(0xffffffffu, m, o);
-            if (lane >= o) {
-                s += s2;
-                m = max(m, m2);
-            }
+            if (lane >= o) s += s2;
         }
-        int exM = __shfl_up_sync(0xffffffffu, m, 1);
-        if (lane == 0) exM = -1;
-        if (lane == 31) {
-            wSum[warp] = s;
-            wMax[warp] = m;
-        }
+        if (lane == 31) wSum[warp] = s;
         __syncthreads();
-        if (warp == 0) {
-            int ws = wSum[lane], wm = wMax[lane];
+        const int w = wSum[lane];
+        const int before = warpSum(lane < warp ? w : 0), all = warpSum(w);
+        if (i < n) count[i] = carry + before + s - v;
+        carry += all;
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ int8_t termOf(unsigned w, int c) { return (int8_t)(w >> (8 * c)); }
+
+// The reward as the advantages use it.  Adds its magnitude, and what clipping took of it, which the
+// reference leaves at all of it without standardisation; summed apart, the small excess keeps the
+// digits that the difference of two large sums would lose.
+__device__ __forceinline__ float gaeReward(const GaeArgs& a, float rew, float& sum, float& excess) {
+    if (!(a.returnStd > 0.0f)) {
+        sum += fabsf(rew);
+        excess += fabsf(rew);
+        return rew;
+    }
+    const float r = rew / a.returnStd;
+    float used = r;
+    if (a.clipRange > 0.0f) used = fminf(fmaxf(r, -a.clipRange), a.clipRange);
+    sum += fabsf(r);
+    excess += fabsf(r) - fabsf(used);
+    return used;
+}
+
+// The recurrence of GAECuda.cu:77-113 over rows [stop, end], backward.  Its rows hold what does not
+// depend on later steps (sD the delta, sR the reward), four read ahead of the chain; they take the
+// advantages and the returns.  A segment's last step starts from zero carries, so that the factors
+// (1 - done)(1 - trunc), which are 1 at every other step, need not be applied.
+__device__ __forceinline__ void gaeWalk(float* sD, float* sR, int end, int stop, float gl, float gamma, float& adv,
+                                        float& ret) {
+    int rel = end;
+    for (; rel - 3 >= stop; rel -= 4) {
+        float d[4], r[4];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int s2 = __shfl_up_sync(0xffffffffu, ws, o);
-                const int m2 = __shfl_up_sync(0xffffffffu, wm, o);
-                if (lane >= o) {
-                    ws += s2;
-                    wm = max(wm, m2);
-                }
-            }
-            wSum[lane] = ws;
-            wMax[lane] = wm;
+        for (int k = 0; k < 4; ++k) {
+            d[k] = sD[padIdx(rel - k)];
+            r[k] = sR[padIdx(rel - k)];
         }
-        __syncthreads();
-        const int addS = carrySum + (warp ? wSum[warp - 1] : 0);
-        const int addM = max(carryMax, warp ? wMax[warp - 1] : -1);
-        if (i < n) pre[i] = make_int2(addS + s - v.x, max(addM, exM));
-        __syncthreads();
-        if (threadIdx.x == 1023) {
-            carrySum = addS + s;
-            carryMax = max(addM, m);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ret = r[k] + ret * gamma;
+            adv = d[k] + gl * adv;
+            sD[padIdx(rel - k)] = adv;
+            sR[padIdx(rel - k)] = ret;
         }
-        __syncthreads();
+    }
+    for (; rel >= stop; --rel) {
+        ret = sR[padIdx(rel)] + ret * gamma;
+        adv = sD[padIdx(rel)] + gl * adv;
+        sD[padIdx(rel)] = adv;
+        sR[padIdx(rel)] = ret;
     }
 }
 
-// One backward step of GAECuda.cu:77-113 (the same operations in the same order).
-struct GaeCarry {
-    float adv, ret, rew, clipped;
-};
-
-__device__ __forceinline__ void gaeStep(const GaeArgs& a, float rew, int8_t terminal, float val, float nextVal,
-                                        int truncBefore, GaeCarry& c, float& advOut, float& retOut) {
-    const float done = terminal == kTermNormal ? 1.0f : 0.0f;
-    const float trunc = terminal == kTermTruncated ? 1.0f : 0.0f;
-    float curReward;
-    if (a.returnStd > 0.0f) {
-        curReward = rew / a.returnStd;
-        c.rew += fabsf(curReward);
-        if (a.clipRange > 0.0f) curReward = fminf(fmaxf(curReward, -a.clipRange), a.clipRange);
-        c.clipped += fabsf(curReward);
-    } else {
-        curReward = rew;
-        c.rew += fabsf(curReward);
-    }
-    float nextValPred;
-    if (terminal == kTermTruncated) {
-        const int idx = a.numTruncs - truncBefore - 1;
-        // a count that does not match the truncated steps reads nothing out of range
-        nextValPred = (idx >= 0 && idx < a.numTruncs) ? __ldg(a.truncVals + idx) : 0.0f;
-    } else if (terminal == kTermNormal) {
-        nextValPred = 0.0f;
-    } else {
-        nextValPred = nextVal;
-    }
-    const float predReturn = curReward + a.gamma * nextValPred * (1.0f - done);
-    const float delta = predReturn - val;
-    const float notDoneNotTrunc = (1.0f - done) * (1.0f - trunc);
-    const float curReturn = rew + c.ret * a.gamma * notDoneNotTrunc;
-    retOut = curReturn;
-    c.adv = delta + a.gamma * a.lambda * notDoneNotTrunc * c.adv;
-    advOut = c.adv;
-    c.ret = curReturn;
-}
-
-// The same step for a running element (terminal 0), the only kind a segment holds before its
-// end: done = trunc = 0 make the reference's factors (1 - done) and (1 - done)(1 - trunc)
-// exactly 1, and multiplying by 1 changes no finite value, so the products are dropped.
-__device__ __forceinline__ void gaeStepRunning(const GaeArgs& a, float rew, float val, float nextVal, GaeCarry& c,
-                                               float& advOut, float& retOut) {
-    float curReward;
-    if (a.returnStd > 0.0f) {
-        curReward = rew / a.returnStd;
-        c.rew += fabsf(curReward);
-        if (a.clipRange > 0.0f) curReward = fminf(fmaxf(curReward, -a.clipRange), a.clipRange);
-        c.clipped += fabsf(curReward);
-    } else {
-        curReward = rew;
-        c.rew += fabsf(curReward);
-    }
-    const float predReturn = curReward + a.gamma * nextVal;
-    const float delta = predReturn - val;
-    const float curReturn = rew + c.ret * a.gamma;
-    retOut = curReturn;
-    c.adv = delta + a.gamma * a.lambda * c.adv;
-    advOut = c.adv;
-    c.ret = curReturn;
-}
-
+// Elements j .. j + 3 of a row, zero from len on.
 template <bool kVec>
-__global__ void __launch_bounds__(kGaeThreads) gaeSegmentKernel(GaeArgs a) {
-    extern __shared__ float4 gaeSmem[];
-    float* sRew = reinterpret_cast<float*>(gaeSmem);  // rewards, overwritten by advantages
-    float* sRet = sRew + kPadded;
-    float* sVal = sRet + kPadded;
-    int* sSeg = reinterpret_cast<int*>(sVal + kPadded + 4);
-    int8_t* sTerm = reinterpret_cast<int8_t*>(sSeg + kGaeChunk + 4);
-    __shared__ int sWarpCount[kGaeThreads / 32];
-    __shared__ float2 sWarpSum[kGaeThreads / 32];
-    __shared__ int sTotal;
+__device__ __forceinline__ void gaeLoad4(const float* __restrict__ p, int j, int len, float* v) {
+    if (kVec && j + 4 <= len) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(p + j));
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = x.z;
+        v[3] = x.w;
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = j + c < len ? __ldg(p + j + c) : 0.0f;
+    }
+}
+template <bool kVec>
+__device__ __forceinline__ unsigned gaeTerm4(const int8_t* __restrict__ p, int j, int len) {
+    if (kVec && j + 4 <= len) return __ldg(reinterpret_cast<const unsigned*>(p + j));
+    unsigned w = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (j + c < len) w |= (unsigned)(uint8_t)__ldg(p + j + c) << (8 * c);
+    return w;
+}
+// Results of elements j .. j + 3 that lie in [from, to).
+template <bool kVec>
+__device__ __forceinline__ void gaeStore4(const GaeArgs& a, int base, int j, int from, int to, const float* sD,
+                                          const float* sR, const float* val) {
+    if (j >= to || j + 4 <= from) return;
+    float d[4], r[4], g[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        d[c] = sD[padIdx(j + c)];
+        r[c] = sR[padIdx(j + c)];
+        g[c] = val[c] + d[c];
+    }
+    if (kVec && j >= from && j + 4 <= to) {
+        *reinterpret_cast<float4*>(a.adv + base + j) = make_float4(d[0], d[1], d[2], d[3]);
+        *reinterpret_cast<float4*>(a.ret + base + j) = make_float4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<float4*>(a.tgt + base + j) = make_float4(g[0], g[1], g[2], g[3]);
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (j + c >= from && j + c < to) {
+            a.adv[base + j + c] = d[c];
+            a.ret[base + j + c] = r[c];
+            a.tgt[base + j + c] = g[c];
+        }
+}
+
+// One block per chunk.  What a step needs besides the carries (reward, delta) is computed for every
+// element in parallel, in the threads that loaded it, four elements to a load; a thread then walks
+// each segment that ends among 16 elements of its own, two multiplies and two adds a step; the
+// threads that hold the values write the results.  A segment that began in an earlier chunk goes on
+// through windows of kGaeHalo elements, staged and written by the whole block and walked by one
+// thread.
+//
+// The buffer is bound by its bytes (9 read, 12 written per element) as long as segments are short
+// against a chunk, else by the walk's chain.
+template <bool kVec>
+__global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
+    __shared__ float sD[kPadded], sR[kPadded];
+    __shared__ unsigned sEnd[kGaeWords], sTrunc[kGaeWords];  // a bit per element: ends of segments, truncations
+    __shared__ int sBefore[kGaeWords], sCount[kGaeThreads / 32], sMax[kGaeThreads / 32];
+    __shared__ float2 sWarpSum[kGaeThreads / 32], sCarry;
     __shared__ bool sLastBlock;
 
+    const uint32_t all = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int base = blockIdx.x * kGaeChunk;
     const int len = min(kGaeChunk, a.T - base);
-
-    // 1. stage the chunk (coalesced; terminals as 4-byte words when aligned)
-#pragma unroll
-    for (int k = 0; k < kGaePerThread; ++k) {
-        const int j = k * kGaeThreads + tid;
-        if (j < len) {
-            sRew[padIdx(j)] = __ldg(a.rews + base + j);
-            sVal[padIdx(j)] = __ldg(a.vals + base + j);
-        }
-    }
-    if (kVec) {
-#pragma unroll
-        for (int k = 0; k < kGaePerThread / 4; ++k) {
-            const int w = k * kGaeThreads + tid;
-            if (4 * w + 4 <= len) {
-                reinterpret_cast<int*>(sTerm)[w] = __ldg(reinterpret_cast<const int*>(a.term + base) + w);
-            } else {
-                for (int b = 4 * w; b < len && b < 4 * w + 4; ++b) sTerm[b] = __ldg(a.term + base + b);
-            }
-        }
-    } else {
-        for (int j = tid; j < len; j += kGaeThreads) sTerm[j] = __ldg(a.term + base + j);
-    }
-    if (tid == 0) {
-        // the value after the chunk; past the buffer the reference reads valPreds[T] only
-        // for a non-terminal final step (GAECuda.cu:101-102)
-        const int nxt = base + len;
-        float v = 0.0f;
-        if (nxt < a.T) v = __ldg(a.vals + nxt);
-        else if (__ldg(a.term + a.T - 1) == 0) v = __ldg(a.vals + a.T);
-        sVal[padIdx(len)] = v;
-    }
-    __syncthreads();
-
-    // 2. list the segments that end in this chunk: nonzero terminals, and the buffer's last
-    //    element when it is not terminal (the trailing run)
     const bool lastChunk = base + len == a.T;
-    const int own0 = tid * kGaePerThread;
-    unsigned endMask = 0, truncMask = 0;
-    {
-        const uint4 w = reinterpret_cast<const uint4*>(sTerm)[tid];  // bytes past len are not read below
-        const unsigned words[4] = {w.x, w.y, w.z, w.w};
+    // past the buffer the reference reads valPreds[T] only for a non-terminal final step
+    // (GAECuda.cu:101-102)
+    const int lenVal = len + (!lastChunk || __ldg(a.term + a.T - 1) == 0);
+
+    // 1. the chunk's elements; bits of the segments' ends (nonzero terminals, and the buffer's last
+    //    element) and of the truncations; truncations before the chunk
+    float rew[4][4], val[4][4], after[4];
+    unsigned term[4];
 #pragma unroll
-        for (int k = 0; k < kGaePerThread; ++k) {
-            const int j = own0 + k;
-            if (j < len) {
-                const int8_t t = (int8_t)(words[k >> 2] >> (8 * (k & 3)));
-                if (t != 0 || (lastChunk && j == len - 1)) endMask |= 1u << k;
-                if (t == kTermTruncated) truncMask |= 1u << k;
+    for (int k = 0; k < 4; ++k) {
+        const int j = 4 * (k * kGaeThreads + tid);
+        term[k] = gaeTerm4<kVec>(a.term + base, j, len);
+        gaeLoad4<kVec>(a.rews + base, j, len, rew[k]);
+        if (kVec && j + 4 <= len) gaeLoad4<true>(a.vals + base, j, len, val[k]);
+        else gaeLoad4<false>(a.vals + base, j, lenVal, val[k]);
+        after[k] = lane == 31 && j + 4 < lenVal ? __ldg(a.vals + base + j + 4) : 0.0f;
+    }
+    cudaGridDependencySynchronize();  // from here on the counts and the ticket
+    int before = 0;
+    if (a.count) {
+        if (a.counted) before = tid == 0 ? __ldcg(a.count + blockIdx.x) : 0;
+        else
+            for (int i = tid; i < (int)blockIdx.x; i += kGaeThreads) before += __ldcg(a.count + i);
+    }
+    before = warpSum(before);
+    if (lane == 0) sCount[warp] = before;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int j = 4 * (k * kGaeThreads + tid);
+        const float first = __shfl_down_sync(all, val[k][0], 1);
+        if (lane != 31) after[k] = first;
+        unsigned ends = 0, truncs = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int8_t t = termOf(term[k], c);
+            if (j + c < len && (t != 0 || (lastChunk && j + c == len - 1))) ends |= 1u << c;
+            if (t == kTermTruncated) truncs |= 1u << c;
+        }
+        unsigned e = ends << (4 * (lane & 7)), r = truncs << (4 * (lane & 7));
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            e |= __shfl_xor_sync(all, e, o);
+            r |= __shfl_xor_sync(all, r, o);
+        }
+        if ((lane & 7) == 0) {
+            sEnd[j >> 5] = e;
+            sTrunc[j >> 5] = r;
+        }
+    }
+    __syncthreads();
+    before = 0;
+#pragma unroll
+    for (int w = 0; w < kGaeThreads / 32; ++w) before += sCount[w];
+    if (warp == 0) {
+        // truncations before each word
+        for (int w0 = 0; w0 < kGaeWords; w0 += 32) {
+            const int n = __popc(sTrunc[w0 + lane]);
+            int s = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int s2 = __shfl_up_sync(all, s, o);
+                if (lane >= o) s += s2;
+            }
+            sBefore[w0 + lane] = before + s - n;
+            before += __shfl_sync(all, s, 31);
+        }
+    }
+    __syncthreads();
+
+    // 2. reward and delta of every element
+    float accRew = 0.0f, accExcess = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int j = 4 * (k * kGaeThreads + tid);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (j + c >= len) break;
+            const int8_t t = termOf(term[k], c);
+            float next = c < 3 ? val[k][c < 3 ? c + 1 : 3] : after[k];
+            if (t == kTermNormal) next = 0.0f;
+            if (t == kTermTruncated) {
+                const int bit = (j + c) & 31;
+                const int idx = a.numTruncs - (sBefore[j >> 5] + __popc(sTrunc[j >> 5] & ((1u << bit) - 1u))) - 1;
+                // a count that does not match the truncated steps reads nothing out of range
+                next = idx >= 0 && idx < a.numTruncs ? __ldg(a.truncVals + idx) : 0.0f;
+            }
+            const float done = t == kTermNormal ? 1.0f : 0.0f;
+            const float r = gaeReward(a, rew[k][c], accRew, accExcess);
+            sD[padIdx(j + c)] = (r + a.gamma * next * (1.0f - done)) - val[k][c];
+            sR[padIdx(j + c)] = rew[k][c];
+        }
+    }
+    __syncthreads();
+
+    // 3. a thread per 16 elements, backward from each end among them
+    const float gl = a.gamma * a.lambda;
+    for (unsigned ends = sEnd[tid >> 1] >> (16 * (tid & 1)) & 0xffffu; ends; ends &= ends - 1u) {
+        const int end = kGaePerThread * tid + __ffs((int)ends) - 1;
+        int w = end >> 5;
+        unsigned earlier = sEnd[w] & ((1u << (end & 31)) - 1u);
+        while (!earlier && w > 0) earlier = sEnd[--w];
+        const int start = earlier ? 32 * w + 32 - __clz((int)earlier) : 0;
+        float adv = 0.0f, ret = 0.0f;
+        gaeWalk(sD, sR, end, start, gl, a.gamma, adv, ret);
+        if (!earlier) sCarry = make_float2(adv, ret);
+    }
+    __syncthreads();
+
+    // 4. the elements of the segments that end here
+    int owned = 0;
+    for (int w0 = 0; w0 < kGaeWords; w0 += 32) {
+        const unsigned e = sEnd[w0 + lane];
+        owned = max(owned, e ? 32 * (w0 + lane) + 32 - __clz((int)e) : 0);
+    }
+    owned = warpMax(owned);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        gaeStore4<kVec>(a, base, 4 * (k * kGaeThreads + tid), 0, owned, sD, sR, val[k]);
+
+    // 5. the part of the first of them in earlier chunks
+    for (int lo = base; owned > 0 && lo > 0;) {
+        const int hi = lo;
+        lo -= kGaeHalo;
+        const int j = 4 * tid;
+        const unsigned t = gaeTerm4<kVec>(a.term + lo, j, kGaeHalo);
+        int last = -1;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (termOf(t, c) != 0) last = j + c;
+        last = warpMax(last);
+        __syncthreads();  // the rows and sMax are read until here
+        if (lane == 0) sMax[warp] = last;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kGaeThreads / 32; ++w) last = max(last, sMax[w]);
+        const int start = last + 1;
+        if (start == hi - lo) break;
+        const bool mine = j + 4 > start;
+        float r[4], v[5], sum = 0.0f;
+        if (mine) {
+            gaeLoad4<kVec>(a.rews + lo, j, kGaeHalo, r);
+            gaeLoad4<kVec>(a.vals + lo, j, kGaeHalo, v);
+            v[4] = __ldg(a.vals + lo + j + 4);  // lo + j + 4 <= base
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                sD[padIdx(j + c)] = (gaeReward(a, r[c], sum, sum) + a.gamma * v[c + 1] * (1.0f - 0.0f)) - v[c];
+                sR[padIdx(j + c)] = r[c];
             }
         }
-    }
-    // block exclusive scan of (ends | truncations << 16)
-    const int packed = __popc(endMask) | (__popc(truncMask) << 16);
-    int incl = packed;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) sWarpCount[warp] = incl;
-    __syncthreads();
-    if (tid == 0) {
-        int run = 0;
-        for (int w = 0; w < kGaeThreads / 32; ++w) {
-            const int c = sWarpCount[w];
-            sWarpCount[w] = run;
-            run += c;
+        __syncthreads();
+        if (tid == 0) {
+            float2 carry = sCarry;
+            gaeWalk(sD, sR, kGaeHalo - 1, start, gl, a.gamma, carry.x, carry.y);
+            sCarry = carry;
         }
-        sTotal = run;
-    }
-    __syncthreads();
-    {
-        const int ex = incl - packed + sWarpCount[warp];
-        int idx = ex & 0xffff;
-        int trb = ex >> 16;
-#pragma unroll
-        for (int k = 0; k < kGaePerThread; ++k) {
-            if (endMask >> k & 1u) sSeg[idx++] = (own0 + k) | (trb << kPosBits);
-            if (truncMask >> k & 1u) ++trb;
-        }
-    }
-    __syncthreads();
-    const int nSeg = sTotal & 0xffff;
-    const int2 pre = a.pre[blockIdx.x];
-
-    // 3. one thread per segment, backward from its end
-    float accRew = 0.0f, accClipped = 0.0f;
-    for (int s = tid; s < nSeg; s += kGaeThreads) {
-        const int e = sSeg[s];
-        const int endRel = e & kPosMask;
-        const int truncBefore = pre.x + (e >> kPosBits);
-        const int start = s == 0 ? pre.y + 1 : base + (sSeg[s - 1] & kPosMask) + 1;
-        const int stopRel = max(start - base, 0);
-        GaeCarry c{0.0f, 0.0f, 0.0f, 0.0f};
-        float adv, ret;
-        // the segment's end carries its terminal
-        float nextVal = sVal[padIdx(endRel)];
-        gaeStep(a, sRew[padIdx(endRel)], sTerm[endRel], nextVal, sVal[padIdx(endRel + 1)], truncBefore, c, adv, ret);
-        sRew[padIdx(endRel)] = adv;
-        sRet[padIdx(endRel)] = ret;
-        // every earlier step of the segment is running
-#pragma unroll 4
-        for (int rel = endRel - 1; rel >= stopRel; --rel) {
-            const float val = sVal[padIdx(rel)];
-            gaeStepRunning(a, sRew[padIdx(rel)], val, nextVal, c, adv, ret);
-            sRew[padIdx(rel)] = adv;
-            sRet[padIdx(rel)] = ret;
-            nextVal = val;
-        }
-        // a segment that began in an earlier chunk continues in global memory
-        for (int step = base - 1; step >= start; --step) {
-            const float val = __ldg(a.vals + step);
-            gaeStepRunning(a, __ldg(a.rews + step), val, nextVal, c, adv, ret);
-            a.adv[step] = adv;
-            a.ret[step] = ret;
-            a.tgt[step] = val + adv;
-            nextVal = val;
-        }
-        accRew += c.rew;
-        accClipped += c.clipped;
-    }
-    __syncthreads();
-
-    // 4. write back the elements of the segments that end here (coalesced)
-    const int owned = nSeg > 0 ? (sSeg[nSeg - 1] & kPosMask) + 1 : 0;
-#pragma unroll
-    for (int k = 0; k < kGaePerThread; ++k) {
-        const int j = k * kGaeThreads + tid;
-        if (j < owned) {
-            const float adv = sRew[padIdx(j)];
-            a.adv[base + j] = adv;
-            a.ret[base + j] = sRet[padIdx(j)];
-            a.tgt[base + j] = sVal[padIdx(j)] + adv;
-        }
+        __syncthreads();
+        if (mine) gaeStore4<kVec>(a, lo, j, start, kGaeHalo, sD, sR, v);
+        if (start > 0) break;
     }
 
-    // 5. clip-portion sums: block partial, then the last block adds the partials in order
+    // 6. clip-portion sums: block partial, then the last block adds the partials in order
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        accRew += __shfl_xor_sync(0xffffffffu, accRew, o);
-        accClipped += __shfl_xor_sync(0xffffffffu, accClipped, o);
+        accRew += __shfl_xor_sync(all, accRew, o);
+        accExcess += __shfl_xor_sync(all, accExcess, o);
     }
-    if (lane == 0) sWarpSum[warp] = make_float2(accRew, accClipped);
+    if (lane == 0) sWarpSum[warp] = make_float2(accRew, accExcess);
     __syncthreads();
     if (tid == 0) {
         float r = 0.0f, cl = 0.0f;
@@ -446,18 +445,20 @@ __global__ void __launch_bounds__(kGaeThreads) gaeSegmentKernel(GaeArgs a) {
             tr += sWarpSum[w].x;
             tc += sWarpSum[w].y;
         }
-        *a.clipPortion = (tr - tc) / fmaxf(tr, 1e-7f);
+        *a.clipPortion = tc / fmaxf(tr, 1e-7f);
     }
 }
 
-// Per-device scratch, grown on demand (chunk rows + the ticket).
+// Per-device scratch: a slot of chunk rows and a ticket for each stream that calls, so that calls on
+// several streams run side by side; slot 0 is for calls under stream capture.  The slots are
+// allocated together and grown on demand; a stream beyond them takes the slot used longest ago.
+constexpr int kGaeSlots = 16;
 struct GaeScratch {
     int capacity = 0;
-    int2* sum = nullptr;
-    int2* pre = nullptr;
+    int* count = nullptr;     // kGaeSlots rows of `capacity`
     float2* part = nullptr;
     unsigned* ticket = nullptr;
-    bool smemSet = false;
+    unsigned long long stream[kGaeSlots] = {}, used[kGaeSlots] = {}, calls = 0;
 };
 
 std::mutex g_gaeMu;
@@ -473,36 +474,40 @@ struct GaeHostStage {
 };
 std::vector<GaeHostStage> g_gaeHost;
 
-rsb_status ensureScratch(int dev, int nChunks, GaeScratch*& out) {
+rsb_status ensureScratch(int dev, int nChunks, cudaStream_t st, GaeScratch*& out, int& slot) {
     if ((int)g_gaeScratch.size() <= dev) g_gaeScratch.resize(dev + 1);
     GaeScratch& s = g_gaeScratch[dev];
-    if (!s.smemSet) {
-        if (cudaFuncSetAttribute(gaeSegmentKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemSegment) != cudaSuccess ||
-            cudaFuncSetAttribute(gaeSegmentKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemSegment) != cudaSuccess)
-            return RSB_ERR_CUDA;
-        s.smemSet = true;
-    }
     if (s.capacity < nChunks) {
         // the old rows may still be read by work queued earlier on any stream
         if (s.capacity > 0 && cudaDeviceSynchronize() != cudaSuccess) return RSB_ERR_CUDA;
-        cudaFree(s.sum);
-        cudaFree(s.pre);
+        cudaFree(s.count);
         cudaFree(s.part);
-        if (!s.ticket && cudaMalloc(&s.ticket, sizeof(unsigned)) != cudaSuccess) return RSB_ERR_NOMEM;
+        if (!s.ticket && cudaMalloc(&s.ticket, sizeof(unsigned) * kGaeSlots) != cudaSuccess) return RSB_ERR_NOMEM;
         const int cap = nChunks < 64 ? 64 : nChunks;
         s.capacity = 0;
-        s.sum = nullptr;
-        s.pre = nullptr;
+        s.count = nullptr;
         s.part = nullptr;
-        if (cudaMalloc(&s.sum, sizeof(int2) * cap) != cudaSuccess ||
-            cudaMalloc(&s.pre, sizeof(int2) * cap) != cudaSuccess ||
-            cudaMalloc(&s.part, sizeof(float2) * cap) != cudaSuccess)
+        if (cudaMalloc(&s.count, sizeof(int) * cap * kGaeSlots) != cudaSuccess ||
+            cudaMalloc(&s.part, sizeof(float2) * cap * kGaeSlots) != cudaSuccess)
             return RSB_ERR_NOMEM;
         s.capacity = cap;
     }
     out = &s;
+    slot = 0;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) return RSB_ERR_CUDA;
+    if (capture != cudaStreamCaptureStatusNone) return RSB_OK;
+    unsigned long long id = 0;
+    if (cudaStreamGetId(st, &id) != cudaSuccess) return RSB_ERR_CUDA;
+    int oldest = 1;
+    for (slot = 1; slot < kGaeSlots && !(s.used[slot] && s.stream[slot] == id); ++slot)
+        if (s.used[slot] < s.used[oldest]) oldest = slot;
+    if (slot == kGaeSlots) {
+        slot = oldest;
+        if (s.used[slot] && cudaDeviceSynchronize() != cudaSuccess) return RSB_ERR_CUDA;
+        s.stream[slot] = id;
+    }
+    s.used[slot] = ++s.calls;
     return RSB_OK;
 }
 
@@ -517,7 +522,8 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     if (cudaGetDevice(&dev) != cudaSuccess) return RSB_ERR_CUDA;
     const int nChunks = (T + kGaeChunk - 1) / kGaeChunk;
     GaeScratch* s = nullptr;
-    const rsb_status rc = ensureScratch(dev, nChunks, s);
+    int slot = 0;
+    const rsb_status rc = ensureScratch(dev, nChunks, st, s, slot);
     if (rc != RSB_OK) return rc;
     GaeArgs a;
     a.rews = rews;
@@ -535,16 +541,34 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     a.lambda = p.lambda;
     a.returnStd = p.return_std;
     a.clipRange = p.clip_range;
-    a.pre = s->pre;
-    a.part = s->part;
-    a.ticket = s->ticket;
-    const bool vec = (reinterpret_cast<uintptr_t>(terminals) & 15) == 0;
-    if (vec) gaeSummaryKernel<true><<<nChunks, kGaeThreads, 0, st>>>(terminals, T, s->sum);
-    else gaeSummaryKernel<false><<<nChunks, kGaeThreads, 0, st>>>(terminals, T, s->sum);
-    gaeScanKernel<<<1, 1024, 0, st>>>(s->sum, nChunks, s->pre);
-    if (cudaMemsetAsync(s->ticket, 0, sizeof(unsigned), st) != cudaSuccess) return RSB_ERR_CUDA;
-    if (vec) gaeSegmentKernel<true><<<nChunks, kGaeThreads, kSmemSegment, st>>>(a);
-    else gaeSegmentKernel<false><<<nChunks, kGaeThreads, kSmemSegment, st>>>(a);
+    int* const count = s->count + (size_t)slot * s->capacity;
+    a.part = s->part + (size_t)slot * s->capacity;
+    a.ticket = s->ticket + slot;
+    a.count = numTruncs > 0 ? count : nullptr;
+    a.counted = nChunks > kGaeDirect;
+    auto aligned = [](const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; };
+    if (a.count) {
+        if (aligned(terminals, 16)) gaeSummaryKernel<true><<<nChunks, kGaeThreads, 0, st>>>(terminals, T, count, a.ticket);
+        else gaeSummaryKernel<false><<<nChunks, kGaeThreads, 0, st>>>(terminals, T, count, a.ticket);
+        if (a.counted) gaeScanKernel<<<1, 1024, 0, st>>>(count, nChunks);
+    } else if (cudaMemsetAsync(a.ticket, 0, sizeof(unsigned), st) != cudaSuccess) {
+        return RSB_ERR_CUDA;
+    }
+    // four elements to a load and a store where every row allows it
+    const bool vec = aligned(terminals, 4) && aligned(rews, 16) && aligned(valPreds, 16) && aligned(advantages, 16) &&
+                     aligned(targetValues, 16) && aligned(returns, 16);
+    // it may start while the kernel before it runs: that kernel's results are read after a wait
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nChunks);
+    cfg.blockDim = dim3(kGaeThreads);
+    cfg.stream = st;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = a.count ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, vec ? gaeSegmentKernel<true> : gaeSegmentKernel<false>, a) != cudaSuccess)
+        return RSB_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? RSB_OK : RSB_ERR_CUDA;
 }
 
