@@ -124,14 +124,15 @@ __global__ void __launch_bounds__(1024) gaeScanKernel(int* __restrict__ count, i
 }
 
 __device__ __forceinline__ int8_t termOf(unsigned w, int c) { return (int8_t)(w >> (8 * c)); }
+// Bit c of the result: byte c of a comparison's mask (0 or 255).
+__device__ __forceinline__ unsigned bytesToBits(unsigned mask) { return (mask & 0x01010101u) * 0x01020408u >> 24 & 15u; }
 
-// The reward as the advantages use it.  Adds its magnitude, and what clipping took of it, which the
-// reference leaves at all of it without standardisation; summed apart, the small excess keeps the
-// digits that the difference of two large sums would lose.
+// The reward as the advantages use it.  Adds its magnitude and what clipping took of it; summed
+// apart, the small excess keeps the digits that the difference of two large sums would lose.
+template <bool kScaled>
 __device__ __forceinline__ float gaeReward(const GaeArgs& a, float rew, float& sum, float& excess) {
-    if (!(a.returnStd > 0.0f)) {
+    if (!kScaled) {
         sum += fabsf(rew);
-        excess += fabsf(rew);
         return rew;
     }
     const float r = rew / a.returnStd;
@@ -143,33 +144,36 @@ __device__ __forceinline__ float gaeReward(const GaeArgs& a, float rew, float& s
 }
 
 // The recurrence of GAECuda.cu:77-113 over rows [stop, end], backward.  Its rows hold what does not
-// depend on later steps (sD the delta, sR the reward), four read ahead of the chain; they take the
-// advantages and the returns.  A segment's last step starts from zero carries, so that the factors
-// (1 - done)(1 - trunc), which are 1 at every other step, need not be applied.
+// depend on later steps (sD the delta, sR the reward), an aligned four of them read ahead of the
+// chain; they take the advantages and the returns.  A segment's last step starts from zero carries,
+// so that the factors (1 - done)(1 - trunc), which are 1 at every other step, need not be applied.
 __device__ __forceinline__ void gaeWalk(float* sD, float* sR, int end, int stop, float gl, float gamma, float& adv,
                                         float& ret) {
+    auto one = [&](int at) {
+        ret = sR[at] + ret * gamma;
+        adv = sD[at] + gl * adv;
+        sD[at] = adv;
+        sR[at] = ret;
+    };
     int rel = end;
+    for (; rel >= stop && (rel & 3) != 3; --rel) one(padIdx(rel));
     for (; rel - 3 >= stop; rel -= 4) {
+        const int at = padIdx(rel - 3);
         float d[4], r[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            d[k] = sD[padIdx(rel - k)];
-            r[k] = sR[padIdx(rel - k)];
+            d[k] = sD[at + k];
+            r[k] = sR[at + k];
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 3; k >= 0; --k) {
             ret = r[k] + ret * gamma;
             adv = d[k] + gl * adv;
-            sD[padIdx(rel - k)] = adv;
-            sR[padIdx(rel - k)] = ret;
+            sD[at + k] = adv;
+            sR[at + k] = ret;
         }
     }
-    for (; rel >= stop; --rel) {
-        ret = sR[padIdx(rel)] + ret * gamma;
-        adv = sD[padIdx(rel)] + gl * adv;
-        sD[padIdx(rel)] = adv;
-        sR[padIdx(rel)] = ret;
-    }
+    for (; rel >= stop; --rel) one(padIdx(rel));
 }
 
 // Elements j .. j + 3 of a row, zero from len on.
@@ -200,11 +204,12 @@ template <bool kVec>
 __device__ __forceinline__ void gaeStore4(const GaeArgs& a, int base, int j, int from, int to, const float* sD,
                                           const float* sR, const float* val) {
     if (j >= to || j + 4 <= from) return;
+    const int at = padIdx(j);
     float d[4], r[4], g[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        d[c] = sD[padIdx(j + c)];
-        r[c] = sR[padIdx(j + c)];
+        d[c] = sD[at + c];
+        r[c] = sR[at + c];
         g[c] = val[c] + d[c];
     }
     if (kVec && j >= from && j + 4 <= to) {
@@ -224,14 +229,18 @@ __device__ __forceinline__ void gaeStore4(const GaeArgs& a, int base, int j, int
 
 // One block per chunk.  What a step needs besides the carries (reward, delta) is computed for every
 // element in parallel, in the threads that loaded it, four elements to a load; a thread then walks
-// each segment that ends among 16 elements of its own, two multiplies and two adds a step; the
+// each segment that ends among 32 elements of its own, two multiplies and two adds a step; the
 // threads that hold the values write the results.  A segment that began in an earlier chunk goes on
 // through windows of kGaeHalo elements, staged and written by the whole block and walked by one
 // thread.
 //
-// The buffer is bound by its bytes (9 read, 12 written per element) as long as segments are short
-// against a chunk, else by the walk's chain.
-template <bool kVec>
+// What bounds it: 393,216 x 32 elements (266 MB, 41 us at the rate of a copy) take 64 us in calls
+// side by side, against 77 us with bounds, terminals and padding worked out for every element and 81
+// us with the arithmetic in the walk as well; the rest is instructions and the waits between the
+// phases.  More blocks on a multiprocessor do not shorten it (five or six of 48 or 40 registers: 77
+// and 81 us before those instructions went).  257 episodes of 400 uneven steps: 10 us, against 23 us
+// when a segment went on through global memory step by step.
+template <bool kVec, bool kScaled>
 __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
     __shared__ float sD[kPadded], sR[kPadded];
     __shared__ unsigned sEnd[kGaeWords], sTrunc[kGaeWords];  // a bit per element: ends of segments, truncations
@@ -252,6 +261,7 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
     //    element) and of the truncations; truncations before the chunk
     float rew[4][4], val[4][4], after[4];
     unsigned term[4];
+    if (tid < kGaeWords) sEnd[tid] = sTrunc[tid] = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int j = 4 * (k * kGaeThreads + tid);
@@ -270,27 +280,19 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
     }
     before = warpSum(before);
     if (lane == 0) sCount[warp] = before;
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int j = 4 * (k * kGaeThreads + tid);
         const float first = __shfl_down_sync(all, val[k][0], 1);
         if (lane != 31) after[k] = first;
-        unsigned ends = 0, truncs = 0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int8_t t = termOf(term[k], c);
-            if (j + c < len && (t != 0 || (lastChunk && j + c == len - 1))) ends |= 1u << c;
-            if (t == kTermTruncated) truncs |= 1u << c;
-        }
-        unsigned e = ends << (4 * (lane & 7)), r = truncs << (4 * (lane & 7));
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            e |= __shfl_xor_sync(all, e, o);
-            r |= __shfl_xor_sync(all, r, o);
-        }
-        if ((lane & 7) == 0) {
-            sEnd[j >> 5] = e;
-            sTrunc[j >> 5] = r;
+        // elements past the buffer have terminals of 0
+        unsigned ends = bytesToBits(__vcmpne4(term[k], 0));
+        if (lastChunk && j >> 2 == (len - 1) >> 2) ends |= 1u << ((len - 1) & 3);
+        if (ends) {
+            atomicOr(&sEnd[j >> 5], ends << (j & 31));
+            const unsigned truncs = bytesToBits(__vcmpeq4(term[k], 0x01010101u * kTermTruncated));
+            if (truncs) atomicOr(&sTrunc[j >> 5], truncs << (j & 31));
         }
     }
     __syncthreads();
@@ -313,14 +315,13 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
     }
     __syncthreads();
 
-    // 2. reward and delta of every element
+    // 2. reward and delta of every element (past the buffer: zeros)
     float accRew = 0.0f, accExcess = 0.0f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int j = 4 * (k * kGaeThreads + tid);
+        const int j = 4 * (k * kGaeThreads + tid), at = padIdx(4 * tid) + k * padIdx(4 * kGaeThreads);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if (j + c >= len) break;
             const int8_t t = termOf(term[k], c);
             float next = c < 3 ? val[k][c < 3 ? c + 1 : 3] : after[k];
             if (t == kTermNormal) next = 0.0f;
@@ -330,18 +331,18 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
                 // a count that does not match the truncated steps reads nothing out of range
                 next = idx >= 0 && idx < a.numTruncs ? __ldg(a.truncVals + idx) : 0.0f;
             }
-            const float done = t == kTermNormal ? 1.0f : 0.0f;
-            const float r = gaeReward(a, rew[k][c], accRew, accExcess);
-            sD[padIdx(j + c)] = (r + a.gamma * next * (1.0f - done)) - val[k][c];
-            sR[padIdx(j + c)] = rew[k][c];
+            const float r = gaeReward<kScaled>(a, rew[k][c], accRew, accExcess);
+            sD[at + c] = (r + a.gamma * next) - val[k][c];
+            sR[at + c] = rew[k][c];
         }
     }
+    if (!kScaled) accExcess = accRew;
     __syncthreads();
 
-    // 3. a thread per 16 elements, backward from each end among them
+    // 3. a thread per 32 elements, backward from each end among them
     const float gl = a.gamma * a.lambda;
-    for (unsigned ends = sEnd[tid >> 1] >> (16 * (tid & 1)) & 0xffffu; ends; ends &= ends - 1u) {
-        const int end = kGaePerThread * tid + __ffs((int)ends) - 1;
+    for (unsigned ends = tid < kGaeWords ? sEnd[tid] : 0u; ends; ends &= ends - 1u) {
+        const int end = 32 * tid + __ffs((int)ends) - 1;
         int w = end >> 5;
         unsigned earlier = sEnd[w] & ((1u << (end & 31)) - 1u);
         while (!earlier && w > 0) earlier = sEnd[--w];
@@ -389,8 +390,8 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
             v[4] = __ldg(a.vals + lo + j + 4);  // lo + j + 4 <= base
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                sD[padIdx(j + c)] = (gaeReward(a, r[c], sum, sum) + a.gamma * v[c + 1] * (1.0f - 0.0f)) - v[c];
-                sR[padIdx(j + c)] = r[c];
+                sD[padIdx(j) + c] = (gaeReward<kScaled>(a, r[c], sum, sum) + a.gamma * v[c + 1]) - v[c];
+                sR[padIdx(j) + c] = r[c];
             }
         }
         __syncthreads();
@@ -557,6 +558,8 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     // four elements to a load and a store where every row allows it
     const bool vec = aligned(terminals, 4) && aligned(rews, 16) && aligned(valPreds, 16) && aligned(advantages, 16) &&
                      aligned(targetValues, 16) && aligned(returns, 16);
+    const auto kernel = p.return_std > 0.0f ? (vec ? gaeSegmentKernel<true, true> : gaeSegmentKernel<false, true>)
+                                            : (vec ? gaeSegmentKernel<true, false> : gaeSegmentKernel<false, false>);
     // it may start while the kernel before it runs: that kernel's results are read after a wait
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -567,7 +570,7 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     cfg.stream = st;
     cfg.attrs = &overlap;
     cfg.numAttrs = a.count ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, vec ? gaeSegmentKernel<true> : gaeSegmentKernel<false>, a) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, kernel, a) != cudaSuccess)
         return RSB_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? RSB_OK : RSB_ERR_CUDA;
 }
