@@ -354,7 +354,7 @@ def run_ours(args, rank, world, dist):
 
         value, total_ms, _, queries = timed(steps, clocks, _Replay)
         step_times = kernel_steps
-        extra["graph"] = {"api": "rsb_env_graph_capture / rsb_env_graph_launch", "launches_per_replay": 6,
+        extra["graph"] = {"api": "rsb_env_graph_capture / rsb_env_graph_launch", "launches_per_replay": 5 + (1 if wl.num_arenas <= 2048 else 12 * wl.tick_skip),
                           "note": "action sampling (torch) launched outside the graph"}
         ex_value = value
     else:
@@ -538,10 +538,8 @@ def run_ours(args, rank, world, dist):
     # roofline of the step kernel (the dominant launch): algorithmic bytes = persistent
     # state read + written per launch (the library reports it), over the kernel's own time
     alg_bytes = batch.stats()["state_bytes_per_step"]
-    # DRAM traffic of a settled 3v3 step-kernel launch, measured by ncu on 8,192 arenas
-    # (dram__bytes_read.sum + dram__bytes_write.sum = 58,409 B per arena, the threads' local
-    # memory), scaled by the arenas; no capture exists for other team sizes
-    traffic = 58409 * wl.num_arenas if (wl.team_size == 3 and not wl.mixed) else None
+    # one launch for all phases and ticks of a small batch, else a launch per phase and tick
+    step_launches = 1 if wl.num_arenas <= 2048 else 12 * wl.tick_skip
     kernel_s = statistics.mean(step_times) / 1e3
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / kernel_s / 1e9
@@ -553,16 +551,14 @@ def run_ours(args, rank, world, dist):
         "warmup": args.warmup, "ms_per_step": total_ms / steps, "higher_is_better": True,
         "scaling": "strong" if wl.strong else "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded random states)", "config": cfg,
-        "roofline": {"bound": "hbm", "kernel": "stepKernel", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                     "traffic_source": "ncu dram bytes of a settled 3v3 x 8192 launch, scaled by arenas"
-                     if traffic else None,
+        "roofline": {"bound": "hbm", "kernel": "the step's phases (stepBlockKernel up to 2,048 arenas)", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                     "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
                      "bytes_per_launch": alg_bytes, "kernel_ms": kernel_s * 1e3,
                      "kernel_share": statistics.mean(step_times) / (total_ms / steps)},
         "e2e": {"value": e2e_value, "unit": "arena-ticks/s", "h2d_bytes_per_step": int(statistics.mean(h2d)),
                 "d2h_bytes_per_step": int(statistics.mean(d2h))},
-        # per env step: action expansion, (culler,) step, obs + masks, rewards + terminals, reset
-        "gpu_launches": steps * ((6 if learned is not None else 5) + (1 if wl.graph else 0)),
+        # per env step: action expansion, (culler,) the step's phases, obs + masks, rewards + terminals, reset
+        "gpu_launches": steps * ((5 if learned is not None else 4) + step_launches + (1 if wl.graph else 0)),
         "learned_cull": learned,
         "state_ring": ring,
         "ball_prediction": pred,
@@ -936,12 +932,11 @@ def run_gae(args, rank, world, dist, steps, warmup, reference_device=False):
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (ms / 1e3) / 1e9
     res = {"value": T * world / (ms / 1e3), "unit": "elements/s", "ms_per_call": ms, "elements": T,
-           "roofline": {"bound": "hbm", "kernel": "gaeSegmentKernel (+ summary and scan)", "achieved": achieved,
+           "roofline": {"bound": "hbm", "kernel": "gaeSegmentKernel (+ summary)", "achieved": achieved,
                         "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                        # ncu dram__bytes_read.sum + write.sum of gaeSegmentKernel on this buffer
-                        "traffic": 213854464 if T == GAE_PLAYERS * GAE_STEPS else None,
+                        "traffic": None,
                         "peak_kind": peak_kind, "bytes_per_call": alg_bytes},
-           "gpu_launches": 3 * steps, "clocks": cs.summary()}
+           "gpu_launches": 2 * steps, "clocks": cs.summary()}
     if not reference_device:
         # e2e through the host entry point: copies in, kernels, copies out
         e2e = []
