@@ -13,7 +13,7 @@
 
 namespace rsb {
 
-constexpr int BALL_LIST = 128;         // triangles a list holds
+constexpr int BALL_LIST = 96;          // triangles a list holds
 constexpr int BALL_LIST_NONE = -1;     // not made yet
 constexpr int BALL_LIST_OVER = -2;     // more triangles than it holds: the meshes are queried
 constexpr float BALL_MARGIN = 2.f;      // Bullet units (100 uu: two ticks of flight at the top speed)

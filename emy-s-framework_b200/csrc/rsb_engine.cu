@@ -413,9 +413,11 @@ __device__ __noinline__ int warpBallList(const EngineView& D, V3 at, V3 mn, V3 m
 // PRED_WARPS * SMs * 32 balls on: narrower warps spread the contacts, but each holds its own lines
 // of local memory and of code.  16,384 balls, 360 ticks, three such calls side by side, with 2, 4,
 // 8, 16, 32 and 64 warps per SM: 5.7, 6.0, 7.4, 9.5, 12.1 and 17.0 ms each; 1,024 balls with 2, 4
-// and 8: 1.1, 1.3 and 1.7 ms.  One thread per ball on the general tick, whose arena lies in local
-// memory, took 17.0 ms; this takes 5.1 ms.
-constexpr int PRED_THREADS = 64, PRED_WARPS = 2;
+// and 8: 1.1, 1.3 and 1.7 ms.  Those were blocks of two warps.  Warps that share a multiprocessor
+// share its fetched code: blocks of one, two and four warps take 8.4, 5.1 and 3.5 ms for the 16,384
+// balls (four are as many as static shared memory holds lists for).  One thread per ball on the
+// general tick, whose arena lies in local memory, took 17.0 ms.
+constexpr int PRED_THREADS = 128, PRED_WARPS = 2;
 __global__ void __launch_bounds__(PRED_THREADS) predictBallKernel(const __grid_constant__ EngineView D, PredSlices s,
                                                                   rsb_ball_state* out, int width) {
     __shared__ uint16_t lists[PRED_THREADS][BALL_LIST], hits[PRED_THREADS][BALL_LIST];
