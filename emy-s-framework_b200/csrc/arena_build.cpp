@@ -545,6 +545,7 @@ bool buildArenaStatic(const std::string& folder, ArenaStaticHost& out) {
 
     S.triInfo = out.triInfo.data();
     S.bpCells = out.bpCells.data();
+    for (uint32_t c : out.bpCells) out.cellStatics = std::max(out.cellStatics, __builtin_popcount(c));
 
     // ---- mesh occupancy grid (see ArenaStatic::occ): 64 uu voxels over the arena, a mesh bit each
     {

@@ -16,6 +16,7 @@ struct ArenaStaticHost {
     std::vector<BvhNode> leaves;
     std::vector<TriEdgeInfo> triInfo;
     std::vector<uint32_t> bpCells;
+    int cellStatics = 0;  // the most static objects in a cell of bpCells
     std::vector<uint16_t> occ, occAhead;
     std::vector<uint32_t> voxOff, voxList;
     std::vector<uint16_t> occDist;

@@ -63,8 +63,7 @@ enum : int {
     QC_WORDS
 };
 constexpr int NUM_TASK_TYPES = 4;  // QC_CARMESH .. QC_CARCAR
-// The most pairs of each type that an arena can have, and contact blocks (MAX_BLOCKS manifolds
-// hold contacts in one tick; more are dropped, as in the one-thread tick).
+// The most pairs of each type that an arena can have.
 constexpr int CAP_CARMESH = MAX_CARS * MAX_MESHES, CAP_BALLMESH = MAX_MESHES, CAP_CARBALL = MAX_CARS,
               CAP_CARCAR = MAX_CARS * (MAX_CARS - 1) / 2, CAP_PLANE = MAX_BODIES * NUM_PLANES;
 constexpr int CAP_RESULTS = CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL + CAP_CARCAR + CAP_PLANE;
@@ -75,6 +74,12 @@ RSB_HD int resultBase(int type) {  // per arena: first result of the type
          : type == QC_CARCAR ? CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL
                              : CAP_CARMESH + CAP_BALLMESH + CAP_CARBALL + CAP_CARCAR;
 }
+// ... and the most that can hold contacts in one tick, where a broadphase cell has at most
+// `cellStatics` static objects: a body's pairs with static objects are those of one cell.  The point
+// pool has a place for each.  Of an arena's manifolds with contacts the first MAX_BLOCKS in dispatch
+// order keep them (solveCallbacks, as the one-thread tick), but the points are stored as the pairs
+// finish, in any order and side by side with other arenas'.
+RSB_HD int contactPairs(int cars, int cellStatics) { return (1 + cars) * cellStatics + cars * (cars + 1) / 2; }
 
 struct PairTask {
     uint32_t a;
@@ -125,8 +130,8 @@ struct StepTemp {
     uint32_t* rayQ;      // rays near meshes [4 * MAX_CARS * N], then as many places for the others
     PairTask* tasks;     // per type, [cap * N], at resultBase(type) * N
     PairResult* results;
-    MPoint* blocks;      // [MAX_BLOCKS * N][MAX_POINTS]
-    uint32_t blockCap;
+    MPoint* blocks;      // [blockCap][MAX_POINTS]
+    uint32_t blockCap, arenaBlocks;  // places in all, and to an arena
     uint32_t* solveQ;    // arenas with pairs of bodies [N]
     uint32_t* bodyQ;     // bodies with contacts in the others, b * N + a [MAX_BODIES * N]
     uint32_t* first;     // first candidate of each pair and their number << 26, as results
@@ -994,7 +999,7 @@ RSB_HD void storePair(const EngineView& D, const StepTemp& T, int a, WT& W, cons
             MPoint* dst = T.blocks + (size_t)MAX_POINTS * r.block;
             for (int k = 0; k < m.n; k++) dst[k] = m.pt[k];
         } else {
-            r.n = 0;  // more blocks than the whole batch may hold: the contacts are dropped
+            r.n = 0;  // out of range: the pool has a place for every pair
             r.block = r.flags = 0;
             W.status |= WS_OVERFLOW;
         }

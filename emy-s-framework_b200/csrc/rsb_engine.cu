@@ -572,7 +572,8 @@ static bool allocStep(rsb_handle* h) {
         p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(h->dStep + off);
         off += count * sizeof(*p);
     };
-    T.blockCap = (uint32_t)(MAX_BLOCKS * N);
+    T.arenaBlocks = (uint32_t)std::max(1, contactPairs(h->maxCars, h->host->cellStatics));
+    T.blockCap = T.arenaBlocks * (uint32_t)N;
     T.candCap = (uint32_t)(CAP_CANDIDATES * N);
     for (int pass = 0; pass < 2; pass++) {
         off = 0;

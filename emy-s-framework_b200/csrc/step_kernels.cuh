@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) stepBlockKernel(const __grid
     StepTemp T = T0;
     T.count = count;
     T.candCap = (uint32_t)(CAP_CANDIDATES * (a0 + n));
-    T.blockCap = (uint32_t)(MAX_BLOCKS * (a0 + n));
+    T.blockCap = T.arenaBlocks * (uint32_t)(a0 + n);
     if (tid == 0) {
         base[QC_RAY] = base[QC_BODYRAY] = (uint32_t)(4 * MAX_CARS * a0);
         base[QC_CARMESH] = (uint32_t)(CAP_CARMESH * a0);
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) stepBlockKernel(const __grid
         base[QC_CARBALL] = (uint32_t)(CAP_CARBALL * a0);
         base[QC_CARCAR] = (uint32_t)(CAP_CARCAR * a0);
         base[QC_PLANE] = (uint32_t)(CAP_PLANE * a0);
-        base[QC_BLOCK] = (uint32_t)(MAX_BLOCKS * a0);
+        base[QC_BLOCK] = T.arenaBlocks * (uint32_t)a0;
         base[QC_SOLVE] = (uint32_t)a0;
         base[QC_BODY] = (uint32_t)(MAX_BODIES * a0);
         base[QC_TRI] = (uint32_t)(CAP_CANDIDATES * a0);
