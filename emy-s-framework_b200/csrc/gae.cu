@@ -450,10 +450,105 @@ __global__ void __launch_bounds__(kGaeThreads, 4) gaeSegmentKernel(GaeArgs a) {
     }
 }
 
-// Per-device scratch: a slot of chunk rows and a ticket for each stream that calls, so that calls on
-// several streams run side by side; slot 0 is for calls under stream capture.  The slots are
-// allocated together and grown on demand; a stream beyond them takes the slot used longest ago.
-constexpr int kGaeSlots = 16;
+// What a call works in: a row of counts, a row of partial sums and a ticket, in one allocation.
+struct GaeRows {
+    int capacity = 0;  // chunks
+    int* count = nullptr;
+    float2* part = nullptr;
+    unsigned* ticket = nullptr;
+};
+bool allocRows(int nChunks, GaeRows& r) {
+    const size_t cap = (size_t)(nChunks < 64 ? 64 : nChunks);
+    char* p = nullptr;
+    if (cudaMalloc(&p, (sizeof(float2) + sizeof(int)) * cap + sizeof(unsigned)) != cudaSuccess) return false;
+    r.capacity = (int)cap;
+    r.part = reinterpret_cast<float2*>(p);
+    r.count = reinterpret_cast<int*>(r.part + cap);
+    r.ticket = reinterpret_cast<unsigned*>(r.count + cap);
+    return true;
+}
+
+// Allocations that this thread makes while a stream is captured are not part of the capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// The rows of a captured call belong to the graph it is captured into: replays of two graphs, or of
+// two calls in one, may run side by side, and at any time while the graph lives.  The graph and its
+// executables give them back when the last of them is gone; a later capture takes them again, and
+// what is more than kGaeReturned is freed by the next call that is not captured.
+constexpr size_t kGaeReturned = 16;
+struct GaeGraphRows {
+    int dev;
+    GaeRows rows;
+};
+struct GaeReturnedRows {
+    std::mutex mu;
+    std::vector<GaeGraphRows*> list;
+};
+GaeReturnedRows& gaeReturned() {
+    static GaeReturnedRows* r = new GaeReturnedRows;  // graphs may be destroyed as late as at exit
+    return *r;
+}
+void CUDART_CB gaeGiveBack(void* p) {  // may call nothing of CUDA
+    GaeReturnedRows& r = gaeReturned();
+    std::lock_guard<std::mutex> lock(r.mu);
+    r.list.push_back(static_cast<GaeGraphRows*>(p));
+}
+rsb_status rowsForGraph(int dev, int nChunks, cudaGraph_t graph, GaeRows& out) {
+    GaeReturnedRows& r = gaeReturned();
+    GaeGraphRows* g = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(r.mu);
+        for (size_t i = 0; i < r.list.size() && !g; ++i)
+            if (r.list[i]->dev == dev && r.list[i]->rows.capacity >= nChunks) {
+                g = r.list[i];
+                r.list.erase(r.list.begin() + (ptrdiff_t)i);
+            }
+    }
+    if (!g) {
+        RelaxedCapture relaxed;
+        g = new GaeGraphRows{dev, {}};
+        if (!allocRows(nChunks, g->rows)) {
+            delete g;
+            return RSB_ERR_NOMEM;
+        }
+    }
+    out = g->rows;
+    cudaUserObject_t owner = nullptr;
+    if (cudaUserObjectCreate(&owner, g, gaeGiveBack, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        gaeGiveBack(g);
+        return RSB_ERR_CUDA;
+    }
+    if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaUserObjectRelease(owner, 1);
+        return RSB_ERR_CUDA;
+    }
+    return RSB_OK;
+}
+void freeReturnedRows() {
+    GaeReturnedRows& r = gaeReturned();
+    std::vector<GaeGraphRows*> over;
+    {
+        std::lock_guard<std::mutex> lock(r.mu);
+        while (r.list.size() > kGaeReturned) {
+            over.push_back(r.list.back());
+            r.list.pop_back();
+        }
+    }
+    for (GaeGraphRows* g : over) {
+        RelaxedCapture relaxed;
+        cudaFree(g->rows.part);
+        delete g;
+    }
+}
+
+// Per-device scratch of the other calls: a slot of chunk rows and a ticket for each stream that calls,
+// so that calls on several streams run side by side.  The slots are allocated together and grown on
+// demand; a stream beyond them takes the slot used longest ago.
+constexpr int kGaeSlots = 15;
 struct GaeScratch {
     int capacity = 0;
     int* count = nullptr;     // kGaeSlots rows of `capacity`
@@ -475,7 +570,8 @@ struct GaeHostStage {
 };
 std::vector<GaeHostStage> g_gaeHost;
 
-rsb_status ensureScratch(int dev, int nChunks, cudaStream_t st, GaeScratch*& out, int& slot) {
+rsb_status rowsForStream(int dev, int nChunks, cudaStream_t st, GaeRows& out) {
+    freeReturnedRows();
     if ((int)g_gaeScratch.size() <= dev) g_gaeScratch.resize(dev + 1);
     GaeScratch& s = g_gaeScratch[dev];
     if (s.capacity < nChunks) {
@@ -493,15 +589,11 @@ rsb_status ensureScratch(int dev, int nChunks, cudaStream_t st, GaeScratch*& out
             return RSB_ERR_NOMEM;
         s.capacity = cap;
     }
-    out = &s;
-    slot = 0;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) return RSB_ERR_CUDA;
-    if (capture != cudaStreamCaptureStatusNone) return RSB_OK;
+    int slot = 0;
     unsigned long long id = 0;
     if (cudaStreamGetId(st, &id) != cudaSuccess) return RSB_ERR_CUDA;
-    int oldest = 1;
-    for (slot = 1; slot < kGaeSlots && !(s.used[slot] && s.stream[slot] == id); ++slot)
+    int oldest = 0;
+    for (slot = 0; slot < kGaeSlots && !(s.used[slot] && s.stream[slot] == id); ++slot)
         if (s.used[slot] < s.used[oldest]) oldest = slot;
     if (slot == kGaeSlots) {
         slot = oldest;
@@ -509,6 +601,9 @@ rsb_status ensureScratch(int dev, int nChunks, cudaStream_t st, GaeScratch*& out
         s.stream[slot] = id;
     }
     s.used[slot] = ++s.calls;
+    out.count = s.count + (size_t)slot * s.capacity;
+    out.part = s.part + (size_t)slot * s.capacity;
+    out.ticket = s.ticket + slot;
     return RSB_OK;
 }
 
@@ -522,9 +617,14 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return RSB_ERR_CUDA;
     const int nChunks = (T + kGaeChunk - 1) / kGaeChunk;
-    GaeScratch* s = nullptr;
-    int slot = 0;
-    const rsb_status rc = ensureScratch(dev, nChunks, st, s, slot);
+    GaeRows rows;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(st, &capture, nullptr, &graph) != cudaSuccess ||
+        capture == cudaStreamCaptureStatusInvalidated)
+        return RSB_ERR_CUDA;
+    const rsb_status rc =
+        capture == cudaStreamCaptureStatusActive ? rowsForGraph(dev, nChunks, graph, rows) : rowsForStream(dev, nChunks, st, rows);
     if (rc != RSB_OK) return rc;
     GaeArgs a;
     a.rews = rews;
@@ -542,9 +642,9 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     a.lambda = p.lambda;
     a.returnStd = p.return_std;
     a.clipRange = p.clip_range;
-    int* const count = s->count + (size_t)slot * s->capacity;
-    a.part = s->part + (size_t)slot * s->capacity;
-    a.ticket = s->ticket + slot;
+    int* const count = rows.count;
+    a.part = rows.part;
+    a.ticket = rows.ticket;
     a.count = numTruncs > 0 ? count : nullptr;
     a.counted = nChunks > kGaeDirect;
     auto aligned = [](const void* p, uintptr_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; };
