@@ -457,14 +457,13 @@ struct GaeRows {
     float2* part = nullptr;
     unsigned* ticket = nullptr;
 };
-bool allocRows(int nChunks, GaeRows& r) {
+// `sets` of them, one after another; `first` is the first one.
+bool allocRows(int nChunks, int sets, GaeRows& first) {
     const size_t cap = (size_t)(nChunks < 64 ? 64 : nChunks);
-    char* p = nullptr;
-    if (cudaMalloc(&p, (sizeof(float2) + sizeof(int)) * cap + sizeof(unsigned)) != cudaSuccess) return false;
-    r.capacity = (int)cap;
-    r.part = reinterpret_cast<float2*>(p);
-    r.count = reinterpret_cast<int*>(r.part + cap);
-    r.ticket = reinterpret_cast<unsigned*>(r.count + cap);
+    if (cudaMalloc(&first.part, ((sizeof(float2) + sizeof(int)) * cap + sizeof(unsigned)) * sets) != cudaSuccess) return false;
+    first.capacity = (int)cap;
+    first.count = reinterpret_cast<int*>(first.part + cap * sets);
+    first.ticket = reinterpret_cast<unsigned*>(first.count + cap * sets);
     return true;
 }
 
@@ -511,7 +510,7 @@ rsb_status rowsForGraph(int dev, int nChunks, cudaGraph_t graph, GaeRows& out) {
     if (!g) {
         RelaxedCapture relaxed;
         g = new GaeGraphRows{dev, {}};
-        if (!allocRows(nChunks, g->rows)) {
+        if (!allocRows(nChunks, 1, g->rows)) {
             delete g;
             return RSB_ERR_NOMEM;
         }
@@ -545,16 +544,23 @@ void freeReturnedRows() {
     }
 }
 
-// Per-device scratch of the other calls: a slot of chunk rows and a ticket for each stream that calls,
-// so that calls on several streams run side by side.  The slots are allocated together and grown on
-// demand; a stream beyond them takes the slot used longest ago.
-constexpr int kGaeSlots = 15;
+// Per-device scratch of the other calls, never waited for on the host: rows for each stream that
+// calls, so that calls on several streams run side by side.  The first kGaeOwn streams keep theirs.
+// Beyond them a stream takes, of kGaeShared rows, those used longest ago, and its work waits on the
+// device for the call that had them (an event is recorded after each call in these).  The rows of all
+// are allocated together; a longer buffer makes new ones at least twice as long, which a slot takes
+// when it needs them, and the old ones stay, since work may still use them (all together are at most
+// twice the last).
+constexpr int kGaeOwn = 16, kGaeShared = 8;
+struct GaeSlot {
+    unsigned long long stream = 0, used = 0;  // id of the stream, number of its last call (0: none)
+    GaeRows rows;
+    cudaEvent_t done = nullptr;  // shared slots
+};
 struct GaeScratch {
-    int capacity = 0;
-    int* count = nullptr;     // kGaeSlots rows of `capacity`
-    float2* part = nullptr;
-    unsigned* ticket = nullptr;
-    unsigned long long stream[kGaeSlots] = {}, used[kGaeSlots] = {}, calls = 0;
+    GaeSlot slot[kGaeOwn + kGaeShared];
+    GaeRows rows;  // the first slot's of the last allocation
+    unsigned long long calls = 0;
 };
 
 std::mutex g_gaeMu;
@@ -570,40 +576,37 @@ struct GaeHostStage {
 };
 std::vector<GaeHostStage> g_gaeHost;
 
-rsb_status rowsForStream(int dev, int nChunks, cudaStream_t st, GaeRows& out) {
+rsb_status slotForStream(int dev, int nChunks, cudaStream_t st, GaeSlot*& out) {
     freeReturnedRows();
     if ((int)g_gaeScratch.size() <= dev) g_gaeScratch.resize(dev + 1);
     GaeScratch& s = g_gaeScratch[dev];
-    if (s.capacity < nChunks) {
-        // the old rows may still be read by work queued earlier on any stream
-        if (s.capacity > 0 && cudaDeviceSynchronize() != cudaSuccess) return RSB_ERR_CUDA;
-        cudaFree(s.count);
-        cudaFree(s.part);
-        if (!s.ticket && cudaMalloc(&s.ticket, sizeof(unsigned) * kGaeSlots) != cudaSuccess) return RSB_ERR_NOMEM;
-        const int cap = nChunks < 64 ? 64 : nChunks;
-        s.capacity = 0;
-        s.count = nullptr;
-        s.part = nullptr;
-        if (cudaMalloc(&s.count, sizeof(int) * cap * kGaeSlots) != cudaSuccess ||
-            cudaMalloc(&s.part, sizeof(float2) * cap * kGaeSlots) != cudaSuccess)
-            return RSB_ERR_NOMEM;
-        s.capacity = cap;
-    }
-    int slot = 0;
     unsigned long long id = 0;
     if (cudaStreamGetId(st, &id) != cudaSuccess) return RSB_ERR_CUDA;
-    int oldest = 0;
-    for (slot = 0; slot < kGaeSlots && !(s.used[slot] && s.stream[slot] == id); ++slot)
-        if (s.used[slot] < s.used[oldest]) oldest = slot;
-    if (slot == kGaeSlots) {
-        slot = oldest;
-        if (s.used[slot] && cudaDeviceSynchronize() != cudaSuccess) return RSB_ERR_CUDA;
-        s.stream[slot] = id;
+    GaeSlot *slot = nullptr, *oldest = &s.slot[kGaeOwn];
+    for (int k = 0; k < kGaeOwn + kGaeShared && !slot; ++k) {
+        GaeSlot& c = s.slot[k];
+        if ((c.used && c.stream == id) || (!c.used && k < kGaeOwn)) slot = &c;
+        else if (k >= kGaeOwn && c.used < oldest->used) oldest = &c;
     }
-    s.used[slot] = ++s.calls;
-    out.count = s.count + (size_t)slot * s.capacity;
-    out.part = s.part + (size_t)slot * s.capacity;
-    out.ticket = s.ticket + slot;
+    if (!slot) {
+        slot = oldest;
+        if (!slot->done && cudaEventCreateWithFlags(&slot->done, cudaEventDisableTiming) != cudaSuccess) return RSB_ERR_CUDA;
+        if (slot->used && cudaStreamWaitEvent(st, slot->done, 0) != cudaSuccess) return RSB_ERR_CUDA;
+    }
+    if (slot->rows.capacity < nChunks) {
+        if (s.rows.capacity < nChunks) {
+            RelaxedCapture relaxed;
+            GaeRows rows;
+            if (!allocRows(nChunks > 2 * s.rows.capacity ? nChunks : 2 * s.rows.capacity, kGaeOwn + kGaeShared, rows))
+                return RSB_ERR_NOMEM;
+            s.rows = rows;
+        }
+        const size_t k = (size_t)(slot - s.slot), at = k * s.rows.capacity;
+        slot->rows = GaeRows{s.rows.capacity, s.rows.count + at, s.rows.part + at, s.rows.ticket + k};
+    }
+    slot->stream = id;
+    slot->used = ++s.calls;
+    out = slot;
     return RSB_OK;
 }
 
@@ -618,14 +621,16 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     if (cudaGetDevice(&dev) != cudaSuccess) return RSB_ERR_CUDA;
     const int nChunks = (T + kGaeChunk - 1) / kGaeChunk;
     GaeRows rows;
+    GaeSlot* slot = nullptr;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
     if (cudaStreamGetCaptureInfo(st, &capture, nullptr, &graph) != cudaSuccess ||
         capture == cudaStreamCaptureStatusInvalidated)
         return RSB_ERR_CUDA;
-    const rsb_status rc =
-        capture == cudaStreamCaptureStatusActive ? rowsForGraph(dev, nChunks, graph, rows) : rowsForStream(dev, nChunks, st, rows);
+    const rsb_status rc = capture == cudaStreamCaptureStatusActive ? rowsForGraph(dev, nChunks, graph, rows)
+                                                                   : slotForStream(dev, nChunks, st, slot);
     if (rc != RSB_OK) return rc;
+    if (slot) rows = slot->rows;
     GaeArgs a;
     a.rews = rews;
     a.term = terminals;
@@ -672,6 +677,7 @@ rsb_status launchGae(const float* rews, const int8_t* terminals, const float* va
     cfg.numAttrs = a.count ? 1 : 0;
     if (cudaLaunchKernelEx(&cfg, kernel, a) != cudaSuccess)
         return RSB_ERR_CUDA;
+    if (slot && slot->done && cudaEventRecord(slot->done, st) != cudaSuccess) return RSB_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? RSB_OK : RSB_ERR_CUDA;
 }
 

@@ -544,11 +544,12 @@ rsb_status rsb_ring_stats_get(rsb_handle* h, rsb_ring_stats* out);
  *     elements; *rew_clip_portion = (sum|r/std| - sum|clip(r/std)|) / max(sum|r/std|, 1e-7),
  *     summed in another order than the reference's atomics (equal within float rounding).
  * All pointers are device pointers; stream is a cudaStream_t as void* (NULL = legacy default
- * stream).  The library keeps a small per-device scratch (grown on demand, as the
- * reference's is); calls on one device are serialised on the host, and work queued on two
- * streams must not overlap.  A call under stream capture works in scratch of its own, which its
- * graph keeps and gives back when it is destroyed; such graphs may be replayed side by side.
- * Three kernel launches, no host synchronisation. */
+ * stream).  The library keeps a small per-device scratch for each stream that calls (grown on
+ * demand, as the reference's is); calls on one device are serialised on the host, and their
+ * work on several streams may overlap (beyond 16 streams some wait on the device for others').
+ * A call under stream capture works in scratch of its own, which its graph keeps and gives back
+ * when it is destroyed; such graphs may be replayed side by side.  One to three kernel launches,
+ * no host synchronisation. */
 typedef struct rsb_gae_params {
     float gamma;       /* 0.99 by default */
     float lambda;      /* 0.95 */
