@@ -206,6 +206,12 @@ class DevArray:
         self.__cuda_array_interface__ = {"data": (ptr, False), "shape": shape, "typestr": typestr, "version": 3}
 
 
+def step_launches(batch, ticks):
+    """Kernels of one rsb_step: one for all phases and ticks of a small batch, unless a configuration of
+    the kernels of each phase and tick is pinned or tuned."""
+    return 1 if batch.step_config()["block"] == 256 else 12 * ticks
+
+
 def reduce_max(value, dist, device=None):
     """The largest value over the ranks (timing of the slowest rank)."""
     if dist is None:
@@ -354,7 +360,7 @@ def run_ours(args, rank, world, dist):
 
         value, total_ms, _, queries = timed(steps, clocks, _Replay)
         step_times = kernel_steps
-        extra["graph"] = {"api": "rsb_env_graph_capture / rsb_env_graph_launch", "launches_per_replay": 5 + (1 if wl.num_arenas <= 2048 else 12 * wl.tick_skip),
+        extra["graph"] = {"api": "rsb_env_graph_capture / rsb_env_graph_launch", "launches_per_replay": 5 + step_launches(batch, wl.tick_skip),
                           "note": "action sampling (torch) launched outside the graph"}
         ex_value = value
     else:
@@ -538,8 +544,6 @@ def run_ours(args, rank, world, dist):
     # roofline of the step kernel (the dominant launch): algorithmic bytes = persistent
     # state read + written per launch (the library reports it), over the kernel's own time
     alg_bytes = batch.stats()["state_bytes_per_step"]
-    # one launch for all phases and ticks of a small batch, else a launch per phase and tick
-    step_launches = 1 if wl.num_arenas <= 2048 else 12 * wl.tick_skip
     kernel_s = statistics.mean(step_times) / 1e3
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / kernel_s / 1e9
@@ -551,14 +555,14 @@ def run_ours(args, rank, world, dist):
         "warmup": args.warmup, "ms_per_step": total_ms / steps, "higher_is_better": True,
         "scaling": "strong" if wl.strong else "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded random states)", "config": cfg,
-        "roofline": {"bound": "hbm", "kernel": "the step's phases (stepBlockKernel up to 2,048 arenas)", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "the step's phases, " + ("one kernel" if step_launches(batch, 1) == 1 else "a kernel each"), "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
                      "bytes_per_launch": alg_bytes, "kernel_ms": kernel_s * 1e3,
                      "kernel_share": statistics.mean(step_times) / (total_ms / steps)},
         "e2e": {"value": e2e_value, "unit": "arena-ticks/s", "h2d_bytes_per_step": int(statistics.mean(h2d)),
                 "d2h_bytes_per_step": int(statistics.mean(d2h))},
         # per env step: action expansion, (culler,) the step's phases, obs + masks, rewards + terminals, reset
-        "gpu_launches": steps * ((5 if learned is not None else 4) + step_launches + (1 if wl.graph else 0)),
+        "gpu_launches": steps * ((5 if learned is not None else 4) + step_launches(batch, wl.tick_skip) + (1 if wl.graph else 0)),
         "learned_cull": learned,
         "state_ring": ring,
         "ball_prediction": pred,

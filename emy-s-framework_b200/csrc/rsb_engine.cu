@@ -218,7 +218,7 @@ static const int kStepResidency[] = {0, 1, 2, 3, 4, 6};
 // 1892 with 250; a kernel per phase 742 / 1955.  3v3 x 1,023, 4 ticks: 496 / 1365
 // with 64 blocks, 783 / 1147 with 128, 551 / 1387 with a kernel per phase, which is the faster one
 // once 64 blocks of 32 arenas are full.
-constexpr int kStepBlockGrid = 64;
+constexpr int kStepBlockGrid = 64, kStepBlockMax = kStepBlockGrid * PHASE_ARENAS;
 constexpr int kNumStepResidency = sizeof(kStepResidency) / sizeof(kStepResidency[0]);
 
 // Fills the triangles' query data (TriData) on the device.
@@ -918,7 +918,7 @@ static cudaError_t launchStep(rsb_handle* h, const EngineView& D, int v, int b, 
 // The default launch: one kernel while its blocks hold the batch, a kernel per phase beyond; a
 // configuration that was set or tuned is taken as it is.
 static int stepVariantFor(const rsb_handle* h) {
-    return !h->stepPinned && h->N <= kStepBlockGrid * PHASE_ARENAS ? -1 : h->stepVariant;
+    return !h->stepPinned && h->N <= kStepBlockMax ? -1 : h->stepVariant;
 }
 
 rsb_status rsb_step(rsb_handle* h, int32_t ticks, void* stream) {
@@ -1058,8 +1058,22 @@ rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32
     return RSB_OK;
 }
 
+rsb_status rsb_get_step_config(const rsb_handle* h, rsb_tune_entry* out) {
+    if (!h || !out) return RSB_ERR_INVALID;
+    const int v = stepVariantFor(h);
+    *out = v < 0 ? rsb_tune_entry{1, BLOCK_THREADS, 0.f, 0, 0}
+                 : rsb_tune_entry{kStepVariants[v].minBlocks, kStepBlocks[h->stepBlock], 0.f,
+                                  kStepVariants[v].persistent ? 1 : 0, kStepResidency[h->stepResidency]};
+    return RSB_OK;
+}
+
 rsb_status rsb_set_step_config(rsb_handle* h, const rsb_tune_entry* cfg) {
     if (!h || !cfg) return RSB_ERR_INVALID;
+    if (cfg->min_blocks == 1 && cfg->block == BLOCK_THREADS && !cfg->persistent && cfg->warps_per_sm == 0 &&
+        h->N <= kStepBlockMax) {
+        h->stepPinned = false;  // the default of such a batch
+        return RSB_OK;
+    }
     int r = -1;
     for (int k = 0; k < kNumStepResidency; k++)
         if (kStepResidency[k] == cfg->warps_per_sm) r = k;

@@ -211,6 +211,7 @@ _SIGS = {
     "rsb_reset_done": [_P, C.c_uint64, C.c_int32, _P],
     "rsb_autotune": [_P, C.c_int32, _P, C.c_int32, _P],
     "rsb_set_step_config": [_P, _P],
+    "rsb_get_step_config": [_P, _P],
     "rsb_culler_log": [_P, _P],
     "rsb_set_cull_mode": [_P, C.c_int32],
     "rsb_culler_train": [_P, _P, _P],
@@ -604,7 +605,8 @@ class Batch:
         self._check(self.lib.rsb_build_rewards_terminals(self._h, step_ticks, C.c_void_p(stream or 0)))
 
     def autotune(self, ticks: int = 8) -> list[dict]:
-        """rsb_autotune: times the step kernel's launch configurations, keeps the fastest."""
+        """rsb_autotune: times the launch configurations of the step's queue kernels and keeps the fastest, or
+        the default where that is faster (step_config tells)."""
         out = (TuneEntry * 64)()
         n = C.c_int32()
         self._check(self.lib.rsb_autotune(self._h, ticks, out, 64, C.byref(n)))
@@ -612,10 +614,17 @@ class Batch:
                  "warps_per_sm": e.warps_per_sm} for e in out[:min(n.value, 64)]]
 
     def set_step_config(self, min_blocks: int, block: int, persistent: bool = False, warps_per_sm: int = 0):
-        """rsb_set_step_config: pins a launch configuration of the step kernel."""
+        """rsb_set_step_config: pins a launch configuration of the step (1, 256: the one-kernel step)."""
         e = TuneEntry(min_blocks=min_blocks, block=block, ms=0.0, persistent=1 if persistent else 0,
                       warps_per_sm=warps_per_sm)
         self._check(self.lib.rsb_set_step_config(self._h, C.byref(e)))
+
+    def step_config(self) -> dict:
+        """rsb_get_step_config: the launch configuration in use, as set_step_config takes it."""
+        e = TuneEntry()
+        self._check(self.lib.rsb_get_step_config(self._h, C.byref(e)))
+        return {"min_blocks": e.min_blocks, "block": e.block, "persistent": bool(e.persistent),
+                "warps_per_sm": e.warps_per_sm}
 
     # ---------------------------------------------------------------- learned culler
     def set_cull_mode(self, mode: int):

@@ -396,8 +396,10 @@ rsb_status rsb_get_arena_info_at(rsb_handle* h, int32_t arena, rsb_arena_info* o
 rsb_status rsb_predict_ball(rsb_handle* h, const int32_t* slice_ticks, int32_t n_slices, rsb_ball_state* out,
                             size_t out_count, void* stream);
 
-/* One candidate launch configuration of the step's queue kernels (wheel rays near meshes or
- * bodies, contact pairs, islands) and the measured time of the step. */
+/* One launch configuration of the step and its measured time.  Batches of up to 2,048 arenas are
+ * stepped by one kernel by default, which is {1, 256, ms, 0, 0}; every other entry is a kernel per
+ * phase and tick, with its own choices for the queue kernels (the register budget for wheel rays near
+ * bodies and for triangles, the block size and grid for these and for combining contacts). */
 typedef struct rsb_tune_entry {
     int32_t min_blocks;   /* register budget: at least this many 128-thread blocks per SM */
     int32_t block;        /* threads per block (one queued item per thread) */
@@ -407,13 +409,17 @@ typedef struct rsb_tune_entry {
 } rsb_tune_entry;
 
 /* Times every launch configuration of the step's queue kernels on a device copy of the current
- * arena state (the handle's own state is not advanced), keeps the fastest for later
- * rsb_step calls, and reports every candidate in out[0..cap).  Allocates the scratch copy
+ * arena state (the handle's own state is not advanced), and reports them in out[0..cap).  Keeps
+ * the fastest for later rsb_step calls, or the default where that is faster (it is timed too, but
+ * not reported; rsb_get_step_config tells which was kept).  Allocates the scratch copy
  * of the state on its first call.  No counterpart in the reference. */
 rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32_t cap, int32_t* count);
-/* Selects a launch configuration (min_blocks, block, persistent as rsb_autotune reports them),
- * e.g. one tuned in an earlier run; RSB_ERR_INVALID if no such configuration exists. */
+/* Selects a launch configuration (min_blocks, block, persistent as rsb_autotune or
+ * rsb_get_step_config report them), e.g. one tuned in an earlier run; RSB_ERR_INVALID if no such
+ * configuration exists (the one-kernel step: if the batch is larger than it takes). */
 rsb_status rsb_set_step_config(rsb_handle* h, const rsb_tune_entry* cfg);
+/* The launch configuration that rsb_step uses now (ms = 0). */
+rsb_status rsb_get_step_config(const rsb_handle* h, rsb_tune_entry* out);
 
 /* ---- learned culler (no counterpart in the reference) ----
  * A 3 -> 64 -> 64 -> 1 MLP (BF16 weights, FP32 accumulation) estimates the distance (uu)
