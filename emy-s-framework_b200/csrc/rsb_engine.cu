@@ -765,20 +765,27 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
 
     if (cudaSetDevice(h->device) != cudaSuccess) return fail(nullptr, RSB_ERR_CUDA, "cudaSetDevice failed");
     {
-        // kernels with a large thread-local frame (EPA scratch, solver rows, the ball-only world):
-        // make the per-thread stack limit cover the largest (the default limit is 1 KB), and give
-        // the L1 its largest share in those that use no shared memory to speak of
-        size_t need = 0;
-        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)meshRayKernel, (const void*)solveBodyKernel,
-                                     (const void*)combineKernel};
+        // The per-thread stack limit covers the largest thread-local frame (solver rows, EPA scratch, the
+        // one-kernel step's spills), so that no launch has to grow the device's local memory: a first
+        // launch that did took half a second.  The kernels of the first list also give the L1 its largest
+        // share: they use little shared memory, or (predictBallKernel, 48 KB a block) live on their local
+        // memory: 16,384 balls, 360 ticks, three calls side by side 3.7 ms against 4.5 with the default
+        // share, 1,024 balls equal, 65,536 balls alone 16.1 against 14.9.
+        std::vector<const void*> fns{(const void*)predictBallKernel, (const void*)findKernel, (const void*)meshRayKernel,
+                                     (const void*)solveBodyKernel, (const void*)combineKernel};
         for (const StepVariant& v : kStepVariants)
             for (StepFn f : {v.ray, v.triangle}) fns.push_back((const void*)f);
+        for (const void* f : fns) cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+        for (StepFn f : {(StepFn)rayKernel, (StepFn)driveKernel, (StepFn)deepKernel, (StepFn)solveKernel, (StepFn)finishKernel})
+            fns.push_back((const void*)f);
+        fns.push_back((const void*)pairKernel);
+        fns.push_back((const void*)stepBlockKernel);
+        size_t need = 0;
         for (const void* f : fns) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, f) != cudaSuccess)
                 return fail(nullptr, RSB_ERR_CUDA, "cudaFuncGetAttributes failed");
-            need = std::max(need, ((fa.localSizeBytes + 4096) + 1023) / 1024 * 1024);
-            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+            need = std::max(need, (fa.localSizeBytes + 1023) / 1024 * 1024);
         }
         if (cudaFuncSetAttribute(stepBlockKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockShared)) !=
             cudaSuccess)
