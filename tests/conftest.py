@@ -30,6 +30,19 @@ def load_pkg():
     return mod
 
 
+def pytest_collection_modifyitems(config, items):
+    """Where the reference's meshes or the oracle are not at hand, the tests that use neither run first, so
+    that `-x` does not end the run before them."""
+    if os.path.exists(ORACLE_LIB) and os.path.isdir(os.path.join(load_pkg().MESHES_DIR, "soccar")):
+        return
+
+    def needs(it):
+        return (not {"meshes_dir", "oracle_lib", "oracle"}.isdisjoint(it.fixturenames) or
+                "ORACLE_LIB" in it.function.__code__.co_names)
+
+    items.sort(key=needs)
+
+
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200); compares the engine with the oracle")
 
