@@ -189,11 +189,11 @@ static rsb_status cudaFail(rsb_handle* h, const char* what, cudaError_t e) {
 
 // ------------------------------------------------------------------ kernels
 
-// The queue kernels of a step (heavy rays, contacts, islands) for one register budget: MINB is
-// the minimum number of 128-thread blocks per SM the compiler must fit.  Their grids loop over
-// the queues: either wide enough for every item to get a thread of its own, or (persistent)
-// only as many blocks as are resident at once.  The autotuner picks the variant and the block
-// size.
+// The queue kernels of a step that come in several register budgets (rays near bodies, triangles): MINB
+// is the minimum number of 128-thread blocks per SM the compiler must fit.  The grids of these and of
+// combineKernel loop over the queues: either wide enough for every item to get a thread of its own, or
+// (persistent) only as many blocks as are resident at once.  The autotuner picks the variant and the
+// block size of the three; the other kernels' grids and blocks are fixed.
 typedef void (*StepFn)(EngineView, StepTemp);
 struct StepVariant {
     StepFn ray, triangle;
@@ -411,9 +411,10 @@ __device__ __noinline__ int warpBallList(const EngineView& D, V3 at, V3 mn, V3 m
 // and contacts, which differ from ball to ball: 14,000 cycles for a tick of a warp in which a ball
 // touches something, 3,000 for one in which all fly.  A warp still takes a full 32 balls from
 // PRED_WARPS * SMs * 32 balls on: narrower warps spread the contacts, but each holds its own lines
-// of local memory and of code.  16,384 balls, 360 ticks, three such calls side by side, with 2, 4,
-// 8, 16, 32 and 64 warps per SM: 5.7, 6.0, 7.4, 9.5, 12.1 and 17.0 ms each; 1,024 balls with 2, 4
-// and 8: 1.1, 1.3 and 1.7 ms.  Those were blocks of two warps.  Warps that share a multiprocessor
+// of local memory and of code.  360 ticks, ms per call of three side by side / of one alone, with 1, 2,
+// 4 and 8 warps per SM: 1,024 balls 1.10 / 2.09, 1.01 / 2.04, 1.09 / 1.87, 1.18 / 2.29; 4,096 balls
+// 1.77 / 4.26, 1.65 / 3.69, 1.69 / 3.47, 1.94 / 4.23; 16,384 balls 3.74 / 6.48, 3.73 / 6.48, 3.88 /
+// 7.06, 4.63 / 7.55.  Warps that share a multiprocessor
 // share its fetched code: blocks of one, two and four warps take 8.4, 5.1 and 3.5 ms for the 16,384
 // balls (four are as many as static shared memory holds lists for).  One thread per ball on the
 // general tick, whose arena lies in local memory, took 17.0 ms.
