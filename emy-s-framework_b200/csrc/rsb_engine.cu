@@ -767,8 +767,8 @@ rsb_status rsb_create(const rsb_config* cfg, rsb_handle** out) {
     if (cudaSetDevice(h->device) != cudaSuccess) return fail(nullptr, RSB_ERR_CUDA, "cudaSetDevice failed");
     {
         // The per-thread stack limit covers the largest thread-local frame (solver rows, EPA scratch, the
-        // one-kernel step's spills), so that no launch has to grow the device's local memory: a first
-        // launch that did took half a second.  The kernels of the first list also give the L1 its largest
+        // one-kernel step's spills), so that no launch has to wait for the device and grow its local
+        // memory.  The kernels of the first list also give the L1 its largest
         // share: they use little shared memory, or (predictBallKernel, 48 KB a block) live on their local
         // memory: 16,384 balls, 360 ticks, three calls side by side 3.7 ms against 4.5 with the default
         // share, 1,024 balls equal, 65,536 balls alone 16.1 against 14.9.
