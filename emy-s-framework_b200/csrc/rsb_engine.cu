@@ -990,6 +990,8 @@ rsb_status rsb_autotune(rsb_handle* h, int32_t ticks, rsb_tune_entry* out, int32
     const size_t words = wBall + wCar + wPad + wArena;
     if (!h->dScratch && cudaMalloc((void**)&h->dScratch, words * 4) != cudaSuccess)
         return fail(h, RSB_ERR_NOMEM, "autotune scratch allocation failed");
+    // the candidates work in the step's buffers, which steps queued on any stream may still use
+    RSB_CUDA(cudaDeviceSynchronize());
     EngineView D = devView(h);
     D.ball = h->dScratch;
     D.car = D.ball + wBall;
