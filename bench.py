@@ -42,6 +42,22 @@ def load_pkg():
     return mod
 
 
+UNAVAILABLE = "oracle/_ref is not built: the reference's sources and meshes are not at hand"
+GENERATED = "generated arena of perf/cases.py (8,700 triangles in 14 meshes): the reference's soccar meshes are not at hand"
+
+
+def arena_meshes(pkg):
+    """(folder of the arena meshes, None), or a generated arena and what it is where the reference's are not staged."""
+    if os.path.isdir(os.path.join(pkg.MESHES_DIR, "soccar")):
+        return pkg.MESHES_DIR, None
+    if "rsb_bench_arena" not in sys.modules:
+        spec = importlib.util.spec_from_file_location("rsb_bench_arena", os.path.join(ROOT, "perf", "cases.py"))
+        mod = importlib.util.module_from_spec(spec)
+        sys.modules["rsb_bench_arena"] = mod
+        spec.loader.exec_module(mod)
+    return sys.modules["rsb_bench_arena"]._arena(), GENERATED
+
+
 def measured_peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -252,7 +268,7 @@ def run_ours(args, rank, world, dist):
         wl.shard(rank, world)
     rewards = rsb.default_rewards(pkg.engine_library(), episode_max_ticks=EPISODE_TICKS)
     batch = rsb.Batch(pkg.engine_library(), wl.num_arenas, team_size=wl.team_size or None,
-                      team_sizes=wl.team_sizes(), meshes_path=pkg.MESHES_DIR, device=dev, seed=0x5EED0000 + rank,
+                      team_sizes=wl.team_sizes(), meshes_path=arena_meshes(pkg)[0], device=dev, seed=0x5EED0000 + rank,
                       rewards=rewards, cull_mode=rsb.RSB_CULL_EXACT)
     lut = rsb.default_action_lut(batch.lib)
     batch.set_action_lut(lut)
@@ -548,6 +564,8 @@ def run_ours(args, rank, world, dist):
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / kernel_s / 1e9
     cfg = wl.config() | {"parallelism": f"arena-shards x{world}"}
+    if arena_meshes(pkg)[1]:
+        cfg["arena"] = GENERATED
     if learned is not None:
         cfg["narrowphase"] = "learned cull (exact BVH for every body the bound does not clear)"
     res = {
@@ -737,7 +755,7 @@ def stress_events(pkg, trained, wl, rank, dev, steps, arenas=None):
     mk = []
     for mode in (rsb.RSB_CULL_EXACT, rsb.RSB_CULL_LEARNED):
         b = rsb.Batch(pkg.engine_library(), n, team_size=wl.team_size or None,
-                      team_sizes=wl.team_sizes(), meshes_path=pkg.MESHES_DIR, device=dev, seed=0x5EED0000 + rank,
+                      team_sizes=wl.team_sizes(), meshes_path=arena_meshes(pkg)[0], device=dev, seed=0x5EED0000 + rank,
                       rewards=rsb.default_rewards(pkg.engine_library(), episode_max_ticks=EPISODE_TICKS),
                       cull_mode=mode)
         b.set_action_lut(lut)
@@ -806,8 +824,9 @@ def config_summaries(args, rank, world, dist):
                                  "voxel_culled_fraction": lc["voxel_bound"]["culled_fraction"]}
         if rank == 0 and world == 1 and not args.no_cpu_baseline:
             ref = cpu_reference(a, sample_s=4.0)
-            s["reference_cpu"] = {"value": ref["value"], "cores": ref["cores"], "sample": ref["sample"]}
-            s["vs_reference_cpu"] = r["value"] / ref["value"]
+            if "unavailable" not in ref:
+                s["reference_cpu"] = {"value": ref["value"], "cores": ref["cores"], "sample": ref["sample"]}
+                s["vs_reference_cpu"] = r["value"] / ref["value"]
         out[name] = s
     return out
 
@@ -851,6 +870,8 @@ def gae_cpu_baseline(rews, term, vals, trunc):
     C restatement of it when that library is absent."""
     import ctypes as C
 
+    if not os.path.exists(GAE_LIB_REF) and not os.path.exists(GAE_LIB_PORT):
+        return {"unavailable": UNAVAILABLE}
     T = len(rews)
     outs = [np.zeros(T, np.float32) for _ in range(3)]
     clip = np.zeros(1, np.float32)
@@ -963,6 +984,8 @@ def cpu_reference(args, sample_s=10.0, threads=None):
     terminal conditions, then the finished arenas reset.  (The CPU reference has no
     high-contact start; that preset's CPU sample starts from random states.)"""
     pkg = load_pkg()
+    if not os.path.exists(ORACLE_LIB) or arena_meshes(pkg)[1]:
+        return {"unavailable": UNAVAILABLE}
     rsb = pkg.rsb
     lib = rsb.load_library(ORACLE_LIB)
     threads = threads or os.cpu_count() or 1
@@ -1009,6 +1032,9 @@ def gae_line(args, res, world, impl=None):
 
 
 def run_reference(args):
+    lib = GAE_LIB_REF if args.config == "gae" else ORACLE_LIB
+    if not os.path.exists(lib) or (args.config != "gae" and arena_meshes(load_pkg())[1]):
+        return {"impl": "reference", "unavailable": UNAVAILABLE}
     if args.config == "gae":
         # the reference's own implementation of this path is its device GAE
         # (RocketSimCuda/src/GAECuda.cu), built from its tree for sm_100a
